@@ -29,7 +29,7 @@ CPP_SOURCES = ["fn_node.cpp", "fn_compile.cpp", "fn_runtime.cpp", "fn_batch.cpp"
                "fn_jit.cpp", "fn_ipc.cpp", "fn_live.cpp", "fn_capi_mesh.cpp"]
 
 # Headers handed to NVRTC at run time (in this order), embedded into the library.
-JIT_HEADERS = ["fn_types.h", "fn_device.cuh", "fn_eval.cuh"]
+JIT_HEADERS = ["fn_types.h", "fn_device.cuh", "fn_eval.cuh", "fn_column.cuh"]
 JIT_SRC = os.path.join(OUT, "fn_embedded_src.gen.cpp")
 
 CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fvisibility=hidden", "-Wall",

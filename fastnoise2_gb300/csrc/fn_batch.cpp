@@ -187,11 +187,16 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     // variant when it is built (a variant not built yet is queued for a background build and
     // variant 0 runs meanwhile), or the variant a tuning run forces.
     std::vector<BatchKernel> kernels(n);
+    std::vector<PointArgs> args(n);
+    std::vector<char> column(n, 0);                 // grid requests walked in columns
+    double column_work = 0;                         // their 32-point steps
+    for (size_t i = 0; i < n; ++i) args[i] = items[i].args;
     bool jit = true;
     for (size_t i = 0; jit && i < n; ++i) jit = items[i].args.total < (1ll << 32);   // 32-bit point indices
     {
         const int forced = tuning_in ? tuning_in->variant : -1;
-        std::map<uint64_t, BatchKernel> chosen;
+        struct Tree { BatchKernel kernel; JitKernels jk; };
+        std::map<uint64_t, Tree> chosen;
         for (size_t i = 0; jit && i < n; ++i) {
             auto it = chosen.find(progs[i].hash);
             if (it == chosen.end()) {
@@ -205,11 +210,20 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
                     ok = jit_batch_kernel(progs[i].hash, 0, bk);
                 }
                 if (!ok) { jit = false; break; }
-                it = chosen.emplace(progs[i].hash, bk).first;
+                Tree t;
+                t.kernel = bk;
+                if (forced >= 0 || !jit_lookup(progs[i].hash, t.jk)) t.jk = JitKernels();   // a forced variant is run as asked
+                it = chosen.emplace(progs[i].hash, t).first;
             }
-            kernels[i] = it->second;
+            kernels[i] = it->second.kernel;
+            if (it->second.jk.batch_column && jit_column_grid(args[i], it->second.jk)) {
+                kernels[i] = BatchKernel{it->second.jk.batch_column, 256};
+                column[i] = 1;
+                column_work += (double)args[i].col_steps * ((args[i].col_plane + 31) / 32);
+            }
         }
     }
+    if (!jit) std::fill(column.begin(), column.end(), 0);
     if (!jit) {                                     // interpreter batch: count a use of each program
         std::vector<uint64_t> seen;
         for (size_t i = 0; i < n; ++i)
@@ -230,8 +244,15 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     if (tuning_in) tuning = *tuning_in;
     else Autotuner::instance().lookup(signature_, tuning);
     const uint32_t tp = std::max<uint32_t>(256, tuning.tile_points);
+    // Column units: about four rounds of 16 warps per SM over the whole batch, so that short
+    // batches still spread, and at most 64 steps (longer ones gain under 5 % of set-up).
+    const unsigned col_len = (unsigned)std::min(64.0, std::max(4.0, column_work / (64.0 * num_sms())));
+    std::vector<uint32_t> tiles(n);
     size_t n_items = 0;
-    for (size_t i = 0; i < n; ++i) n_items += tiles_for(items[i].args.total, tp);
+    for (size_t i = 0; i < n; ++i) {
+        tiles[i] = column[i] ? jit_column_tiles(args[i], col_len) : tiles_for(items[i].args.total, tp);
+        n_items += tiles[i];
+    }
     if (n_items > 0xFFFFFFFFull) { set_error(-4, "batch too large"); return -4; }
     if (!reserve(n, n_items)) return -3;
 
@@ -274,7 +295,7 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     for (size_t i = 0; i < n; ++i) {
         BatchRequest& r = reqs[i];
         std::memset(&r, 0, sizeof r);
-        r.args = items[i].args;
+        r.args = args[i];
         r.prog = progs[i].dptr;
         r.jit_slot = -1;
         r.prog_bytes = progs[i].bytes;
@@ -283,7 +304,7 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         r.host_minmax = items[i].host_minmax;
         r.host_done = items[i].host_done;
         r.host_time = items[i].host_time;
-        r.n_tiles = tiles_for(items[i].args.total, tp);
+        r.n_tiles = tiles[i];
         states[i].mn_enc = 0xFFFFFFFFu;
         states[i].mx_enc = 0u;
         states[i].tiles_done = 0u;

@@ -1,0 +1,312 @@
+// fn_column.cuh -- noise evaluated along a column of a uniform grid.
+//
+// The specialised column kernels (fn_jit.cpp) give every lane one position across the
+// grid's last axis and walk it along that axis, so all lanes of a warp share the last
+// coordinate.  Where a node's position is still separable (its last component depends on the
+// last grid axis alone, the others on the other axes alone), everything the lattice
+// contributes changes only when that coordinate enters another cell, and everything that
+// depends on the other axes never changes.  The structs below keep those parts in registers
+// between steps.  What depends on the column's coordinate alone (cell, offset, easing curve)
+// is the same for all lanes: the lanes compute 32 steps' worth at a time into shared memory,
+// one step each, and every step reads its entry with one broadcast load.  A step then runs
+// the reference's remaining arithmetic, the same operations in the same order on the same
+// operands, so results equal the point functions of fn_device.cuh.
+//
+// Bound by: instruction issue.  A Perlin octave in 3D costs ~17 instructions a step (a packed
+// fma per corner pair, packed lerps) against ~200 for the point function, whose integer
+// hashing and gradient selection (the half-rate ALU pipe) move to the plane rebuild, ~115
+// instructions once per cell.
+#pragma once
+
+#include "fn_device.cuh"
+
+namespace fnd {
+
+// Keeps a value the same but hides where it came from: computations on the result are not
+// hoisted out of the (rare) branch they are needed in, where they would hold registers.
+FND float opaque(float v)
+{
+    asm volatile("" : "+f"(v));
+    return v;
+}
+
+FND float nan_() { return __int_as_float(0x7fffffff); }
+
+// Two floats in one register pair and the packed FP32 operations on them: each half rounds
+// like the scalar operation, in one issue slot.
+typedef unsigned long long f32x2;
+FND f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+FND void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+FND f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+FND f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+FND f32x2 lerp2(f32x2 a, f32x2 b, f32x2 t) { return fma2(t, sub2(b, a), a); }
+
+// The gradient dot of one lattice corner as a function of the offset t along the last axis,
+// for fixed offsets across it: dot = fma(s, t, g) with s in {-1, 0, 1}.  s * t is exact, so
+// the fma rounds once, as the reference's sum of two signed offsets does (3D, 4D).
+FND void grad_col3(int h, float x, float y, float& s, float& g)
+{
+    // the second offset is y (h & 12 == 0), x (h & 13 == 12) or the column's own; a zero
+    // second offset and the column's signed weight are exclusive
+    const bool takes_y = (h & 12) == 0, takes_x = (h & 13) == 12;
+    const float u = flip((h & 8) ? y : x, h << 31), sign = flip(1.0f, h << 30);
+    s = takes_y ? 0.0f : (takes_x ? 0.0f : sign);
+    g = fmaf(takes_y ? y : (takes_x ? x : 0.0f), sign, u);
+}
+FND void grad_col4(int h, float x, float y, float z, float& s, float& g)
+{
+    const bool any34 = (h & 24) != 0, b4 = (h & 16) != 0, both34 = (h & 24) == 24;
+    const float ab = flip(any34 ? x : y, h << 31) + flip(b4 ? y : z, h << 30);
+    s = both34 ? 0.0f : flip(1.0f, h << 29);
+    g = both34 ? ab + flip(z, h << 29) : ab;
+}
+
+// Cell bookkeeping shared by the columns.  prepare() fills the lane's table entry (offset,
+// offset - 1, easing, cell) for the coordinate Z of step `lane` and returns the ballot of
+// steps that enter another cell than the step before (a NaN cell always does).  enter() says
+// whether the kept upper plane becomes the lower one (1, the usual step to the next cell) or
+// both planes are new (0).
+struct ColCell {
+    float cell;
+    int icell;
+    FND void init() { cell = nan_(); icell = 0; }
+    template <typename Ease>
+    FND unsigned prepare(float4* tab, unsigned lane, float Z, Ease&& ease)
+    {
+        const float zs = floorf(Z), z0 = Z - zs;
+        tab[lane] = make_float4(z0, z0 - 1.0f, ease(z0), zs);
+        const float before = __shfl_up_sync(0xffffffffu, zs, 1);
+        return __ballot_sync(0xffffffffu, zs != (lane ? before : cell));
+    }
+    FND int enter(float zs, int& zi)
+    {
+        zi = cvti(zs);
+        const int from = (cell == cell && zi == iadd(icell, 1)) ? 1 : 0;
+        cell = zs;
+        icell = zi;
+        return from;
+    }
+};
+
+// Lattice cell and offsets of the fixed axes (recomputed at each rebuild: cheaper than the
+// registers that would hold them).
+template <int D>
+FND void col_lattice(const float* q, int (*c)[2], float (*f)[2])
+{
+#pragma unroll
+    for (int k = 0; k < D - 1; ++k) {
+        const float fl = floorf(q[k]);
+        c[k][0] = imul(cvti(fl), kPrimes[k]);
+        c[k][1] = iadd(c[k][0], kPrimes[k]);
+        f[k][0] = q[k] - fl;
+        f[k][1] = f[k][0] - 1.0f;
+    }
+}
+
+// `pos(q)` writes the D - 1 fixed coordinates (already scaled by the node's frequency).
+// The lower and the upper lattice plane run as the two halves of packed operations (256^3
+// FBm(Perlin): 142 us; scalar operations 151 us; the point kernel 515 us).  The rebuild loop
+// works on scalars and packs at its end: kept pairs updated half by half inside the loop came
+// out of the compiler with both halves new (tests/test_gpu_column.py would show it).
+template <int D>
+struct PerlinCol {
+    static constexpr int N = 1 << (D - 1);        // corners of one lattice plane
+    f32x2 s[N], g[N];                             // (lower, upper) plane: dot = fma(s, t, g)
+    float ease[D - 1];
+    ColCell at;
+
+    template <typename Pos>
+    FND void init(Pos&& pos)
+    {
+        float q[D - 1];
+        pos(q);
+#pragma unroll
+        for (int k = 0; k < D - 1; ++k) ease[k] = quintic(q[k] - floorf(q[k]));
+#pragma unroll
+        for (int m = 0; m < N; ++m) s[m] = g[m] = 0;
+        at.init();
+    }
+    FND unsigned prepare(float4* tab, unsigned lane, float Z)
+    {
+        return at.prepare(tab, lane, Z, [](float t) { return quintic(t); });
+    }
+    template <typename Pos>
+    FND void enter(int seed, float zs, Pos&& pos)
+    {
+        if (zs != at.cell) {
+            int zi;
+            float q[D - 1], f[D - 1][2];
+            int c[D - 1][2];
+            pos(q);
+            col_lattice<D>(q, c, f);
+            float ls[N], lg[N], hs[N], hg[N];
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                unpack2(s[m], ls[m], hs[m]);
+                unpack2(g[m], lg[m], hg[m]);
+            }
+#pragma unroll 1
+            for (int k = at.enter(zs, zi); k < 2; ++k) {
+                const int zh = seed ^ imul(iadd(zi, k), kPrimes[D - 1]);
+#pragma unroll
+                for (int m = 0; m < N; ++m) {
+                    const int b0 = m & 1, b1 = (m >> 1) & 1, b2 = (m >> 2) & 1;
+                    int h = zh ^ c[0][b0] ^ c[1][b1];
+                    if constexpr (D == 4) h ^= c[2 % (D - 1)][b2];
+                    h = hash_mix(h);
+                    ls[m] = hs[m];
+                    lg[m] = hg[m];
+                    if constexpr (D == 3) grad_col3(h, f[0][b0], f[1][b1], hs[m], hg[m]);
+                    else grad_col4(h, f[0][b0], f[1][b1], f[2 % (D - 1)][b2], hs[m], hg[m]);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                s[m] = pack2(ls[m], hs[m]);
+                g[m] = pack2(lg[m], hg[m]);
+            }
+        }
+    }
+    FND float eval(const float4& e) const
+    {
+        const f32x2 z = pack2(e.x, e.y);
+        f32x2 v[N];
+#pragma unroll
+        for (int m = 0; m < N; ++m) v[m] = fma2(s[m], z, g[m]);
+#pragma unroll
+        for (int k = 0; k < D - 1; ++k) {
+            const f32x2 t = pack2(ease[k], ease[k]);
+#pragma unroll
+            for (int j = 0; j < (N >> (k + 1)); ++j) v[j] = lerp2(v[2 * j], v[2 * j + 1], t);
+        }
+        float lo, hi;
+        unpack2(v[0], lo, hi);
+        return lerp(lo, hi, e.z);
+    }
+};
+
+// 2D: dot = fma(1 + sqrt 2, a, b) with (a, b) the signed offsets, in either order; the one
+// along the column is p * t, the other is kept (q), so a = fma(pa, t, qa), b = fma(pb, t, qb)
+// with one of each pair zero.
+template <>
+struct PerlinCol<2> {
+    float pa[2][2], qa[2][2], pb[2][2], qb[2][2];   // [plane][x corner]
+    float ease;
+    ColCell at;
+
+    template <typename Pos>
+    FND void init(Pos&& pos)
+    {
+        float q[1];
+        pos(q);
+        ease = quintic(q[0] - floorf(q[0]));
+#pragma unroll
+        for (int m = 0; m < 4; ++m) pa[m >> 1][m & 1] = qa[m >> 1][m & 1] = pb[m >> 1][m & 1] = qb[m >> 1][m & 1] = 0.0f;
+        at.init();
+    }
+    FND unsigned prepare(float4* tab, unsigned lane, float Y)
+    {
+        return at.prepare(tab, lane, Y, [](float t) { return quintic(t); });
+    }
+    template <typename Pos>
+    FND void enter(int seed, float ys, Pos&& pos)
+    {
+        if (ys != at.cell) {
+            int yi;
+            float q[1], f[1][2];
+            int c[1][2];
+            pos(q);
+            col_lattice<2>(q, c, f);
+#pragma unroll 1
+            for (int k = at.enter(ys, yi); k < 2; ++k) {
+                const int yh = seed ^ imul(iadd(yi, k), kPrimeY);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    pa[0][m] = pa[1][m]; qa[0][m] = qa[1][m]; pb[0][m] = pb[1][m]; qb[0][m] = qb[1][m];
+                    const int h = hash_mix(yh ^ c[0][m]);
+                    const bool swap = (h << 29) < 0;
+                    const float xv = flip(f[0][m], h << 31), sy = flip(1.0f, h << 30);
+                    pa[1][m] = swap ? sy : 0.0f;
+                    qa[1][m] = swap ? 0.0f : xv;
+                    pb[1][m] = swap ? 0.0f : sy;
+                    qb[1][m] = swap ? xv : 0.0f;
+                }
+            }
+        }
+    }
+    FND float eval(const float4& e) const
+    {
+        float d[2][2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float t = k ? e.y : e.x;
+                d[k][m] = fmaf(1.0f + (float)kRoot2, fmaf(pa[k][m], t, qa[k][m]), fmaf(pb[k][m], t, qb[k][m]));
+            }
+        return lerp(lerp(d[0][0], d[0][1], ease), lerp(d[1][0], d[1][1], ease), e.z);
+    }
+};
+
+// Value noise: a lattice plane interpolated across the fixed axes is one number; a step is
+// the easing curve and the last lerp.
+template <int D>
+struct ValueCol {
+    static constexpr int N = 1 << (D - 1);
+    float lo, hi;
+    ColCell at;
+
+    template <typename Pos>
+    FND void init(Pos&&) { lo = hi = 0.0f; at.init(); }
+    FND unsigned prepare(float4* tab, unsigned lane, float Z)
+    {
+        return at.prepare(tab, lane, Z, [](float t) { return hermite(t); });
+    }
+    template <typename Pos>
+    FND void enter(int seed, float zs, Pos&& pos)
+    {
+        if (zs != at.cell) {
+            int zi;
+            float q[D - 1], f[D - 1][2];
+            int c[D - 1][2];
+            pos(q);
+            col_lattice<D>(q, c, f);
+#pragma unroll 1
+            for (int k = at.enter(zs, zi); k < 2; ++k) {
+                const int zh = seed ^ imul(iadd(zi, k), kPrimes[D - 1]);
+                float v[N];
+#pragma unroll
+                for (int m = 0; m < N; ++m) {
+                    int h = zh ^ c[0][m & 1];
+                    if constexpr (D >= 3) h ^= c[1 % (D - 1)][(m >> 1) & 1];
+                    if constexpr (D == 4) h ^= c[2 % (D - 1)][(m >> 2) & 1];
+                    v[m] = valcoord(h);
+                }
+#pragma unroll
+                for (int a = 0; a < D - 1; ++a)
+#pragma unroll
+                    for (int j = 0; j < (N >> (a + 1)); ++j) v[j] = lerp(v[2 * j], v[2 * j + 1], hermite(f[a][0]));
+                lo = hi;
+                hi = v[0];
+            }
+        }
+    }
+    FND float eval(const float4& e) const { return lerp(lo, hi, e.z); }
+};
+
+}  // namespace fnd

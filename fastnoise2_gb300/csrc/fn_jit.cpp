@@ -49,6 +49,9 @@ std::string lit(float f)
 
 std::string r(int i) { return "r" + std::to_string(i); }
 
+constexpr int kColMaxRegs = 200;       // registers of column state a kernel may hold
+constexpr int kColMaxTable = 370;       // float4 of shared table per warp (8 warps within 48 KB of static shared memory)
+
 const char* noise_fn(int kind)
 {
     switch (kind) {
@@ -59,14 +62,155 @@ const char* noise_fn(int kind)
     }
 }
 
-// One program -> `__device__ float <name>(int seed, float x, float y, float z, float w)`.
+// Column evaluation of a program over a uniform grid (fn_column.cuh): the noise
+// instructions whose position is separable -- every component but the last depends on the
+// grid's fixed axes only, the last on the column's axis only, all through constant scales
+// and offsets -- keep their lattice state between the steps of a column.
+struct ColState {
+    int pc = 0;                        // instruction
+    std::string type;                  // state struct of fn_column.cuh
+    std::vector<std::string> pos;      // fixed components as expressions of the root position
+    std::string along;                 // the last component, as an expression of the column's coordinate
+    std::string jitter;                // cellular states: the jitter
+    ColumnRate rate;                   // lattice cells per unit along the grid's axes
+    int table = 0, table_size = 0;     // its part of the warp's shared table, in float4
+};
+struct ColPlan {
+    std::vector<ColState> states;
+    int regs = 0;                      // registers the states hold
+    int table = 0;                     // float4 of shared table per warp
+
+    const ColState* at(int pc) const
+    {
+        for (auto& st : states) if (st.pc == pc) return &st;
+        return nullptr;
+    }
+};
+
+ColPlan column_plan(const CompiledProgram& prog)
+{
+    ColPlan plan;
+    const FnProgramHeader* h = reinterpret_cast<const FnProgramHeader*>(prog.blob.data());
+    const FnInstr* ins = fn_program_instrs(h);
+    const float* P = fn_program_params(h);
+    // what is known of a register: a constant, a function of the fixed axes (with its
+    // expression), of the column's axis (with the product of its scales), or neither
+    struct Reg {
+        enum { kOther, kConst, kFixed, kColumn } kind = kOther;
+        std::string expr;
+        float scale = 0.0f;            // product of its scales (a constant's value)
+        int axis = 0;                  // grid axis it depends on
+    };
+    std::vector<Reg> R((size_t)std::max<int>(h->n_regs, h->dim));
+    const char* root[4] = {"x", "y", "z", "w"};
+    for (int k = 0; k < h->dim; ++k) {
+        R[(size_t)k].kind = k == h->dim - 1 ? Reg::kColumn : Reg::kFixed;
+        R[(size_t)k].expr = root[k];
+        R[(size_t)k].scale = 1.0f;
+        R[(size_t)k].axis = k;
+    }
+    // a state for the instruction, if its position is separable and the kernel has room
+    auto add_state = [&](int pc, const std::string& type, float freq, int regs, int table, bool cellular) -> ColState* {
+        const FnInstr& I = ins[pc];
+        bool ok = R[(size_t)(I.a + I.dim - 1)].kind == Reg::kColumn && plan.regs + regs <= kColMaxRegs &&
+                  plan.states.size() < kMaxColumnStates && plan.table + table <= kColMaxTable;
+        for (int k = 0; k < I.dim - 1; ++k)
+            ok = ok && (R[(size_t)(I.a + k)].kind == Reg::kFixed || R[(size_t)(I.a + k)].kind == Reg::kConst);
+        if (!ok) return nullptr;
+        ColState st;
+        st.pc = pc;
+        st.type = type;
+        st.rate.cellular = cellular;
+        for (int k = 0; k < I.dim; ++k) {
+            const Reg& r = R[(size_t)(I.a + k)];
+            if (k < I.dim - 1) st.pos.push_back(r.expr + " * " + lit(freq));
+            else st.along = r.expr + " * " + lit(freq);
+            if (r.kind != Reg::kConst) st.rate.scale[r.axis] = std::max(st.rate.scale[r.axis], std::fabs(r.scale * freq));
+        }
+        st.table = plan.table;
+        st.table_size = table;
+        plan.table += table;
+        plan.regs += regs;
+        plan.states.push_back(st);
+        return &plan.states.back();
+    };
+    for (int pc = 0; pc < h->n_instr; ++pc) {
+        const FnInstr& I = ins[pc];
+        const int D = I.dim;
+        auto scaled = [&](const Reg& a, float f) {
+            Reg r = a;
+            if (r.kind == Reg::kConst) r.kind = Reg::kFixed;
+            if (!r.expr.empty()) r.expr = "(" + r.expr + " * " + lit(f) + ")";
+            r.scale *= f;
+            return r;
+        };
+        auto set_other = [&](int reg, int n) { for (int k = 0; k < n; ++k) if (reg + k < (int)R.size()) R[(size_t)(reg + k)] = Reg(); };
+        switch (I.op) {
+        case FN_OP_CONST:
+            R[I.dst] = Reg();
+            R[I.dst].kind = Reg::kConst;
+            R[I.dst].expr = lit(P[I.prm]);
+            R[I.dst].scale = P[I.prm];
+            break;
+        case FN_OP_MOV: R[I.dst] = R[I.a]; break;
+        case FN_OP_SCALE_POS: case FN_OP_SCALE_POS_V: {
+            std::vector<Reg> t;
+            for (int k = 0; k < D; ++k) t.push_back(scaled(R[(size_t)(I.a + k)], P[I.prm + (I.op == FN_OP_SCALE_POS_V ? k : 0)]));
+            for (int k = 0; k < D; ++k) R[(size_t)(I.dst + k)] = t[(size_t)k];
+            break;
+        }
+        case FN_OP_OFFSET_POS: {
+            const int off[4] = {I.b, I.c, I.d, I.e};
+            std::vector<Reg> t;
+            for (int k = 0; k < D; ++k) {
+                Reg r = R[(size_t)(I.a + k)];
+                const Reg& o = R[(size_t)off[k]];
+                if (r.kind == Reg::kConst) r.kind = Reg::kFixed;
+                if (o.kind != Reg::kConst || r.kind == Reg::kOther) r = Reg();
+                else r.expr = "(" + r.expr + " + " + o.expr + ")";
+                t.push_back(r);
+            }
+            for (int k = 0; k < D; ++k) R[(size_t)(I.dst + k)] = t[(size_t)k];
+            break;
+        }
+        case FN_OP_NOISE:
+            if (I.aux == FN_NOISE_PERLIN)
+                add_state(pc, "PerlinCol<" + std::to_string(D) + ">", P[I.prm], D == 2 ? 18 : D == 3 ? 20 : 38, 32, false);
+            else if (I.aux == FN_NOISE_VALUE)
+                add_state(pc, "ValueCol<" + std::to_string(D) + ">", P[I.prm], 4, 32, false);
+            R[I.dst] = Reg();
+            break;
+        case FN_OP_CELL_LOOKUP: set_other(I.dst, D); break;
+        // in-place operands and multi-register results
+        case FN_OP_SUB_POS: set_other(I.dst, D); break;
+        case FN_OP_ROTATE2: set_other(I.dst, 2); break;
+        case FN_OP_ROTATE3: set_other(I.dst, 3); break;
+        case FN_OP_ROTPLANE: set_other(I.dst, std::max(3, D)); break;
+        case FN_OP_WARP_GRAD: case FN_OP_WARP_SIMPLEX:
+            set_other(I.dst, D);
+            if (I.c != FN_REG_NONE) set_other(I.c, 1);
+            break;
+        case FN_OP_FRACT_INIT: case FN_OP_FRACT_AMP: case FN_OP_FRACT_ACC: case FN_OP_DWF_AMP:
+            set_other(I.dst, 1);
+            if (I.a != FN_REG_NONE) set_other(I.a, 1);
+            if (I.b != FN_REG_NONE) set_other(I.b, 1);
+            break;
+        default: set_other(I.dst, 1); break;
+        }
+    }
+    return plan;
+}
+
+// One program -> `__device__ float <name>(int seed, float x, float y, float z, float w)`;
+// with a column plan the function also takes the column's state, `struct <name>_state`.
 // Its per-cell sub-programs (node-driven Minkowski P) come first, each as a
 // function `<name>_s<j>` plus a functor `<name>_s<j>_mk` the cellular walk calls
 // with the cell's offset vector.
-void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostringstream& o)
+void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostringstream& o, const ColPlan* col = nullptr)
 {
+    const std::string sub_prefix = name + "_s";
     for (size_t j = 0; j < prog.subs.size(); ++j) {
-        const std::string sub = name + "_s" + std::to_string(j);
+        const std::string sub = sub_prefix + std::to_string(j);
         emit_eval(prog.subs[j], sub, o);
         const int sd = prog.subs[j].dim;
         o << "struct " << sub << "_mk {\n    int seed;\n    static constexpr bool kNode = true;\n"
@@ -80,10 +224,42 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
     auto mk = [&](const FnInstr& I) {   // trailing functor argument of a cellular call
         return I.d == FN_REG_NONE ? std::string() : ", " + name + "_s" + std::to_string(I.d) + "_mk{seed}";
     };
-    o << "__device__ __forceinline__ float " << name << "(int seed, float x, float y, float z, float w)\n{\n";
-    o << "    (void)x; (void)y; (void)z; (void)w;\n";
     const char* root[4] = {"x", "y", "z", "w"};
+    if (col) {
+        o << "struct " << name << "_state {\n";
+        for (auto& st : col->states) {
+            o << "    fnd::" << st.type << " s" << st.pc << ";\n"
+              << "    static __device__ __forceinline__ void pos" << st.pc << "(float x, float y, float z, float* q)\n    {\n"
+              << "        x = fnd::opaque(x); y = fnd::opaque(y); z = fnd::opaque(z);\n";
+            for (size_t k = 0; k < st.pos.size(); ++k) o << "        q[" << k << "] = " << st.pos[k] << ";\n";
+            o << "    }\n";
+        }
+        const char* zc = root[h->dim - 1];
+        o << "    __device__ __forceinline__ void init(float x, float y, float z)\n    {\n";
+        for (auto& st : col->states)
+            o << "        s" << st.pc << ".init([&](float* q) { pos" << st.pc << "(x, y, z, q); });\n";
+        o << "    }\n    __device__ __forceinline__ unsigned prepare(float4* tab, unsigned lane, float " << zc << ")\n    {\n        return 0u";
+        for (auto& st : col->states) o << " | s" << st.pc << ".prepare(tab + " << st.table << ", lane, " << st.along << ")";
+        o << ";\n    }\n    __device__ __forceinline__ void enter(int seed, float4* tab, unsigned j, float x, float y, float z)\n    {\n";
+        for (auto& st : col->states)
+            o << "        s" << st.pc << ".enter(fnd::iadd(seed, " << ins[st.pc].seed << "), "
+              << (st.rate.cellular ? "tab + " + std::to_string(st.table) + ", j, " + st.jitter : "tab[" + std::to_string(st.table) + " + j].w")
+              << ", [&](float* q) { pos" << st.pc << "(x, y, z, q); });\n";
+        o << "    }\n};\n";
+    }
+    o << "__device__ __forceinline__ float " << name << "(int seed, float x, float y, float z, float w"
+      << (col ? ", const " + name + "_state& S, const float4* tab, unsigned j" : std::string()) << ")\n{\n";
+    o << "    (void)x; (void)y; (void)z; (void)w;\n";
     for (int i = 0; i < nregs; ++i) o << "    float " << r(i) << " = " << (i < h->dim ? root[i] : "0.0f") << ";\n";
+    // What is known of a register's value (beyond NaN): a constant, a noise output of bounded
+    // size, the strength a gradient warp returned.  A weighted strength of constant 0 makes the
+    // amplitude factor of an octave lerp(1, t, 0) = fma(0, t - 1, 1), which is 1 for every finite
+    // t; a NaN t comes from a NaN noise (already in the sum) or NaN positions, so the result is
+    // NaN with or without it.  The factor (and the warp's square root) is then left out:
+    // FBm(Simplex) octaves lose 5 of ~150 instructions, a warp octave ~20 of ~190.
+    enum Known { kUnknown, kConst, kBounded, kWarpStrength };
+    struct { Known what = kUnknown; float value = 0.0f; } known[FN_MAX_REGS + 4];
+    auto is_zero = [&](int reg) { return known[reg].what == kConst && known[reg].value == 0.0f; };
     for (int pc = 0; pc < h->n_instr; ++pc) {
         const FnInstr& I = ins[pc];
         const int D = I.dim;
@@ -102,6 +278,9 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
               << "; cp.distFunc = " << (I.aux & 15) << "; cp.minkowski = " << p(mk_index) << ";";
             return c.str();
         };
+        const ColState* cell = col ? col->at(pc) : nullptr;
+        const std::string cell_state = "S.s" + std::to_string(pc), cell_tab = cell ? "tab + " + std::to_string(cell->table) + ", j" : std::string();
+        auto fast = [&](const char* call) { return cell ? cell_state + ".fast ? " + cell_state + "." + call + cell_tab + ") : " : std::string(); };
         o << "    { // op " << (int)I.op << "\n";
         switch (I.op) {
         case FN_OP_CONST: o << "        " << r(I.dst) << " = " << p(0) << ";\n"; break;
@@ -141,6 +320,11 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             break;
         case FN_OP_NOISE: {
             o << "        const float f = " << p(0) << ";\n";
+            if (const ColState* st = col ? col->at(pc) : nullptr) {
+                o << "        " << r(I.dst) << " = fnd::scale_out(S.s" << pc << ".eval(tab[" << st->table << " + j]), " << p(1) << ", " << p(2)
+                  << ", " << p(3) << ");\n";
+                break;
+            }
             o << "        " << r(I.dst) << " = fnd::scale_out(fnd::" << noise_fn(I.aux) << D << "(" << sd;
             for (int j = 0; j < D; ++j) o << ", " << r(I.a + j) << " * f";
             o << "), " << p(1) << ", " << p(2) << ", " << p(3) << ");\n";
@@ -160,12 +344,14 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             break;
         case FN_OP_CELL_VALUE:
             o << "        const float pp[" << D << "] = " << pos(I.a) << ";\n        " << cellp(3) << "\n";
-            o << "        " << r(I.dst) << " = fnd::scale_out(fnd::cellular_value<" << D << ">(" << sd << ", pp, cp, " << ((I.aux >> 4) & 3)
-              << mk(I) << "), -fnd::kValueBounds, " << p(1) << ", " << p(2) << ");\n";
+            o << "        " << r(I.dst) << " = fnd::scale_out(" << fast("value(") << "fnd::cellular_value<" << D << ">(" << sd << ", pp, cp, "
+              << ((I.aux >> 4) & 3) << mk(I) << "), -fnd::kValueBounds, " << p(1) << ", " << p(2) << ");\n";
             break;
         case FN_OP_CELL_DIST:
             o << "        const float pp[" << D << "] = " << pos(I.a) << ";\n        " << cellp(3) << "\n";
-            o << "        float dist[4]; fnd::cellular_distances<" << D << ", "
+            o << "        float dist[4];\n        ";
+            if (cell) o << "if (" << cell_state << ".fast) " << cell_state << ".distances(" << cell_tab << ", dist); else ";
+            o << "fnd::cellular_distances<" << D << ", "
               << std::max((I.aux >> 4) & 3, (I.aux >> 8) & 3) + 1 << ">(" << sd << ", pp, cp, dist" << mk(I) << ");\n";
             o << "        float nmax; const float v = fnd::cellular_return<" << D << ">(dist, cp.distFunc, " << ((I.aux >> 4) & 3) << ", "
               << ((I.aux >> 8) & 3) << ", " << ((I.aux >> 12) & 7) << ", nmax);\n";
@@ -173,7 +359,9 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             break;
         case FN_OP_CELL_LOOKUP:
             o << "        const float pp[" << D << "] = " << pos(I.a) << ";\n        " << cellp(2) << "\n";
-            o << "        float oo[" << D << "]; fnd::cellular_lookup_pos<" << D << ">(" << sd << ", pp, cp, " << p(1) << ", oo" << mk(I) << ");\n";
+            o << "        float oo[" << D << "];\n        ";
+            if (cell) o << "if (" << cell_state << ".fast) " << cell_state << ".lookup(" << cell_tab << ", " << p(1) << ", oo); else ";
+            o << "fnd::cellular_lookup_pos<" << D << ">(" << sd << ", pp, cp, " << p(1) << ", oo" << mk(I) << ");\n";
             for (int j = 0; j < D; ++j) o << "        " << r(I.dst + j) << " = oo[" << j << "];\n";
             break;
         case FN_OP_WARP_GRAD: case FN_OP_WARP_SIMPLEX:
@@ -197,6 +385,10 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             o << "        " << r(I.b) << " = 1.0f;\n";
             break;
         case FN_OP_FRACT_AMP:
+            if (is_zero(I.c) && known[I.a].what == kBounded) {
+                o << "        " << r(I.b) << " = " << r(I.b) << " * " << r(I.d) << ";\n";
+                break;
+            }
             o << "        const float t = " << (I.aux ? "1.0f - " + r(I.a) : "(" + r(I.a) + " + 1.0f) * 0.5f") << ";\n";
             o << "        const float amp = " << r(I.b) << " * fnd::lerp(1.0f, t, " << r(I.c) << ");\n";
             o << "        " << r(I.b) << " = amp * " << r(I.d) << ";\n";
@@ -206,6 +398,10 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             else o << "        " << r(I.dst) << " = " << r(I.dst) << " + " << r(I.a) << " * " << r(I.b) << ";\n";
             break;
         case FN_OP_DWF_AMP:
+            if (is_zero(I.c) && known[I.a].what == kWarpStrength) {
+                o << "        " << r(I.b) << " = " << r(I.b) << " * " << r(I.d) << ";\n";
+                break;
+            }
             o << "        const float s = sqrtf(" << r(I.a) << "); " << r(I.a) << " = s;\n";
             o << "        const float amp = " << r(I.b) << " * fnd::lerp(1.0f, 1.0f - s, " << r(I.c) << ");\n";
             o << "        " << r(I.b) << " = amp * " << r(I.d) << ";\n";
@@ -261,9 +457,81 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             break;
         }
         o << "    }\n";
+        switch (I.op) {
+        case FN_OP_MOV: known[I.dst] = known[I.a]; break;
+        case FN_OP_CONST: known[I.dst].what = kConst; known[I.dst].value = P[I.prm]; break;
+        case FN_OP_NOISE: {
+            const bool bounded = std::fabs(P[I.prm + 1]) * std::fabs(P[I.prm + 2]) < 1e30f && std::fabs(P[I.prm + 3]) < 1e30f;
+            known[I.dst].what = bounded ? kBounded : kUnknown;
+            break;
+        }
+        case FN_OP_FRACT_INIT: case FN_OP_FRACT_ACC: known[I.dst].what = known[I.b].what = kUnknown; break;   // a keeps its size (abs)
+        case FN_OP_FRACT_AMP: known[I.b].what = kUnknown; break;
+        case FN_OP_DWF_AMP: known[I.a].what = known[I.b].what = kUnknown; break;
+        default:
+            for (int j = 0; j < 4; ++j) known[I.dst + j].what = kUnknown;
+            if ((I.op == FN_OP_WARP_GRAD || I.op == FN_OP_WARP_SIMPLEX) && I.c != FN_REG_NONE)
+                known[I.c].what = I.op == FN_OP_WARP_GRAD ? kWarpStrength : kUnknown;
+            break;
+        }
     }
     o << "    return " << r(h->out_reg) << ";\n}\n\n";
 }
+
+// Unit `u` of a column launch: 32 neighbouring points of the grid's plane (all axes but the
+// last; one per lane, lanes past the plane repeat its last point and store nothing), walked
+// along the last axis for up to A.col_len steps.
+void emit_column_unit(const CompiledProgram& prog, const std::string& eval, const std::string& name, std::ostringstream& o)
+{
+    const int D = prog.dim;
+    const char* pv[4] = {"px", "py", "pz", "pw"};
+    const std::string fixed = std::string("px, ") + (D > 2 ? "py" : "0.0f") + ", " + (D > 3 ? "pz" : "0.0f");
+    o << "__device__ __forceinline__ void " << name << "(const fn::PointArgs& A, float* __restrict__ out, unsigned u, float4* tab, float& mn, float& mx)\n{\n"
+      << "    const unsigned plane = A.col_plane, chunks = (plane + 31u) >> 5;\n"
+      << "    const unsigned seg = u / chunks, p = (u - seg * chunks) * 32u + (threadIdx.x & 31u);\n"
+      << "    const bool live = p < plane;\n"
+      << "    unsigned r = live ? p : plane - 1u;\n";
+    for (int j = 0; j < D - 1; ++j) {
+        if (j < D - 2)
+            o << "    const unsigned q" << j << " = fne::fast_div(r, A.divm[" << j << "], A.divs[" << j << "]);\n"
+              << "    const float " << pv[j] << " = fmaf(fnd::cvtf((int)(r - q" << j << " * (unsigned)A.count[" << j << "])), A.step[" << j
+              << "], A.offset[" << j << "]); r = q" << j << ";\n";
+        else
+            o << "    const float " << pv[j] << " = fmaf(fnd::cvtf((int)r), A.step[" << j << "], A.offset[" << j << "]);\n";
+    }
+    o << "    const unsigned t0 = seg * A.col_len, t1 = A.col_steps - t0 < A.col_len ? A.col_steps : t0 + A.col_len;\n"
+      << "    float* dst = out + (unsigned long long)t0 * plane + p;\n"
+      << "    const unsigned lane = threadIdx.x & 31u;\n"
+      << "    " << eval << "_state S;\n    S.init(" << fixed << ");\n"
+      << "#pragma unroll 1\n"
+      << "    for (unsigned tb = t0; tb < t1; tb += 32u) {\n"
+      << "        const unsigned fresh = S.prepare(tab, lane, fmaf(fnd::cvtf((int)(A.col_first + tb + lane)), A.step[" << D - 1
+      << "], A.offset[" << D - 1 << "]));\n"
+      << "        __syncwarp();\n"
+      << "        const unsigned n = t1 - tb < 32u ? t1 - tb : 32u;\n"
+      << "        for (unsigned j = 0; j < n;) {\n"
+      << "            if ((fresh >> j) & 1u) S.enter(A.seed, tab, j, " << fixed << ");\n"
+      << "            const unsigned ahead = (fresh >> j) >> 1, run = ahead ? j + (unsigned)__ffs((int)ahead) : n, stop = run < n ? run : n;\n"
+      << "#pragma unroll 1\n"
+      << "            for (; j < stop; ++j, dst += plane) {\n"
+      << "                const float " << pv[D - 1] << " = fmaf(fnd::cvtf((int)(A.col_first + tb + j)), A.step[" << D - 1 << "], A.offset[" << D - 1 << "]);\n"
+      << "                const float v = " << eval << "(A.seed";
+    for (int j = 0; j < 4; ++j) o << ", " << (j < D ? pv[j] : "0.0f");
+    o << ", S, tab, j);\n"
+      << "                if (live) *dst = v;\n"
+      << "                fne::fold(v, mn, mx);\n"
+      << "            }\n"
+      << "        }\n"
+      << "        __syncwarp();\n"
+      << "    }\n}\n\n";
+}
+
+// 256-thread blocks per SM a column kernel is bounded to, by the registers its state holds
+// beside the ~25 the step itself needs.  Keeping every octave's state is worth more than warps:
+// FBm(Perlin) 4D 32^4 takes 23 us with five states and one block, 37 us with four, 54 us with two
+// octaves' states and two blocks; FBm(Perlin) 256^3 (100 registers of state) 137 us with two
+// blocks, 156 with one, 243 with three (spills).
+int column_blocks(const ColPlan& plan) { return plan.regs <= 16 ? 4 : plan.regs <= 36 ? 3 : plan.regs <= 104 ? 2 : 1; }
 
 // Per-call kernels for program k: grid / position array / tileable.
 //
@@ -273,9 +541,22 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
 // parks the values in shared memory; with ppl == 4 the warp then writes the
 // chunk as 32 float4 stores (512 contiguous bytes per warp).  Small calls use
 // ppl == 1 so that their few points spread over as many SMs as possible.
-void emit_percall(const CompiledProgram& prog, int k, std::ostringstream& o)
+void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::ostringstream& o)
 {
     const int D = prog.dim;
+    if (!plan.states.empty()) {
+        const std::string id = std::to_string(k);
+        emit_column_unit(prog, "fnjit_ceval_" + id, "fnjit_colunit_" + id, o);
+        o << "extern \"C\" __global__ void __launch_bounds__(256, " << column_blocks(plan) << ") fnjit_col_" << id
+          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax)\n{\n"
+          << "    __shared__ float4 tab[8][" << plan.table << "];\n"
+          << "    __shared__ float smn[8], smx[8];\n"
+          << "    float mn = fne::inf(), mx = -fne::inf();\n"
+          << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
+          << "        fnjit_colunit_" << id << "(A, out, u, tab[threadIdx.x >> 5], mn, mx);\n"
+          << "    fne::grid_minmax(mn, mx, work, dminmax, smn, smx);\n"
+          << "}\n\n";
+    }
     const char* pv[4] = {"px", "py", "pz", "pw"};
     std::string call = "fnjit_eval_" + std::to_string(k) + "(A.seed";
     for (int j = 0; j < 4; ++j) call += std::string(", ") + (j < D ? pv[j] : "0.0f");
@@ -493,6 +774,36 @@ void emit_batch(const std::vector<const CompiledProgram*>& progs, std::ostringst
     }
 }
 
+// The batch kernel of a tree's grid requests walked in columns: a work item is eight
+// consecutive units of one request, one per warp.
+void emit_batch_column(const CompiledProgram& prog, size_t k, const ColPlan& plan, std::ostringstream& o)
+{
+    const std::string id = std::to_string(k);
+    emit_column_unit(prog, "fnjit_ceval_" + id, "fnjit_colunit_" + id, o);
+    o << "extern \"C\" __global__ void __launch_bounds__(256, " << column_blocks(plan) << ") fnjit_bcol_" << id
+      << "(fn::BatchHeader* hdr, const fn::BatchRequest* __restrict__ reqs, fn::BatchState* states,\n"
+         "    const uint2* __restrict__ items, fn::BatchGroup* grp)\n{\n"
+         "    __shared__ float4 tab[8][" << plan.table << "];\n"
+         "    __shared__ unsigned int s_item;\n"
+         "    __shared__ float smn[8], smx[8];\n"
+         "    const unsigned int first = grp->item_begin, last = grp->item_end;\n"
+         "    for (;;) {\n"
+         "        if (threadIdx.x == 0) s_item = first + atomicAdd(&grp->head, 1u);\n"
+         "        __syncthreads();\n"
+         "        const unsigned int it = s_item;\n"
+         "        __syncthreads();\n"
+         "        if (it >= last) break;\n"
+         "        const uint2 item = items[it];\n"
+         "        const fn::BatchRequest& rq = reqs[item.x];\n"
+         "        const fn::PointArgs args = rq.args;\n"
+         "        const unsigned u = item.y * 8u + (threadIdx.x >> 5);\n"
+         "        float mn = fne::inf(), mx = -fne::inf();\n"
+         "        if (u < args.col_units) fnjit_colunit_" << id << "(args, rq.out, u, tab[threadIdx.x >> 5], mn, mx);\n"
+         "        fne::block_minmax(mn, mx, smn, smx);\n"
+         "        if (threadIdx.x == 0) fne::finish_tile(rq, states + item.x, hdr, mn, mx);\n"
+         "    }\n}\n\n";
+}
+
 struct Module {
     cudaLibrary_t lib = nullptr;
     std::vector<uint64_t> hashes;
@@ -513,6 +824,13 @@ std::string jit_batch_source(const std::vector<const CompiledProgram*>& progs, i
     o << "// generated by fn_jit.cpp: batch module, variant " << variant << "\n" << embedded_device_source() << "\n";
     for (size_t k = 0; k < progs.size(); ++k) emit_eval(*progs[k], "fnjit_eval_" + std::to_string(k), o);
     emit_batch(progs, o, variant);
+    if (variant == 0)
+        for (size_t k = 0; k < progs.size(); ++k) {
+            const ColPlan plan = column_plan(*progs[k]);
+            if (plan.states.empty()) continue;
+            emit_eval(*progs[k], "fnjit_ceval_" + std::to_string(k), o, &plan);
+            emit_batch_column(*progs[k], k, plan, o);
+        }
     return o.str();
 }
 
@@ -521,7 +839,9 @@ std::string jit_percall_source(const CompiledProgram& prog)
     std::ostringstream o;
     o << "// generated by fn_jit.cpp: per-call module\n" << embedded_device_source() << "\n";
     emit_eval(prog, "fnjit_eval_0", o);
-    emit_percall(prog, 0, o);
+    const ColPlan plan = column_plan(prog);
+    if (!plan.states.empty()) emit_eval(prog, "fnjit_ceval_0", o, &plan);
+    emit_percall(prog, 0, plan, o);
     return o.str();
 }
 
@@ -742,23 +1062,30 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
     }
     std::unordered_map<uint64_t, JitKernels> found;
     std::unordered_map<uint64_t, cudaKernel_t> batch;
+    std::vector<ColPlan> plans;
+    for (auto* p : progs) plans.push_back(column_plan(*p));
     bool ok = true;
     for (size_t k = 0; ok && k < progs.size(); ++k) {
         cudaLibrary_t lib = mods[1 + k]->lib;
         JitKernels jk;
         jk.slot = (int)k;
+        for (auto& st : plans[k].states)
+            if (st.type[0] != 'V') jk.column_rates[jk.n_column_rates++] = st.rate;
         cudaKernel_t bk = nullptr;
         ok = cudaLibraryGetKernel(&jk.grid, lib, "fnjit_grid_0") == cudaSuccess &&
              cudaLibraryGetKernel(&jk.positions, lib, "fnjit_pos_0") == cudaSuccess &&
              (progs[k]->dim != 4 || cudaLibraryGetKernel(&jk.tileable, lib, "fnjit_tile_0") == cudaSuccess) &&
              (progs[k]->dim != 3 || (cudaLibraryGetKernel(&jk.solid, lib, "fnjit_solid_0") == cudaSuccess &&
                                      cudaLibraryGetKernel(&jk.list, lib, "fnjit_list_0") == cudaSuccess)) &&
+             (plans[k].states.empty() ||
+              (cudaLibraryGetKernel(&jk.column, lib, "fnjit_col_0") == cudaSuccess &&
+               cudaLibraryGetKernel(&jk.batch_column, mods[0]->lib, ("fnjit_bcol_" + std::to_string(k)).c_str()) == cudaSuccess)) &&
              cudaLibraryGetKernel(&bk, mods[0]->lib, ("fnjit_batch_" + std::to_string(k)).c_str()) == cudaSuccess;
-        const cudaKernel_t kern[3] = {jk.grid, jk.positions, jk.tileable};
-        for (int j = 0; ok && j < 3; ++j) {
+        const cudaKernel_t kern[4] = {jk.grid, jk.positions, jk.tileable, jk.column};
+        for (int j = 0; ok && j < 4; ++j) {
             int n = 0;
             if (kern[j] && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)kern[j], 256, 0) == cudaSuccess && n > 0)
-                jk.resident[j] = n;
+                (j < 3 ? jk.resident[j] : jk.column_resident) = n;
             else
                 cudaGetLastError();
         }
@@ -1052,6 +1379,81 @@ bool jit_auto_wait(int timeout_ms)
     return a.idle_cv.wait_for(lk, std::chrono::milliseconds(timeout_ms), idle);
 }
 
+constexpr double kColMaxGroups = 3.0;
+
+// Whether the grid of `a` is to be walked in columns (a tree without a column kernel, other
+// point sources and partial planes are not); sets its plane, steps and first step.
+bool jit_column_grid(PointArgs& a, const JitKernels& jk)
+{
+    if (a.src != kSrcGrid || a.total <= 0 || a.total > (1ll << 31) || !jk.column) return false;
+    long long plane = 1;
+    for (int k = 0; k < a.dim - 1; ++k) plane *= a.count[k];
+    if (plane <= 0 || a.total % plane || a.base % plane) return false;
+    // A step that crosses into another lattice cell rebuilds a Perlin state at about the cost
+    // of the point function: FBm(Perlin) 128^3 (69.7 us with the point kernel) takes 27, 39, 53,
+    // 70 and 86 us at 0.06, 0.25, 0.40, 0.62 and 0.79 crossings a step.  Value states never lose.
+    // A cellular state also builds one neighbourhood per distinct cell of a warp's lanes.
+    double rate = 0;
+    for (int k = 0; k < jk.n_column_rates; ++k) {
+        const ColumnRate& c = jk.column_rates[k];
+        double r = std::fabs((double)c.scale[a.dim - 1] * a.step[a.dim - 1]);
+        if (c.cellular) {
+            double groups = 1, left = 32;          // lanes not yet spread over an axis
+            for (int j = 0; j < a.dim - 1; ++j) {
+                const double spread = std::min<double>(left, a.count[j]);
+                groups *= 1 + (spread - 1) * std::fabs((double)c.scale[j] * a.step[j]);
+                left = std::max(1.0, left / a.count[j]);
+            }
+            if (!(groups <= kColMaxGroups)) return false;
+        }
+        rate += r < 1.0 ? r : 1.0;
+    }
+    if (jk.n_column_rates && !(rate < 0.6 * jk.n_column_rates)) return false;
+    a.col_plane = (unsigned)plane;
+    a.col_steps = (unsigned)(a.total / plane);
+    a.col_first = a.base / (unsigned)plane;
+    return true;
+}
+
+unsigned column_chunks(const PointArgs& a) { return (a.col_plane + 31) / 32; }
+
+// Cut the columns into units of at most `len` steps, evenly.
+void column_cut(PointArgs& a, unsigned len)
+{
+    const unsigned segs = (a.col_steps + len - 1) / len;
+    a.col_len = (a.col_steps + segs - 1) / segs;
+    a.col_units = column_chunks(a) * ((a.col_steps + a.col_len - 1) / a.col_len);
+}
+
+// Steps per unit of a launch that has the GPU to itself: setting a unit up costs about 7 steps
+// (FBm(Perlin) 256^3: 221, 170, 147 us at 8, 16, 32 steps a unit), and an SM works on
+// `column_resident` blocks of 8 units at once, so minimise (blocks of the busiest SM, at least
+// the resident ones) x (set-up + length).
+void column_cut_alone(PointArgs& a, const JitKernels& jk)
+{
+    constexpr double kInit = 7.0;
+    const unsigned n = a.col_steps, chunks = column_chunks(a);
+    const double sms = num_sms(), fill = std::max(1, jk.column_resident);
+    unsigned best = 1;
+    double best_cost = 1e300;
+    for (int w = 1; w <= 16; ++w) {
+        const unsigned fit = (unsigned)std::min<double>(n, std::max(1.0, std::floor(w * sms * 8.0 / chunks)));
+        const unsigned len = (n + fit - 1) / fit;
+        const double units = (double)chunks * ((n + len - 1) / len);
+        const double cost = std::max(fill, std::ceil(units / (8.0 * sms))) * (kInit + len);
+        if (cost < best_cost) { best_cost = cost; best = len; }
+    }
+    column_cut(a, best);
+}
+
+unsigned jit_column_tiles(PointArgs& args, unsigned len)
+{
+    // a request with fewer units than a block has warps is cut finer
+    const unsigned long long work = (unsigned long long)column_chunks(args) * args.col_steps;
+    column_cut(args, (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(len, (work + 7) / 8)));
+    return (args.col_units + 7) / 8;
+}
+
 bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax, cudaStream_t stream,
                 cudaError_t& err)
 {
@@ -1059,6 +1461,14 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     JitKernels jk;
     if (args.total <= 0 || args.total > (1ll << 31) || !jit_lookup(hash, jk)) return false;
     const int which = args.src == kSrcGrid ? 0 : args.src == kSrcPositions ? 1 : 2;
+    PointArgs c = args;
+    if (which == 0 && jit_column_grid(c, jk)) {
+        column_cut_alone(c, jk);
+        const unsigned grid = std::min<unsigned>((c.col_units + 7) / 8, (unsigned)kMaxReduceBlocks);
+        void* params[] = {&c, &out, &work, &dminmax};
+        err = cudaLaunchKernel((const void*)jk.column, dim3(grid), dim3(256), params, 0, stream);
+        return true;
+    }
     cudaKernel_t k = which == 0 ? jk.grid : which == 1 ? jk.positions : jk.tileable;
     if (!k) return false;
     const int sms = num_sms();

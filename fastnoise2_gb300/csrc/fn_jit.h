@@ -23,12 +23,24 @@
 
 namespace fn {
 
+constexpr int kMaxColumnStates = 10;
+
+struct ColumnRate {                   // lattice cells per unit along the grid's axes, of one column state
+    float scale[4] = {};
+    bool cellular = false;
+};
+
 struct JitKernels {
     cudaKernel_t grid = nullptr;      // GenUniformGrid for the program's dimensionality
     cudaKernel_t positions = nullptr; // GenPositionArray
     cudaKernel_t tileable = nullptr;  // GenTileable2D (4D programs only)
     cudaKernel_t solid = nullptr;     // chunk meshing (3D programs): classification bitmasks of a grid
     cudaKernel_t list = nullptr;      // chunk meshing (3D programs): grid values at listed point indices
+    cudaKernel_t column = nullptr;    // grids walked along their last axis (trees with separable lattice noise)
+    cudaKernel_t batch_column = nullptr;   // the same for a batch's grid requests
+    ColumnRate column_rates[kMaxColumnStates];   // of its Perlin and cellular states
+    int n_column_rates = 0;
+    int column_resident = 1;          // its 256-thread blocks per SM at once
     int slot = -1;                    // index in the module's batch kernel
     int resident[3] = {1, 1, 1};      // 256-thread blocks per SM of grid / positions / tileable at once
 };
@@ -80,6 +92,12 @@ bool jit_build_batch_variants(const std::vector<const CompiledProgram*>& progs, 
 
 // The batch kernel of `hash` in `variant`, or false when it is not built (or JIT is off).
 bool jit_batch_kernel(uint64_t hash, int variant, BatchKernel& out);
+
+// Whether a grid is to be walked in columns by the kernels `jk` (fn_column.cuh); if so `args`
+// gets its plane and steps.  jit_column_tiles cuts it into units of at most `len` steps and
+// returns a batch's work items for it (eight units each).
+bool jit_column_grid(PointArgs& args, const JitKernels& jk);
+unsigned jit_column_tiles(PointArgs& args, unsigned len);
 
 // Queue a background build of the batch variants of `prog` (a tuning table loaded in this
 // process may name variants that have not been built yet).

@@ -29,6 +29,9 @@ struct PointArgs {
     // Index of this launch's first point in the whole request (0 unless a large grid is
     // generated slab by slab): positions come from base + i, output and min/max cover i only.
     unsigned int base;
+    // Column launches (grids walked along their last axis): points of the plane across it, steps
+    // of this launch along it and the index of the first, steps per work unit and units.
+    unsigned int col_plane, col_steps, col_first, col_len, col_units;
 };
 
 // Per-launch reduction workspace.  Every block folds its min/max into the two
