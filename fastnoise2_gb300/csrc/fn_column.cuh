@@ -309,4 +309,185 @@ struct ValueCol {
     FND float eval(const float4& e) const { return lerp(lo, hi, e.z); }
 };
 
+// Cellular noise with a constant jitter and (squared) Euclidean distance, 2D and 3D.  A
+// step's 3^D cells are the same while the column stays in its cell: the warp computes the
+// jittered points of each distinct cell neighbourhood its lanes need (one lane per cell) into
+// shared memory, and every lane keeps each cell's squared distance across the column, so a
+// step is two fmas and a comparison per cell, in the reference's order, without pruning.
+// Neighbourhoods beyond kGroups per warp and positions past 1e9 (or NaN) take the point
+// function; `fast` says which, the same for all lanes.
+enum ColCellKind { kColValue, kColDistance, kColLookup };
+
+template <int D, ColCellKind Kind, int NS = 1>
+struct CellCol {
+    static constexpr int N = D == 3 ? 27 : 9, kGroups = 4;
+    float part[N];                                // squared distance across the column
+    int icell;
+    unsigned slot;                                // first cell of this lane's neighbourhood in the table
+    bool fast;
+
+    // per warp behind the 32 step entries: kGroups x N cells (direction and scale, or the cell
+    // point for kColLookup), then their hashes (kColValue)
+    static constexpr int kTable = 32 + kGroups * N + (Kind == kColValue ? N : 0);
+
+    template <typename Pos>
+    FND void init(Pos&&)
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) part[i] = 0.0f;
+        icell = 0x7fffffff;
+        slot = 0;
+        fast = false;
+    }
+    // entry: the column offsets of the three cell planes as the walk of this kind computes them
+    // (kColLookup: the coordinate), and the plane's base cell (INT_MIN: no fast cell)
+    FND unsigned prepare(float4* tab, unsigned lane, float p)
+    {
+        const int base = fabs_(p) < 1e9f ? iadd(cvti(p), -1) : (int)0x80000000;
+        const float c0 = cvtf(base), c1 = c0 + 1.0f, c2 = c1 + 1.0f;
+        float4 e;
+        if (Kind == kColValue) { e.x = c0 - p; e.y = e.x + 1.0f; e.z = e.y + 1.0f; }
+        else if (Kind == kColDistance) { e.x = c0 - p; e.y = c1 - p; e.z = c2 - p; }
+        else { e.x = e.y = e.z = p; }
+        e.w = __int_as_float(base);
+        tab[lane] = e;
+        const int before = __shfl_up_sync(0xffffffffu, base, 1);
+        return __ballot_sync(0xffffffffu, base != (lane ? before : icell));
+    }
+    template <typename Pos>
+    FND void enter(int seed, float4* tab, unsigned j, float jitter, Pos&& pos)
+    {
+        const int base = __float_as_int(tab[j].w);
+        if (base == icell) return;
+        icell = base;
+        float q[D - 1];
+        int cb[D - 1];
+        pos(q);
+        bool sane = base != (int)0x80000000;
+#pragma unroll
+        for (int k = 0; k < D - 1; ++k) {
+            sane = sane && fabs_(q[k]) < 1e9f;
+            cb[k] = iadd(cvti(q[k]), -1);
+        }
+        fast = __all_sync(0xffffffffu, sane) != 0;
+        if (!fast) return;
+        float4* cells = tab + 32;
+        int* hashes = reinterpret_cast<int*>(cells + kGroups * N);
+        const int lane = (int)(threadIdx.x & 31u);
+        const int at[3] = {D == 3 ? lane / 9 : lane / 3, D == 3 ? (lane / 3) % 3 : lane % 3, lane % 3};
+        unsigned todo = 0xffffffffu, groups = 0;
+        __syncwarp();
+#pragma unroll 1
+        do {
+            const int leader = __ffs((int)todo) - 1;
+            int c[D];
+            float cf[D];
+            bool mine = true;
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const int b = k == D - 1 ? base : __shfl_sync(0xffffffffu, cb[k % (D - 1)], leader);
+                if (k < D - 1) mine = mine && cb[k % (D - 1)] == b;
+                c[k] = imul(iadd(b, at[k]), kPrimes[k]);
+                cf[k] = cvtf(b);
+                if (at[k] > 0) cf[k] += 1.0f;
+                if (at[k] > 1) cf[k] += 1.0f;
+            }
+            if (lane < N) {
+                const int h = cell_hash<D>(seed, c);
+                float d[D + 1];
+                cell_dir_raw<D>(h, d);
+                cell_dir_scale<D>(jitter, d);
+                float4 e;
+                if (Kind == kColLookup) {
+                    e.x = fmaf(d[0], d[D], cf[0]);
+                    e.y = fmaf(d[1], d[D], cf[1]);
+                    e.z = D == 3 ? fmaf(d[2 % D], d[D], cf[2 % D]) : 0.0f;
+                    e.w = 0.0f;
+                } else {
+                    e = D == 3 ? make_float4(d[0], d[1], d[2 % D], d[D]) : make_float4(d[0], 0.0f, d[1], d[D]);
+                }
+                cells[groups * N + lane] = e;
+                if (Kind == kColValue) hashes[groups * N + lane] = h;
+            }
+            if (mine) slot = groups * N;
+            todo &= ~__ballot_sync(0xffffffffu, mine);
+            ++groups;
+        } while (todo && groups < (unsigned)kGroups);
+        __syncwarp();
+        fast = todo == 0;
+        if (!fast) return;
+        float t[D - 1][3];
+#pragma unroll
+        for (int k = 0; k < D - 1; ++k) {
+            const float c0 = cvtf(cb[k]), c1 = c0 + 1.0f, c2 = c1 + 1.0f;
+            t[k][0] = c0 - q[k];
+            t[k][1] = Kind == kColValue ? t[k][0] + 1.0f : c1 - q[k];
+            t[k][2] = Kind == kColValue ? t[k][1] + 1.0f : c2 - q[k];
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float4 e = cells[slot + i];
+            const int i0 = D == 3 ? i / 9 : i / 3, i1 = D == 3 ? (i / 3) % 3 : 0;
+            const float o0 = Kind == kColLookup ? e.x - q[0] : fmaf(e.x, e.w, t[0][i0]);
+            part[i] = o0 * o0;
+            if (D == 3) {
+                const float o1 = Kind == kColLookup ? e.y - q[1 % (D - 1)] : fmaf(e.y, e.w, t[1 % (D - 1)][i1]);
+                part[i] = fmaf(o1, o1, part[i]);
+            }
+        }
+    }
+    // squared distance of cell i at step entry e
+    FND float dist2(const float4* cells, const float4& e, int i) const
+    {
+        const float t = i % 3 == 0 ? e.x : (i % 3 == 1 ? e.y : e.z);
+        float o;
+        if (Kind == kColLookup) {
+            o = (D == 3 ? cells[slot + i].z : cells[slot + i].y) - t;
+        } else {
+            const float2 ds = reinterpret_cast<const float2*>(cells + slot + i)[1];
+            o = fmaf(ds.x, ds.y, t);
+        }
+        return fmaf(o, o, part[i]);
+    }
+    // index of the closest cell, the first of equals
+    FND int closest(const float4* tab, unsigned j) const
+    {
+        const float4* cells = tab + 32;
+        const float4 e = tab[j];
+        float best = dist2(cells, e, 0);
+        int at = 0;
+#pragma unroll
+        for (int i = 1; i < N; ++i) {
+            const float d = dist2(cells, e, i);
+            const bool closer = d < best;
+            best = closer ? d : best;
+            at = closer ? i : at;
+        }
+        return at;
+    }
+    FND float value(const float4* tab, unsigned j) const
+    {
+        return cvtf(reinterpret_cast<const int*>(tab + 32 + kGroups * N)[slot + closest(tab, j)]);
+    }
+    FND void distances(const float4* tab, unsigned j, float* dist) const
+    {
+        const float4* cells = tab + 32;
+        const float4 e = tab[j];
+        dist[0] = dist[1] = dist[2] = dist[3] = __int_as_float(0x7F800000);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float d = dist2(cells, e, i);
+            if (NS > 1) dist[1] = fmaxf(fminf(dist[1], d), dist[0]);
+            dist[0] = fminf(dist[0], d);
+        }
+    }
+    FND void lookup(const float4* tab, unsigned j, float scale, float* out) const
+    {
+        const float4 e = tab[32 + slot + closest(tab, j)];
+        out[0] = e.x * scale;
+        out[1] = e.y * scale;
+        if (D == 3) out[2 % D] = e.z * scale;
+    }
+};
+
 }  // namespace fnd

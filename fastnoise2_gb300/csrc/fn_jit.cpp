@@ -180,7 +180,24 @@ ColPlan column_plan(const CompiledProgram& prog)
                 add_state(pc, "ValueCol<" + std::to_string(D) + ">", P[I.prm], 4, 32, false);
             R[I.dst] = Reg();
             break;
-        case FN_OP_CELL_LOOKUP: set_other(I.dst, D); break;
+        case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: {
+            // constant jitter, no size jitter, distances that are sums of squares (the 2D value
+            // walk takes the root of Euclidean ones), the closest cell or two
+            const int df = I.aux & 15, slots = I.op == FN_OP_CELL_DIST ? std::max((I.aux >> 4) & 3, (I.aux >> 8) & 3) + 1 : ((I.aux >> 4) & 3) + 1;
+            const Reg jit = R[I.b];
+            const bool sums = df == 1 || (df == 0 && !(I.op == FN_OP_CELL_VALUE && D == 2));
+            if (D < 4 && sums && jit.kind == Reg::kConst && std::isfinite(jit.scale) && I.c == FN_REG_NONE && I.d == FN_REG_NONE &&
+                (I.op == FN_OP_CELL_LOOKUP || slots <= (I.op == FN_OP_CELL_DIST ? 2 : 1))) {
+                const std::string kind = I.op == FN_OP_CELL_VALUE ? "kColValue" : I.op == FN_OP_CELL_DIST ? "kColDistance" : "kColLookup";
+                const int cells = D == 3 ? 27 : 9;
+                ColState* st = add_state(pc, "CellCol<" + std::to_string(D) + ", fnd::" + kind + ", " + std::to_string(I.op == FN_OP_CELL_DIST ? slots : 1) + ">",
+                                         P[I.prm], cells + 4, 32 + 4 * cells + (I.op == FN_OP_CELL_VALUE ? cells : 0), true);
+                if (st) st->jitter = "fnd::CellConst<" + std::to_string(D) + ">::jitter * " + lit(jit.scale);
+            }
+            if (I.op == FN_OP_CELL_LOOKUP) set_other(I.dst, D);
+            else R[I.dst] = Reg();
+            break;
+        }
         // in-place operands and multi-register results
         case FN_OP_SUB_POS: set_other(I.dst, D); break;
         case FN_OP_ROTATE2: set_other(I.dst, 2); break;
@@ -527,11 +544,12 @@ void emit_column_unit(const CompiledProgram& prog, const std::string& eval, cons
 }
 
 // 256-thread blocks per SM a column kernel is bounded to, by the registers its state holds
-// beside the ~25 the step itself needs.  Keeping every octave's state is worth more than warps:
-// FBm(Perlin) 4D 32^4 takes 23 us with five states and one block, 37 us with four, 54 us with two
-// octaves' states and two blocks; FBm(Perlin) 256^3 (100 registers of state) 137 us with two
-// blocks, 156 with one, 243 with three (spills).
-int column_blocks(const ColPlan& plan) { return plan.regs <= 16 ? 4 : plan.regs <= 36 ? 3 : plan.regs <= 104 ? 2 : 1; }
+// beside the ~25-60 the step itself needs.  Keeping every state is worth more than warps:
+// FBm(Perlin) 4D 32^4 takes 23 us with five octaves' states and one block, 37 us with four, 54 us
+// with two octaves' and two blocks; FBm(Perlin) 256^3 (100 registers of state) 142 us with two
+// blocks, 156 with one, 243 with three (spills); terrain and CellularLookup 160^3 (31 registers)
+// 269 and 55 us with two blocks, 279 and 60 with three, 290 and 66 with four.
+int column_blocks(const ColPlan& plan) { return plan.regs <= 16 ? 4 : plan.regs <= 104 ? 2 : 1; }
 
 // Per-call kernels for program k: grid / position array / tileable.
 //

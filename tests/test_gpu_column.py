@@ -20,6 +20,13 @@ TREES = {
                              RHS=N("Multiply", LHS=N("DomainOffset", Source=N("Value", Feature_Scale=6.0)).set("Offset", 3.25, 0)
                                                 .set("Offset", -7.5, 1).set("Offset", 0.125, 2),
                                    RHS=N("Simplex", Feature_Scale=12.0))),
+    "CellValue": lambda: N("CellularValue", Feature_Scale=21.0, Seed_Offset=4),
+    "CellDistance": lambda: N("CellularDistance", Feature_Scale=34.0, Grid_Jitter=0.7).set("Distance Function", "Euclidean")
+                              .set("Return Type", "Index0Sub1"),
+    "CellClosest": lambda: N("CellularDistance", Feature_Scale=9.0, Grid_Jitter=-1.4),
+    "CellLookup": lambda: N("CellularLookup", Feature_Scale=27.0, Lookup=N("Perlin", Feature_Scale=40.0)),
+    "CellTies": lambda: N("CellularValue", Feature_Scale=8.0, Grid_Jitter=0.0),
+    "Terrain": trees.terrain_c2,
 }
 SHAPES = {2: [(1, 1), (31, 33), (33, 64), (70, 65), (5, 200)],
           3: [(1, 1, 1), (5, 3, 2), (33, 1, 31), (7, 9, 33), (16, 16, 16), (11, 6, 97)],
