@@ -72,6 +72,42 @@ FND float lerp(float a, float b, float t) { return fmaf(t, b - a, a); }
 FND float hermite(float t) { return t * t * fmaf(-t, 2.0f, 3.0f); }
 FND float quintic(float t) { return t * t * t * fmaf(t, fmaf(t, 6.0f, -15.0f), 10.0f); }
 
+#ifdef FN_GRADIENT_TABLE
+// Gradient directions by hash, per component, in shared memory (specialised kernels that use 3D
+// or 4D gradient noise fill it with gradient_init() first): component k of direction h is
+// table[k * 32 + (h & 31)], -1, 0 or 1; 3D directions repeat after 16.  Products with them are
+// exact, so the fmas add the direction's signed offsets in the reference's order (a zero's sign
+// can differ; every user ends in scale_out, which adds a nonzero bound).  Three or four
+// conflict-free loads and fmas replace 12 or 17 instructions, 9 of them on the half-rate ALU
+// pipe that bounds simplex noise: FBm(Simplex) 160^3 71.7 -> 67.7 us, terrain 268 -> 256 us.
+template <int D>
+FND float* gradient_table()
+{
+    __shared__ float t[D * 32];
+    return t;
+}
+template <int D>
+FND void gradient_init()
+{
+    float* t = gradient_table<D>();
+    if (threadIdx.x < 32u) {
+        const int h = (int)threadIdx.x;
+        // the axes of the direction's signed terms, in ascending significance of their sign bits
+        const int a = D == 3 ? ((h & 8) ? 1 : 0) : ((h & 24) ? 0 : 1);
+        const int b = D == 3 ? ((h & 4) ? ((h & 9) == 8 ? 0 : 2) : ((h & 8) ? 2 : 1)) : ((h & 16) ? 1 : 2);
+        const int c = D == 3 ? -1 : ((h & 24) == 24 ? 2 : 3);
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+            t[k * 32 + h] = k == a ? ((h & 1) ? -1.0f : 1.0f) : k == b ? ((h & 2) ? -1.0f : 1.0f) : k == c ? ((h & 4) ? -1.0f : 1.0f) : 0.0f;
+    }
+    __syncthreads();
+}
+FND float grad3(int h, float x, float y, float z)
+{
+    const float* t = gradient_table<3>() + (h & 31);
+    return fmaf(t[64], z, fmaf(t[32], y, t[0] * x));
+}
+#else
 // GetGradientDotCommon, portable branch (Utils.inl:132-158)
 FND float grad3(int h, float x, float y, float z)
 {
@@ -81,6 +117,7 @@ FND float grad3(int h, float x, float y, float z)
     const float v = b2 ? (x_case ? x : z) : (b3 ? z : y);
     return flip(u, h << 31) + flip(v, h << 30);
 }
+#endif
 // GetGradientDotPerlin 2D, portable branch (Utils.inl:181-190)
 FND float grad2(int h, float x, float y)
 {
@@ -89,6 +126,13 @@ FND float grad2(int h, float x, float y)
     bool s = (h << 29) < 0;
     return fmaf(1.0f + (float)kRoot2, s ? y : x, s ? x : y);
 }
+#ifdef FN_GRADIENT_TABLE
+FND float grad4(int h, float x, float y, float z, float w)
+{
+    const float* t = gradient_table<4>() + (h & 31);
+    return fmaf(t[96], w, fmaf(t[64], z, fmaf(t[32], y, t[0] * x)));
+}
+#else
 // GetGradientDotPerlin 4D, portable branch (Utils.inl:205-218)
 FND float grad4(int h, float x, float y, float z, float w)
 {
@@ -99,6 +143,7 @@ FND float grad4(int h, float x, float y, float z, float w)
     const float c = both34 ? z : w;
     return (flip(a, h << 31) + flip(b, h << 30)) + flip(c, h << 29);
 }
+#endif
 
 // Sin / Cos: Cody-Waite reduction by pi/2 (three-part constant), Taylor
 // polynomials on [-pi/4, pi/4] evaluated by Horner with fmaf.

@@ -79,6 +79,7 @@ struct ColPlan {
     std::vector<ColState> states;
     int regs = 0;                      // registers the states hold
     int table = 0;                     // float4 of shared table per warp
+    float setup = 0.0f;                // set-up of a unit, in steps (see below)
 
     const ColState* at(int pc) const
     {
@@ -109,8 +110,25 @@ ColPlan column_plan(const CompiledProgram& prog)
         R[(size_t)k].scale = 1.0f;
         R[(size_t)k].axis = k;
     }
+    // Instructions of setting a state up and of a step of it, and of a step of the other
+    // instructions, roughly (from instruction counts of the kernels): their ratio decides how
+    // short a unit may be.
+    double setup = 30, step = 15;
+    auto generic_cost = [&](const FnInstr& I) -> double {
+        const int d = I.dim - 2;
+        static const double simplex[3] = {90, 130, 230}, super[3] = {130, 380, 900}, lattice[3] = {90, 200, 440}, warp[3] = {70, 190, 500},
+                            cells[3] = {200, 700, 2400};
+        switch (I.op) {
+        case FN_OP_NOISE: return I.aux == FN_NOISE_SIMPLEX ? simplex[d] : I.aux == FN_NOISE_SUPERSIMPLEX ? super[d] : lattice[d];
+        case FN_OP_WARP_GRAD: return warp[d];
+        case FN_OP_WARP_SIMPLEX: return 2 * warp[d];
+        case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: return cells[d];
+        default: return 4;
+        }
+    };
     // a state for the instruction, if its position is separable and the kernel has room
-    auto add_state = [&](int pc, const std::string& type, float freq, int regs, int table, bool cellular) -> ColState* {
+    auto add_state = [&](int pc, const std::string& type, float freq, int regs, int table, bool cellular, double setup_cost,
+                         double step_cost) -> ColState* {
         const FnInstr& I = ins[pc];
         bool ok = R[(size_t)(I.a + I.dim - 1)].kind == Reg::kColumn && plan.regs + regs <= kColMaxRegs &&
                   plan.states.size() < kMaxColumnStates && plan.table + table <= kColMaxTable;
@@ -131,12 +149,15 @@ ColPlan column_plan(const CompiledProgram& prog)
         st.table_size = table;
         plan.table += table;
         plan.regs += regs;
+        setup += setup_cost;
+        step += step_cost;
         plan.states.push_back(st);
         return &plan.states.back();
     };
     for (int pc = 0; pc < h->n_instr; ++pc) {
         const FnInstr& I = ins[pc];
         const int D = I.dim;
+        const size_t had = plan.states.size();
         auto scaled = [&](const Reg& a, float f) {
             Reg r = a;
             if (r.kind == Reg::kConst) r.kind = Reg::kFixed;
@@ -175,9 +196,10 @@ ColPlan column_plan(const CompiledProgram& prog)
         }
         case FN_OP_NOISE:
             if (I.aux == FN_NOISE_PERLIN)
-                add_state(pc, "PerlinCol<" + std::to_string(D) + ">", P[I.prm], D == 2 ? 18 : D == 3 ? 20 : 38, 32, false);
+                add_state(pc, "PerlinCol<" + std::to_string(D) + ">", P[I.prm], D == 2 ? 18 : D == 3 ? 20 : 38, 32, false,
+                          D == 2 ? 90 : D == 3 ? 140 : 280, D == 2 ? 22 : D == 3 ? 17 : 32);
             else if (I.aux == FN_NOISE_VALUE)
-                add_state(pc, "ValueCol<" + std::to_string(D) + ">", P[I.prm], 4, 32, false);
+                add_state(pc, "ValueCol<" + std::to_string(D) + ">", P[I.prm], 4, 32, false, 60, 4);
             R[I.dst] = Reg();
             break;
         case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: {
@@ -191,7 +213,8 @@ ColPlan column_plan(const CompiledProgram& prog)
                 const std::string kind = I.op == FN_OP_CELL_VALUE ? "kColValue" : I.op == FN_OP_CELL_DIST ? "kColDistance" : "kColLookup";
                 const int cells = D == 3 ? 27 : 9;
                 ColState* st = add_state(pc, "CellCol<" + std::to_string(D) + ", fnd::" + kind + ", " + std::to_string(I.op == FN_OP_CELL_DIST ? slots : 1) + ">",
-                                         P[I.prm], cells + 4, 32 + 4 * cells + (I.op == FN_OP_CELL_VALUE ? cells : 0), true);
+                                         P[I.prm], cells + 4, 32 + 4 * cells + (I.op == FN_OP_CELL_VALUE ? cells : 0), true,
+                                         D == 3 ? 300 : 150, D == 3 ? 190 : 65);
                 if (st) st->jitter = "fnd::CellConst<" + std::to_string(D) + ">::jitter * " + lit(jit.scale);
             }
             if (I.op == FN_OP_CELL_LOOKUP) set_other(I.dst, D);
@@ -214,8 +237,28 @@ ColPlan column_plan(const CompiledProgram& prog)
             break;
         default: set_other(I.dst, 1); break;
         }
+        if (plan.states.size() == had) step += generic_cost(I);
     }
+    plan.setup = (float)(setup / step);
     return plan;
+}
+
+// Statements that fill the shared gradient tables (fn_device.cuh) a kernel of `prog` reads: of
+// the dimensionalities of its gradient noises, per-cell sub-programs included, but for those
+// that are column states.
+void gradient_dims(const CompiledProgram& prog, const ColPlan* col, bool* used)
+{
+    const FnProgramHeader* h = reinterpret_cast<const FnProgramHeader*>(prog.blob.data());
+    const FnInstr* ins = fn_program_instrs(h);
+    for (int pc = 0; pc < h->n_instr; ++pc)
+        if (ins[pc].op == FN_OP_NOISE && ins[pc].aux != FN_NOISE_VALUE && !(col && col->at(pc))) used[ins[pc].dim] = true;
+    for (auto& sub : prog.subs) gradient_dims(sub, nullptr, used);
+}
+std::string gradient_setup(const CompiledProgram& prog, const ColPlan* col = nullptr)
+{
+    bool used[5] = {};
+    gradient_dims(prog, col, used);
+    return std::string(used[3] ? "    fnd::gradient_init<3>();\n" : "") + (used[4] ? "    fnd::gradient_init<4>();\n" : "");
 }
 
 // One program -> `__device__ float <name>(int seed, float x, float y, float z, float w)`;
@@ -569,6 +612,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax)\n{\n"
           << "    __shared__ float4 tab[8][" << plan.table << "];\n"
           << "    __shared__ float smn[8], smx[8];\n"
+          << gradient_setup(prog, &plan)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
           << "        fnjit_colunit_" << id << "(A, out, u, tab[threadIdx.x >> 5], mn, mx);\n"
@@ -585,6 +629,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned ppl)\n{\n"
           << "    __shared__ float4 stage[8][32];\n"
           << "    __shared__ float smn[8], smx[8];\n"
+          << gradient_setup(prog)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    const unsigned total = (unsigned)A.total;\n"
           << "    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;\n"
@@ -666,6 +711,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "(fn::PointArgs A, unsigned* __restrict__ above, unsigned* __restrict__ solid, fn::MinMaxWork* work, float* dminmax,\n"
           << "    float iso, unsigned ppl)\n{\n"
           << "    __shared__ float smn[8], smx[8];\n"
+          << gradient_setup(prog)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    const unsigned total = (unsigned)A.total;\n"
           << "    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;\n"
@@ -691,6 +737,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "}\n\n";
         o << "extern \"C\" __global__ void __launch_bounds__(256, 4) fnjit_list_" << k
           << "(fn::PointArgs A, const unsigned* __restrict__ idx, const unsigned* __restrict__ count, float* __restrict__ out)\n{\n"
+          << gradient_setup(prog)
           << "    const unsigned n = *count;\n"
           << "    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {\n"
           << "        const unsigned i = idx[j];\n"
@@ -770,6 +817,7 @@ void emit_batch(const std::vector<const CompiledProgram*>& progs, std::ostringst
              "    const uint2* __restrict__ items, fn::BatchGroup* grp)\n{\n"
              "    __shared__ unsigned int s_item;\n"
              "    __shared__ float smn[" << bv.threads / 32 << "], smx[" << bv.threads / 32 << "];\n"
+          << gradient_setup(*progs[k]) <<
              "    const unsigned int first = grp->item_begin, last = grp->item_end;\n"
              "    const unsigned int tile_points = hdr->tile_points;\n"
              "    for (;;) {\n"
@@ -804,6 +852,7 @@ void emit_batch_column(const CompiledProgram& prog, size_t k, const ColPlan& pla
          "    __shared__ float4 tab[8][" << plan.table << "];\n"
          "    __shared__ unsigned int s_item;\n"
          "    __shared__ float smn[8], smx[8];\n"
+      << gradient_setup(prog, &plan) <<
          "    const unsigned int first = grp->item_begin, last = grp->item_end;\n"
          "    for (;;) {\n"
          "        if (threadIdx.x == 0) s_item = first + atomicAdd(&grp->head, 1u);\n"
@@ -839,7 +888,7 @@ std::atomic<bool> g_enabled{true};
 std::string jit_batch_source(const std::vector<const CompiledProgram*>& progs, int variant)
 {
     std::ostringstream o;
-    o << "// generated by fn_jit.cpp: batch module, variant " << variant << "\n" << embedded_device_source() << "\n";
+    o << "// generated by fn_jit.cpp: batch module, variant " << variant << "\n#define FN_GRADIENT_TABLE\n" << embedded_device_source() << "\n";
     for (size_t k = 0; k < progs.size(); ++k) emit_eval(*progs[k], "fnjit_eval_" + std::to_string(k), o);
     emit_batch(progs, o, variant);
     if (variant == 0)
@@ -855,7 +904,7 @@ std::string jit_batch_source(const std::vector<const CompiledProgram*>& progs, i
 std::string jit_percall_source(const CompiledProgram& prog)
 {
     std::ostringstream o;
-    o << "// generated by fn_jit.cpp: per-call module\n" << embedded_device_source() << "\n";
+    o << "// generated by fn_jit.cpp: per-call module\n#define FN_GRADIENT_TABLE\n" << embedded_device_source() << "\n";
     emit_eval(prog, "fnjit_eval_0", o);
     const ColPlan plan = column_plan(prog);
     if (!plan.states.empty()) emit_eval(prog, "fnjit_ceval_0", o, &plan);
@@ -1087,6 +1136,7 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
         cudaLibrary_t lib = mods[1 + k]->lib;
         JitKernels jk;
         jk.slot = (int)k;
+        jk.column_setup = plans[k].setup;
         for (auto& st : plans[k].states)
             if (st.type[0] != 'V') jk.column_rates[jk.n_column_rates++] = st.rate;
         cudaKernel_t bk = nullptr;
@@ -1443,13 +1493,13 @@ void column_cut(PointArgs& a, unsigned len)
     a.col_units = column_chunks(a) * ((a.col_steps + a.col_len - 1) / a.col_len);
 }
 
-// Steps per unit of a launch that has the GPU to itself: setting a unit up costs about 7 steps
-// (FBm(Perlin) 256^3: 221, 170, 147 us at 8, 16, 32 steps a unit), and an SM works on
-// `column_resident` blocks of 8 units at once, so minimise (blocks of the busiest SM, at least
-// the resident ones) x (set-up + length).
+// Steps per unit of a launch that has the GPU to itself: setting a unit up costs
+// `column_setup` steps (about 7 for FBm(Perlin): 256^3 takes 221, 170, 147 us at 8, 16, 32 steps
+// a unit; a fraction of one for a terrain tree), and an SM works on `column_resident` blocks of
+// 8 units at once, so minimise (blocks of the busiest SM, at least the resident ones) x
+// (set-up + length).
 void column_cut_alone(PointArgs& a, const JitKernels& jk)
 {
-    constexpr double kInit = 7.0;
     const unsigned n = a.col_steps, chunks = column_chunks(a);
     const double sms = num_sms(), fill = std::max(1, jk.column_resident);
     unsigned best = 1;
@@ -1458,7 +1508,7 @@ void column_cut_alone(PointArgs& a, const JitKernels& jk)
         const unsigned fit = (unsigned)std::min<double>(n, std::max(1.0, std::floor(w * sms * 8.0 / chunks)));
         const unsigned len = (n + fit - 1) / fit;
         const double units = (double)chunks * ((n + len - 1) / len);
-        const double cost = std::max(fill, std::ceil(units / (8.0 * sms))) * (kInit + len);
+        const double cost = std::max(fill, std::ceil(units / (8.0 * sms))) * (jk.column_setup + len);
         if (cost < best_cost) { best_cost = cost; best = len; }
     }
     column_cut(a, best);

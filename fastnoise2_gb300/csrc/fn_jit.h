@@ -40,6 +40,7 @@ struct JitKernels {
     cudaKernel_t batch_column = nullptr;   // the same for a batch's grid requests
     ColumnRate column_rates[kMaxColumnStates];   // of its Perlin and cellular states
     int n_column_rates = 0;
+    float column_setup = 1.0f;        // set-up of a unit of columns, in steps
     int column_resident = 1;          // its 256-thread blocks per SM at once
     int slot = -1;                    // index in the module's batch kernel
     int resident[3] = {1, 1, 1};      // 256-thread blocks per SM of grid / positions / tileable at once
