@@ -16,6 +16,13 @@ using fnd::fmin_;
 // +infinity (a bit pattern, so that NVRTC, which lacks the compiler builtins, accepts it)
 __device__ __forceinline__ float inf() { return __int_as_float(0x7f800000); }
 
+// Overlap of consecutive launches on a stream (programmatic dependent launch; no effect in
+// launches without that attribute).  let_stream_continue: the next launch may take SM slots
+// this one leaves free from here on.  wait_for_stream: the stream's earlier work is complete
+// and its memory visible; before the first access to memory other launches may touch.
+__device__ __forceinline__ void let_stream_continue() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Root position of point i (Generator.inl:104-105, 160-162, 225-228, 295-297, 400-406).
 __device__ __forceinline__ void root_position(const fn::PointArgs& a, long long i, float* R)
 {
@@ -131,6 +138,7 @@ __device__ __forceinline__ void grid_minmax(float mn, float mx, fn::MinMaxWork* 
 {
     block_minmax(mn, mx, smn, smx);
     if (threadIdx.x != 0) return;
+    wait_for_stream();                           // the workspace may be an earlier launch's
     if (mn <= mx) {
         atomicMax(&work->mn_key, ~enc_ordered(mn));
         atomicMax(&work->mx_key, enc_ordered(mx));

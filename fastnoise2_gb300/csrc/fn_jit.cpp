@@ -569,6 +569,7 @@ void emit_column_unit(const CompiledProgram& prog, const std::string& eval, cons
       << "], A.offset[" << D - 1 << "]));\n"
       << "        __syncwarp();\n"
       << "        const unsigned n = t1 - tb < 32u ? t1 - tb : 32u;\n"
+      << "        fne::wait_for_stream();\n"
       << "        for (unsigned j = 0; j < n;) {\n"
       << "            if ((fresh >> j) & 1u) S.enter(A.seed, tab, j, " << fixed << ");\n"
       << "            const unsigned ahead = (fresh >> j) >> 1, run = ahead ? j + (unsigned)__ffs((int)ahead) : n, stop = run < n ? run : n;\n"
@@ -612,6 +613,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax)\n{\n"
           << "    __shared__ float4 tab[8][" << plan.table << "];\n"
           << "    __shared__ float smn[8], smx[8];\n"
+          << "    fne::let_stream_continue();\n"
           << gradient_setup(prog, &plan)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
@@ -625,10 +627,12 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
     call += ")";
 
     auto kernel = [&](const char* name, const std::string& prologue, const std::string& position) {
+        // prologue: before the first point (a kernel that reads the caller's arrays waits there)
         o << "extern \"C\" __global__ void __launch_bounds__(256, 4) " << name << "_" << k
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned ppl)\n{\n"
           << "    __shared__ float4 stage[8][32];\n"
           << "    __shared__ float smn[8], smx[8];\n"
+          << "    fne::let_stream_continue();\n"
           << gradient_setup(prog)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    const unsigned total = (unsigned)A.total;\n"
@@ -651,6 +655,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "            st[t * 32u + lane] = v;\n"
           << "        }\n"
           << "        __syncwarp();\n"
+          << "        fne::wait_for_stream();\n"
           << "        if (ppl == 4u && aligned && base + 128u <= total) {\n"
           << "            reinterpret_cast<float4*>(out + base)[lane] = stage[warp][lane];\n"
           << "        } else {\n"
@@ -686,7 +691,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
         std::ostringstream pos;
         for (int j = 0; j < D; ++j)
             pos << "                const float " << pv[j] << " = A.offset[" << j << "] + __ldg(A.pos[" << j << "] + i + A.base);\n";
-        kernel("fnjit_pos", "", pos.str());
+        kernel("fnjit_pos", "    fne::wait_for_stream();\n", pos.str());
     }
     // tileable (4D programs): Generator.inl:370-433
     if (D == 4) {
@@ -1522,6 +1527,23 @@ unsigned jit_column_tiles(PointArgs& args, unsigned len)
     return (args.col_units + 7) / 8;
 }
 
+// Launch a per-call kernel so that it may start while the stream's previous kernel drains
+// (programmatic dependent launch): its blocks take free SM slots, compute their first points
+// and wait for that kernel before they touch memory (fne::wait_for_stream).
+cudaError_t launch_overlapped(cudaKernel_t k, unsigned grid, void** params, cudaStream_t stream)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, (const void*)k, params);
+}
+
 bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax, cudaStream_t stream,
                 cudaError_t& err)
 {
@@ -1534,7 +1556,7 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
         column_cut_alone(c, jk);
         const unsigned grid = std::min<unsigned>((c.col_units + 7) / 8, (unsigned)kMaxReduceBlocks);
         void* params[] = {&c, &out, &work, &dminmax};
-        err = cudaLaunchKernel((const void*)jk.column, dim3(grid), dim3(256), params, 0, stream);
+        err = launch_overlapped(jk.column, grid, params, stream);
         return true;
     }
     cudaKernel_t k = which == 0 ? jk.grid : which == 1 ? jk.positions : jk.tileable;
@@ -1559,7 +1581,7 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     if (blocks < 1) blocks = 1;
     PointArgs a = args;
     void* params[] = {&a, &out, &work, &dminmax, &ppl};
-    err = cudaLaunchKernel((const void*)k, dim3((unsigned)blocks), dim3(256), params, 0, stream);
+    err = launch_overlapped(k, (unsigned)blocks, params, stream);
     return true;
 }
 
