@@ -46,6 +46,17 @@ FND float fmax_(float a, float b) { return a > b ? a : b; }
 FND float fabs_(float a) { return __int_as_float(__float_as_int(a) & 0x7FFFFFFF); }
 FND float flip(float v, int s) { return __int_as_float(__float_as_int(v) ^ (s & (int)0x80000000)); }
 FND float flipm(float v, bool m) { return m ? __int_as_float(__float_as_int(v) ^ (int)0x80000000) : v; }
+// By the sign bit of m: v negated where it is set; the lattice neighbour on the upper side
+// (c + P, given) or, where it is set, on the lower one (c - P)
+FND float flips(float v, float m) { return __int_as_float((__float_as_int(m) & (int)0x80000000) ^ __float_as_int(v)); }
+FND int sided(int upper, int prime, float m)
+{
+    // in assembly, as a shift and a multiply-add (FMA pipe): written out, the compiler turns
+    // it back into a compare and selects
+    int r;
+    asm("{ .reg .u32 s; shr.u32 s, %1, 31; mad.lo.s32 %0, s, %2, %3; }" : "=r"(r) : "r"(__float_as_uint(m)), "r"((int)(0u - (unsigned)prime * 2u)), "r"(upper));
+    return r;
+}
 FND int cvti(float x)
 {
     // cvt.rni saturates: below -2^31 (and -inf) it already gives INT_MIN, as x86 does; at or
@@ -59,6 +70,7 @@ FND int imul(int a, int b) { return (int)((unsigned)a * (unsigned)b); }
 FND int iadd(int a, int b) { return (int)((unsigned)a + (unsigned)b); }
 FND float invsqrt(float x) { return 1.0f / sqrtf(x); }
 
+FND int hashm(int v) { return imul(v, kHashA); }
 FND int hash_mix(int v) { int h = imul(v, kHashA); return (h >> 15) ^ h; }
 FND int hash(int seed, int a, int b) { int h = imul(seed ^ a ^ b, kHashA); return (h >> 15) ^ h; }
 FND int hash(int seed, int a, int b, int c) { int h = imul(seed ^ a ^ b ^ c, kHashA); return (h >> 15) ^ h; }
@@ -102,9 +114,16 @@ FND void gradient_init()
     }
     __syncthreads();
 }
-FND float grad3(int h, float x, float y, float z)
+// the table entry of hash product p (hash_mix(p') before its mix): byte offset 4 * (mix & 31)
+template <int D>
+FND const float* gradient_of(int p)
 {
-    const float* t = gradient_table<3>() + (h & 31);
+    const unsigned at = (((unsigned)p >> 13) ^ ((unsigned)p << 2)) & 124u;
+    return reinterpret_cast<const float*>(reinterpret_cast<const char*>(gradient_table<D>()) + at);
+}
+FND float gdot3(int p, float x, float y, float z)
+{
+    const float* t = gradient_of<3>(p);
     return fmaf(t[64], z, fmaf(t[32], y, t[0] * x));
 }
 #else
@@ -117,6 +136,7 @@ FND float grad3(int h, float x, float y, float z)
     const float v = b2 ? (x_case ? x : z) : (b3 ? z : y);
     return flip(u, h << 31) + flip(v, h << 30);
 }
+FND float gdot3(int p, float x, float y, float z) { return grad3((p >> 15) ^ p, x, y, z); }
 #endif
 // GetGradientDotPerlin 2D, portable branch (Utils.inl:181-190)
 FND float grad2(int h, float x, float y)
@@ -127,9 +147,9 @@ FND float grad2(int h, float x, float y)
     return fmaf(1.0f + (float)kRoot2, s ? y : x, s ? x : y);
 }
 #ifdef FN_GRADIENT_TABLE
-FND float grad4(int h, float x, float y, float z, float w)
+FND float gdot4(int p, float x, float y, float z, float w)
 {
-    const float* t = gradient_table<4>() + (h & 31);
+    const float* t = gradient_of<4>(p);
     return fmaf(t[96], w, fmaf(t[64], z, fmaf(t[32], y, t[0] * x)));
 }
 #else
@@ -143,6 +163,7 @@ FND float grad4(int h, float x, float y, float z, float w)
     const float c = both34 ? z : w;
     return (flip(a, h << 31) + flip(b, h << 30)) + flip(c, h << 29);
 }
+FND float gdot4(int p, float x, float y, float z, float w) { return grad4((p >> 15) ^ p, x, y, z, w); }
 #endif
 
 // Sin / Cos: Cody-Waite reduction by pi/2 (three-part constant), Taylor
@@ -299,10 +320,10 @@ FND float simplex3(int seed, float x, float y, float z)
     float f3 = f0 - (unskew + (float)(3.0 / 4.0));
     f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f);
     f0 *= f0; f0 *= f0; f1 *= f1; f1 *= f1; f2 *= f2; f2 *= f2; f3 *= f3; f3 *= f3;
-    float g0 = grad3(hash(seed, xp, yp, zp), dx0, dy0, dz0);
-    float g1 = grad3(hash(seed, mx1 ? iadd(xp, kPrimeX) : xp, my1 ? iadd(yp, kPrimeY) : yp, mz1 ? zp : iadd(zp, kPrimeZ)), dx1, dy1, dz1);
-    float g2 = grad3(hash(seed, nx2 ? iadd(xp, kPrimeX) : xp, ny2 ? yp : iadd(yp, kPrimeY), nz2 ? zp : iadd(zp, kPrimeZ)), dx2, dy2, dz2);
-    float g3 = grad3(hash(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ)), dx3, dy3, dz3);
+    float g0 = gdot3(hashhb(seed, xp, yp, zp), dx0, dy0, dz0);
+    float g1 = gdot3(hashhb(seed, mx1 ? iadd(xp, kPrimeX) : xp, my1 ? iadd(yp, kPrimeY) : yp, mz1 ? zp : iadd(zp, kPrimeZ)), dx1, dy1, dz1);
+    float g2 = gdot3(hashhb(seed, nx2 ? iadd(xp, kPrimeX) : xp, ny2 ? yp : iadd(yp, kPrimeY), nz2 ? zp : iadd(zp, kPrimeZ)), dx2, dy2, dz2);
+    float g3 = gdot3(hashhb(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ)), dx3, dy3, dz3);
     return fmaf(g3, f3, fmaf(g2, f2, fmaf(g1, f1, g0 * f0)));
 }
 
@@ -340,11 +361,11 @@ FND float simplex4(int seed, float x, float y, float z, float w)
     float f4 = f0 + fmaf(unskew, (float)(-4.0 * (kRoot5 + 3.0) / (kRoot5 + 5.0)), (float)(-4.0 / 5.0));
     f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f); f4 = fmaxf(f4, 0.0f);
     f0 *= f0; f0 *= f0; f1 *= f1; f1 *= f1; f2 *= f2; f2 *= f2; f3 *= f3; f3 *= f3; f4 *= f4; f4 *= f4;
-    float g0 = grad4(hash(seed, xp, yp, zp, wp), dx0, dy0, dz0, dw0);
-    float g1 = grad4(hash(seed, rx > 2 ? iadd(xp, kPrimeX) : xp, ry > 2 ? iadd(yp, kPrimeY) : yp, rz > 2 ? iadd(zp, kPrimeZ) : zp, rw > 2 ? iadd(wp, kPrimeW) : wp), dx1, dy1, dz1, dw1);
-    float g2 = grad4(hash(seed, rx > 1 ? iadd(xp, kPrimeX) : xp, ry > 1 ? iadd(yp, kPrimeY) : yp, rz > 1 ? iadd(zp, kPrimeZ) : zp, rw > 1 ? iadd(wp, kPrimeW) : wp), dx2, dy2, dz2, dw2);
-    float g3 = grad4(hash(seed, rx > 0 ? iadd(xp, kPrimeX) : xp, ry > 0 ? iadd(yp, kPrimeY) : yp, rz > 0 ? iadd(zp, kPrimeZ) : zp, rw > 0 ? iadd(wp, kPrimeW) : wp), dx3, dy3, dz3, dw3);
-    float g4 = grad4(hash(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ), iadd(wp, kPrimeW)), dx4, dy4, dz4, dw4);
+    float g0 = gdot4(hashhb(seed, xp, yp, zp, wp), dx0, dy0, dz0, dw0);
+    float g1 = gdot4(hashhb(seed, rx > 2 ? iadd(xp, kPrimeX) : xp, ry > 2 ? iadd(yp, kPrimeY) : yp, rz > 2 ? iadd(zp, kPrimeZ) : zp, rw > 2 ? iadd(wp, kPrimeW) : wp), dx1, dy1, dz1, dw1);
+    float g2 = gdot4(hashhb(seed, rx > 1 ? iadd(xp, kPrimeX) : xp, ry > 1 ? iadd(yp, kPrimeY) : yp, rz > 1 ? iadd(zp, kPrimeZ) : zp, rw > 1 ? iadd(wp, kPrimeW) : wp), dx2, dy2, dz2, dw2);
+    float g3 = gdot4(hashhb(seed, rx > 0 ? iadd(xp, kPrimeX) : xp, ry > 0 ? iadd(yp, kPrimeY) : yp, rz > 0 ? iadd(zp, kPrimeZ) : zp, rw > 0 ? iadd(wp, kPrimeW) : wp), dx3, dy3, dz3, dw3);
+    float g4 = gdot4(hashhb(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ), iadd(wp, kPrimeW)), dx4, dy4, dz4, dw4);
     return fmaf(g0, f0, fmaf(g1, f1, fmaf(g2, f2, fmaf(g3, f3, g4 * f4))));
 }
 
@@ -408,7 +429,7 @@ FND float supersimplex2(int seed, float x, float y)
 FND void ss_consider(float& maxScore, int& bits, float score, int b)
 {
     bits = score > maxScore ? b : bits;
-    maxScore = fmax_(maxScore, score);
+    maxScore = fmaxf(maxScore, score);           // only compared and added to: a zero's sign and NaN cannot show
 }
 
 FND float supersimplex3(int seed, float x, float y, float z)
@@ -446,59 +467,64 @@ FND float supersimplex3(int seed, float x, float y, float z)
     float cs = (float)(1 + 3 * kReflect) * sum;
     float value, stemA, stemB;
     {
-        float g = grad3(hash(seed, xp, yp, zp), dx, dy, dz);
+        float g = gdot3(hashhb(seed, xp, yp, zp), dx, dy, dz);
         float fb = fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA))) * 0.5f;
         stemA = fb - (float)(kDA * 0.5);
         stemB = fb - (float)(kDB * 0.5);
         value = (fb * fb) * (fb * fb) * g;
     }
+    // Every other vertex lies on one of two opposite sides, chosen by a comparison a < b.  Its
+    // outcome is the sign of a - b (of a + 0 against zero), so offsets are flipped by that sign
+    // bit and lattice coordinates stepped by it through a multiply-add, which keeps compares,
+    // selects and adds off the half-rate ALU pipe.
+    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ);   // the positive side
     {
-        bool m = xyzn < 0.0f;
-        float off = flipm((float)(3 * kReflect + 1), m);
-        float g = grad3(hash(seed, iadd(xp, m ? -kPrimeX : kPrimeX), iadd(yp, m ? -kPrimeY : kPrimeY), iadd(zp, m ? -kPrimeZ : kPrimeZ)), dx - off, dy - off, dz - off);
+        float m = xyzn + 0.0f;
+        float off = flips((float)(3 * kReflect + 1), m);
+        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), sided(yq, kPrimeY, m), sided(zq, kPrimeZ, m)), dx - off, dy - off, dz - off);
         float fb = fmaxf(fmaf(off, cs, stemA), 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = xyzn < zn;
-        float o0 = flipm((float)(2 * kReflect), m);
-        float g = grad3(hash(seed, iadd(xp, m ? -kPrimeX : kPrimeX), iadd(yp, m ? -kPrimeY : kPrimeY), zp), dx, dy, dz - o0);
-        float fb = fminf(flipm(dz, m) - stemB, 0.0f);
+        float m = xyzn - zn;
+        float o0 = flips((float)(2 * kReflect), m);
+        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), sided(yq, kPrimeY, m), zp), dx, dy, dz - o0);
+        float fb = fminf(flips(dz, m) - stemB, 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = xyzn < yn;
-        float o0 = flipm((float)(2 * kReflect), m);
-        float g = grad3(hash(seed, iadd(xp, m ? -kPrimeX : kPrimeX), yp, iadd(zp, m ? -kPrimeZ : kPrimeZ)), dx, dy - o0, dz);
-        float fb = fminf(flipm(dy, m) - stemB, 0.0f);
+        float m = xyzn - yn;
+        float o0 = flips((float)(2 * kReflect), m);
+        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), yp, sided(zq, kPrimeZ, m)), dx, dy - o0, dz);
+        float fb = fminf(flips(dy, m) - stemB, 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = xyzn < xn;
-        float o0 = flipm((float)(2 * kReflect), m);
-        float g = grad3(hash(seed, xp, iadd(yp, m ? -kPrimeY : kPrimeY), iadd(zp, m ? -kPrimeZ : kPrimeZ)), dx - o0, dy, dz);
-        float fb = fminf(flipm(dx, m) - stemB, 0.0f);
+        float m = xyzn - xn;
+        float o0 = flips((float)(2 * kReflect), m);
+        float g = gdot3(hashhb(seed, xp, sided(yq, kPrimeY, m), sided(zq, kPrimeZ, m)), dx - o0, dy, dz);
+        float fb = fminf(flips(dx, m) - stemB, 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = xn < 0.0f;
-        float o0 = flipm((float)kReflect, m);
-        float g = grad3(hash(seed, iadd(xp, m ? -kPrimeX : kPrimeX), yp, zp), dx + o0, dy - o0, dz - o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flipm(dx, m), 0.0f);
+        float m = xn + 0.0f;
+        float o0 = flips((float)kReflect, m);
+        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), yp, zp), dx + o0, dy - o0, dz - o0);
+        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dx, m), 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = yn < 0.0f;
-        float o0 = flipm((float)kReflect, m);
-        float g = grad3(hash(seed, xp, iadd(yp, m ? -kPrimeY : kPrimeY), zp), dx - o0, dy + o0, dz - o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flipm(dy, m), 0.0f);
+        float m = yn + 0.0f;
+        float o0 = flips((float)kReflect, m);
+        float g = gdot3(hashhb(seed, xp, sided(yq, kPrimeY, m), zp), dx - o0, dy + o0, dz - o0);
+        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dy, m), 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     {
-        bool m = zn < 0.0f;
-        float o0 = flipm((float)kReflect, m);
-        float g = grad3(hash(seed, xp, yp, iadd(zp, m ? -kPrimeZ : kPrimeZ)), dx - o0, dy - o0, dz + o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flipm(dz, m), 0.0f);
+        float m = zn + 0.0f;
+        float o0 = flips((float)kReflect, m);
+        float g = gdot3(hashhb(seed, xp, yp, sided(zq, kPrimeZ, m)), dx - o0, dy - o0, dz + o0);
+        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dz, m), 0.0f);
         value = fmaf((fb * fb) * (fb * fb), g, value);
     }
     return value;
@@ -552,88 +578,89 @@ FND float supersimplex4(int seed, float x, float y, float z, float w)
     float cs = (float)(1 + 4 * kU) * sum;
     float value, stemA, stemB;
     {
-        float g = grad4(hash(seed, xp, yp, zp, wp), dx, dy, dz, dw);
+        float g = gdot4(hashhb(seed, xp, yp, zp, wp), dx, dy, dz, dw);
         float fb = fmaf(-dw, dw, fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA)))) * 0.5f;
         stemA = fb - (float)(kDA * 0.5);
         stemB = fb - (float)(kDB * 0.5);
         value = (fb * fb) * (fb * fb) * g;
     }
-#define FND_P(m, base, P) iadd(base, (m) ? -(P) : (P))
+    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ), wq = iadd(wp, kPrimeW);   // as in 3D
+#define FND_P(m, base, P) sided(base, P, m)
 #define FND_ACC(fbexpr, gexpr) { float g_ = (gexpr); float fb_ = fmaxf((fbexpr), 0.0f); value = fmaf((fb_ * fb_) * (fb_ * fb_), g_, value); }
     {
-        bool m = xyzwn < 0.0f;
-        float o = flipm((float)(4 * kU + 1), m);
-        FND_ACC(fmaf(o, cs, stemA), grad4(hash(seed, FND_P(m, xp, kPrimeX), FND_P(m, yp, kPrimeY), FND_P(m, zp, kPrimeZ), FND_P(m, wp, kPrimeW)), dx - o, dy - o, dz - o, dw - o));
+        float m = xyzwn + 0.0f;
+        float o = flips((float)(4 * kU + 1), m);
+        FND_ACC(fmaf(o, cs, stemA), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o, dy - o, dz - o, dw - o));
     }
     {
-        bool m = xyzwn < wn;
-        float o1 = flipm((float)(3 * kU + 1), m), o0 = flipm((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flipm(dw, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), FND_P(m, yp, kPrimeY), FND_P(m, zp, kPrimeZ), wp), dx - o1, dy - o1, dz - o1, dw - o0));
+        float m = xyzwn - wn;
+        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
+        FND_ACC(fmaf(o1, cs, stemB) - flips(dw, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), wp), dx - o1, dy - o1, dz - o1, dw - o0));
     }
     {
-        bool m = xyzwn < zn;
-        float o1 = flipm((float)(3 * kU + 1), m), o0 = flipm((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flipm(dz, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), FND_P(m, yp, kPrimeY), zp, FND_P(m, wp, kPrimeW)), dx - o1, dy - o1, dz - o0, dw - o1));
+        float m = xyzwn - zn;
+        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
+        FND_ACC(fmaf(o1, cs, stemB) - flips(dz, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), zp, FND_P(m, wq, kPrimeW)), dx - o1, dy - o1, dz - o0, dw - o1));
     }
     {
-        bool m = xyzwn < yn;
-        float o1 = flipm((float)(3 * kU + 1), m), o0 = flipm((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flipm(dy, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), yp, FND_P(m, zp, kPrimeZ), FND_P(m, wp, kPrimeW)), dx - o1, dy - o0, dz - o1, dw - o1));
+        float m = xyzwn - yn;
+        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
+        FND_ACC(fmaf(o1, cs, stemB) - flips(dy, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o1, dy - o0, dz - o1, dw - o1));
     }
     {
-        bool m = xyzwn < xn;
-        float o1 = flipm((float)(3 * kU + 1), m), o0 = flipm((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flipm(dx, m), grad4(hash(seed, xp, FND_P(m, yp, kPrimeY), FND_P(m, zp, kPrimeZ), FND_P(m, wp, kPrimeW)), dx - o0, dy - o1, dz - o1, dw - o1));
+        float m = xyzwn - xn;
+        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
+        FND_ACC(fmaf(o1, cs, stemB) - flips(dx, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o0, dy - o1, dz - o1, dw - o1));
     }
     {
-        bool m = xn < 0.0f;
-        float o1 = flipm((float)(kU + 1), m), o0 = flipm((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flipm(dx, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), yp, zp, wp), dx - o1, dy - o0, dz - o0, dw - o0));
+        float m = xn + 0.0f;
+        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
+        FND_ACC(fmaf(o0, cs, stemA) + flips(dx, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, zp, wp), dx - o1, dy - o0, dz - o0, dw - o0));
     }
     {
-        bool m = xn < -yn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dx + dy, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), FND_P(m, yp, kPrimeY), zp, wp), dx - o1, dy - o1, dz - o0, dw - o0));
+        float m = xn + yn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dy, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), zp, wp), dx - o1, dy - o1, dz - o0, dw - o0));
     }
     {
-        bool m = xn < -zn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dx + dz, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), yp, FND_P(m, zp, kPrimeZ), wp), dx - o1, dy - o0, dz - o1, dw - o0));
+        float m = xn + zn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dz, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, FND_P(m, zq, kPrimeZ), wp), dx - o1, dy - o0, dz - o1, dw - o0));
     }
     {
-        bool m = xn < -wn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dx + dw, m), grad4(hash(seed, FND_P(m, xp, kPrimeX), yp, zp, FND_P(m, wp, kPrimeW)), dx - o1, dy - o0, dz - o0, dw - o1));
+        float m = xn + wn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dw, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, zp, FND_P(m, wq, kPrimeW)), dx - o1, dy - o0, dz - o0, dw - o1));
     }
     {
-        bool m = yn < 0.0f;
-        float o1 = flipm((float)(kU + 1), m), o0 = flipm((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flipm(dy, m), grad4(hash(seed, xp, FND_P(m, yp, kPrimeY), zp, wp), dx - o0, dy - o1, dz - o0, dw - o0));
+        float m = yn + 0.0f;
+        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
+        FND_ACC(fmaf(o0, cs, stemA) + flips(dy, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), zp, wp), dx - o0, dy - o1, dz - o0, dw - o0));
     }
     {
-        bool m = yn < -zn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dy + dz, m), grad4(hash(seed, xp, FND_P(m, yp, kPrimeY), FND_P(m, zp, kPrimeZ), wp), dx - o0, dy - o1, dz - o1, dw - o0));
+        float m = yn + zn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dy + dz, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), wp), dx - o0, dy - o1, dz - o1, dw - o0));
     }
     {
-        bool m = yn < -wn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dy + dw, m), grad4(hash(seed, xp, FND_P(m, yp, kPrimeY), zp, FND_P(m, wp, kPrimeW)), dx - o0, dy - o1, dz - o0, dw - o1));
+        float m = yn + wn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dy + dw, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), zp, FND_P(m, wq, kPrimeW)), dx - o0, dy - o1, dz - o0, dw - o1));
     }
     {
-        bool m = zn < 0.0f;
-        float o1 = flipm((float)(kU + 1), m), o0 = flipm((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flipm(dz, m), grad4(hash(seed, xp, yp, FND_P(m, zp, kPrimeZ), wp), dx - o0, dy - o0, dz - o1, dw - o0));
+        float m = zn + 0.0f;
+        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
+        FND_ACC(fmaf(o0, cs, stemA) + flips(dz, m), gdot4(hashhb(seed, xp, yp, FND_P(m, zq, kPrimeZ), wp), dx - o0, dy - o0, dz - o1, dw - o0));
     }
     {
-        bool m = zn < -wn;
-        float o1 = flipm((float)(2 * kU + 1), m), o0 = flipm((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flipm(dz + dw, m), grad4(hash(seed, xp, yp, FND_P(m, zp, kPrimeZ), FND_P(m, wp, kPrimeW)), dx - o0, dy - o0, dz - o1, dw - o1));
+        float m = zn + wn;
+        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
+        FND_ACC(fmaf(o0, cs, stemB) + flips(dz + dw, m), gdot4(hashhb(seed, xp, yp, FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o0, dy - o0, dz - o1, dw - o1));
     }
     {
-        bool m = wn < 0.0f;
-        float o1 = flipm((float)(kU + 1), m), o0 = flipm((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flipm(dw, m), grad4(hash(seed, xp, yp, zp, FND_P(m, wp, kPrimeW)), dx - o0, dy - o0, dz - o0, dw - o1));
+        float m = wn + 0.0f;
+        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
+        FND_ACC(fmaf(o0, cs, stemA) + flips(dw, m), gdot4(hashhb(seed, xp, yp, zp, FND_P(m, wq, kPrimeW)), dx - o0, dy - o0, dz - o0, dw - o1));
     }
 #undef FND_P
 #undef FND_ACC
@@ -663,10 +690,10 @@ FND float perlin3(int seed, float x, float y, float z)
     float u = quintic(xf0), v = quintic(yf0), s = quintic(zf0);
     // seed ^ y ^ z shared by each x pair of corners (xor reassociated: the same hashes)
     const int a00 = seed ^ y0 ^ z0, a10 = seed ^ y1 ^ z0, a01 = seed ^ y0 ^ z1, a11 = seed ^ y1 ^ z1;
-    return lerp(lerp(lerp(grad3(hash_mix(a00 ^ x0), xf0, yf0, zf0), grad3(hash_mix(a00 ^ x1), xf1, yf0, zf0), u),
-                     lerp(grad3(hash_mix(a10 ^ x0), xf0, yf1, zf0), grad3(hash_mix(a10 ^ x1), xf1, yf1, zf0), u), v),
-                lerp(lerp(grad3(hash_mix(a01 ^ x0), xf0, yf0, zf1), grad3(hash_mix(a01 ^ x1), xf1, yf0, zf1), u),
-                     lerp(grad3(hash_mix(a11 ^ x0), xf0, yf1, zf1), grad3(hash_mix(a11 ^ x1), xf1, yf1, zf1), u), v), s);
+    return lerp(lerp(lerp(gdot3(hashm(a00 ^ x0), xf0, yf0, zf0), gdot3(hashm(a00 ^ x1), xf1, yf0, zf0), u),
+                     lerp(gdot3(hashm(a10 ^ x0), xf0, yf1, zf0), gdot3(hashm(a10 ^ x1), xf1, yf1, zf0), u), v),
+                lerp(lerp(gdot3(hashm(a01 ^ x0), xf0, yf0, zf1), gdot3(hashm(a01 ^ x1), xf1, yf0, zf1), u),
+                     lerp(gdot3(hashm(a11 ^ x0), xf0, yf1, zf1), gdot3(hashm(a11 ^ x1), xf1, yf1, zf1), u), v), s);
 }
 
 FND float perlin4(int seed, float x, float y, float z, float w)
@@ -677,7 +704,7 @@ FND float perlin4(int seed, float x, float y, float z, float w)
     float xf0 = x - xs, yf0 = y - ys, zf0 = z - zs, wf0 = w - ws;
     float xf1 = xf0 - 1.0f, yf1 = yf0 - 1.0f, zf1 = zf0 - 1.0f, wf1 = wf0 - 1.0f;
     float u = quintic(xf0), v = quintic(yf0), s = quintic(zf0), q = quintic(wf0);
-#define G(a, b, c, d, fa, fb, fc, fd) grad4(hash_mix((seed ^ b ^ c ^ d) ^ a), fa, fb, fc, fd)
+#define G(a, b, c, d, fa, fb, fc, fd) gdot4(hashm((seed ^ b ^ c ^ d) ^ a), fa, fb, fc, fd)
     return lerp(
         lerp(lerp(lerp(G(x0, y0, z0, w0, xf0, yf0, zf0, wf0), G(x1, y0, z0, w0, xf1, yf0, zf0, wf0), u),
                   lerp(G(x0, y1, z0, w0, xf0, yf1, zf0, wf0), G(x1, y1, z0, w0, xf1, yf1, zf0, wf0), u), v),
