@@ -26,7 +26,10 @@ namespace {
 struct MeshCtx {
     float* dens = nullptr;
     size_t dens_cap = 0;
-    float* dminmax = nullptr;
+    // What a chunk reports, read back in one copy: words 0.. the mesher's totals and heights
+    // (bloxel faces, air, solid; DMC vertices, quads, air, solid), words 4, 5 OutputMinMax.
+    unsigned* result = nullptr;
+    float* dminmax = nullptr;          // in result
     MeshScratch scratch;
     DmcScratch dmc;
     SparseScratch sp;                  // the sparse density form (trees with specialised kernels)
@@ -34,7 +37,7 @@ struct MeshCtx {
     ~MeshCtx()
     {
         if (dens) cudaFree(dens);
-        if (dminmax) cudaFree(dminmax);
+        if (result) cudaFree(result);
         if (scratch.counts) cudaFree(scratch.counts);
         if (dmc.offsets) cudaFree(dmc.offsets);
         if (sp.stored) cudaFree(sp.stored);
@@ -74,7 +77,10 @@ struct MeshCtx {
 
     bool reserve(size_t densities, size_t voxels)
     {
-        if (!dminmax && !cuda_ok(cudaMalloc(&dminmax, 2 * sizeof(float)), "cudaMalloc(mesh minmax)")) return false;
+        if (!result) {
+            if (!cuda_ok(cudaMalloc(&result, 8 * sizeof(unsigned)), "cudaMalloc(mesh result)")) return false;
+            dminmax = reinterpret_cast<float*>(result + 4);
+        }
         if (!host && !cuda_ok(cudaMallocHost(&host, 8 * sizeof(unsigned)), "cudaMallocHost(mesh read-back)")) return false;
         if (densities > dens_cap) {
             if (dens) cudaFree(dens);
@@ -86,13 +92,13 @@ struct MeshCtx {
             if (scratch.counts) cudaFree(scratch.counts);
             scratch = MeshScratch();
             const size_t nb = (voxels + 1023) / 1024;
-            unsigned* block = nullptr;                  // counts | offsets | block totals | total | air, solid
-            if (!cuda_ok(cudaMalloc(&block, (2 * voxels + nb + 4) * sizeof(unsigned)), "cudaMalloc(mesh scan)")) return false;
+            unsigned* block = nullptr;                  // counts | offsets | block totals
+            if (!cuda_ok(cudaMalloc(&block, (2 * voxels + nb) * sizeof(unsigned)), "cudaMalloc(mesh scan)")) return false;
             scratch.counts = block;
             scratch.offsets = block + voxels;
             scratch.block_totals = block + 2 * voxels;
-            scratch.total = block + 2 * voxels + nb;
-            scratch.airsolid = block + 2 * voxels + nb + 1;
+            scratch.total = result;
+            scratch.airsolid = result + 1;
             scratch.cap_voxels = voxels;
         }
         return true;
@@ -105,23 +111,24 @@ struct MeshCtx {
         if (dmc.offsets) cudaFree(dmc.offsets);
         dmc = DmcScratch();
         const size_t tiles = (cells + 2047) / 2048;
-        // uint2: offsets | tile sums | total; uint32: masks | air, solid | list counters |
-        // vertex items | quad items; then cases (uint8)
-        const size_t pairs = cells + tiles + 1, words = cells + 4 + 4 * vcells + 3 * cells;
+        // uint2: offsets | tile sums; uint32: masks | list counters | vertex items | quad items;
+        // then cases and cut axes (uint8)
+        const size_t pairs = cells + tiles, words = cells + 2 + 4 * vcells + 3 * cells;
         char* block = nullptr;
-        if (!cuda_ok(cudaMalloc(&block, pairs * sizeof(uint2) + words * sizeof(unsigned) + vcells), "cudaMalloc(dmc scratch)"))
+        if (!cuda_ok(cudaMalloc(&block, pairs * sizeof(uint2) + words * sizeof(unsigned) + vcells + cells), "cudaMalloc(dmc scratch)"))
             return false;
         uint2* p = reinterpret_cast<uint2*>(block);
         dmc.offsets = p;
         dmc.tile_sums = p + cells;
-        dmc.total = p + cells + tiles;
+        dmc.total = reinterpret_cast<uint2*>(result);
         unsigned* w = reinterpret_cast<unsigned*>(p + pairs);
         dmc.masks = w;
-        dmc.airsolid = w + cells;
-        dmc.counters = w + cells + 2;
-        dmc.vert_items = w + cells + 4;
-        dmc.quad_items = w + cells + 4 + 4 * vcells;
+        dmc.airsolid = result + 2;
+        dmc.counters = w + cells;
+        dmc.vert_items = w + cells + 2;
+        dmc.quad_items = w + cells + 2 + 4 * vcells;
         dmc.cases = reinterpret_cast<unsigned char*>(w + words);
+        dmc.cell_axes = dmc.cases + vcells;
         dmc.cap_cells = cells;
         return true;
     }
@@ -235,8 +242,7 @@ bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStr
                    : cuda_ok(launch_bloxel(m.dens, size, upAxisZ != 0, (float)px, (float)py, (float)pz, iso, m.dminmax, m.scratch,
                                            verts, (unsigned)mesh->vertexCapacity, mesh->indices, (unsigned)mesh->indexCapacity, s),
                              "bloxel mesher");
-        if (!queued || !cuda_ok(cudaMemcpyAsync(host8, m.scratch.total, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read back"))
-            return false;
+        if (!queued) return false;
     } else {
         const bool queued =
             sparse ? cuda_ok(launch_dmc_sparse_prepare(m.sp, size, upAxisZ != 0, iso, m.dminmax, m.dmc, s), "dual marching cubes mesher") &&
@@ -247,12 +253,9 @@ bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStr
                    : cuda_ok(launch_dmc(m.dens, size, upAxisZ != 0, px, py, pz, iso, m.dminmax, m.dmc, verts,
                                         (unsigned)mesh->vertexCapacity, mesh->indices, (unsigned)mesh->indexCapacity, s),
                              "dual marching cubes mesher");
-        if (!queued ||
-            !cuda_ok(cudaMemcpyAsync(host8, m.dmc.total, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read back") ||
-            !cuda_ok(cudaMemcpyAsync(host8 + 2, m.dmc.airsolid, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read back"))
-            return false;
+        if (!queued) return false;
     }
-    return cuda_ok(cudaMemcpyAsync(host8 + 4, m.dminmax, 2 * sizeof(float), cudaMemcpyDeviceToHost, s), "read back");
+    return cuda_ok(cudaMemcpyAsync(host8, m.result, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read back");
 }
 
 // Fill a chunk's results from its read-back (after the stream has finished); FN_OK or

@@ -31,6 +31,7 @@ struct DmcScratch {
     unsigned* vert_items = nullptr;    // 4 (size+1)^3: every (vertex cell, piece) at most once
     unsigned* quad_items = nullptr;    // 3 size^3: every cut edge at most once
     unsigned char* cases = nullptr;    // (size+1)^3 marching-cubes cases
+    unsigned char* cell_axes = nullptr;   // per cell: its cut axes
     size_t cap_cells = 0;
 };
 
