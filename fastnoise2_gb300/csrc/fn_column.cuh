@@ -32,30 +32,6 @@ FND float opaque(float v)
 
 FND float nan_() { return __int_as_float(0x7fffffff); }
 
-// Two floats in one register pair and the packed FP32 operations on them: each half rounds
-// like the scalar operation, in one issue slot.
-typedef unsigned long long f32x2;
-FND f32x2 pack2(float lo, float hi)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-FND void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-FND f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-FND f32x2 sub2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-FND f32x2 lerp2(f32x2 a, f32x2 b, f32x2 t) { return fma2(t, sub2(b, a), a); }
-
 // The gradient dot of one lattice corner as a function of the offset t along the last axis,
 // for fixed offsets across it: dot = fma(s, t, g) with s in {-1, 0, 1}.  s * t is exact, so
 // the fma rounds once, as the reference's sum of two signed offsets does (3D, 4D).

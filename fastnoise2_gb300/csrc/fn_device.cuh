@@ -263,6 +263,76 @@ FND float mod_(float a, float b) { return a - truncf(a / b) * b; }
 // VariableRange::ScaleOutput (BasicGenerators.inl:27-30); mul = (1/(max-min))*rangeScale
 FND float scale_out(float v, float nmin, float mul, float rmin) { return fmaf(mul, v - nmin, rmin); }
 
+// Two floats in one register pair and the packed FP32 operations on them: each half rounds
+// like the scalar operation, in one issue slot.
+typedef unsigned long long f32x2;
+FND f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+FND void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+FND f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+FND f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+FND f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+FND f32x2 lerp2(f32x2 a, f32x2 b, f32x2 t) { return fma2(t, sub2(b, a), a); }
+
+// Two lattice vertices a, b of a simplex kernel, in this order: value + f^4 g for each, with f
+// its falloff, p its hash product and x, y, z(, w) its offset.  With the gradient table the
+// falloff powers and the dots of both run as packed operations (5 and 6 instructions instead of
+// 10 and 12): FBm(Simplex) 160^3 67.9 -> 65.5 us, terrain 3D 248 -> 243 us, 4D 32^4 217 -> 210 us.
+FND float add_pair3(float value, float fa, int pa, float xa, float ya, float za, float fb, int pb, float xb, float yb, float zb)
+{
+#ifdef FN_GRADIENT_TABLE
+    const float *ta = gradient_of<3>(pa), *tb = gradient_of<3>(pb);
+    f32x2 f = pack2(fa, fb);
+    f = mul2(f, f);
+    f = mul2(f, f);
+    const f32x2 g = fma2(pack2(ta[64], tb[64]), pack2(za, zb), fma2(pack2(ta[32], tb[32]), pack2(ya, yb), mul2(pack2(ta[0], tb[0]), pack2(xa, xb))));
+    float ga, gb;
+    unpack2(f, fa, fb);
+    unpack2(g, ga, gb);
+    return fmaf(fb, gb, fmaf(fa, ga, value));
+#else
+    fa *= fa; fa *= fa; fb *= fb; fb *= fb;
+    return fmaf(fb, gdot3(pb, xb, yb, zb), fmaf(fa, gdot3(pa, xa, ya, za), value));
+#endif
+}
+FND float add_pair4(float value, float fa, int pa, float xa, float ya, float za, float wa, float fb, int pb, float xb, float yb, float zb, float wb)
+{
+#ifdef FN_GRADIENT_TABLE
+    const float *ta = gradient_of<4>(pa), *tb = gradient_of<4>(pb);
+    f32x2 f = pack2(fa, fb);
+    f = mul2(f, f);
+    f = mul2(f, f);
+    const f32x2 g = fma2(pack2(ta[96], tb[96]), pack2(wa, wb), fma2(pack2(ta[64], tb[64]), pack2(za, zb),
+                         fma2(pack2(ta[32], tb[32]), pack2(ya, yb), mul2(pack2(ta[0], tb[0]), pack2(xa, xb)))));
+    float ga, gb;
+    unpack2(f, fa, fb);
+    unpack2(g, ga, gb);
+    return fmaf(fb, gb, fmaf(fa, ga, value));
+#else
+    fa *= fa; fa *= fa; fb *= fb; fb *= fb;
+    return fmaf(fb, gdot4(pb, xb, yb, zb, wb), fmaf(fa, gdot4(pa, xa, ya, za, wa), value));
+#endif
+}
+
 // ---------------------------------------------------------------- Simplex
 
 FND float simplex2(int seed, float x, float y)
@@ -281,11 +351,16 @@ FND float simplex2(int seed, float x, float y)
     float dy1 = (xgey ? dy0 + 1.0f : dy0) - (float)(kUnskew2 + 1);
     float dx2 = dx0 - (float)(kUnskew2 * 2 + 1);
     float dy2 = dy0 - (float)(kUnskew2 * 2 + 1);
-    float f0 = fmaf(-dx0, dx0, fmaf(-dy0, dy0, 0.5f));
-    float f1 = fmaf(-dx1, dx1, fmaf(-dy1, dy1, 0.5f));
-    float f2 = f0 + fmaf(unskew, (float)(-4.0 * (kRoot3 + 2.0) / (kRoot3 + 3.0)), (float)(-2.0 / 3.0));
-    f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); f2 = fmaxf(f2, 0.0f);
-    f0 *= f0; f0 *= f0; f1 *= f1; f1 *= f1; f2 *= f2; f2 *= f2;
+    // vertices 0 and 1 packed, negated: d.d - 1/2 rounds as 1/2 - d.d does
+    const f32x2 dx01 = pack2(dx0, dx1), dy01 = pack2(dy0, dy1);
+    float n0, n1, f0, f1;
+    unpack2(fma2(dx01, dx01, fma2(dy01, dy01, pack2(-0.5f, -0.5f))), n0, n1);
+    float f2 = fmaf(unskew, (float)(-4.0 * (kRoot3 + 2.0) / (kRoot3 + 3.0)), (float)(-2.0 / 3.0)) - n0;
+    f32x2 f01 = pack2(fminf(n0, 0.0f), fminf(n1, 0.0f));
+    f01 = mul2(f01, f01);
+    unpack2(mul2(f01, f01), f0, f1);
+    f2 = fmaxf(f2, 0.0f);
+    f2 *= f2; f2 *= f2;
     float g0 = grad2(hash(seed, xp, yp), dx0, dy0);
     float g1 = grad2(hash(seed, xgey ? iadd(xp, kPrimeX) : xp, xgey ? yp : iadd(yp, kPrimeY)), dx1, dy1);
     float g2 = grad2(hash(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY)), dx2, dy2);
@@ -315,16 +390,19 @@ FND float simplex3(int seed, float x, float y, float z)
     float dz2 = nz2 ? dz0 + 1.0f : dz0;
     constexpr float R = (float)0.6;
     float f0 = fmaf(-dz0, dz0, fmaf(-dy0, dy0, fmaf(-dx0, dx0, R)));
-    float f1 = fmaf(-dz1, dz1, fmaf(-dy1, dy1, fmaf(-dx1, dx1, R)));
-    float f2 = fmaf(-dz2, dz2, fmaf(-dy2, dy2, fmaf(-dx2, dx2, R)));
+    // vertices 1 and 2 packed, negated: d.d - R rounds as R - d.d does
+    const f32x2 dx12 = pack2(dx1, dx2), dy12 = pack2(dy1, dy2), dz12 = pack2(dz1, dz2);
+    float n1, n2;
+    unpack2(fma2(dz12, dz12, fma2(dy12, dy12, fma2(dx12, dx12, pack2(-R, -R)))), n1, n2);
     float f3 = f0 - (unskew + (float)(3.0 / 4.0));
-    f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f);
-    f0 *= f0; f0 *= f0; f1 *= f1; f1 *= f1; f2 *= f2; f2 *= f2; f3 *= f3; f3 *= f3;
-    float g0 = gdot3(hashhb(seed, xp, yp, zp), dx0, dy0, dz0);
-    float g1 = gdot3(hashhb(seed, mx1 ? iadd(xp, kPrimeX) : xp, my1 ? iadd(yp, kPrimeY) : yp, mz1 ? zp : iadd(zp, kPrimeZ)), dx1, dy1, dz1);
-    float g2 = gdot3(hashhb(seed, nx2 ? iadd(xp, kPrimeX) : xp, ny2 ? yp : iadd(yp, kPrimeY), nz2 ? zp : iadd(zp, kPrimeZ)), dx2, dy2, dz2);
-    float g3 = gdot3(hashhb(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ)), dx3, dy3, dz3);
-    return fmaf(g3, f3, fmaf(g2, f2, fmaf(g1, f1, g0 * f0)));
+    f32x2 f03 = pack2(fmaxf(f0, 0.0f), fmaxf(f3, 0.0f));
+    f03 = mul2(f03, f03);
+    unpack2(mul2(f03, f03), f0, f3);
+    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ);
+    const int p1 = hashhb(seed, mx1 ? xq : xp, my1 ? yq : yp, mz1 ? zp : zq), p2 = hashhb(seed, nx2 ? xq : xp, ny2 ? yp : yq, nz2 ? zp : zq);
+    const float v = add_pair3(f0 * gdot3(hashhb(seed, xp, yp, zp), dx0, dy0, dz0), fminf(n1, 0.0f), p1, dx1, dy1, dz1,
+                              fminf(n2, 0.0f), p2, dx2, dy2, dz2);
+    return fmaf(gdot3(hashhb(seed, xq, yq, zq), dx3, dy3, dz3), f3, v);
 }
 
 FND float simplex4(int seed, float x, float y, float z, float w)
@@ -387,43 +465,28 @@ FND float supersimplex2(int seed, float x, float y)
     bool fy = fmaf(dys, -2.0f, dxs) < boundary;
     float unskew = (float)kUnskew2 * (dxs + dys);
     float dxb = dxs + unskew, dyb = dys + unskew;
-    float fb0 = fmaf(-dxb, dxb, fmaf(-dyb, dyb, R));
-    float value;
-    {
-        float g = grad2(hash(seed, xp, yp), dxb, dyb);
-        float f = fb0; f *= f; f *= f;
-        value = f * g;
-    }
-    {
-        float g = grad2(hash(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY)), dxb - (float)(2 * kUnskew2 + 1), dyb - (float)(2 * kUnskew2 + 1));
-        float f = fmaf(unskew, (float)(-4.0 * (kRoot3 + 2.0) / (kRoot3 + 3.0)), fb0 - R);
-        f *= f; f *= f;
-        value = fmaf(f, g, value);
-    }
-    float xyd = fxy ? (float)(kUnskew2 + 1) : (float)(-kUnskew2);
+    const float fb0 = fmaf(-dxb, dxb, fmaf(-dyb, dyb, R));
+    const float g0 = grad2(hash(seed, xp, yp), dxb, dyb);
+    const float g1 = grad2(hash(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY)), dxb - (float)(2 * kUnskew2 + 1), dyb - (float)(2 * kUnskew2 + 1));
+    f32x2 f = pack2(fb0, fmaf(unskew, (float)(-4.0 * (kRoot3 + 2.0) / (kRoot3 + 3.0)), fb0 - R));
+    f = mul2(f, f);
+    float f0, f1, f2, f3;
+    unpack2(mul2(f, f), f0, f1);
+    const float xyd = fxy ? (float)(kUnskew2 + 1) : (float)(-kUnskew2);
     dxb = dxb - xyd;
     dyb = dyb - xyd;
-    {
-        int xa = fx ? iadd(xp, (int)((unsigned)kPrimeX * 2u)) : xp;
-        int h = hash(seed, fxy ? xa : iadd(xa, -kPrimeX), fxy ? iadd(yp, kPrimeY) : yp);
-        float dx = dxb - (fx ? (float)(1 + 2 * kUnskew2) : -1.0f);
-        float dy = fx ? dyb - (float)(2 * kUnskew2) : dyb;
-        float g = grad2(h, dx, dy);
-        float f = fmaxf(fmaf(-dx, dx, fmaf(-dy, dy, R)), 0.0f);
-        f *= f; f *= f;
-        value = fmaf(f, g, value);
-    }
-    {
-        int ya = fy ? iadd(yp, (int)((unsigned)kPrimeY * 2u)) : yp;
-        int h = hash(seed, fxy ? iadd(xp, kPrimeX) : xp, fxy ? ya : iadd(ya, -kPrimeY));
-        float dx = fy ? dxb - (float)(2 * kUnskew2) : dxb;
-        float dy = dyb - (fy ? (float)(1 + 2 * kUnskew2) : -1.0f);
-        float g = grad2(h, dx, dy);
-        float f = fmaxf(fmaf(-dx, dx, fmaf(-dy, dy, R)), 0.0f);
-        f *= f; f *= f;
-        value = fmaf(f, g, value);
-    }
-    return value;
+    const int xa = fx ? iadd(xp, (int)((unsigned)kPrimeX * 2u)) : xp, ya = fy ? iadd(yp, (int)((unsigned)kPrimeY * 2u)) : yp;
+    const float dx2 = dxb - (fx ? (float)(1 + 2 * kUnskew2) : -1.0f), dy2 = fx ? dyb - (float)(2 * kUnskew2) : dyb;
+    const float dx3 = fy ? dxb - (float)(2 * kUnskew2) : dxb, dy3 = dyb - (fy ? (float)(1 + 2 * kUnskew2) : -1.0f);
+    const float g2 = grad2(hash(seed, fxy ? xa : iadd(xa, -kPrimeX), fxy ? iadd(yp, kPrimeY) : yp), dx2, dy2);
+    const float g3 = grad2(hash(seed, fxy ? iadd(xp, kPrimeX) : xp, fxy ? ya : iadd(ya, -kPrimeY)), dx3, dy3);
+    // the last two vertices packed, negated: d.d - R rounds as R - d.d does
+    const f32x2 dx23 = pack2(dx2, dx3), dy23 = pack2(dy2, dy3);
+    unpack2(fma2(dx23, dx23, fma2(dy23, dy23, pack2(-R, -R))), f2, f3);
+    f = pack2(fminf(f2, 0.0f), fminf(f3, 0.0f));
+    f = mul2(f, f);
+    unpack2(mul2(f, f), f2, f3);
+    return fmaf(f3, g3, fmaf(f2, g2, fmaf(f1, g1, f0 * g0)));
 }
 
 FND void ss_consider(float& maxScore, int& bits, float score, int b)
@@ -465,67 +528,36 @@ FND float supersimplex3(int seed, float x, float y, float z)
     float unskew = (float)kReflect * sum;
     float dx = dxs + unskew, dy = dys + unskew, dz = dzs + unskew;
     float cs = (float)(1 + 3 * kReflect) * sum;
-    float value, stemA, stemB;
-    {
-        float g = gdot3(hashhb(seed, xp, yp, zp), dx, dy, dz);
-        float fb = fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA))) * 0.5f;
-        stemA = fb - (float)(kDA * 0.5);
-        stemB = fb - (float)(kDB * 0.5);
-        value = (fb * fb) * (fb * fb) * g;
-    }
+    const float fb0 = fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA))) * 0.5f;
+    const float stemA = fb0 - (float)(kDA * 0.5), stemB = fb0 - (float)(kDB * 0.5);
     // Every other vertex lies on one of two opposite sides, chosen by a comparison a < b.  Its
     // outcome is the sign of a - b (of a + 0 against zero), so offsets are flipped by that sign
     // bit and lattice coordinates stepped by it through a multiply-add, which keeps compares,
     // selects and adds off the half-rate ALU pipe.
     const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ);   // the positive side
-    {
-        float m = xyzn + 0.0f;
-        float off = flips((float)(3 * kReflect + 1), m);
-        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), sided(yq, kPrimeY, m), sided(zq, kPrimeZ, m)), dx - off, dy - off, dz - off);
-        float fb = fmaxf(fmaf(off, cs, stemA), 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
+    float value;
+    {   // the closest vertex and <1,1,1> or <-1,-1,-1>
+        const float m = xyzn + 0.0f, off = flips((float)(3 * kReflect + 1), m);
+        value = add_pair3(0.0f, fb0, hashhb(seed, xp, yp, zp), dx, dy, dz, fmaxf(fmaf(off, cs, stemA), 0.0f),
+                          hashhb(seed, sided(xq, kPrimeX, m), sided(yq, kPrimeY, m), sided(zq, kPrimeZ, m)), dx - off, dy - off, dz - off);
     }
-    {
-        float m = xyzn - zn;
-        float o0 = flips((float)(2 * kReflect), m);
-        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), sided(yq, kPrimeY, m), zp), dx, dy, dz - o0);
-        float fb = fminf(flips(dz, m) - stemB, 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
+    {   // <1,1,0> and <1,0,1> or their negatives
+        const float ma = xyzn - zn, mb = xyzn - yn;
+        const float oa = flips((float)(2 * kReflect), ma), ob = flips((float)(2 * kReflect), mb);
+        value = add_pair3(value, fminf(flips(dz, ma) - stemB, 0.0f), hashhb(seed, sided(xq, kPrimeX, ma), sided(yq, kPrimeY, ma), zp), dx, dy, dz - oa,
+                          fminf(flips(dy, mb) - stemB, 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), yp, sided(zq, kPrimeZ, mb)), dx, dy - ob, dz);
     }
-    {
-        float m = xyzn - yn;
-        float o0 = flips((float)(2 * kReflect), m);
-        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), yp, sided(zq, kPrimeZ, m)), dx, dy - o0, dz);
-        float fb = fminf(flips(dy, m) - stemB, 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
+    {   // <0,1,1> and <1,0,0> or their negatives
+        const float ma = xyzn - xn, mb = xn + 0.0f;
+        const float oa = flips((float)(2 * kReflect), ma), ob = flips((float)kReflect, mb);
+        value = add_pair3(value, fminf(flips(dx, ma) - stemB, 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, ma), sided(zq, kPrimeZ, ma)), dx - oa, dy, dz,
+                          fmaxf(fmaf(ob, cs, stemA) + flips(dx, mb), 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), yp, zp), dx + ob, dy - ob, dz - ob);
     }
-    {
-        float m = xyzn - xn;
-        float o0 = flips((float)(2 * kReflect), m);
-        float g = gdot3(hashhb(seed, xp, sided(yq, kPrimeY, m), sided(zq, kPrimeZ, m)), dx - o0, dy, dz);
-        float fb = fminf(flips(dx, m) - stemB, 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
-    }
-    {
-        float m = xn + 0.0f;
-        float o0 = flips((float)kReflect, m);
-        float g = gdot3(hashhb(seed, sided(xq, kPrimeX, m), yp, zp), dx + o0, dy - o0, dz - o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dx, m), 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
-    }
-    {
-        float m = yn + 0.0f;
-        float o0 = flips((float)kReflect, m);
-        float g = gdot3(hashhb(seed, xp, sided(yq, kPrimeY, m), zp), dx - o0, dy + o0, dz - o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dy, m), 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
-    }
-    {
-        float m = zn + 0.0f;
-        float o0 = flips((float)kReflect, m);
-        float g = gdot3(hashhb(seed, xp, yp, sided(zq, kPrimeZ, m)), dx - o0, dy - o0, dz + o0);
-        float fb = fmaxf(fmaf(o0, cs, stemA) + flips(dz, m), 0.0f);
-        value = fmaf((fb * fb) * (fb * fb), g, value);
+    {   // <0,1,0> and <0,0,1> or their negatives
+        const float ma = yn + 0.0f, mb = zn + 0.0f;
+        const float oa = flips((float)kReflect, ma), ob = flips((float)kReflect, mb);
+        value = add_pair3(value, fmaxf(fmaf(oa, cs, stemA) + flips(dy, ma), 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, ma), zp), dx - oa, dy + oa, dz - oa,
+                          fmaxf(fmaf(ob, cs, stemA) + flips(dz, mb), 0.0f), hashhb(seed, xp, yp, sided(zq, kPrimeZ, mb)), dx - ob, dy - ob, dz + ob);
     }
     return value;
 }
@@ -576,94 +608,57 @@ FND float supersimplex4(int seed, float x, float y, float z, float w)
     float ud = (float)kU * sum;
     float dx = dxs + ud, dy = dys + ud, dz = dzs + ud, dw = dws + ud;
     float cs = (float)(1 + 4 * kU) * sum;
-    float value, stemA, stemB;
+    const float fb0 = fmaf(-dw, dw, fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA)))) * 0.5f;
+    const float stemA = fb0 - (float)(kDA * 0.5), stemB = fb0 - (float)(kDB * 0.5);
+    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ), wq = iadd(wp, kPrimeW);   // sides as in 3D
+    float value;
     {
-        float g = gdot4(hashhb(seed, xp, yp, zp, wp), dx, dy, dz, dw);
-        float fb = fmaf(-dw, dw, fmaf(-dz, dz, fmaf(-dy, dy, fmaf(-dx, dx, (float)kDA)))) * 0.5f;
-        stemA = fb - (float)(kDA * 0.5);
-        stemB = fb - (float)(kDB * 0.5);
-        value = (fb * fb) * (fb * fb) * g;
-    }
-    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ), wq = iadd(wp, kPrimeW);   // as in 3D
-#define FND_P(m, base, P) sided(base, P, m)
-#define FND_ACC(fbexpr, gexpr) { float g_ = (gexpr); float fb_ = fmaxf((fbexpr), 0.0f); value = fmaf((fb_ * fb_) * (fb_ * fb_), g_, value); }
-    {
-        float m = xyzwn + 0.0f;
-        float o = flips((float)(4 * kU + 1), m);
-        FND_ACC(fmaf(o, cs, stemA), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o, dy - o, dz - o, dw - o));
+        const float mb = xyzwn + 0.0f, ob = flips((float)(4 * kU + 1), mb);
+        value = add_pair4(0.0f, fb0, hashhb(seed, xp, yp, zp, wp), dx, dy, dz, dw,
+                          fmaxf(fmaf(ob, cs, stemA), 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), sided(yq, kPrimeY, mb), sided(zq, kPrimeZ, mb), sided(wq, kPrimeW, mb)), dx - ob, dy - ob, dz - ob, dw - ob);
     }
     {
-        float m = xyzwn - wn;
-        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flips(dw, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), wp), dx - o1, dy - o1, dz - o1, dw - o0));
+        const float ma = xyzwn - wn, o1a = flips((float)(3 * kU + 1), ma), o0a = flips((float)(3 * kU), ma);
+        const float mb = xyzwn - zn, o1b = flips((float)(3 * kU + 1), mb), o0b = flips((float)(3 * kU), mb);
+        value = add_pair4(value, fmaxf(fmaf(o1a, cs, stemB) - flips(dw, ma), 0.0f), hashhb(seed, sided(xq, kPrimeX, ma), sided(yq, kPrimeY, ma), sided(zq, kPrimeZ, ma), wp), dx - o1a, dy - o1a, dz - o1a, dw - o0a,
+                          fmaxf(fmaf(o1b, cs, stemB) - flips(dz, mb), 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), sided(yq, kPrimeY, mb), zp, sided(wq, kPrimeW, mb)), dx - o1b, dy - o1b, dz - o0b, dw - o1b);
     }
     {
-        float m = xyzwn - zn;
-        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flips(dz, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), zp, FND_P(m, wq, kPrimeW)), dx - o1, dy - o1, dz - o0, dw - o1));
+        const float ma = xyzwn - yn, o1a = flips((float)(3 * kU + 1), ma), o0a = flips((float)(3 * kU), ma);
+        const float mb = xyzwn - xn, o1b = flips((float)(3 * kU + 1), mb), o0b = flips((float)(3 * kU), mb);
+        value = add_pair4(value, fmaxf(fmaf(o1a, cs, stemB) - flips(dy, ma), 0.0f), hashhb(seed, sided(xq, kPrimeX, ma), yp, sided(zq, kPrimeZ, ma), sided(wq, kPrimeW, ma)), dx - o1a, dy - o0a, dz - o1a, dw - o1a,
+                          fmaxf(fmaf(o1b, cs, stemB) - flips(dx, mb), 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, mb), sided(zq, kPrimeZ, mb), sided(wq, kPrimeW, mb)), dx - o0b, dy - o1b, dz - o1b, dw - o1b);
     }
     {
-        float m = xyzwn - yn;
-        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flips(dy, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o1, dy - o0, dz - o1, dw - o1));
+        const float ma = xn + 0.0f, o1a = flips((float)(kU + 1), ma), o0a = flips((float)kU, ma);
+        const float mb = xn + yn, o1b = flips((float)(2 * kU + 1), mb), o0b = flips((float)(2 * kU), mb);
+        value = add_pair4(value, fmaxf(fmaf(o0a, cs, stemA) + flips(dx, ma), 0.0f), hashhb(seed, sided(xq, kPrimeX, ma), yp, zp, wp), dx - o1a, dy - o0a, dz - o0a, dw - o0a,
+                          fmaxf(fmaf(o0b, cs, stemB) + flips(dx + dy, mb), 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), sided(yq, kPrimeY, mb), zp, wp), dx - o1b, dy - o1b, dz - o0b, dw - o0b);
     }
     {
-        float m = xyzwn - xn;
-        float o1 = flips((float)(3 * kU + 1), m), o0 = flips((float)(3 * kU), m);
-        FND_ACC(fmaf(o1, cs, stemB) - flips(dx, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o0, dy - o1, dz - o1, dw - o1));
+        const float ma = xn + zn, o1a = flips((float)(2 * kU + 1), ma), o0a = flips((float)(2 * kU), ma);
+        const float mb = xn + wn, o1b = flips((float)(2 * kU + 1), mb), o0b = flips((float)(2 * kU), mb);
+        value = add_pair4(value, fmaxf(fmaf(o0a, cs, stemB) + flips(dx + dz, ma), 0.0f), hashhb(seed, sided(xq, kPrimeX, ma), yp, sided(zq, kPrimeZ, ma), wp), dx - o1a, dy - o0a, dz - o1a, dw - o0a,
+                          fmaxf(fmaf(o0b, cs, stemB) + flips(dx + dw, mb), 0.0f), hashhb(seed, sided(xq, kPrimeX, mb), yp, zp, sided(wq, kPrimeW, mb)), dx - o1b, dy - o0b, dz - o0b, dw - o1b);
     }
     {
-        float m = xn + 0.0f;
-        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flips(dx, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, zp, wp), dx - o1, dy - o0, dz - o0, dw - o0));
+        const float ma = yn + 0.0f, o1a = flips((float)(kU + 1), ma), o0a = flips((float)kU, ma);
+        const float mb = yn + zn, o1b = flips((float)(2 * kU + 1), mb), o0b = flips((float)(2 * kU), mb);
+        value = add_pair4(value, fmaxf(fmaf(o0a, cs, stemA) + flips(dy, ma), 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, ma), zp, wp), dx - o0a, dy - o1a, dz - o0a, dw - o0a,
+                          fmaxf(fmaf(o0b, cs, stemB) + flips(dy + dz, mb), 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, mb), sided(zq, kPrimeZ, mb), wp), dx - o0b, dy - o1b, dz - o1b, dw - o0b);
     }
     {
-        float m = xn + yn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dy, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), FND_P(m, yq, kPrimeY), zp, wp), dx - o1, dy - o1, dz - o0, dw - o0));
+        const float ma = yn + wn, o1a = flips((float)(2 * kU + 1), ma), o0a = flips((float)(2 * kU), ma);
+        const float mb = zn + 0.0f, o1b = flips((float)(kU + 1), mb), o0b = flips((float)kU, mb);
+        value = add_pair4(value, fmaxf(fmaf(o0a, cs, stemB) + flips(dy + dw, ma), 0.0f), hashhb(seed, xp, sided(yq, kPrimeY, ma), zp, sided(wq, kPrimeW, ma)), dx - o0a, dy - o1a, dz - o0a, dw - o1a,
+                          fmaxf(fmaf(o0b, cs, stemA) + flips(dz, mb), 0.0f), hashhb(seed, xp, yp, sided(zq, kPrimeZ, mb), wp), dx - o0b, dy - o0b, dz - o1b, dw - o0b);
     }
     {
-        float m = xn + zn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dz, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, FND_P(m, zq, kPrimeZ), wp), dx - o1, dy - o0, dz - o1, dw - o0));
+        const float ma = zn + wn, o1a = flips((float)(2 * kU + 1), ma), o0a = flips((float)(2 * kU), ma);
+        const float mb = wn + 0.0f, o1b = flips((float)(kU + 1), mb), o0b = flips((float)kU, mb);
+        value = add_pair4(value, fmaxf(fmaf(o0a, cs, stemB) + flips(dz + dw, ma), 0.0f), hashhb(seed, xp, yp, sided(zq, kPrimeZ, ma), sided(wq, kPrimeW, ma)), dx - o0a, dy - o0a, dz - o1a, dw - o1a,
+                          fmaxf(fmaf(o0b, cs, stemA) + flips(dw, mb), 0.0f), hashhb(seed, xp, yp, zp, sided(wq, kPrimeW, mb)), dx - o0b, dy - o0b, dz - o0b, dw - o1b);
     }
-    {
-        float m = xn + wn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dx + dw, m), gdot4(hashhb(seed, FND_P(m, xq, kPrimeX), yp, zp, FND_P(m, wq, kPrimeW)), dx - o1, dy - o0, dz - o0, dw - o1));
-    }
-    {
-        float m = yn + 0.0f;
-        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flips(dy, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), zp, wp), dx - o0, dy - o1, dz - o0, dw - o0));
-    }
-    {
-        float m = yn + zn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dy + dz, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), FND_P(m, zq, kPrimeZ), wp), dx - o0, dy - o1, dz - o1, dw - o0));
-    }
-    {
-        float m = yn + wn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dy + dw, m), gdot4(hashhb(seed, xp, FND_P(m, yq, kPrimeY), zp, FND_P(m, wq, kPrimeW)), dx - o0, dy - o1, dz - o0, dw - o1));
-    }
-    {
-        float m = zn + 0.0f;
-        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flips(dz, m), gdot4(hashhb(seed, xp, yp, FND_P(m, zq, kPrimeZ), wp), dx - o0, dy - o0, dz - o1, dw - o0));
-    }
-    {
-        float m = zn + wn;
-        float o1 = flips((float)(2 * kU + 1), m), o0 = flips((float)(2 * kU), m);
-        FND_ACC(fmaf(o0, cs, stemB) + flips(dz + dw, m), gdot4(hashhb(seed, xp, yp, FND_P(m, zq, kPrimeZ), FND_P(m, wq, kPrimeW)), dx - o0, dy - o0, dz - o1, dw - o1));
-    }
-    {
-        float m = wn + 0.0f;
-        float o1 = flips((float)(kU + 1), m), o0 = flips((float)kU, m);
-        FND_ACC(fmaf(o0, cs, stemA) + flips(dw, m), gdot4(hashhb(seed, xp, yp, zp, FND_P(m, wq, kPrimeW)), dx - o0, dy - o0, dz - o0, dw - o1));
-    }
-#undef FND_P
-#undef FND_ACC
     return value;
 }
 
@@ -690,10 +685,23 @@ FND float perlin3(int seed, float x, float y, float z)
     float u = quintic(xf0), v = quintic(yf0), s = quintic(zf0);
     // seed ^ y ^ z shared by each x pair of corners (xor reassociated: the same hashes)
     const int a00 = seed ^ y0 ^ z0, a10 = seed ^ y1 ^ z0, a01 = seed ^ y0 ^ z1, a11 = seed ^ y1 ^ z1;
+#ifdef FN_GRADIENT_TABLE
+    // the two z planes as the halves of packed operations
+    const f32x2 zf = pack2(zf0, zf1), uu = pack2(u, u), vv = pack2(v, v);
+    auto corner = [&](int lo, int hi, float xf, float yf) {
+        const float *a = gradient_of<3>(hashm(lo)), *b = gradient_of<3>(hashm(hi));
+        return fma2(pack2(a[64], b[64]), zf, fma2(pack2(a[32], b[32]), pack2(yf, yf), mul2(pack2(a[0], b[0]), pack2(xf, xf))));
+    };
+    float lo, hi;
+    unpack2(lerp2(lerp2(corner(a00 ^ x0, a01 ^ x0, xf0, yf0), corner(a00 ^ x1, a01 ^ x1, xf1, yf0), uu),
+                  lerp2(corner(a10 ^ x0, a11 ^ x0, xf0, yf1), corner(a10 ^ x1, a11 ^ x1, xf1, yf1), uu), vv), lo, hi);
+    return lerp(lo, hi, s);
+#else
     return lerp(lerp(lerp(gdot3(hashm(a00 ^ x0), xf0, yf0, zf0), gdot3(hashm(a00 ^ x1), xf1, yf0, zf0), u),
                      lerp(gdot3(hashm(a10 ^ x0), xf0, yf1, zf0), gdot3(hashm(a10 ^ x1), xf1, yf1, zf0), u), v),
                 lerp(lerp(gdot3(hashm(a01 ^ x0), xf0, yf0, zf1), gdot3(hashm(a01 ^ x1), xf1, yf0, zf1), u),
                      lerp(gdot3(hashm(a11 ^ x0), xf0, yf1, zf1), gdot3(hashm(a11 ^ x1), xf1, yf1, zf1), u), v), s);
+#endif
 }
 
 FND float perlin4(int seed, float x, float y, float z, float w)
