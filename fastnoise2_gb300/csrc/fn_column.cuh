@@ -466,4 +466,108 @@ struct CellCol {
     }
 };
 
+// DomainWarpGradient at a separable position, 2D and 3D: the corner vectors of the lattice cell
+// are the same while the column stays in it.  The warp keeps those of each distinct cell of its
+// lanes in shared memory (converted, one lane per corner), a lane its corners' weights across
+// the column; a step is one broadcast load and a packed and a scalar fma per corner (46
+// instructions in 3D against ~150 with hashing and conversions).  More than kGroups cells per
+// warp take the point function (`fast`).
+template <int D>
+struct WarpCol {
+    static constexpr int N = 1 << D, kGroups = 4, kTable = 32 + kGroups * N;
+    float weight[N / 2];                          // of the corners across the column
+    int icell;
+    unsigned slot;
+    bool fast;
+
+    template <typename Pos>
+    FND void init(Pos&& pos)
+    {
+        float q[D - 1], s[2][2];
+        pos(q);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            s[k][1] = hermite(q[k % (D - 1)] - floorf(q[k % (D - 1)]));
+            s[k][0] = 1.0f - s[k][1];
+        }
+#pragma unroll
+        for (int m = 0; m < N / 2; ++m) weight[m] = D == 2 ? s[0][m] : s[0][m & 1] * s[1][m >> 1];
+        icell = 0x7fffffff;
+        slot = 0;
+        fast = false;
+    }
+    // entry: weights of the lower and the upper plane, -, the cell
+    FND unsigned prepare(float4* tab, unsigned lane, float p)
+    {
+        const float fl = floorf(p), s1 = hermite(p - fl);
+        const int cell = cvti(fl);
+        tab[lane] = make_float4(1.0f - s1, s1, 0.0f, __int_as_float(cell));
+        const int before = __shfl_up_sync(0xffffffffu, cell, 1);
+        return __ballot_sync(0xffffffffu, cell != (lane ? before : icell));
+    }
+    template <typename Pos>
+    FND void enter(int seed, float4* tab, unsigned j, float, Pos&& pos)
+    {
+        const int cell = __float_as_int(tab[j].w);
+        if (cell == icell) return;
+        icell = cell;
+        float q[D - 1];
+        int cb[D - 1];
+        pos(q);
+#pragma unroll
+        for (int k = 0; k < D - 1; ++k) cb[k] = cvti(floorf(q[k]));
+        const int lane = (int)(threadIdx.x & 31u);
+        unsigned todo = 0xffffffffu, groups = 0;
+        __syncwarp();
+#pragma unroll 1
+        do {
+            const int leader = __ffs((int)todo) - 1;
+            int c[D];
+            bool mine = true;
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const int b = k == D - 1 ? cell : __shfl_sync(0xffffffffu, cb[k % (D - 1)], leader);
+                if (k < D - 1) mine = mine && cb[k % (D - 1)] == b;
+                c[k] = imul(iadd(b, (lane >> k) & 1), kPrimes[k]);
+            }
+            if (lane < N) {
+                const int h = cell_hash<D>(seed, c);
+                tab[32 + groups * N + lane] = D == 2 ? make_float4(cvtf(h & 0xffff), cvtf((int)srl(h, 16)), 0.0f, 0.0f)
+                                                     : make_float4(cvtf(h & 0x3ff), cvtf((h >> 11) & 0x3ff), cvtf((int)srl(h, 22)), 0.0f);
+            }
+            if (mine) slot = groups * N;
+            todo &= ~__ballot_sync(0xffffffffu, mine);
+            ++groups;
+        } while (todo && groups < (unsigned)kGroups);
+        __syncwarp();
+        fast = todo == 0;
+    }
+    FND float warp(const float4* tab, unsigned j, float amp, const float* axis, float* io) const
+    {
+        const float4 e = tab[j];
+        const float4* corners = tab + 32 + slot;
+        f32x2 v01 = 0;
+        float wv[D];
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const float4 c = corners[m];
+            const float t = weight[m & (N / 2 - 1)] * (m < N / 2 ? e.x : e.y);
+            const f32x2 tt = pack2(t, t), c01 = pack2(c.x, c.y);
+            v01 = m == 0 ? mul2(tt, c01) : fma2(tt, c01, v01);
+            if (D == 3) wv[2 % D] = m == 0 ? t * c.z : fmaf(t, c.z, wv[2 % D]);
+        }
+        unpack2(v01, wv[0], wv[1]);
+        constexpr float normalise = D == 2 ? 1.0f / (0xffff / 2.0f) : 1.0f / (0x3ff / 2.0f);
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            wv[k] = fmaf(wv[k], normalise, -1.0f);
+            io[k] = fmaf(wv[k], amp * axis[k], io[k]);
+        }
+        float r = wv[D - 1] * wv[D - 1];
+#pragma unroll
+        for (int k = D - 2; k >= 0; --k) r = fmaf(wv[k], wv[k], r);
+        return r;
+    }
+};
+
 }  // namespace fnd

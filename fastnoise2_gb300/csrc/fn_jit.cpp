@@ -227,6 +227,11 @@ ColPlan column_plan(const CompiledProgram& prog)
         case FN_OP_ROTATE3: set_other(I.dst, 3); break;
         case FN_OP_ROTPLANE: set_other(I.dst, std::max(3, D)); break;
         case FN_OP_WARP_GRAD: case FN_OP_WARP_SIMPLEX:
+            if (I.op == FN_OP_WARP_GRAD && D < 4) {
+                ColState* st = add_state(pc, "WarpCol<" + std::to_string(D) + ">", P[I.prm], D == 2 ? 4 : 6, 32 + (4 << D), true,
+                                         D == 2 ? 80 : 120, D == 2 ? 28 : 46);
+                if (st) st->jitter = "0.0f";
+            }
             set_other(I.dst, D);
             if (I.c != FN_REG_NONE) set_other(I.c, 1);
             break;
@@ -431,7 +436,8 @@ void emit_eval(const CompiledProgram& prog, const std::string& name, std::ostrin
             o << "        const float axis[" << D << "] = {";
             for (int j = 0; j < D; ++j) o << (j ? ", " : "") << p(1 + j);
             if (I.op == FN_OP_WARP_GRAD)
-                o << "};\n        const float st = fnd::warp_gradient<" << D << ">(" << sd << ", " << r(I.b) << ", sp, axis, io);\n";
+                o << "};\n        const float st = " << (cell ? cell_state + ".fast ? " + cell_state + ".warp(" + cell_tab + ", " + r(I.b) + ", axis, io) : " : std::string())
+                  << "fnd::warp_gradient<" << D << ">(" << sd << ", " << r(I.b) << ", sp, axis, io);\n";
             else
                 o << "};\n        const float st = fnd::warp_simplex<" << D << ">(" << sd << ", " << r(I.b) << ", sp, axis, io, "
                   << ((I.aux & 1) ? "true" : "false") << ", " << ((I.aux & 2) ? "true" : "false") << ");\n";
@@ -592,8 +598,9 @@ void emit_column_unit(const CompiledProgram& prog, const std::string& eval, cons
 // FBm(Perlin) 4D 32^4 takes 23 us with five octaves' states and one block, 37 us with four, 54 us
 // with two octaves' and two blocks; FBm(Perlin) 256^3 (100 registers of state) 142 us with two
 // blocks, 156 with one, 243 with three (spills); terrain and CellularLookup 160^3 (31 registers)
-// 269 and 55 us with two blocks, 279 and 60 with three, 290 and 66 with four.
-int column_blocks(const ColPlan& plan) { return plan.regs <= 16 ? 4 : plan.regs <= 104 ? 2 : 1; }
+// 269 and 55 us with two blocks, 279 and 60 with three, 290 and 66 with four; terrain 2048^2 (17
+// registers) 105 us with four, 109 with two.
+int column_blocks(const ColPlan& plan) { return plan.regs <= 20 ? 4 : plan.regs <= 104 ? 2 : 1; }
 
 // Per-call kernels for program k: grid / position array / tileable.
 //

@@ -27,6 +27,10 @@ TREES = {
     "CellLookup": lambda: N("CellularLookup", Feature_Scale=27.0, Lookup=N("Perlin", Feature_Scale=40.0)),
     "CellTies": lambda: N("CellularValue", Feature_Scale=8.0, Grid_Jitter=0.0),
     "Terrain": trees.terrain_c2,
+    "Warp": lambda: N("DomainWarpGradient", Source=N("Value", Feature_Scale=6.0), Warp_Amplitude=5.0, Feature_Scale=23.0, Seed_Offset=2)
+                      .set("Amplitude Scaling", 0.5, 0),
+    "WarpIndependent": lambda: N("DomainWarpFractalIndependent", Octaves=3, Weighted_Strength=0.3,
+                                 Domain_Warp_Source=N("DomainWarpGradient", Source=N("Perlin"), Warp_Amplitude=8.0, Feature_Scale=40.0)),
 }
 SHAPES = {2: [(1, 1), (31, 33), (33, 64), (70, 65), (5, 200)],
           3: [(1, 1, 1), (5, 3, 2), (33, 1, 31), (7, 9, 33), (16, 16, 16), (11, 6, 97)],
