@@ -42,7 +42,10 @@ def library_path() -> str:
 
 
 _lib = None
+_grid_host = {}                 # generation calls by dimensionality, set once the library is loaded
+_grid_device = {}
 _FP = ctypes.POINTER(ctypes.c_float)
+_MinMax = ctypes.c_float * 2
 
 
 def _declare(L):
@@ -173,7 +176,10 @@ def lib():
         if not os.path.exists(_LIB_PATH):
             raise ImportError(f"{_LIB_PATH} is missing: build it with `python -m fastnoise2_gb300.build` "
                               "(this package has no CPU fallback)")
-        _lib = _declare(ctypes.CDLL(_LIB_PATH))
+        L = _declare(ctypes.CDLL(_LIB_PATH))
+        _grid_host.update({2: L.fnGenUniformGrid2D, 3: L.fnGenUniformGrid3D, 4: L.fnGenUniformGrid4D})
+        _grid_device.update({2: L.fnGenUniformGrid2DDevice, 3: L.fnGenUniformGrid3DDevice, 4: L.fnGenUniformGrid4DDevice})
+        _lib = L
     return _lib
 
 
@@ -186,6 +192,16 @@ def _check():
 
 def _fp(a: np.ndarray):
     return a.ctypes.data_as(_FP)
+
+
+def _seed32(v) -> int:
+    """A seed of the device calls: an int32 (a plain int in range without the numpy round trip)."""
+    return v if type(v) is int and -0x80000000 <= v <= 0x7FFFFFFF else int(np.int32(v))
+
+
+def _address(a: np.ndarray) -> int:
+    """Where an array's data starts (`a.ctypes.data` builds an object for it)."""
+    return a.__array_interface__["data"][0]
 
 
 def _i32(v) -> int:
@@ -747,18 +763,19 @@ class Node:
     # -- generation (host memory, reference-compatible) ----------------------
     def gen_uniform_grid(self, offset: Sequence[float], count: Sequence[int], step: Sequence[float], seed: int,
                          out: Optional[np.ndarray] = None) -> Tuple[np.ndarray, Tuple[float, float]]:
-        dim = len(count)
-        total = math.prod(max(int(c), 0) for c in count)
+        total = 1
+        for c in count:
+            total *= max(int(c), 0)
         if out is None:
             out = np.empty(max(total, 1), np.float32)
-        mm = np.zeros(2, np.float32)
-        L = lib()
-        f = {2: L.fnGenUniformGrid2D, 3: L.fnGenUniformGrid3D, 4: L.fnGenUniformGrid4D}.get(dim)
+        lib()
+        f = _grid_host.get(len(count))
         if f is None:
             raise ValueError("dimension must be 2, 3 or 4")
-        f(self._h, out.ctypes.data, *offset, *count, *step, _i32(seed), mm.ctypes.data)
+        mm = _MinMax()
+        f(self._h, _address(out), *offset, *count, *step, _i32(seed), ctypes.addressof(mm))
         _check()
-        return out[:total], (float(mm[0]), float(mm[1]))
+        return out[:total], (mm[0], mm[1])
 
     def gen_uniform_grid_2d(self, offset, count, step, seed, out=None):
         return self.gen_uniform_grid(offset, count, step, seed, out)
@@ -808,11 +825,9 @@ class Node:
     def gen_uniform_grid_device(self, out_ptr: int, offset, count, step, seed: int, minmax_ptr: int = 0,
                                 stream: int = 0) -> None:
         """Queue a grid into device memory `out_ptr` on `stream` (a cudaStream_t value)."""
-        L = lib()
-        dim = len(count)
-        f = {2: L.fnGenUniformGrid2DDevice, 3: L.fnGenUniformGrid3DDevice, 4: L.fnGenUniformGrid4DDevice}[dim]
-        rc = f(self._h, out_ptr, *map(float, offset), *map(int, count), *map(float, step), int(np.int32(seed)),
-               minmax_ptr or None, stream or None)
+        lib()
+        rc = _grid_device[len(count)](self._h, out_ptr, *map(float, offset), *map(int, count), *map(float, step), _seed32(seed),
+                                      minmax_ptr or None, stream or None)
         if rc != 0:
             _check()
 

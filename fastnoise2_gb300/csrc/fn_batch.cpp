@@ -10,6 +10,7 @@
 #include <cstring>
 #include <fstream>
 #include <sstream>
+#include <unordered_map>
 
 namespace fn {
 
@@ -23,7 +24,7 @@ uint32_t tiles_for(long long total, uint32_t tile_points)
     return (uint32_t)((total + tile_points - 1) / tile_points);
 }
 
-uint64_t batch_signature(const std::vector<BatchItem>& items, const std::vector<DeviceProgram>& progs)
+uint64_t batch_signature(const std::vector<BatchItem>& items, const std::vector<uint64_t>& hashes)
 {
     // multiset of (program, size class): independent of request order and of node addresses
     std::vector<uint64_t> keys;
@@ -31,7 +32,7 @@ uint64_t batch_signature(const std::vector<BatchItem>& items, const std::vector<
     for (size_t i = 0; i < items.size(); ++i) {
         int lg = 0;
         while ((1ll << lg) < items[i].args.total && lg < 62) ++lg;
-        keys.push_back(progs[i].hash * 0x9E3779B97F4A7C15ull ^ ((uint64_t)items[i].args.src << 60) ^ ((uint64_t)lg << 48));
+        keys.push_back(hashes[i] * 0x9E3779B97F4A7C15ull ^ ((uint64_t)items[i].args.src << 60) ^ ((uint64_t)lg << 48));
     }
     std::sort(keys.begin(), keys.end());
     return fnv1a64(keys.data(), keys.size() * sizeof(uint64_t));
@@ -168,114 +169,117 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
 {
     const size_t n = items.size();
     if (n == 0) return 0;
-    std::vector<DeviceProgram> progs(n);
+    // A batch has few trees: each is looked up once, not once per request.
+    struct Tree {
+        DeviceProgram prog;
+        BatchKernel kernel;            // its specialised batch kernel
+        JitKernels jk;                 // its column kernel, unless a variant is forced
+        int group[2] = {-1, -1};       // launch group of its point / column requests
+    };
+    std::vector<Tree> trees;
+    std::unordered_map<uintptr_t, uint32_t> tree_index;
+    tree_of_.resize(n);
     uint32_t max_bytes = 16;
     points_ = 0;
+    bool jit = true;
     for (size_t i = 0; i < n; ++i) {
-        if (!items[i].node || items[i].args.total < 0 || (items[i].args.total > 0 && !items[i].dout)) {
+        const BatchItem& it = items[i];
+        if (!it.node || it.args.total < 0 || (it.args.total > 0 && !it.dout)) {
             set_error(-1, "batch request " + std::to_string(i) + ": invalid arguments");
             return -1;
         }
-        if (!get_program(items[i].node, items[i].args.dim, progs[i])) return last_error();
-        std::string err;
-        if (!jit_ensure(progs[i].host, err)) { set_error(-2, "batch request " + std::to_string(i) + ": " + err); return -2; }
-        max_bytes = std::max(max_bytes, progs[i].bytes);
-        points_ += (uint64_t)std::max(0ll, items[i].args.total);
+        const auto known = tree_index.emplace(reinterpret_cast<uintptr_t>(it.node) * 8 + (uintptr_t)it.args.dim, (uint32_t)trees.size());
+        if (known.second) {
+            trees.emplace_back();
+            DeviceProgram& prog = trees.back().prog;
+            if (!get_program(it.node, it.args.dim, prog)) return last_error();
+            std::string err;
+            if (!jit_ensure(prog.host, err)) { set_error(-2, "batch request " + std::to_string(i) + ": " + err); return -2; }
+            max_bytes = std::max(max_bytes, prog.bytes);
+        }
+        tree_of_[i] = known.first->second;
+        points_ += (uint64_t)it.args.total;
+        jit = jit && it.args.total < (1ll << 32);   // 32-bit point indices
     }
-    signature_ = batch_signature(items, progs);
     // Specialised batch kernels when every program of the batch has one: each tree's tuned
     // variant when it is built (a variant not built yet is queued for a background build and
     // variant 0 runs meanwhile), or the variant a tuning run forces.
-    std::vector<BatchKernel> kernels(n);
-    std::vector<PointArgs> args(n);
-    std::vector<char> column(n, 0);                 // grid requests walked in columns
-    double column_work = 0;                         // their 32-point steps
-    for (size_t i = 0; i < n; ++i) args[i] = items[i].args;
-    bool jit = true;
-    for (size_t i = 0; jit && i < n; ++i) jit = items[i].args.total < (1ll << 32);   // 32-bit point indices
-    {
-        const int forced = tuning_in ? tuning_in->variant : -1;
-        struct Tree { BatchKernel kernel; JitKernels jk; };
-        std::map<uint64_t, Tree> chosen;
-        for (size_t i = 0; jit && i < n; ++i) {
-            auto it = chosen.find(progs[i].hash);
-            if (it == chosen.end()) {
-                BatchKernel bk;
-                const int v = forced >= 0 ? forced : Autotuner::instance().tree_variant(progs[i].hash);
-                bool ok = jit_batch_kernel(progs[i].hash, v, bk);
-                if (!ok && !jit_is_specialised(progs[i].hash) && jit_try_cached(progs[i].host))   // an earlier process built it
-                    ok = jit_batch_kernel(progs[i].hash, v, bk);
-                if (!ok && v != 0) {
-                    if (forced < 0) jit_request_batch_variants(progs[i].host);
-                    ok = jit_batch_kernel(progs[i].hash, 0, bk);
-                }
-                if (!ok) { jit = false; break; }
-                Tree t;
-                t.kernel = bk;
-                if (forced >= 0 || !jit_lookup(progs[i].hash, t.jk)) t.jk = JitKernels();   // a forced variant is run as asked
-                it = chosen.emplace(progs[i].hash, t).first;
-            }
-            kernels[i] = it->second.kernel;
-            if (it->second.jk.batch_column && jit_column_grid(args[i], it->second.jk)) {
-                kernels[i] = BatchKernel{it->second.jk.batch_column, 256};
-                column[i] = 1;
-                column_work += (double)args[i].col_steps * ((args[i].col_plane + 31) / 32);
-            }
+    const int forced = tuning_in ? tuning_in->variant : -1;
+    for (size_t t = 0; jit && t < trees.size(); ++t) {
+        Tree& tr = trees[t];
+        const uint64_t hash = tr.prog.hash;
+        const int v = forced >= 0 ? forced : Autotuner::instance().tree_variant(hash);
+        bool ok = jit_batch_kernel(hash, v, tr.kernel);
+        if (!ok && !jit_is_specialised(hash) && jit_try_cached(tr.prog.host))   // an earlier process built it
+            ok = jit_batch_kernel(hash, v, tr.kernel);
+        if (!ok && v != 0) {
+            if (forced < 0) jit_request_batch_variants(tr.prog.host);
+            ok = jit_batch_kernel(hash, 0, tr.kernel);
         }
+        if (!ok) { jit = false; break; }
+        if (forced >= 0 || !jit_lookup(hash, tr.jk)) tr.jk = JitKernels();   // a forced variant is run as asked
     }
-    if (!jit) std::fill(column.begin(), column.end(), 0);
-    if (!jit) {                                     // interpreter batch: count a use of each program
-        std::vector<uint64_t> seen;
-        for (size_t i = 0; i < n; ++i)
-            if (std::find(seen.begin(), seen.end(), progs[i].hash) == seen.end()) {
-                seen.push_back(progs[i].hash);
-                jit_note_interpreted(progs[i].host);
-            }
-    }
+    if (!jit)                                       // interpreter batch: count a use of each program
+        for (size_t t = 0; t < trees.size(); ++t) {
+            bool seen = false;
+            for (size_t u = 0; u < t; ++u) seen = seen || trees[u].prog.hash == trees[t].prog.hash;
+            if (!seen) jit_note_interpreted(trees[t].prog.host);
+        }
     if (!jit)
         for (size_t i = 0; i < n; ++i)
-            if (progs[i].host->needs_specialisation() && items[i].args.total > 0) {
+            if (trees[tree_of_[i]].prog.host->needs_specialisation() && items[i].args.total > 0) {
                 set_error(-2, "batch request " + std::to_string(i) + ": the tree needs specialised kernels, which this batch "
                               "cannot use (specialisation disabled or a request of 2^32 points or more)");
                 return -2;
             }
-    if (jit) signature_ = signature_ * 0x100000001B3ull + 0x4A17;   // tuned separately from the interpreter
+    // the signature sorts a key per request: only for a tuning run, or to look one up
+    signature_ = 0;
+    if (tuning_in || Autotuner::instance().any()) {
+        std::vector<uint64_t> hashes;
+        for (uint32_t t : tree_of_) hashes.push_back(trees[t].prog.hash);
+        signature_ = batch_signature(items, hashes);
+        if (jit) signature_ = signature_ * 0x100000001B3ull + 0x4A17;   // tuned separately from the interpreter
+    }
     BatchTuning tuning;
     if (tuning_in) tuning = *tuning_in;
     else Autotuner::instance().lookup(signature_, tuning);
     const uint32_t tp = std::max<uint32_t>(256, tuning.tile_points);
+    // Grid requests of trees with a column kernel are walked in columns.
+    columns_.assign(n, ColumnShape());
+    double column_work = 0;                         // their 32-point steps
+    for (size_t i = 0; jit && i < n; ++i) {
+        const JitKernels& jk = trees[tree_of_[i]].jk;
+        if (jk.batch_column && jit_column_grid(items[i].args, jk, columns_[i]))
+            column_work += (double)columns_[i].steps * column_chunks(columns_[i]);
+    }
     // Column units: about four rounds of 16 warps per SM over the whole batch, so that short
     // batches still spread, and at most 64 steps (longer ones gain under 5 % of set-up).
     const unsigned col_len = (unsigned)std::min(64.0, std::max(4.0, column_work / (64.0 * num_sms())));
-    std::vector<uint32_t> tiles(n);
+    // One group per distinct kernel, in first-appearance order (the interpreter: one for all).
+    std::vector<BatchKernel> gkernel;
+    std::vector<size_t> gitems;                     // work items per group
+    tiles_.resize(n);
+    group_of_.resize(n);
     size_t n_items = 0;
     for (size_t i = 0; i < n; ++i) {
-        tiles[i] = column[i] ? jit_column_tiles(args[i], col_len) : tiles_for(items[i].args.total, tp);
-        n_items += tiles[i];
+        const bool column = columns_[i].plane != 0;
+        tiles_[i] = column ? column_tiles(columns_[i], col_len) : tiles_for(items[i].args.total, tp);
+        Tree& tr = trees[tree_of_[i]];
+        int& g = tr.group[column ? 1 : 0];
+        if (g < 0) {
+            const BatchKernel bk = !jit ? BatchKernel{nullptr, 256} : column ? BatchKernel{tr.jk.batch_column, 256} : tr.kernel;
+            for (g = 0; g < (int)gkernel.size() && gkernel[(size_t)g].kernel != bk.kernel; ++g) {}
+            if (g == (int)gkernel.size()) {
+                gkernel.push_back(bk);
+                gitems.push_back(0);
+            }
+        }
+        group_of_[i] = (uint32_t)g;
+        gitems[(size_t)g] += tiles_[i];
+        n_items += tiles_[i];
     }
     if (n_items > 0xFFFFFFFFull) { set_error(-4, "batch too large"); return -4; }
     if (!reserve(n, n_items)) return -3;
-
-    // Requests per group: all of them for the interpreter, one group per
-    // distinct specialised kernel (first-appearance order) otherwise.
-    std::vector<std::vector<uint32_t>> members;
-    std::vector<BatchKernel> gkernel;
-    if (jit) {
-        std::map<cudaKernel_t, size_t> index;
-        for (size_t i = 0; i < n; ++i) {
-            auto it = index.find(kernels[i].kernel);
-            if (it == index.end()) {
-                it = index.emplace(kernels[i].kernel, members.size()).first;
-                members.emplace_back();
-                gkernel.push_back(kernels[i]);
-            }
-            members[it->second].push_back((uint32_t)i);
-        }
-    } else {
-        members.emplace_back();
-        gkernel.push_back(BatchKernel{nullptr, 256});          // the interpreter's batch kernel: 256 threads
-        for (size_t i = 0; i < n; ++i) members[0].push_back((uint32_t)i);
-    }
 
     // The staging buffer is reused: the previous launch's upload must have been consumed.
     if (!staged_ && !cuda_ok(cudaEventCreateWithFlags(&staged_, cudaEventDisableTiming), "event")) return -3;
@@ -295,16 +299,18 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     for (size_t i = 0; i < n; ++i) {
         BatchRequest& r = reqs[i];
         std::memset(&r, 0, sizeof r);
-        r.args = args[i];
-        r.prog = progs[i].dptr;
+        const DeviceProgram& prog = trees[tree_of_[i]].prog;
+        r.args = items[i].args;
+        if (columns_[i].plane) column_args(r.args, columns_[i]);
+        r.prog = prog.dptr;
         r.jit_slot = -1;
-        r.prog_bytes = progs[i].bytes;
+        r.prog_bytes = prog.bytes;
         r.out = items[i].dout;
         r.minmax = items[i].dminmax;
         r.host_minmax = items[i].host_minmax;
         r.host_done = items[i].host_done;
         r.host_time = items[i].host_time;
-        r.n_tiles = tiles[i];
+        r.n_tiles = tiles_[i];
         states[i].mn_enc = 0xFFFFFFFFu;
         states[i].mx_enc = 0u;
         states[i].tiles_done = 0u;
@@ -312,24 +318,29 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         last_minmax_[i] = items[i].dminmax;
     }
     const int sms = num_sms();
-    groups_.assign(members.size(), Group());
-    size_t k = 0;
+    groups_.assign(gkernel.size(), Group());
+    std::vector<size_t> next(gkernel.size());       // next item of each group
+    for (size_t g = 0, k = 0; g < gkernel.size(); ++g) {
+        next[g] = k;
+        k += gitems[g];
+    }
     int total_grid = 0;
-    for (size_t g = 0; g < members.size(); ++g) {
+    for (size_t g = 0; g < gkernel.size(); ++g) {
         Group& gr = groups_[g];
         gr.jit = gkernel[g].kernel;
         gr.threads = gkernel[g].threads;
-        gr.item_begin = (uint32_t)k;
-        for (uint32_t i : members[g])
-            for (uint32_t t = 0; t < reqs[i].n_tiles; ++t) its[k++] = make_uint2(i, t);
-        gr.item_end = (uint32_t)k;
+        gr.item_begin = (uint32_t)next[g];
+        gr.item_end = (uint32_t)(next[g] + gitems[g]);
         grps[g].item_begin = gr.item_begin;
         grps[g].item_end = gr.item_end;
         grps[g].head = 0;
         grps[g].pad = 0;
         int occ = tuning.ctas_per_sm;
         if (occ <= 0 && gr.jit) {
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)gr.jit, gr.threads, 0) != cudaSuccess || occ < 1) occ = 1;
+            int& known = occupancy_[gr.jit];
+            if (!known && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&known, (const void*)gr.jit, gr.threads, 0) != cudaSuccess || known < 1))
+                known = 1;
+            occ = known;
         } else if (occ <= 0) {
             occ = batch_occupancy(256, max_bytes);
         }
@@ -339,6 +350,11 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         if (grid < 1) grid = 1;
         gr.grid = (int)grid;
         total_grid += gr.grid;
+    }
+    for (size_t i = 0; i < n; ++i) {
+        uint2* at = its + next[group_of_[i]];
+        for (uint32_t t = 0; t < tiles_[i]; ++t) at[t] = make_uint2((unsigned)i, t);
+        next[group_of_[i]] += tiles_[i];
     }
     const size_t bytes = off_items_ + n_items * sizeof(uint2);
     const uint32_t smem = jit ? 0 : max_bytes;
@@ -384,6 +400,12 @@ bool Autotuner::lookup(uint64_t sig, BatchTuning& out)
     if (it == table_.end()) return false;
     out = it->second.first;
     return true;
+}
+
+bool Autotuner::any()
+{
+    std::lock_guard<std::mutex> lk(mu_);
+    return !table_.empty();
 }
 
 void Autotuner::store(uint64_t sig, const BatchTuning& t, double ms)

@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "fn_jit.h"
 #include "fn_kernels.cuh"
 #include "fn_runtime.h"
 
@@ -46,7 +47,7 @@ public:
     // Device copy of the last launch's per-request state (for min/max read-back).
     BatchState* device_states() const { return d_states_; }
     const std::vector<float*>& last_device_minmax() const { return last_minmax_; }
-    uint64_t last_signature() const { return signature_; }
+    uint64_t last_signature() const { return signature_; }   // of a launch with a tuning
     uint64_t last_points() const { return points_; }
     // Shape of the last launch: work items, bytes uploaded, tile size, CTAs, kernel kind.
     uint64_t last_items() const { return items_; }
@@ -93,6 +94,10 @@ private:
     std::vector<Group> last_groups_;    // shape of the previous launch (a graph is captured for a repeated shape)
     uint32_t last_smem_ = 0;
     std::vector<float*> last_minmax_;
+    // per request of a launch, kept to save their allocation: tree, column shape, work items, group
+    std::vector<uint32_t> tree_of_, tiles_, group_of_;
+    std::vector<ColumnShape> columns_;
+    std::map<cudaKernel_t, int> occupancy_;
     uint64_t signature_ = 0;
     uint64_t points_ = 0;
     uint64_t items_ = 0, upload_bytes_ = 0;
@@ -108,6 +113,7 @@ class Autotuner {
 public:
     static Autotuner& instance();
     bool lookup(uint64_t signature, BatchTuning& out);
+    bool any();                                              // a batch signature has been tuned or loaded
     void store(uint64_t signature, const BatchTuning& t, double ms);
     std::vector<BatchTuning> candidates() const;
     int tree_variant(uint64_t program_hash);                 // 0 when the tree has not been tuned
@@ -121,7 +127,7 @@ private:
     std::map<uint64_t, std::pair<int, double>> trees_;
 };
 
-uint64_t batch_signature(const std::vector<BatchItem>& items, const std::vector<DeviceProgram>& progs);
+uint64_t batch_signature(const std::vector<BatchItem>& items, const std::vector<uint64_t>& program_hashes);
 uint32_t tiles_for(long long total, uint32_t tile_points);
 
 }  // namespace fn

@@ -386,8 +386,8 @@ void set_divisor(PointArgs& a, int k, int count)
 {
     const uint64_t d = count > 0 ? (uint64_t)count : 1u;
     if (d == 1) { a.divm[k] = 0; a.divs[k] = 0; return; }
-    unsigned s = 0;
-    while ((1ull << s) < d) ++s;
+    const unsigned s = 32u - (unsigned)__builtin_clz((unsigned)d - 1u);
+    if ((d & (d - 1)) == 0) { a.divm[k] = 1; a.divs[k] = s; return; }
     a.divm[k] = (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
     a.divs[k] = s;
 }
@@ -482,6 +482,7 @@ bool request_args(const fnGenRequest& r, PointArgs& a)
 
 struct BatchCtx {
     BatchRunner runner;
+    std::vector<BatchItem> items;          // of the current call, kept to save the allocation
     float* dminmax = nullptr;
     float* hminmax = nullptr;
     size_t cap = 0;
@@ -539,7 +540,7 @@ int run_batch(const fnGenRequest* reqs, int n, void* stream, int flags, const Ba
     if (n == 0) return FN_OK;
     if (!thread_ctx()) return FN_ERR_CUDA;
     if (b ? !reserve_batch(b, (size_t)n) : !(b = batch_ctx((size_t)n))) return FN_ERR_CUDA;
-    std::vector<BatchItem> items;
+    std::vector<BatchItem>& items = b->items;
     int rc = build_items(reqs, n, b, items);
     if (rc) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);

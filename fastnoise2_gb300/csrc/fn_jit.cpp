@@ -1461,48 +1461,48 @@ bool jit_auto_wait(int timeout_ms)
 
 constexpr double kColMaxGroups = 3.0;
 
-// Whether the grid of `a` is to be walked in columns (a tree without a column kernel, other
-// point sources and partial planes are not); sets its plane, steps and first step.
-bool jit_column_grid(PointArgs& a, const JitKernels& jk)
+// A tree without a column kernel, other point sources and partial planes are not walked.
+bool jit_column_grid(const PointArgs& a, const JitKernels& jk, ColumnShape& shape)
 {
     if (a.src != kSrcGrid || a.total <= 0 || a.total > (1ll << 31) || !jk.column) return false;
     long long plane = 1;
     for (int k = 0; k < a.dim - 1; ++k) plane *= a.count[k];
-    if (plane <= 0 || a.total % plane || a.base % plane) return false;
+    if (plane <= 0) return false;
+    if ((a.base || a.total != plane * a.count[a.dim - 1]) && (a.total % plane || a.base % plane)) return false;
     // A step that crosses into another lattice cell rebuilds a Perlin state at about the cost
     // of the point function: FBm(Perlin) 128^3 (69.7 us with the point kernel) takes 27, 39, 53,
     // 70 and 86 us at 0.06, 0.25, 0.40, 0.62 and 0.79 crossings a step.  Value states never lose.
-    // A cellular state also builds one neighbourhood per distinct cell of a warp's lanes.
-    double rate = 0;
+    // A cellular or warp state also builds one neighbourhood per distinct cell of a warp's lanes.
+    float rate = 0;
     for (int k = 0; k < jk.n_column_rates; ++k) {
         const ColumnRate& c = jk.column_rates[k];
-        double r = std::fabs((double)c.scale[a.dim - 1] * a.step[a.dim - 1]);
+        const float r = std::fabs(c.scale[a.dim - 1] * a.step[a.dim - 1]);
         if (c.cellular) {
-            double groups = 1, left = 32;          // lanes not yet spread over an axis
+            float groups = 1, left = 32;           // lanes not yet spread over an axis
             for (int j = 0; j < a.dim - 1; ++j) {
-                const double spread = std::min<double>(left, a.count[j]);
-                groups *= 1 + (spread - 1) * std::fabs((double)c.scale[j] * a.step[j]);
-                left = std::max(1.0, left / a.count[j]);
+                const float spread = std::min<float>(left, (float)a.count[j]);
+                groups *= 1 + (spread - 1) * std::fabs(c.scale[j] * a.step[j]);
+                left = std::max(1.0f, left / (float)a.count[j]);
             }
             if (!(groups <= kColMaxGroups)) return false;
         }
-        rate += r < 1.0 ? r : 1.0;
+        rate += r < 1.0f ? r : 1.0f;
     }
-    if (jk.n_column_rates && !(rate < 0.6 * jk.n_column_rates)) return false;
-    a.col_plane = (unsigned)plane;
-    a.col_steps = (unsigned)(a.total / plane);
-    a.col_first = a.base / (unsigned)plane;
+    if (jk.n_column_rates && !(rate < 0.6f * (float)jk.n_column_rates)) return false;
+    shape.plane = (unsigned)plane;
+    shape.steps = a.base || a.total != plane * a.count[a.dim - 1] ? (unsigned)(a.total / plane) : (unsigned)a.count[a.dim - 1];
+    shape.first = a.base ? a.base / (unsigned)plane : 0u;
     return true;
 }
 
-unsigned column_chunks(const PointArgs& a) { return (a.col_plane + 31) / 32; }
+namespace {
 
 // Cut the columns into units of at most `len` steps, evenly.
-void column_cut(PointArgs& a, unsigned len)
+void column_cut(ColumnShape& s, unsigned len)
 {
-    const unsigned segs = (a.col_steps + len - 1) / len;
-    a.col_len = (a.col_steps + segs - 1) / segs;
-    a.col_units = column_chunks(a) * ((a.col_steps + a.col_len - 1) / a.col_len);
+    const unsigned segs = (s.steps + len - 1) / len;
+    s.len = (s.steps + segs - 1) / segs;
+    s.units = column_chunks(s) * ((s.steps + s.len - 1) / s.len);
 }
 
 // Steps per unit of a launch that has the GPU to itself: setting a unit up costs
@@ -1510,28 +1510,40 @@ void column_cut(PointArgs& a, unsigned len)
 // a unit; a fraction of one for a terrain tree), and an SM works on `column_resident` blocks of
 // 8 units at once, so minimise (blocks of the busiest SM, at least the resident ones) x
 // (set-up + length).
-void column_cut_alone(PointArgs& a, const JitKernels& jk)
+void column_cut_alone(ColumnShape& s, const JitKernels& jk)
 {
-    const unsigned n = a.col_steps, chunks = column_chunks(a);
-    const double sms = num_sms(), fill = std::max(1, jk.column_resident);
+    const unsigned n = s.steps, chunks = column_chunks(s), slots = 8u * (unsigned)num_sms(),
+                   fill = (unsigned)std::max(1, jk.column_resident);
     unsigned best = 1;
-    double best_cost = 1e300;
-    for (int w = 1; w <= 16; ++w) {
-        const unsigned fit = (unsigned)std::min<double>(n, std::max(1.0, std::floor(w * sms * 8.0 / chunks)));
-        const unsigned len = (n + fit - 1) / fit;
-        const double units = (double)chunks * ((n + len - 1) / len);
-        const double cost = std::max(fill, std::ceil(units / (8.0 * sms))) * (jk.column_setup + len);
+    float best_cost = 1e30f;
+    for (unsigned w = 1; w <= 16; ++w) {
+        const unsigned fit = std::min(n, std::max(1u, w * slots / chunks)), len = (n + fit - 1) / fit;
+        const unsigned long long units = (unsigned long long)chunks * ((n + len - 1) / len);
+        const unsigned load = (unsigned)((units + slots - 1) / slots);
+        const float cost = (float)std::max(fill, load) * (jk.column_setup + (float)len);
         if (cost < best_cost) { best_cost = cost; best = len; }
+        if (len == 1) break;
     }
-    column_cut(a, best);
+    column_cut(s, best);
 }
 
-unsigned jit_column_tiles(PointArgs& args, unsigned len)
+}  // namespace
+
+unsigned column_tiles(ColumnShape& s, unsigned len)
 {
     // a request with fewer units than a block has warps is cut finer
-    const unsigned long long work = (unsigned long long)column_chunks(args) * args.col_steps;
-    column_cut(args, (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(len, (work + 7) / 8)));
-    return (args.col_units + 7) / 8;
+    const unsigned long long work = (unsigned long long)column_chunks(s) * s.steps;
+    column_cut(s, (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(len, (work + 7) / 8)));
+    return (s.units + 7) / 8;
+}
+
+void column_args(PointArgs& a, const ColumnShape& s)
+{
+    a.col_plane = s.plane;
+    a.col_steps = s.steps;
+    a.col_first = s.first;
+    a.col_len = s.len;
+    a.col_units = s.units;
 }
 
 // Launch a per-call kernel so that it may start while the stream's previous kernel drains
@@ -1558,10 +1570,12 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     JitKernels jk;
     if (args.total <= 0 || args.total > (1ll << 31) || !jit_lookup(hash, jk)) return false;
     const int which = args.src == kSrcGrid ? 0 : args.src == kSrcPositions ? 1 : 2;
-    PointArgs c = args;
-    if (which == 0 && jit_column_grid(c, jk)) {
-        column_cut_alone(c, jk);
-        const unsigned grid = std::min<unsigned>((c.col_units + 7) / 8, (unsigned)kMaxReduceBlocks);
+    ColumnShape shape;
+    if (which == 0 && jit_column_grid(args, jk, shape)) {
+        column_cut_alone(shape, jk);
+        PointArgs c = args;
+        column_args(c, shape);
+        const unsigned grid = std::min<unsigned>((shape.units + 7) / 8, (unsigned)kMaxReduceBlocks);
         void* params[] = {&c, &out, &work, &dminmax};
         err = launch_overlapped(jk.column, grid, params, stream);
         return true;

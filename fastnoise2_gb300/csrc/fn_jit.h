@@ -94,11 +94,19 @@ bool jit_build_batch_variants(const std::vector<const CompiledProgram*>& progs, 
 // The batch kernel of `hash` in `variant`, or false when it is not built (or JIT is off).
 bool jit_batch_kernel(uint64_t hash, int variant, BatchKernel& out);
 
-// Whether a grid is to be walked in columns by the kernels `jk` (fn_column.cuh); if so `args`
-// gets its plane and steps.  jit_column_tiles cuts it into units of at most `len` steps and
-// returns a batch's work items for it (eight units each).
-bool jit_column_grid(PointArgs& args, const JitKernels& jk);
-unsigned jit_column_tiles(PointArgs& args, unsigned len);
+// A grid walked in columns (PointArgs' col_ fields): points of the plane across the last axis
+// (0: not walked in columns), steps along it and the index of the first, steps per unit, units.
+struct ColumnShape {
+    unsigned plane = 0, steps = 0, first = 0, len = 0, units = 0;
+};
+
+// Whether a grid is to be walked in columns by the kernels `jk` (fn_column.cuh); if so `shape`
+// gets its plane and steps.  column_tiles cuts it into units of at most `len` steps and returns
+// a batch's work items for it (eight units each).
+bool jit_column_grid(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
+inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
+unsigned column_tiles(ColumnShape& shape, unsigned len);
+void column_args(PointArgs& args, const ColumnShape& shape);
 
 // Queue a background build of the batch variants of `prog` (a tuning table loaded in this
 // process may name variants that have not been built yet).
