@@ -562,7 +562,15 @@ FND float supersimplex3(int seed, float x, float y, float z)
     return value;
 }
 
-FND float supersimplex4(int seed, float x, float y, float z, float w)
+// One copy per kernel where specialised: ~750 instructions inlined once per octave overflowed the
+// instruction cache (warps waited for instructions a third of the time): tileable terrain
+// 1024^2 208 -> 190 us.
+#ifdef FN_GRADIENT_TABLE
+__device__ __noinline__
+#else
+FND
+#endif
+float supersimplex4(int seed, float x, float y, float z, float w)
 {
     constexpr double kSkew4 = 1.0 / (kRoot5 + 1.0);
     constexpr double kU = -1.0 / (kRoot5 + 5.0);
