@@ -211,9 +211,11 @@ ColPlan column_plan(const CompiledProgram& prog)
             if (D < 4 && sums && jit.kind == Reg::kConst && std::isfinite(jit.scale) && I.c == FN_REG_NONE && I.d == FN_REG_NONE &&
                 (I.op == FN_OP_CELL_LOOKUP || slots <= (I.op == FN_OP_CELL_DIST ? 2 : 1))) {
                 const std::string kind = I.op == FN_OP_CELL_VALUE ? "kColValue" : I.op == FN_OP_CELL_DIST ? "kColDistance" : "kColLookup";
-                const int cells = D == 3 ? 27 : 9;
+                // CellCol's part of the table (kTable there)
+                const int cells = D == 3 ? 27 : 9, along = (D == 3 ? 12 : 4) * (I.op == FN_OP_CELL_LOOKUP ? 1 : 2);
+                const int cell_table = 32 + 4 * cells + 3 * along + (I.op == FN_OP_CELL_VALUE ? cells : 0);
                 ColState* st = add_state(pc, "CellCol<" + std::to_string(D) + ", fnd::" + kind + ", " + std::to_string(I.op == FN_OP_CELL_DIST ? slots : 1) + ">",
-                                         P[I.prm], cells + 4, 32 + 4 * cells + (I.op == FN_OP_CELL_VALUE ? cells : 0), true,
+                                         P[I.prm], cells + 4, cell_table, true,
                                          D == 3 ? 300 : 150, D == 3 ? 190 : 65);
                 if (st) st->jitter = "fnd::CellConst<" + std::to_string(D) + ">::jitter * " + lit(jit.scale);
             }
