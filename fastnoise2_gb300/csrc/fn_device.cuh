@@ -432,19 +432,22 @@ FND float simplex4(int seed, float x, float y, float z, float w)
     float dz3 = (rz > 0 ? dz0 - 1.0f : dz0) - u3, dw3 = (rw > 0 ? dw0 - 1.0f : dw0) - u3;
     float dx4 = dx0 - u4, dy4 = dy0 - u4, dz4 = dz0 - u4, dw4 = dw0 - u4;
     constexpr float R = (float)0.6;
-    float f0 = fmaf(-dw0, dw0, fmaf(-dz0, dz0, fmaf(-dy0, dy0, fmaf(-dx0, dx0, R))));
-    float f1 = fmaf(-dw1, dw1, fmaf(-dz1, dz1, fmaf(-dy1, dy1, fmaf(-dx1, dx1, R))));
-    float f2 = fmaf(-dw2, dw2, fmaf(-dz2, dz2, fmaf(-dy2, dy2, fmaf(-dx2, dx2, R))));
-    float f3 = fmaf(-dw3, dw3, fmaf(-dz3, dz3, fmaf(-dy3, dy3, fmaf(-dx3, dx3, R))));
-    float f4 = f0 + fmaf(unskew, (float)(-4.0 * (kRoot5 + 3.0) / (kRoot5 + 5.0)), (float)(-4.0 / 5.0));
-    f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f); f4 = fmaxf(f4, 0.0f);
-    f0 *= f0; f0 *= f0; f1 *= f1; f1 *= f1; f2 *= f2; f2 *= f2; f3 *= f3; f3 *= f3; f4 *= f4; f4 *= f4;
-    float g0 = gdot4(hashhb(seed, xp, yp, zp, wp), dx0, dy0, dz0, dw0);
-    float g1 = gdot4(hashhb(seed, rx > 2 ? iadd(xp, kPrimeX) : xp, ry > 2 ? iadd(yp, kPrimeY) : yp, rz > 2 ? iadd(zp, kPrimeZ) : zp, rw > 2 ? iadd(wp, kPrimeW) : wp), dx1, dy1, dz1, dw1);
-    float g2 = gdot4(hashhb(seed, rx > 1 ? iadd(xp, kPrimeX) : xp, ry > 1 ? iadd(yp, kPrimeY) : yp, rz > 1 ? iadd(zp, kPrimeZ) : zp, rw > 1 ? iadd(wp, kPrimeW) : wp), dx2, dy2, dz2, dw2);
-    float g3 = gdot4(hashhb(seed, rx > 0 ? iadd(xp, kPrimeX) : xp, ry > 0 ? iadd(yp, kPrimeY) : yp, rz > 0 ? iadd(zp, kPrimeZ) : zp, rw > 0 ? iadd(wp, kPrimeW) : wp), dx3, dy3, dz3, dw3);
-    float g4 = gdot4(hashhb(seed, iadd(xp, kPrimeX), iadd(yp, kPrimeY), iadd(zp, kPrimeZ), iadd(wp, kPrimeW)), dx4, dy4, dz4, dw4);
-    return fmaf(g0, f0, fmaf(g1, f1, fmaf(g2, f2, fmaf(g3, f3, g4 * f4))));
+    // falloffs negated, vertices 0, 1 and 2, 3 packed: d.d - R rounds as R - d.d does
+    float n0, n1, n2, n3;
+    {
+        const f32x2 x01 = pack2(dx0, dx1), y01 = pack2(dy0, dy1), z01 = pack2(dz0, dz1), w01 = pack2(dw0, dw1);
+        const f32x2 x23 = pack2(dx2, dx3), y23 = pack2(dy2, dy3), z23 = pack2(dz2, dz3), w23 = pack2(dw2, dw3), r = pack2(-R, -R);
+        unpack2(fma2(w01, w01, fma2(z01, z01, fma2(y01, y01, fma2(x01, x01, r)))), n0, n1);
+        unpack2(fma2(w23, w23, fma2(z23, z23, fma2(y23, y23, fma2(x23, x23, r)))), n2, n3);
+    }
+    float f4 = fmaxf(fmaf(unskew, (float)(-4.0 * (kRoot5 + 3.0) / (kRoot5 + 5.0)), (float)(-4.0 / 5.0)) - n0, 0.0f);
+    f4 *= f4; f4 *= f4;
+    const int xq = iadd(xp, kPrimeX), yq = iadd(yp, kPrimeY), zq = iadd(zp, kPrimeZ), wq = iadd(wp, kPrimeW);
+    float v = gdot4(hashhb(seed, xq, yq, zq, wq), dx4, dy4, dz4, dw4) * f4;
+    v = add_pair4(v, fminf(n3, 0.0f), hashhb(seed, rx > 0 ? xq : xp, ry > 0 ? yq : yp, rz > 0 ? zq : zp, rw > 0 ? wq : wp), dx3, dy3, dz3, dw3,
+                  fminf(n2, 0.0f), hashhb(seed, rx > 1 ? xq : xp, ry > 1 ? yq : yp, rz > 1 ? zq : zp, rw > 1 ? wq : wp), dx2, dy2, dz2, dw2);
+    return add_pair4(v, fminf(n1, 0.0f), hashhb(seed, rx > 2 ? xq : xp, ry > 2 ? yq : yp, rz > 2 ? zq : zp, rw > 2 ? wq : wp), dx1, dy1, dz1, dw1,
+                     fminf(n0, 0.0f), hashhb(seed, xp, yp, zp, wp), dx0, dy0, dz0, dw0);
 }
 
 // ---------------------------------------------------------------- SuperSimplex (OpenSimplex2S)
@@ -720,6 +723,23 @@ FND float perlin4(int seed, float x, float y, float z, float w)
     float xf0 = x - xs, yf0 = y - ys, zf0 = z - zs, wf0 = w - ws;
     float xf1 = xf0 - 1.0f, yf1 = yf0 - 1.0f, zf1 = zf0 - 1.0f, wf1 = wf0 - 1.0f;
     float u = quintic(xf0), v = quintic(yf0), s = quintic(zf0), q = quintic(wf0);
+#ifdef FN_GRADIENT_TABLE
+    // the two w planes as the halves of packed operations
+    const f32x2 wf = pack2(wf0, wf1);
+    auto corner = [&](int h, float xf, float yf, float zf) {
+        const float *a = gradient_of<4>(hashm(h ^ w0)), *b = gradient_of<4>(hashm(h ^ w1));
+        return fma2(pack2(a[96], b[96]), wf, fma2(pack2(a[64], b[64]), pack2(zf, zf),
+                    fma2(pack2(a[32], b[32]), pack2(yf, yf), mul2(pack2(a[0], b[0]), pack2(xf, xf)))));
+    };
+    auto face = [&](int z, float zf) {
+        const f32x2 uu = pack2(u, u);
+        return lerp2(lerp2(corner(seed ^ z ^ y0 ^ x0, xf0, yf0, zf), corner(seed ^ z ^ y0 ^ x1, xf1, yf0, zf), uu),
+                     lerp2(corner(seed ^ z ^ y1 ^ x0, xf0, yf1, zf), corner(seed ^ z ^ y1 ^ x1, xf1, yf1, zf), uu), pack2(v, v));
+    };
+    float lo, hi;
+    unpack2(lerp2(face(z0, zf0), face(z1, zf1), pack2(s, s)), lo, hi);
+    return lerp(lo, hi, q);
+#else
 #define G(a, b, c, d, fa, fb, fc, fd) gdot4(hashm((seed ^ b ^ c ^ d) ^ a), fa, fb, fc, fd)
     return lerp(
         lerp(lerp(lerp(G(x0, y0, z0, w0, xf0, yf0, zf0, wf0), G(x1, y0, z0, w0, xf1, yf0, zf0, wf0), u),
@@ -731,6 +751,7 @@ FND float perlin4(int seed, float x, float y, float z, float w)
              lerp(lerp(G(x0, y0, z1, w1, xf0, yf0, zf1, wf1), G(x1, y0, z1, w1, xf1, yf0, zf1, wf1), u),
                   lerp(G(x0, y1, z1, w1, xf0, yf1, zf1, wf1), G(x1, y1, z1, w1, xf1, yf1, zf1, wf1), u), v), s), q);
 #undef G
+#endif
 }
 
 FND float value2(int seed, float x, float y)
@@ -750,8 +771,13 @@ FND float value3(int seed, float x, float y, float z)
     int x1 = iadd(x0, kPrimeX), y1 = iadd(y0, kPrimeY), z1 = iadd(z0, kPrimeZ);
     float u = hermite(x - xs), v = hermite(y - ys), s = hermite(z - zs);
     const int a00 = seed ^ y0 ^ z0, a10 = seed ^ y1 ^ z0, a01 = seed ^ y0 ^ z1, a11 = seed ^ y1 ^ z1;   // shared by x pairs
-    return lerp(lerp(lerp(valcoord(a00 ^ x0), valcoord(a00 ^ x1), u), lerp(valcoord(a10 ^ x0), valcoord(a10 ^ x1), u), v),
-                lerp(lerp(valcoord(a01 ^ x0), valcoord(a01 ^ x1), u), lerp(valcoord(a11 ^ x0), valcoord(a11 ^ x1), u), v), s);
+    // the two z planes as the halves of packed operations
+    auto corner = [&](int lo, int hi) { return pack2(valcoord(lo), valcoord(hi)); };
+    const f32x2 uu = pack2(u, u);
+    float lo, hi;
+    unpack2(lerp2(lerp2(corner(a00 ^ x0, a01 ^ x0), corner(a00 ^ x1, a01 ^ x1), uu),
+                  lerp2(corner(a10 ^ x0, a11 ^ x0), corner(a10 ^ x1, a11 ^ x1), uu), pack2(v, v)), lo, hi);
+    return lerp(lo, hi, s);
 }
 
 FND float value4(int seed, float x, float y, float z, float w)
@@ -760,13 +786,16 @@ FND float value4(int seed, float x, float y, float z, float w)
     int x0 = imul(cvti(xs), kPrimeX), y0 = imul(cvti(ys), kPrimeY), z0 = imul(cvti(zs), kPrimeZ), w0 = imul(cvti(ws), kPrimeW);
     int x1 = iadd(x0, kPrimeX), y1 = iadd(y0, kPrimeY), z1 = iadd(z0, kPrimeZ), w1 = iadd(w0, kPrimeW);
     float u = hermite(x - xs), v = hermite(y - ys), s = hermite(z - zs), q = hermite(w - ws);
-#define V(a, b, c, d) valcoord((seed ^ b ^ c ^ d) ^ a)
-    return lerp(
-        lerp(lerp(lerp(V(x0, y0, z0, w0), V(x1, y0, z0, w0), u), lerp(V(x0, y1, z0, w0), V(x1, y1, z0, w0), u), v),
-             lerp(lerp(V(x0, y0, z1, w0), V(x1, y0, z1, w0), u), lerp(V(x0, y1, z1, w0), V(x1, y1, z1, w0), u), v), s),
-        lerp(lerp(lerp(V(x0, y0, z0, w1), V(x1, y0, z0, w1), u), lerp(V(x0, y1, z0, w1), V(x1, y1, z0, w1), u), v),
-             lerp(lerp(V(x0, y0, z1, w1), V(x1, y0, z1, w1), u), lerp(V(x0, y1, z1, w1), V(x1, y1, z1, w1), u), v), s), q);
-#undef V
+    // the two w planes as the halves of packed operations
+    auto corner = [&](int h) { return pack2(valcoord(h ^ w0), valcoord(h ^ w1)); };
+    auto face = [&](int z) {
+        const f32x2 uu = pack2(u, u);
+        return lerp2(lerp2(corner(seed ^ z ^ y0 ^ x0), corner(seed ^ z ^ y0 ^ x1), uu),
+                     lerp2(corner(seed ^ z ^ y1 ^ x0), corner(seed ^ z ^ y1 ^ x1), uu), pack2(v, v));
+    };
+    float lo, hi;
+    unpack2(lerp2(face(z0), face(z1), pack2(s, s)), lo, hi);
+    return lerp(lo, hi, q);
 }
 
 // ---------------------------------------------------------------- distances (Utils.inl:281-335)
