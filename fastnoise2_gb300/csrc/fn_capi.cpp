@@ -164,11 +164,12 @@ bool pageable_direct(float* p, size_t bytes)
     return at.type == cudaMemoryTypeUnregistered && pageable_direct_supported() && pages_resident(p, bytes);
 }
 
-float* host_direct_view(float* p, size_t bytes)
+float* host_direct_view(float* p, size_t bytes, OutputMemory* memory = nullptr)
 {
     if (!p || !host_direct_allowed()) return nullptr;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (memory) *memory = at.type == cudaMemoryTypeHost ? kPageLocked : kPageable;
     if (at.type == cudaMemoryTypeHost) return pinned_device_view(p, bytes);
     return at.type == cudaMemoryTypeUnregistered && pageable_direct_supported() && pages_resident(p, bytes) ? p : nullptr;
 }
@@ -211,12 +212,12 @@ bool ensure(float*& buf, size_t& cap, size_t n)
 // Launch one generation call: the tree's specialised kernel when one is loaded,
 // the interpreter otherwise.
 cudaError_t launch_points(const DeviceProgram& prog, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax,
-                          cudaStream_t stream)
+                          cudaStream_t stream, OutputMemory memory)
 {
     cudaError_t e;
-    if (jit_launch(prog.hash, args, out, work, dminmax, stream, e)) return e;
+    if (jit_launch(prog.hash, args, out, work, dminmax, stream, e, memory)) return e;
     // the first call on a tree that an earlier process specialised: its kernels from the cache
-    if (args.total > 0 && jit_try_cached(prog.host) && jit_launch(prog.hash, args, out, work, dminmax, stream, e)) return e;
+    if (args.total > 0 && jit_try_cached(prog.host) && jit_launch(prog.hash, args, out, work, dminmax, stream, e, memory)) return e;
     // A tree with per-cell sub-programs cannot run on the interpreter; with no
     // points there is nothing to evaluate and the interpreter only writes min/max.
     if (prog.host->needs_specialisation() && args.total > 0) return cudaErrorNotSupported;
@@ -320,7 +321,9 @@ void gen_host(const void* node, PointArgs args, float* out, float* minmax, const
     // with coherent pageable access): the kernel stores into them directly.  One tree's kernel
     // produces output slower than the host link carries it, so the stores overlap the
     // generation; there is no device buffer, no copy and no slab pipeline to fill and drain.
-    float* direct = total > 0 ? host_direct_view(out, (size_t)total * 4) : nullptr;
+    OutputMemory memory = kDeviceMemory;
+    float* direct = total > 0 ? host_direct_view(out, (size_t)total * 4, &memory) : nullptr;
+    if (!direct) memory = kDeviceMemory;
     if (!work || (!direct && !ensure(ctx->dbuf, ctx->dbuf_cap, (size_t)total))) { fill_nan(out, total, minmax); return; }
     // Position arrays the device can read in place (the same rule as for outputs) are not copied.
     bool pos_direct = args.src == kSrcPositions && total > 0;
@@ -351,7 +354,7 @@ void gen_host(const void* node, PointArgs args, float* out, float* minmax, const
         return;
     }
     // the kernel's last block stores the min/max straight into pinned host memory when it can
-    if (!cuda_ok(launch_points(prog, args, direct ? direct : ctx->dbuf, work, ctx->hminmax_dev, ctx->stream), "launch")) {
+    if (!cuda_ok(launch_points(prog, args, direct ? direct : ctx->dbuf, work, ctx->hminmax_dev, ctx->stream, memory), "launch")) {
         fill_nan(out, total, minmax);
         return;
     }

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 
+#include "fn_jit.h"
 #include "fn_node.h"
 #include "fn_runtime.h"
 #include "fn_types.h"
@@ -22,7 +23,7 @@ PointArgs grid_args(int dim, const float* off, const int* cnt, const float* step
 // Launch one generation call: the tree's specialised kernel when one is loaded,
 // the interpreter otherwise (which may queue the tree for background specialisation).
 cudaError_t launch_points(const DeviceProgram& prog, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax,
-                          cudaStream_t stream);
+                          cudaStream_t stream, OutputMemory memory = kDeviceMemory);
 
 // Specialise trees the interpreter cannot run before their first launch; false (with the
 // error set) when that is impossible.

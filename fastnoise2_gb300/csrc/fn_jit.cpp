@@ -80,6 +80,7 @@ struct ColPlan {
     int regs = 0;                      // registers the states hold
     int table = 0;                     // float4 of shared table per warp
     float setup = 0.0f;                // set-up of a unit, in steps (see below)
+    float step = 0.0f, point = 0.0f;   // issue slots of a step, and of a point of the point kernel
 
     const ColState* at(int pc) const
     {
@@ -113,11 +114,11 @@ ColPlan column_plan(const CompiledProgram& prog)
     // Instructions of setting a state up and of a step of it, and of a step of the other
     // instructions, roughly (from instruction counts of the kernels): their ratio decides how
     // short a unit may be.
-    double setup = 30, step = 15;
+    double setup = 30, step = 15, other = 0, point = 100;
     auto generic_cost = [&](const FnInstr& I) -> double {
         const int d = I.dim - 2;
         static const double simplex[3] = {90, 130, 230}, super[3] = {130, 380, 900}, lattice[3] = {90, 200, 440}, warp[3] = {70, 190, 500},
-                            cells[3] = {200, 700, 2400};
+                            cells[3] = {420, 1300, 2400};
         switch (I.op) {
         case FN_OP_NOISE: return I.aux == FN_NOISE_SIMPLEX ? simplex[d] : I.aux == FN_NOISE_SUPERSIMPLEX ? super[d] : lattice[d];
         case FN_OP_WARP_GRAD: return warp[d];
@@ -244,9 +245,12 @@ ColPlan column_plan(const CompiledProgram& prog)
             break;
         default: set_other(I.dst, 1); break;
         }
-        if (plan.states.size() == had) step += generic_cost(I);
+        if (plan.states.size() == had) other += generic_cost(I);
+        point += generic_cost(I);
     }
-    plan.setup = (float)(setup / step);
+    plan.setup = (float)(setup / (step + other));
+    plan.step = (float)(1.5 * step + other);   // packed operations take two issue slots
+    plan.point = (float)point;
     return plan;
 }
 
@@ -1151,6 +1155,8 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
         JitKernels jk;
         jk.slot = (int)k;
         jk.column_setup = plans[k].setup;
+        jk.column_step = plans[k].step;
+        jk.point_cost = plans[k].point;
         for (auto& st : plans[k].states)
             if (st.type[0] != 'V') jk.column_rates[jk.n_column_rates++] = st.rate;
         cudaKernel_t bk = nullptr;
@@ -1507,12 +1513,25 @@ void column_cut(ColumnShape& s, unsigned len)
     s.units = column_chunks(s) * ((s.steps + s.len - 1) / s.len);
 }
 
-// Steps per unit of a launch that has the GPU to itself: setting a unit up costs
-// `column_setup` steps (about 7 for FBm(Perlin): 256^3 takes 221, 170, 147 us at 8, 16, 32 steps
-// a unit; a fraction of one for a terrain tree), and an SM works on `column_resident` blocks of
-// 8 units at once, so minimise (blocks of the busiest SM, at least the resident ones) x
-// (set-up + length).
-void column_cut_alone(ColumnShape& s, const JitKernels& jk)
+// Cut a launch that has the GPU to itself, and say whether it should be walked in columns at
+// all (false: the point kernel).
+//
+// Steps per unit: setting a unit up costs `column_setup` steps (about 7 for FBm(Perlin): 256^3
+// takes 221, 170, 147 us at 8, 16, 32 steps a unit; a fraction of one for a terrain tree), and an
+// SM works on `column_resident` blocks of 8 units at once, so minimise (blocks of the busiest SM,
+// at least the resident ones) x (set-up + length).
+//
+// Small calls: launches into device memory overlap the launch before them, which a column kernel,
+// with its longer set-up and its registers, does worse (about 4 us a launch to 3).  Back to back,
+// point / column kernel, us: FBm(Perlin) 32^3 3.3 / 7.2, 64^3 7.1 / 9.8, 96^3 19.9 / 14.0;
+// CellularValue 32^3 3.4 / 4.7, 64^3 9.0 / 6.6; terrain 64^3 21.5 / 26.7, 96^3 71 / 55; Value 768^2
+// 3.8 / 4.6.  So both are estimated from their instruction counts.
+//
+// Host outputs: the caller waits for each, so what counts is the length of one warp's work (us of
+// the call: CellularValue 32^3 22.2 / 19.5, FBm(Perlin) 48^3 22.9 / 24.7), and large ones in pageable
+// memory run at the host link, which a column's short rows use less well than the point kernel's
+// runs of 512 bytes (Value 128^3 67 / 77, CellularValue 81 / 77, terrain 205 / 144).
+bool column_cut_alone(ColumnShape& s, const JitKernels& jk, OutputMemory memory)
 {
     const unsigned n = s.steps, chunks = column_chunks(s), slots = 8u * (unsigned)num_sms(),
                    fill = (unsigned)std::max(1, jk.column_resident);
@@ -1526,7 +1545,21 @@ void column_cut_alone(ColumnShape& s, const JitKernels& jk)
         if (cost < best_cost) { best_cost = cost; best = len; }
         if (len == 1) break;
     }
+    // microseconds, at ~9000 warp instructions per SM and microsecond, or ~500 of one warp
+    const float points = (float)s.plane * (float)s.steps;
+    float point_us = points / 32.0f * jk.point_cost / (9000.0f * (float)num_sms());
+    float column_us = best_cost * 8.0f * jk.column_step / 9000.0f;
+    if (memory == kDeviceMemory) {
+        point_us = std::max(point_us, 3.0f);
+        column_us += 4.0f;
+    } else {
+        point_us = std::max(point_us, jk.point_cost / 500.0f);
+        column_us = std::max(column_us, (jk.column_setup + (float)best) * jk.column_step / 500.0f) + 0.7f;
+        if (memory == kPageable) column_us = std::max(column_us, points * 4.0f / 130e3f);
+    }
+    if (!(column_us < point_us)) return false;
     column_cut(s, best);
+    return true;
 }
 
 }  // namespace
@@ -1566,15 +1599,14 @@ cudaError_t launch_overlapped(cudaKernel_t k, unsigned grid, void** params, cuda
 }
 
 bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax, cudaStream_t stream,
-                cudaError_t& err)
+                cudaError_t& err, OutputMemory memory)
 {
     err = cudaSuccess;
     JitKernels jk;
     if (args.total <= 0 || args.total > (1ll << 31) || !jit_lookup(hash, jk)) return false;
     const int which = args.src == kSrcGrid ? 0 : args.src == kSrcPositions ? 1 : 2;
     ColumnShape shape;
-    if (which == 0 && jit_column_grid(args, jk, shape)) {
-        column_cut_alone(shape, jk);
+    if (which == 0 && jit_column_grid(args, jk, shape) && column_cut_alone(shape, jk, memory)) {
         PointArgs c = args;
         column_args(c, shape);
         const unsigned grid = std::min<unsigned>((shape.units + 7) / 8, (unsigned)kMaxReduceBlocks);

@@ -41,6 +41,7 @@ struct JitKernels {
     ColumnRate column_rates[kMaxColumnStates];   // of its Perlin and cellular states
     int n_column_rates = 0;
     float column_setup = 1.0f;        // set-up of a unit of columns, in steps
+    float column_step = 1.0f, point_cost = 1.0f;   // instructions of a step of a column, of a point otherwise
     int column_resident = 1;          // its 256-thread blocks per SM at once
     int slot = -1;                    // index in the module's batch kernel
     int resident[3] = {1, 1, 1};      // 256-thread blocks per SM of grid / positions / tileable at once
@@ -115,11 +116,14 @@ void jit_request_batch_variants(const CompiledProgram* prog);
 // Kernels for a program hash, or false if none have been built.
 bool jit_lookup(uint64_t hash, JitKernels& out);
 
+// Where a kernel stores its output: device memory, or host memory that it writes directly.
+enum OutputMemory { kDeviceMemory, kPageLocked, kPageable };
+
 // Launch the specialised per-call kernel for `hash` if one is loaded (and JIT
 // is enabled); returns false when the caller should use the interpreter.
 // `err` carries the launch status when true is returned.
 bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax, cudaStream_t stream,
-                cudaError_t& err);
+                cudaError_t& err, OutputMemory memory = kDeviceMemory);
 
 // Chunk meshing with a specialised 3D tree (false when none is loaded): bit i of `above` /
 // `solid` = grid point i's value is > iso / <= iso (both 0 for NaN), and OutputMinMax into

@@ -3,7 +3,9 @@ can go wrong -- planes and columns that are no multiple of a warp, of the 32-ste
 unit, cells entered upwards, downwards, skipped or never left, and positions without a cell."""
 import numpy as np
 import pytest
+import torch
 
+import fastnoise2_gb300 as fn
 from oracle.oracle import OracleTree
 from oracle.tree import N
 from tests import trees
@@ -68,3 +70,30 @@ def test_columns_of_extreme_positions(columns, name):
             got, mm = columns[name].gen_uniform_grid(off, (9, 5, 35), (1.0, 1.0, 1.0), -5)
             ref, rmm = oracle.grid(off, (9, 5, 35), (1.0, 1.0, 1.0), -5)
             assert_parity(got, mm, ref, rmm, label=f"{name} {off}")
+
+
+@pytest.mark.parametrize("dim", [2, 3, 4])
+@pytest.mark.parametrize("name", sorted(TREES))
+def test_columns_of_a_batch_match_the_oracle(columns, name, dim):
+    """A batch walks grids of every size in columns; a call of its own does so only where that
+    is the faster route."""
+    oracle = OracleTree(TREES[name]())
+    off = (-7.5, 3.25, -11.0, 2.0)[:dim]
+    grids = [(shape, step) for shape in SHAPES[dim] for step in STEPS]
+    outs = [torch.full((int(np.prod(shape)),), np.nan, device="cuda") for shape, _ in grids]
+    kind = {2: fn.KIND_GRID2D, 3: fn.KIND_GRID3D, 4: fn.KIND_GRID4D}[dim]
+    fn.gen_batch([fn.make_request(columns[name], kind, out.data_ptr(), 77, shape, off, step[:dim])
+                  for out, (shape, step) in zip(outs, grids)])
+    for out, (shape, step) in zip(outs, grids):
+        ref, rmm = oracle.grid(off, shape, step[:dim], 77)
+        assert_parity(out.cpu().numpy(), rmm, ref, rmm, label=f"{name} {shape} {step}")
+
+
+@pytest.mark.parametrize("name", sorted(TREES))
+@pytest.mark.parametrize("shape", [(1003, 1001), (97, 90, 101), (23, 21, 29, 65)])
+def test_calls_large_enough_for_columns(columns, name, shape):
+    oracle = OracleTree(TREES[name]())
+    off, step = (-7.5, 3.25, -11.0, 2.0)[:len(shape)], (1.0, 0.37, -0.9, 1.3)[:len(shape)]
+    got, mm = columns[name].gen_uniform_grid(off, shape, step, 5)
+    ref, rmm = oracle.grid(off, shape, step, 5)
+    assert_parity(got, mm, ref, rmm, label=f"{name} {shape}")
