@@ -20,26 +20,29 @@ using namespace fn::capi;
 namespace {
 
 // Device scratch of one mesher lane: densities, their min/max, the bloxel scan buffers
-// and the dual marching cubes buffers, plus a pinned read-back area for single calls.
-// Single-chunk calls use the thread's lane on the caller's stream; multi-chunk calls
-// spread their chunks over kMeshLanes lanes with their own streams.
+// and the dual marching cubes buffers, plus a pinned read-back area.  Single-chunk calls and
+// multi-chunk dual marching cubes calls use the thread's lane on the caller's stream; other
+// multi-chunk calls spread their chunks over kMeshLanes lanes with their own streams.
 struct MeshCtx {
     float* dens = nullptr;
     size_t dens_cap = 0;
-    // What a chunk reports, read back in one copy: words 0.. the mesher's totals and heights
+    // What a chunk reports in 8 words, read back in one copy: words 0.. the mesher's totals and heights
     // (bloxel faces, air, solid; DMC vertices, quads, air, solid), words 4, 5 OutputMinMax.
     unsigned* result = nullptr;
     float* dminmax = nullptr;          // in result
     MeshScratch scratch;
     DmcScratch dmc;
+    char* dmc_block = nullptr;         // its arrays
+    size_t dmc_cap = 0;
     SparseScratch sp;                  // the sparse density form (trees with specialised kernels)
-    unsigned* host = nullptr;          // pinned read-back of one chunk (see enqueue_chunk)
+    unsigned* host = nullptr;          // pinned read-back, 8 words per chunk
+    size_t host_cap = 0;               // chunks
     ~MeshCtx()
     {
         if (dens) cudaFree(dens);
         if (result) cudaFree(result);
         if (scratch.counts) cudaFree(scratch.counts);
-        if (dmc.offsets) cudaFree(dmc.offsets);
+        if (dmc_block) cudaFree(dmc_block);
         if (sp.stored) cudaFree(sp.stored);
         if (host) cudaFreeHost(host);
     }
@@ -78,10 +81,9 @@ struct MeshCtx {
     bool reserve(size_t densities, size_t voxels)
     {
         if (!result) {
-            if (!cuda_ok(cudaMalloc(&result, 8 * sizeof(unsigned)), "cudaMalloc(mesh result)")) return false;
+            if (!cuda_ok(cudaMalloc(&result, 8 * kDmcChunks * sizeof(unsigned)), "cudaMalloc(mesh result)")) return false;
             dminmax = reinterpret_cast<float*>(result + 4);
         }
-        if (!host && !cuda_ok(cudaMallocHost(&host, 8 * sizeof(unsigned)), "cudaMallocHost(mesh read-back)")) return false;
         if (densities > dens_cap) {
             if (dens) cudaFree(dens);
             dens = nullptr; dens_cap = 0;
@@ -104,32 +106,29 @@ struct MeshCtx {
         return true;
     }
 
-    bool reserve_dmc(int size)
+    bool reserve_dmc(int size, unsigned chunks)
     {
-        const size_t cells = (size_t)size * size * size, vcells = (size_t)(size + 1) * (size + 1) * (size + 1);
-        if (cells <= dmc.cap_cells) return true;
-        if (dmc.offsets) cudaFree(dmc.offsets);
-        dmc = DmcScratch();
-        const size_t tiles = (cells + 2047) / 2048;
-        // uint2: offsets | tile sums; uint32: masks | list counters | vertex items | quad items;
-        // then cases and cut axes (uint8)
-        const size_t pairs = cells + tiles, words = cells + 2 + 4 * vcells + 3 * cells;
-        char* block = nullptr;
-        if (!cuda_ok(cudaMalloc(&block, pairs * sizeof(uint2) + words * sizeof(unsigned) + vcells + cells), "cudaMalloc(dmc scratch)"))
-            return false;
-        uint2* p = reinterpret_cast<uint2*>(block);
-        dmc.offsets = p;
-        dmc.tile_sums = p + cells;
-        dmc.total = reinterpret_cast<uint2*>(result);
-        unsigned* w = reinterpret_cast<unsigned*>(p + pairs);
-        dmc.masks = w;
-        dmc.airsolid = result + 2;
-        dmc.counters = w + cells;
-        dmc.vert_items = w + cells + 2;
-        dmc.quad_items = w + cells + 2 + 4 * vcells;
-        dmc.cases = reinterpret_cast<unsigned char*>(w + words);
-        dmc.cell_axes = dmc.cases + vcells;
-        dmc.cap_cells = cells;
+        const size_t bytes = dmc_scratch(size, chunks, dmc_block, dmc);
+        if (bytes > dmc_cap) {
+            if (dmc_block) cudaFree(dmc_block);
+            dmc_block = nullptr;
+            dmc_cap = 0;
+            if (!cuda_ok(cudaMalloc(&dmc_block, bytes), "cudaMalloc(dmc scratch)")) return false;
+            dmc_cap = bytes;
+            dmc_scratch(size, chunks, dmc_block, dmc);
+        }
+        dmc.result = result;
+        return true;
+    }
+
+    bool reserve_host(size_t chunks)
+    {
+        if (chunks <= host_cap) return true;
+        if (host) cudaFreeHost(host);
+        host = nullptr;
+        host_cap = 0;
+        if (!cuda_ok(cudaMallocHost(&host, chunks * 8 * sizeof(unsigned)), "cudaMallocHost(mesh read-back)")) return false;
+        host_cap = chunks;
         return true;
     }
 };
@@ -137,6 +136,7 @@ thread_local MeshCtx t_mesh;
 
 // FN_MESH_DENSITY_ARRAY (default) or FN_MESH_DENSITY_SPARSE (fnSetMeshDensityForm).
 std::atomic<int> g_mesh_form{FN_MESH_DENSITY_ARRAY};
+bool sparse_form() { return g_mesh_form.load(std::memory_order_relaxed) == FN_MESH_DENSITY_SPARSE; }
 
 constexpr int kMeshLanes = 4;
 
@@ -189,31 +189,43 @@ bool mesh_args_ok(int size, const fnChunkMesh* mesh)
     return mesh && size >= 1 && size <= 256 && mesh->vertexCapacity >= 0 && mesh->indexCapacity >= 0;
 }
 
-// Queue one chunk on `s` with lane `m`: its densities (GenPositionArray3D over the editor's
-// grid positions offset by the chunk position -- MeshNoisePreview.cpp:447-455 bloxel, -1 ..
-// size; :594-603 DMC, -2 .. size+1 -- as a grid of the same exact integer-valued floats; with
-// the z axis up, y and z swap roles), the mesher, and the read-back into host8: bloxel
-// [faces, air, solid], DMC [vertices, quads, air, solid]; [4..5] OutputMinMax.
-bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStream_t s, int size, int px, int py, int pz,
+// A chunk's densities: GenPositionArray3D over the editor's grid positions offset by the chunk
+// position (MeshNoisePreview.cpp:447-455 bloxel, -1 .. size; :594-603 DMC, -2 .. size+1) as a grid
+// of the same exact integer-valued floats; with the z axis up, y and z swap roles.
+int density_side(MeshKind kind, int size) { return size + (kind == kDmc ? 4 : 2); }
+PointArgs density_args(MeshKind kind, int size, const int* p, int seed, int upAxisZ)
+{
+    const int apron = kind == kDmc ? 2 : 1, sg = density_side(kind, size);
+    const float off[3] = {(float)(p[0] - apron), (float)(p[upAxisZ ? 2 : 1] - apron), (float)(p[upAxisZ ? 1 : 2] - apron)};
+    const int cnt[3] = {sg, sg, sg};
+    const float step[3] = {1, 1, 1};
+    return grid_args(3, off, cnt, step, seed);
+}
+
+DmcChunk dmc_chunk(const int* p, const fnChunkMesh& mesh)
+{
+    return DmcChunk{p[0], p[1], p[2], (unsigned)mesh.vertexCapacity, (unsigned)mesh.indexCapacity,
+                    reinterpret_cast<MeshVertex*>(mesh.vertices), mesh.indices};
+}
+
+// Queue one chunk on `s` with lane `m`: its densities, the mesher, and the read-back into host8:
+// bloxel [faces, air, solid], DMC [vertices, quads, air, solid]; [4..5] OutputMinMax.
+bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStream_t s, int size, const int* p,
                    int seed, float iso, int upAxisZ, const fnChunkMesh* mesh, unsigned* host8)
 {
-    const int apron = kind == kDmc ? 2 : 1;
-    const int sg = size + 2 * apron;
+    const int sg = density_side(kind, size), px = p[0], py = p[1], pz = p[2];
     const size_t n_dens = (size_t)sg * sg * sg;
     MinMaxWork* work = work_for_stream(s);
     if (!work) return false;
-    const float off[3] = {(float)(px - apron), (float)((upAxisZ ? pz : py) - apron), (float)((upAxisZ ? py : pz) - apron)};
-    const int cnt[3] = {sg, sg, sg};
-    const float step[3] = {1, 1, 1};
-    const PointArgs args = grid_args(3, off, cnt, step, seed);
+    const PointArgs args = density_args(kind, size, p, seed, upAxisZ);
     // The density array (default): the tree's kernel writes every density of the chunk (9 MB
     // for the editor's 128^3, which stays in L2 between generation and meshing).  The sparse
     // form (fnSetMeshDensityForm, trees with specialised kernels): the densities stay in
     // registers, only their classification against the iso level is stored, and the exact
     // values the passes read are evaluated again at those voxels only.
     bool sparse = false;
-    if (g_mesh_form.load(std::memory_order_relaxed) == FN_MESH_DENSITY_SPARSE && jit_enabled()) {
-        if (!m.reserve(0, kind == kBloxel ? (size_t)size * size * size : 0) || (kind == kDmc && !m.reserve_dmc(size)) ||
+    if (sparse_form() && jit_enabled()) {
+        if (!m.reserve(0, kind == kBloxel ? (size_t)size * size * size : 0) || (kind == kDmc && !m.reserve_dmc(size, 1)) ||
             !m.reserve_sparse(n_dens))
             return false;
         cudaError_t err = cudaSuccess;
@@ -221,7 +233,7 @@ bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStr
         if (sparse && !cuda_ok(err, "densities (classification)")) return false;
     }
     if (!sparse) {
-        if (!m.reserve(n_dens, kind == kBloxel ? (size_t)size * size * size : 0) || (kind == kDmc && !m.reserve_dmc(size)))
+        if (!m.reserve(n_dens, kind == kBloxel ? (size_t)size * size * size : 0) || (kind == kDmc && !m.reserve_dmc(size, 1)))
             return false;
         if (!cuda_ok(launch_points(prog, args, m.dens, work, m.dminmax, s), "densities")) return false;
     }
@@ -244,18 +256,54 @@ bool enqueue_chunk(MeshKind kind, const DeviceProgram& prog, MeshCtx& m, cudaStr
                              "bloxel mesher");
         if (!queued) return false;
     } else {
+        const DmcChunk chunk = dmc_chunk(p, *mesh);
         const bool queued =
-            sparse ? cuda_ok(launch_dmc_sparse_prepare(m.sp, size, upAxisZ != 0, iso, m.dminmax, m.dmc, s), "dual marching cubes mesher") &&
+            sparse ? cuda_ok(launch_dmc_sparse_prepare(m.sp, size, upAxisZ != 0, iso, m.dmc, s), "dual marching cubes mesher") &&
                          needed_values() &&
-                         cuda_ok(launch_dmc_sparse_finish(m.sp, size, upAxisZ != 0, px, py, pz, iso, m.dmc, verts,
-                                                          (unsigned)mesh->vertexCapacity, mesh->indices, (unsigned)mesh->indexCapacity, s),
-                                 "dual marching cubes mesher")
-                   : cuda_ok(launch_dmc(m.dens, size, upAxisZ != 0, px, py, pz, iso, m.dminmax, m.dmc, verts,
-                                        (unsigned)mesh->vertexCapacity, mesh->indices, (unsigned)mesh->indexCapacity, s),
-                             "dual marching cubes mesher");
+                         cuda_ok(launch_dmc_sparse_finish(m.sp, size, upAxisZ != 0, iso, chunk, m.dmc, s), "dual marching cubes mesher")
+                   : cuda_ok(launch_dmc(m.dens, n_dens, size, upAxisZ != 0, iso, &chunk, 1, m.dmc, s), "dual marching cubes mesher");
         if (!queued) return false;
     }
     return cuda_ok(cudaMemcpyAsync(host8, m.result, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read back");
+}
+
+// Dual marching cubes chunks meshed together: their densities one after another, then each pass
+// over all of them (fn_mesh.cu, DmcPass).  As many at once as hold 8 * 128^3 cells (0.8 GB of
+// scratch for 128^3 chunks), at least 4, so that the scratch of larger chunks is that of the four
+// lanes a chunk each would take.
+bool enqueue_dmc_chunks(const DeviceProgram& prog, MeshCtx& m, cudaStream_t s, int size, int count, const int* positions, int seed,
+                        float iso, int upAxisZ, const fnChunkMesh* meshes, unsigned* host)
+{
+    const long long cells = (long long)size * size * size;
+    const int most = (int)std::min<long long>(kDmcChunks, std::max<long long>(4, 8ll * 128 * 128 * 128 / cells));
+    const int groups = (count + most - 1) / most;
+    int group = (count + groups - 1) / groups;
+    const int sg = density_side(kDmc, size);
+    const size_t stride = ((size_t)sg * sg * sg + 31) / 32 * 32;
+    MinMaxWork* work = work_for_stream(s);
+    if (!work) return false;
+    while (!m.reserve(stride * group, 0) || !m.reserve_dmc(size, (unsigned)group)) {
+        if (group == 1) return false;
+        group = (group + 1) / 2;                // no memory for so many: fewer together
+        cudaGetLastError();
+        clear_error();
+    }
+    for (int first = 0; first < count; first += group) {
+        const int n = std::min(group, count - first);
+        DmcChunk chunks[kDmcChunks];
+        for (int k = 0; k < n; ++k) {
+            const int* p = positions + 3 * (size_t)(first + k);
+            chunks[k] = dmc_chunk(p, meshes[first + k]);
+            if (!cuda_ok(launch_points(prog, density_args(kDmc, size, p, seed, upAxisZ), m.dens + stride * k, work, m.dminmax + 8 * k, s),
+                         "densities"))
+                return false;
+        }
+        if (!cuda_ok(launch_dmc(m.dens, stride, size, upAxisZ != 0, iso, chunks, (unsigned)n, m.dmc, s), "dual marching cubes mesher") ||
+            !cuda_ok(cudaMemcpyAsync(host + 8 * (size_t)first, m.result, 8 * (size_t)n * sizeof(unsigned), cudaMemcpyDeviceToHost, s),
+                     "read back"))
+            return false;
+    }
+    return true;
 }
 
 // Fill a chunk's results from its read-back (after the stream has finished); FN_OK or
@@ -292,15 +340,37 @@ int build_chunk_mesh(MeshKind kind, const void* node, int size, int px, int py, 
     if (!ensure_runnable(prog)) return FN_ERR_COMPILE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     MeshCtx& m = t_mesh;
-    if (!m.reserve(0, 0)) return FN_ERR_CUDA;
-    if (!enqueue_chunk(kind, prog, m, s, size, px, py, pz, seed, iso, upAxisZ, mesh, m.host) ||
+    if (!m.reserve(0, 0) || !m.reserve_host(1)) return FN_ERR_CUDA;
+    const int p[3] = {px, py, pz};
+    if (!enqueue_chunk(kind, prog, m, s, size, p, seed, iso, upAxisZ, mesh, m.host) ||
         !cuda_ok(cudaStreamSynchronize(s), "synchronize"))
         return FN_ERR_CUDA;
     return finish_chunk(kind, size, py, iso, m.host, mesh);
 }
 
-// Many chunks: chunk i runs on lane i % kMeshLanes, so the short, latency-bound mesher
-// kernels of neighbouring chunks overlap; the caller's stream orders the whole call.
+bool enqueue_on_lanes(MeshKind kind, const DeviceProgram& prog, MeshLanes& l, cudaStream_t s, int size, int count,
+                      const int* positions, int seed, float iso, int upAxisZ, const fnChunkMesh* meshes)
+{
+    if (!cuda_ok(cudaEventRecord(l.fork, s), "record")) return false;
+    const int lanes = std::min(count, kMeshLanes);
+    for (int k = 0; k < lanes; ++k)
+        if (!cuda_ok(cudaStreamWaitEvent(l.stream[k], l.fork, 0), "wait")) return false;
+    for (int i = 0; i < count; ++i) {
+        const int k = i % kMeshLanes;
+        const int* p = positions + 3 * (size_t)i;
+        if (!enqueue_chunk(kind, prog, l.lane[k], l.stream[k], size, p, seed, iso, upAxisZ, meshes + i,
+                           l.host + 8 * (size_t)i))
+            return false;
+    }
+    for (int k = 0; k < lanes; ++k)
+        if (!cuda_ok(cudaEventRecord(l.join[k], l.stream[k]), "record") || !cuda_ok(cudaStreamWaitEvent(s, l.join[k], 0), "wait"))
+            return false;
+    return true;
+}
+
+// Many chunks.  Dual marching cubes on density arrays: together on the caller's stream.  Else
+// chunk i runs on lane i % kMeshLanes, so the short, latency-bound mesher kernels of
+// neighbouring chunks overlap; the caller's stream orders the whole call.
 int build_chunk_meshes(MeshKind kind, const void* node, int size, int count, const int* positions, int seed, float iso,
                        int upAxisZ, fnChunkMesh* meshes, void* stream)
 {
@@ -313,27 +383,23 @@ int build_chunk_meshes(MeshKind kind, const void* node, int size, int count, con
     DeviceProgram prog;
     if (!get_program(N(node), 3, prog)) return last_error();
     if (!ensure_runnable(prog)) return FN_ERR_COMPILE;
-    MeshLanes* l = mesh_lanes((size_t)count);
-    if (!l) return FN_ERR_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!cuda_ok(cudaEventRecord(l->fork, s), "record")) return FN_ERR_CUDA;
-    const int lanes = std::min(count, kMeshLanes);
-    for (int k = 0; k < lanes; ++k)
-        if (!cuda_ok(cudaStreamWaitEvent(l->stream[k], l->fork, 0), "wait")) return FN_ERR_CUDA;
-    for (int i = 0; i < count; ++i) {
-        const int k = i % kMeshLanes;
-        const int* p = positions + 3 * (size_t)i;
-        if (!enqueue_chunk(kind, prog, l->lane[k], l->stream[k], size, p[0], p[1], p[2], seed, iso, upAxisZ, meshes + i,
-                           l->host + 8 * (size_t)i))
+    const unsigned* host = nullptr;
+    if (kind == kDmc && !(sparse_form() && jit_enabled())) {
+        MeshCtx& m = t_mesh;
+        if (!m.reserve(0, 0) || !m.reserve_host((size_t)count) ||
+            !enqueue_dmc_chunks(prog, m, s, size, count, positions, seed, iso, upAxisZ, meshes, m.host))
             return FN_ERR_CUDA;
+        host = m.host;
+    } else {
+        MeshLanes* l = mesh_lanes((size_t)count);
+        if (!l || !enqueue_on_lanes(kind, prog, *l, s, size, count, positions, seed, iso, upAxisZ, meshes)) return FN_ERR_CUDA;
+        host = l->host;
     }
-    for (int k = 0; k < lanes; ++k)
-        if (!cuda_ok(cudaEventRecord(l->join[k], l->stream[k]), "record") || !cuda_ok(cudaStreamWaitEvent(s, l->join[k], 0), "wait"))
-            return FN_ERR_CUDA;
     if (!cuda_ok(cudaStreamSynchronize(s), "synchronize")) return FN_ERR_CUDA;
     int rc = FN_OK;
     for (int i = 0; i < count; ++i) {
-        const int r = finish_chunk(kind, size, positions[3 * (size_t)i + 1], iso, l->host + 8 * (size_t)i, meshes + i);
+        const int r = finish_chunk(kind, size, positions[3 * (size_t)i + 1], iso, host + 8 * (size_t)i, meshes + i);
         if (r != FN_OK && rc == FN_OK) rc = r;
     }
     if (rc != FN_OK) set_error(rc, "at least one chunk's mesh did not fit its buffers (see its counts)");

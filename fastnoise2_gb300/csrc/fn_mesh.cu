@@ -17,9 +17,12 @@
 // to twelve cut edges, numbered in the order the reference's hash map first sees
 // it; here every reference to a vertex finds its first use directly (the lowest
 // cell / axis / slot among the quads that use it), so the count pass marks the
-// creating references, a scan numbers them, and the quads look their vertices up
-// without a map.
+// creating references and numbers them tile by tile, a scan over the tiles makes
+// the numbers final, and the quads look their vertices up without a map.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "fn_mesh.h"
 
@@ -44,6 +47,8 @@ __device__ __forceinline__ unsigned enc(float f)
 // neither above nor at-or-below the iso level in both forms.
 struct DenseSrc {
     const float* d;
+    size_t stride = 0;       // from one chunk's densities to the next, where several are meshed together
+    __device__ __forceinline__ DenseSrc of_chunk(unsigned c) const { return DenseSrc{d + c * stride, stride}; }
     __device__ __forceinline__ bool above(int i, float iso) const { return d[i] > iso; }
     __device__ __forceinline__ bool solid(int i, float iso) const { return d[i] <= iso; }
     __device__ __forceinline__ float value(int i) const { return d[i]; }
@@ -54,6 +59,7 @@ struct SparseSrc {
     const unsigned* le;      // bit i: density i <= iso
     const uint2* stored;     // per 32 densities: (values stored before them, bit k: density 32w + k is stored)
     const float* vals;
+    __device__ __forceinline__ SparseSrc of_chunk(unsigned) const { return *this; }      // always meshed alone
     __device__ __forceinline__ bool above(int i, float) const { return (__ldg(&gt[i >> 5]) >> (i & 31)) & 1u; }
     __device__ __forceinline__ bool solid(int i, float) const { return (__ldg(&le[i >> 5]) >> (i & 31)) & 1u; }
     __device__ __forceinline__ float value(int i) const
@@ -524,22 +530,6 @@ __device__ __forceinline__ unsigned dmc_case_at(const DmcGrid<S>& g, int x, int 
     return g.cases[((unsigned)(z + 1) * s1 + (unsigned)(y + 1)) * s1 + (unsigned)(x + 1)];
 }
 
-// DmcGetVertIndex's cell code (:774-790)
-template <class S>
-__device__ __forceinline__ unsigned dmc_case(const DmcGrid<S>& g, int i, float iso)
-{
-    unsigned c = 0;
-    c |= g.src.above(i, iso) ? 1u : 0u;
-    c |= g.src.above(i + g.sx, iso) ? 2u : 0u;
-    c |= g.src.above(i + g.sy, iso) ? 4u : 0u;
-    c |= g.src.above(i + g.sx + g.sy, iso) ? 8u : 0u;
-    c |= g.src.above(i + g.sz, iso) ? 16u : 0u;
-    c |= g.src.above(i + g.sx + g.sz, iso) ? 32u : 0u;
-    c |= g.src.above(i + g.sy + g.sz, iso) ? 64u : 0u;
-    c |= g.src.above(i + g.sx + g.sy + g.sz, iso) ? 128u : 0u;
-    return c;
-}
-
 // cut edges from a cell's base corner: bit 0 x (corners 0-1), bit 1 y (0-2), bit 2 z (0-4)
 __device__ __forceinline__ unsigned dmc_axes(unsigned c)
 {
@@ -551,39 +541,32 @@ __device__ __forceinline__ int dmc_slot_offset(int a, int s, int k)
     return -((k == (a + 2) % 3 ? (s & 1) : 0) + (k == (a + 1) % 3 ? (s >> 1) & 1 : 0));
 }
 
-template <class S>
-__device__ __forceinline__ unsigned dmc_key(const DmcGrid<S>& g, unsigned cx, unsigned cy, unsigned cz, unsigned slot)
-{
-    const unsigned n = (unsigned)g.size;
-    return ((cz * n + cy) * n + cx) * 12u + slot;
-}
+// run-time look-ups of dmc_slot_edge (slot = axis * 4 + s), dmc_use_off (bits x, y, z) and dmc_use_slot
+__device__ __forceinline__ unsigned dmc_slot_edge_of(unsigned slot) { return (unsigned)(kDmcSlotEdges >> (4u * slot)) & 0xFu; }
+__device__ __forceinline__ unsigned dmc_use_offset(unsigned e) { return (unsigned)(kDmcUseOffs >> (3u * e)) & 7u; }
+__device__ __forceinline__ unsigned dmc_use_slot_of(unsigned e) { return (unsigned)(kDmcUseSlots >> (4u * e)) & 0xFu; }
 
-// The first quad (in the reference's cell / axis / slot order) that uses the dual vertex
-// (cell w, piece p of case c), as cell index * 12 + axis * 4 + slot: that quad's
-// DmcGetVertIndex call is the one that creates the vertex in the reference's map.  Away
-// from the chunk's faces every quad around w lies in the chunk and the table knows the
-// first; next to them the quads that fall outside are skipped.
+// The edge (of vertex cell w) whose quad is the first in the reference's cell / axis / slot order
+// that uses the dual vertex (w, piece p of case c): that quad's DmcGetVertIndex call is the
+// one that creates the vertex in the reference's map.  Away from the chunk's faces every quad around
+// w lies in the chunk and the table knows the first; next to them the quads that fall outside are
+// skipped.
 template <class S>
-__device__ __forceinline__ unsigned dmc_first_use(const DmcGrid<S>& g, int wx, int wy, int wz, unsigned c, unsigned p)
+__device__ __forceinline__ unsigned dmc_first_edge(const DmcGrid<S>& g, int wx, int wy, int wz, unsigned c, unsigned p)
 {
     const unsigned n = (unsigned)g.size;
-    if ((unsigned)wx < n - 1u && (unsigned)wy < n - 1u && (unsigned)wz < n - 1u) {
-        const int e = __ldg(&kDmc.first[c][p]);
-        const unsigned off = (unsigned)(kDmcUseOffs >> (3 * e)) & 7u;
-        return dmc_key(g, (unsigned)wx + (off & 1u), (unsigned)wy + ((off >> 1) & 1u), (unsigned)wz + (off >> 2),
-                       (unsigned)(kDmcUseSlots >> (4 * e)) & 0xFu);
-    }
-    unsigned best = 0xFFFFFFFFu;
+    if ((unsigned)wx < n - 1u && (unsigned)wy < n - 1u && (unsigned)wz < n - 1u) return __ldg(&kDmc.first[c][p]);
+    unsigned best = 0xFFFFFFFFu, edge = 0u;
     for (unsigned m = __ldg(&kDmc.code[c][p]); m; m &= m - 1u) {
-        const int e = __ffs(m) - 1;
-        const unsigned off = (unsigned)(kDmcUseOffs >> (3 * e)) & 7u;
+        const unsigned e = (unsigned)__ffs(m) - 1u;
+        const unsigned off = dmc_use_offset(e);
         const unsigned cx = (unsigned)(wx + (int)(off & 1u)), cy = (unsigned)(wy + (int)((off >> 1) & 1u)),
                        cz = (unsigned)(wz + (int)(off >> 2));
         if (cx >= n || cy >= n || cz >= n) continue;                // also catches -1
-        const unsigned key = dmc_key(g, cx, cy, cz, (unsigned)(kDmcUseSlots >> (4 * e)) & 0xFu);
-        best = key < best ? key : best;
+        const unsigned key = ((cz * n + cy) * n + cx) * 12u + dmc_use_slot_of(e);
+        if (key < best) { best = key; edge = e; }
     }
-    return best;
+    return edge;
 }
 
 // One quad reference: vertex cell w of slot (a, s) of cell (x, y, z), its case and piece.
@@ -600,8 +583,8 @@ __device__ __forceinline__ DmcRef dmc_ref(const DmcGrid<S>& g, int x, int y, int
     r.wy = y + dmc_slot_offset(a, s, 1);
     r.wz = z + dmc_slot_offset(a, s, 2);
     r.c = dmc_case_at(g, r.wx, r.wy, r.wz);
-    const int e = (int)((kDmcSlotEdges >> (4 * (a * 4 + s))) & 0xFu);
-    r.p = (unsigned)(__ldg(&kDmc.edge_piece[r.c]) >> (4 * e)) & 0xFu;    // the piece holding e (:792-800)
+    const unsigned e = dmc_slot_edge_of((unsigned)(a * 4 + s));
+    r.p = (unsigned)(__ldg(&kDmc.edge_piece[r.c]) >> (4u * e)) & 0xFu;    // the piece holding e (:792-800)
     return r;
 }
 
@@ -632,7 +615,7 @@ __device__ __forceinline__ float3 dmc_point(const DmcGrid<S>& g, int i, unsigned
 }
 
 // NormaliseConstExpr(-LIGHT_DIR) (:21-30): Newton square root until it repeats
-__device__ __forceinline__ float3 dmc_light_dir()
+float3 dmc_light_dir()
 {
     const float x = -kLightX, y = -kLightY, z = -kLightZ;
     const float len2 = x * x + y * y + z * z;
@@ -699,16 +682,66 @@ __device__ __forceinline__ float dmc_light(const DmcGrid<S>& g, int i, float3 v,
     return light < 1.0f ? light : 1.0f;                        // std::min(1.0f, light): NaN -> 1
 }
 
-// Cell counts are scanned in tiles of 2048 cells; the tile sums are accumulated with
-// atomics by the passes that produce the counts, so the scan reads each count once.
-constexpr int kDmcTile = 2048;             // (dmc_cases shifts by 11)
+// Cells are counted and numbered in tiles of 2048.
+constexpr unsigned kDmcTile = 2048;
 
-// Work lists, appended warp by warp.
+// Work lists: a tile's vertices and quads one after another in order, the tiles in any order.
 struct DmcLists {
     unsigned* vert_items;   // packed cell | slot bit << 24, one per vertex
-    unsigned* quad_items;   // packed cell | axis << 24, one per quad
-    unsigned* counters;     // [0] vertex items, [1] quad items
-    uint2* tile_sums;       // per 2048 cells: vertices, quads; then scanned in place
+    unsigned* quad_items;   // packed cell | axis << 24 | (cell's base corner at or below the iso level) << 26, one per quad
+    unsigned short* quad_refs;   // its 4 vertices' dmc_first_edge, 4 bits each
+    unsigned* counters;     // [0] vertex items, [kDmcLine] quad items
+};
+constexpr unsigned kDmcLine = 32;          // words between counters
+
+// What the passes of one chunk work on.  A pass runs over all chunks of a call at once (chunk =
+// blockIdx.y): one after another, a chunk's passes are too short to fill the GPU and each waits
+// for the one before, and beside the density kernels of other chunks they wait for those blocks
+// to end (eight 128^3 chunks of a terrain surface: on
+// four streams 714 us; together, with the passes as they now are, 570 us).
+template <class S>
+struct DmcPass {
+    DmcGrid<S> g;
+    unsigned rcp;           // ceil(2^32 / size)
+    unsigned* marks;
+    unsigned char* cell_axes;
+    uint4* tile_at;
+    uint2* tile_sums;
+    uint2* tile_lists;
+    DmcLists lists;
+    unsigned* result;       // DmcScratch::result
+    __device__ __forceinline__ uint2* total() const { return reinterpret_cast<uint2*>(result); }
+    __device__ __forceinline__ unsigned* airsolid() const { return result + 2; }
+    __device__ __forceinline__ const float* minmax() const { return reinterpret_cast<const float*>(result + 4); }
+    __host__ __device__ __forceinline__ unsigned cells() const { return (unsigned)g.size * (unsigned)g.size * (unsigned)g.size; }
+    __host__ __device__ __forceinline__ unsigned vertex_cells() const
+    {
+        const unsigned s1 = (unsigned)g.size + 1u;
+        return s1 * s1 * s1;
+    }
+    __host__ __device__ __forceinline__ unsigned tiles() const { return (cells() + kDmcTile - 1) / kDmcTile; }
+    __device__ __forceinline__ DmcPass of_chunk(unsigned c) const
+    {
+        const size_t n = cells(), v = vertex_cells();
+        DmcPass p = *this;
+        p.g.src = g.src.of_chunk(c);
+        p.g.cases += c * v;
+        const size_t t = tiles();
+        p.marks += c * n;
+        p.cell_axes += c * t * kDmcTile;
+        p.tile_at += c * t;
+        p.tile_sums += c * t;
+        p.tile_lists += c * t;
+        p.lists.vert_items += c * 4 * v;
+        p.lists.quad_items += c * 3 * n;
+        p.lists.quad_refs += c * 3 * n;
+        p.lists.counters += 2 * kDmcLine * c;
+        p.result += 8 * c;
+        return p;
+    }
+};
+struct DmcChunks {
+    DmcChunk chunk[kDmcChunks];
 };
 
 // Cells travel in the work items as x | y << 8 | z << 16 (sizes are at most 256): the passes
@@ -728,228 +761,210 @@ __device__ __forceinline__ DmcCell dmc_unpack(unsigned item, int size)
     return c;
 }
 
-// Add v to sums[tile] with one atomic per distinct tile among the warp's lanes.
-__device__ __forceinline__ void warp_tile_add(unsigned* sums, unsigned tile, unsigned v)
+// The cell with index t < 2^24: quotients by the chunk size (at most 256) as high halves of a
+// product, exact since t (rcp size - 2^32) < 2^32.
+__device__ __forceinline__ unsigned dmc_pack_index(unsigned t, unsigned size, unsigned rcp)
 {
-    const unsigned group = __match_any_sync(0xffffffffu, tile);
-    const unsigned sum = __reduce_add_sync(group, v);
-    if ((threadIdx.x & 31u) == (unsigned)(__ffs(group) - 1) && sum) atomicAdd(&sums[2 * tile], sum);
+    const unsigned row = __umulhi(t, rcp), z = __umulhi(row, rcp);
+    return dmc_pack(t - row * size, row - z * size, z);
 }
 
-__device__ __forceinline__ unsigned warp_append(unsigned* counter, unsigned n)
-{
-    const int lane = threadIdx.x & 31;
-    unsigned x = n;
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, x, 31);
-    unsigned base = 0;
-    if (lane == 31 && total) base = atomicAdd(counter, total);
-    return __shfl_sync(0xffffffffu, base, 31) + x - n;
-}
-
-// The chunk's counters, before its passes: list counters and tile sums 0, the lowest air
-// height "none", the highest solid 0.
-__global__ void dmc_clear(DmcLists lists, unsigned tiles, unsigned* airsolid)
-{
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < tiles) lists.tile_sums[t] = make_uint2(0u, 0u);
-    if (t < 2) {
-        lists.counters[t] = 0u;
-        airsolid[t] = t == 0 ? 0xFFFFFFFFu : 0u;
-    }
-}
-
-// Case pass: the marching-cubes case of every vertex cell (-1 .. size-1 per axis); for the
-// chunk's own cells also their cut axes, their quads (one per cut axis) in the tile sums and as
-// work items.  A warp takes 31 cells of a row and walks kCaseRun cells along z: the rows'
-// densities become bit words by ballot, a cell's case is eight bits of four words of which two
-// are the previous step's, and four steps' densities are loaded at once.  The quads of a run
-// are appended together, so a warp waits for one atomic per run.  Bound by the latency of the
-// density loads from L2 and the stores: 24.7 -> 18 us for a 128^3 chunk against eight loads,
-// divisions and appends per cell (13.2 -> 7.9 M instructions).
+// Case pass: the cut axes of every cell of the chunk, and the marching-cubes case of every vertex
+// cell (-1 .. size-1 per axis) that the surface may cut; the passes after it ask for no other.  A
+// warp takes 31 cells of a row and walks kCaseRun cells along z: the rows' densities become bit
+// words by ballot, a cell's case is eight bits of four words of which two are the previous
+// step's, and four steps' densities are loaded at once.  Words that are all 0 or all 1 (two steps
+// of three) need no more than their zero axes stored.  Bound by instruction issue and the density loads'
+// latency: eight 128^3 chunks 42 us; 85 us with every case stored and the quads listed here.
 constexpr int kCaseRun = 16;
 
 template <class S>
-__global__ void __launch_bounds__(256) dmc_cases(DmcGrid<S> g, float iso, const float* minmax, unsigned* masks,
-                                                 unsigned char* cell_axes, DmcLists lists)
+__global__ void __launch_bounds__(256) dmc_cases(DmcPass<S> all, float iso)
 {
-    if (early_out(minmax, iso)) return;
+    const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    if (blockIdx.x == 0 && threadIdx.x < 2) {        // what the later passes add to
+        m.lists.counters[threadIdx.x * kDmcLine] = 0u;
+        m.airsolid()[threadIdx.x] = threadIdx.x == 0 ? 0xFFFFFFFFu : 0u;
+    }
+    if (early_out(m.minmax(), iso)) return;
+    const DmcGrid<S>& g = m.g;
     const unsigned s1 = (unsigned)g.size + 1u, lane = threadIdx.x & 31u;
     const unsigned segs = (s1 + 30u) / 31u, runs = (s1 + kCaseRun - 1u) / kCaseRun, units = segs * s1 * runs;
-    unsigned* quad_sums = &lists.tile_sums[0].y;
     for (unsigned u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += (gridDim.x * blockDim.x) >> 5) {
         const unsigned rest = u / segs, xi = (u - rest * segs) * 31u + lane, run = rest / s1, yi = rest - run * s1;
-        const bool live = lane < 31u && xi < s1;
+        const bool live = lane < 31u && xi < s1, cell = live && xi && yi;
         const int base = dmc_index(g, (int)(xi < s1 ? xi : s1) - 1, (int)yi - 1, -1);
         const unsigned z0 = run * kCaseRun, z1 = z0 + kCaseRun < s1 ? z0 + kCaseRun : s1;
-        auto rows = [&](bool lo, bool hi) {          // bits 0, 1: this and the next density of the row, 2, 3: of the row above
-            const unsigned w0 = __ballot_sync(0xffffffffu, lo), w1 = __ballot_sync(0xffffffffu, hi);
-            return ((w0 >> lane) & 3u) | (((w1 >> lane) & 3u) << 2);
-        };
-        const unsigned cell0 = (z0 * g.size + yi - 1u) * g.size + xi - 1u;    // of step z0 + 1, where xi, yi > 0
-        const unsigned row0 = cell0 - lane;                                   // the same of lane 0
-        unsigned low;
+        unsigned l0, l1;                             // bit words of the row and the row above it, this step
         {
             const int i = base + (int)z0 * g.sz;
             const bool a = g.src.above(i, iso), b = g.src.above(i + g.sy, iso);
-            low = rows(a, b);
+            l0 = __ballot_sync(0xffffffffu, a);
+            l1 = __ballot_sync(0xffffffffu, b);
         }
-        unsigned cut[2] = {0u, 0u};                  // cut axes of steps 0-7, 8-15, three bits each
+        for (unsigned zb = z0; zb < z1; zb += 4u) {
+            bool a[4], b[4];
 #pragma unroll
-        for (unsigned h = 0; h < 2u; ++h)
-            for (unsigned q = 0; q < 8u; q += 4u) {
-                const unsigned zb = z0 + h * 8u + q;
-                if (zb >= z1) break;
-                bool a[4], b[4];
+            for (unsigned k = 0; k < 4u; ++k) {
+                const unsigned zn = zb + k + 1u < s1 ? zb + k + 1u : s1;
+                const int i = base + (int)zn * g.sz;
+                a[k] = g.src.above(i, iso);
+                b[k] = g.src.above(i + g.sy, iso);
+            }
 #pragma unroll
-                for (unsigned k = 0; k < 4u; ++k) {
-                    const unsigned zn = zb + k + 1u < s1 ? zb + k + 1u : s1;
-                    const int i = base + (int)zn * g.sz;
-                    a[k] = g.src.above(i, iso);
-                    b[k] = g.src.above(i + g.sy, iso);
-                }
-#pragma unroll
-                for (unsigned k = 0; k < 4u; ++k) {
-                    const unsigned zi = zb + k;
-                    if (zi >= z1) break;
-                    const unsigned high = rows(a[k], b[k]);
-                    const unsigned c = low | high << 4;
-                    low = high;
+            for (unsigned k = 0; k < 4u; ++k) {
+                const unsigned zi = zb + k;
+                if (zi >= z1) break;
+                const unsigned h0 = __ballot_sync(0xffffffffu, a[k]), h1 = __ballot_sync(0xffffffffu, b[k]);
+                unsigned axes = 0u;
+                if ((l0 | l1 | h0 | h1) != 0u && (l0 & l1 & h0 & h1) != 0xffffffffu) {
+                    const unsigned c = ((l0 >> lane) & 3u) | ((l1 >> lane) & 3u) << 2 | ((h0 >> lane) & 3u) << 4 | ((h1 >> lane) & 3u) << 6;
                     if (live) g.cases[(zi * s1 + yi) * s1 + xi] = (unsigned char)c;
-                    if (yi == 0u || zi == 0u) continue;
-                    const unsigned step = (zi - 1u - z0) * g.size * g.size;   // wraps for zi = z0, as cell0 + step does not
-                    const unsigned axes = live && xi ? dmc_axes(c) : 0u;
-                    if (live && xi) cell_axes[cell0 + step] = (unsigned char)axes;
-                    const unsigned mx = __ballot_sync(0xffffffffu, axes & 1u), my = __ballot_sync(0xffffffffu, axes & 2u),
-                                   mz = __ballot_sync(0xffffffffu, axes & 4u);
-                    if (!(mx | my | mz)) continue;
-                    if (axes) masks[cell0 + step] = 0u;
-                    cut[h] |= axes << (3u * (q + k));
-                    // the row's cells lie in one tile, or in two neighbouring ones
-                    // (lane 0 of a row's first 31 cells stands before the row and has none: its
-                    // index may be -1, tile -1, to which nothing is added)
-                    if (lane == 0) {
-                        const int first = (int)(row0 + step), tile = first >> 11, left = (tile + 1) * kDmcTile - first;
-                        const unsigned in = left < 32 ? (1u << left) - 1u : 0xffffffffu;
-                        const unsigned n0 = __popc(mx & in) + __popc(my & in) + __popc(mz & in);
-                        const unsigned n1 = __popc(mx & ~in) + __popc(my & ~in) + __popc(mz & ~in);
-                        if (n0) atomicAdd(&quad_sums[2 * tile], n0);
-                        if (n1) atomicAdd(&quad_sums[2 * tile + 2], n1);
-                    }
+                    axes = dmc_axes(c);
                 }
+                l0 = h0;
+                l1 = h1;
+                if (cell && zi) m.cell_axes[((zi - 1u) * g.size + yi - 1u) * g.size + xi - 1u] = (unsigned char)axes;
             }
-        const unsigned found = __popc(cut[0]) + __popc(cut[1]);
-        if (!__any_sync(0xffffffffu, found != 0u)) continue;
-        unsigned q = warp_append(&lists.counters[1], found);
-#pragma unroll
-        for (unsigned h = 0; h < 2u; ++h)
-            for (unsigned m = cut[h]; m; m &= m - 1u) {
-                const unsigned bit = (unsigned)__ffs(m) - 1u, k = bit / 3u;
-                lists.quad_items[q++] = dmc_pack(xi - 1u, yi - 1u, z0 + h * 8u + k - 1u) | (bit - 3u * k) << 24;
-            }
-    }
-}
-
-// Count pass: one thread per quad; each of its 4 references that is the vertex's first
-// use creates the vertex (bit axis * 4 + slot of the cell's mask) and becomes a vertex item.
-template <class S>
-__global__ void dmc_count(DmcGrid<S> g, unsigned* masks, DmcLists lists)
-{
-    const unsigned items = lists.counters[1];
-    unsigned* vert_sums = &lists.tile_sums[0].x;
-    for (unsigned j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < items; j0 += gridDim.x * blockDim.x) {
-        const unsigned j = j0 + (threadIdx.x & 31u);
-        unsigned bits = 0, t = 0, packed = 0;
-        if (j < items) {
-            const unsigned it = lists.quad_items[j];
-            const DmcCell w = dmc_unpack(it, g.size);
-            packed = it & 0xFFFFFFu;
-            t = w.t;
-            const int a = (int)(it >> 24);
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const DmcRef r = dmc_ref(g, w.x, w.y, w.z, a, s);
-                if (dmc_first_use(g, r.wx, r.wy, r.wz, r.c, r.p) == t * 12u + (unsigned)(a * 4 + s)) bits |= 1u << (a * 4 + s);
-            }
-            if (bits) atomicOr(&masks[t], bits);
         }
-        warp_tile_add(vert_sums, t / kDmcTile, __popc(bits));
-        unsigned v = warp_append(&lists.counters[0], __popc(bits));
-        for (unsigned m = bits; m; m &= m - 1u) lists.vert_items[v++] = packed | (unsigned)(__ffs(m) - 1) << 24;
     }
 }
 
-// Tile offsets: exclusive scan of the tile sums (one block); the grand total lands in `total`.
-__global__ void __launch_bounds__(kScanBlock) dmc_scan_tiles(uint2* tile_sums, unsigned tiles, uint2* total)
+// Count pass: one block per tile of cells, 16 cells a thread.  The tile's quads (one per cut axis)
+// are gathered in shared memory and taken one per thread: each of a quad's 4 references that is
+// the vertex's first use creates the vertex (bit axis * 4 + slot of the cell's marks).  Then
+// the tile's vertices are numbered cell by cell, and both are appended to the work lists with one
+// atomic each.  Bound by the latency of the case look-ups and the barriers; appended warp by warp, with
+// the tiles' sums in global atomics and the cells' offsets scanned in a pass of their own, this
+// waited on the counters: eight 128^3 chunks 50 us against 64 + 73 us.
+constexpr unsigned kDmcOwn = 16, kDmcThreads = kDmcTile / kDmcOwn;
+
+template <class S>
+__global__ void __launch_bounds__(kDmcThreads) dmc_count(DmcPass<S> all, float iso)
 {
+    __shared__ unsigned short quads[3 * kDmcTile];           // cell of the tile | axis << 11
+    __shared__ __align__(16) unsigned marks[kDmcTile / 2];   // two cells a word
+    __shared__ unsigned before[kDmcThreads];                 // vertices that the cells before a thread's create
+    __shared__ unsigned ws[32];
+    __shared__ uint2 s_lists;
+    const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    const DmcGrid<S>& g = m.g;
+    const unsigned n = m.cells(), size = (unsigned)g.size, first = blockIdx.x * kDmcTile, own = threadIdx.x * kDmcOwn;
+    unsigned axes[4] = {0u, 0u, 0u, 0u};
+    if (first + own < n && !early_out(m.minmax(), iso)) {
+        const uint4 v = *reinterpret_cast<const uint4*>(m.cell_axes + first + own);
+        axes[0] = v.x; axes[1] = v.y; axes[2] = v.z; axes[3] = v.w;
+        const unsigned left = n - (first + own);              // the chunk's last cells: nothing behind them
+#pragma unroll
+        for (unsigned k = 0; k < 4u; ++k)
+            if (left < 4u * k + 4u) axes[k] &= left > 4u * k ? (1u << (8u * (left - 4u * k))) - 1u : 0u;
+    }
+    unsigned total;
+    unsigned at = block_exclusive_scan((unsigned)(__popc(axes[0]) + __popc(axes[1]) + __popc(axes[2]) + __popc(axes[3])), ws, total);
+    if (total == 0u) {
+        if (threadIdx.x == 0) m.tile_sums[blockIdx.x] = make_uint2(0u, 0u);
+        return;
+    }
+#pragma unroll
+    for (unsigned k = 0; k < 4u; ++k)
+        for (unsigned a = axes[k]; a; a &= a - 1u) {
+            const unsigned bit = (unsigned)__ffs(a) - 1u;
+            quads[at++] = (unsigned short)((own + 4u * k + (bit >> 3)) | (bit & 7u) << 11);
+        }
+    for (unsigned k = threadIdx.x; k < kDmcTile / 2; k += kDmcThreads) marks[k] = 0u;
+    if (threadIdx.x == 0) s_lists.y = atomicAdd(&m.lists.counters[kDmcLine], total);
+    __syncthreads();
+    for (unsigned j = threadIdx.x; j < total; j += kDmcThreads) {
+        const unsigned q = quads[j], local = q & (kDmcTile - 1u), a = q >> 11;
+        const unsigned packed = dmc_pack_index(first + local, size, m.rcp);
+        const DmcCell w = dmc_unpack(packed, g.size);
+        unsigned bits = 0u, edges = 0u, inside = 0u;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const DmcRef r = dmc_ref(g, w.x, w.y, w.z, (int)a, s);
+            const unsigned e = dmc_first_edge(g, r.wx, r.wy, r.wz, r.c, r.p), slot = a * 4u + (unsigned)s;
+            if (e == dmc_slot_edge_of(slot)) bits |= 1u << slot;
+            edges |= e << (4 * s);
+            if (s == 0) inside = ~r.c & 1u;                   // the quad's own cell
+        }
+        m.lists.quad_items[s_lists.y + j] = packed | a << 24 | inside << 26;
+        m.lists.quad_refs[s_lists.y + j] = (unsigned short)edges;
+        if (bits) atomicOr(&marks[local >> 1], bits << (16u * (local & 1u)));
+    }
+    __syncthreads();
+    unsigned mine = 0u;
+#pragma unroll
+    for (unsigned k = 0; k < kDmcOwn / 2; k += 4u) {
+        const uint4 v = *reinterpret_cast<const uint4*>(marks + own / 2 + k);
+        mine += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
+    unsigned created;
+    before[threadIdx.x] = block_exclusive_scan(mine, ws, created);
+    if (threadIdx.x == 0) {
+        s_lists.x = created ? atomicAdd(&m.lists.counters[0], created) : 0u;
+        m.tile_sums[blockIdx.x] = make_uint2(created, total);
+        m.tile_lists[blockIdx.x] = s_lists;
+    }
+    __syncthreads();
+    // one thread per cell: the first of its quads
+    for (unsigned j = threadIdx.x; j < total; j += kDmcThreads) {
+        const unsigned local = quads[j] & (kDmcTile - 1u), group = local / kDmcOwn;
+        if (j && (quads[j - 1u] & (kDmcTile - 1u)) == local) continue;
+        unsigned at = before[group];
+        for (unsigned k = group * (kDmcOwn / 2); k < local >> 1; ++k) at += __popc(marks[k]);
+        const unsigned word = marks[local >> 1];
+        if (local & 1u) at += __popc(word & 0xFFFFu);
+        const unsigned bits = (word >> (16u * (local & 1u))) & 0xFFFu;
+        m.marks[first + local] = bits | at << 12;
+        if (!bits) continue;
+        const unsigned packed = dmc_pack_index(first + local, size, m.rcp);
+        for (unsigned b = bits; b; b &= b - 1u) m.lists.vert_items[s_lists.x + at++] = packed | (unsigned)(__ffs(b) - 1) << 24;
+    }
+}
+
+// Where each tile's vertices and quads go: exclusive scan of a chunk's tile sums (one block);
+// the grand total lands in the result.
+template <class S>
+__global__ void __launch_bounds__(kScanBlock) dmc_scan_tiles(DmcPass<S> all)
+{
+    const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    const unsigned tiles = m.tiles();
     __shared__ uint2 ws[32];
     uint2 carry = make_uint2(0u, 0u);
     for (unsigned base = 0; base < tiles; base += kScanBlock) {
         const unsigned i = base + threadIdx.x;
-        const uint2 v = i < tiles ? tile_sums[i] : make_uint2(0u, 0u);
+        const uint2 v = i < tiles ? m.tile_sums[i] : make_uint2(0u, 0u);
         uint2 sum;
-        const uint2 ex = block_exclusive_scan(v, ws, sum);
-        if (i < tiles) tile_sums[i] = plus(carry, ex);
+        const uint2 ex = plus(carry, block_exclusive_scan(v, ws, sum));
+        if (v.y) {
+            const uint2 listed = m.tile_lists[i];
+            m.tile_at[i] = make_uint4(ex.x, ex.x - listed.x, ex.y - listed.y, 0u);
+        }
         carry = plus(carry, sum);
         __syncthreads();
     }
-    if (threadIdx.x == 0) *total = carry;
+    if (threadIdx.x == 0) *m.total() = carry;
 }
 
-// Cell offsets within each tile that holds quads (256 threads x 8 cells, staged through
-// shared memory so that global loads and stores stay coalesced).  A cell's counts come from
-// its cut axes (one quad each) and its mask (the vertices it creates).
-__global__ void __launch_bounds__(256) dmc_scan_cells(const unsigned char* cell_axes, const unsigned* masks, uint2* offsets,
-                                                      unsigned n, const uint2* tile_offsets, const uint2* total)
-{
-    __shared__ uint2 tile[kDmcTile];
-    __shared__ uint2 ws[32];
-    const unsigned base = blockIdx.x * kDmcTile;
-    const unsigned next = blockIdx.x + 1u < gridDim.x ? tile_offsets[blockIdx.x + 1].y : total->y;
-    if (next == tile_offsets[blockIdx.x].y) return;             // no quads: nobody reads these offsets
-    for (int k = threadIdx.x; k < kDmcTile; k += 256) {
-        const unsigned t = base + k;
-        uint2 c = make_uint2(0u, 0u);
-        if (t < n) {
-            const unsigned axes = cell_axes[t];
-            if (axes) c = make_uint2(__popc(masks[t]), __popc(axes));
-        }
-        tile[k] = c;
-    }
-    __syncthreads();
-    uint2 local[8];
-    uint2 run = make_uint2(0u, 0u);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        local[k] = run;
-        run = plus(run, tile[threadIdx.x * 8 + k]);
-    }
-    uint2 sum;
-    const uint2 before = plus(tile_offsets[blockIdx.x], block_exclusive_scan(run, ws, sum));
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) tile[threadIdx.x * 8 + k] = plus(before, local[k]);
-    __syncthreads();
-    for (int k = threadIdx.x; k < kDmcTile; k += 256)
-        if (base + k < n) offsets[base + k] = tile[k];
-}
-
-// Vertex pass: one thread per created vertex, written at its cell's scanned offset.
+// The index of the vertex that quad slot `bit` of a cell creates.
 template <class S>
-__global__ void dmc_vertices(DmcGrid<S> g, int3 pos, float iso, const unsigned* masks, const uint2* offsets, const uint2* total,
-                             DmcLists lists, MeshVertex* verts, unsigned vcap)
+__device__ __forceinline__ unsigned dmc_vertex_index(const DmcPass<S>& m, unsigned cell, unsigned bit)
 {
-    __shared__ float3 s_nl;
-    if (threadIdx.x == 0) s_nl = dmc_light_dir();
-    __syncthreads();
-    if (total->x > vcap) return;
-    const float3 nl = s_nl;
-    const unsigned items = lists.counters[0];
+    const unsigned marks = m.marks[cell];
+    return m.tile_at[cell / kDmcTile].x + (marks >> 12) + __popc(marks & ((1u << bit) - 1u));
+}
+
+// Vertex pass: one thread per created vertex; a tile's go to consecutive places.
+template <class S>
+__global__ void dmc_vertices(DmcPass<S> all, float iso, float3 nl, DmcChunks chunks)
+{
+    const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    const DmcGrid<S>& g = m.g;
+    const DmcChunk& chunk = chunks.chunk[blockIdx.y];
+    if (m.total()->x > chunk.vcap) return;
+    const unsigned items = m.lists.counters[0];
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < items; j += gridDim.x * blockDim.x) {
-        const unsigned it = lists.vert_items[j];
+        const unsigned it = m.lists.vert_items[j];
         const DmcCell w = dmc_unpack(it, g.size);
         const unsigned t = w.t, bit = it >> 24;
         const int a = (int)(bit >> 2), s = (int)(bit & 3u), x = w.x, y = w.y, z = w.z;
@@ -957,44 +972,50 @@ __global__ void dmc_vertices(DmcGrid<S> g, int3 pos, float iso, const unsigned* 
         const int wi = dmc_index(g, r.wx, r.wy, r.wz);
         const float3 p = dmc_point(g, wi, __ldg(&kDmc.code[r.c][r.p]), iso);
         const float light = dmc_light(g, wi, p, nl);
-        const unsigned out = offsets[t].x + __popc(masks[t] & ((1u << bit) - 1u));
-        verts[out] = MeshVertex{p.x + dmc_offset(pos.x, x, r.wx), p.y + dmc_offset(pos.y, y, r.wy),
-                                p.z + dmc_offset(pos.z, z, r.wz), light};
+        const unsigned out = m.tile_at[t / kDmcTile].y + j;
+        chunk.verts[out] = MeshVertex{p.x + dmc_offset(chunk.x, x, r.wx), p.y + dmc_offset(chunk.y, y, r.wy),
+                                p.z + dmc_offset(chunk.z, z, r.wz), light};
     }
 }
 
 // Quad pass: one thread per cut edge, 6 indices (:662-674) with the vertex indices found
-// through each vertex's first use; the y-edge quads also give the min air / max solid
+// through each vertex's first use, as the count pass noted it; the y-edge quads also give the min air / max solid
 // heights (:706-724).
 template <class S>
-__global__ void dmc_quads(DmcGrid<S> g, int3 pos, float iso, const unsigned* masks, const uint2* offsets, const uint2* total,
-                          DmcLists lists, const MeshVertex* verts, unsigned vcap, unsigned* idx, unsigned icap, unsigned* airsolid)
+__global__ void dmc_quads(DmcPass<S> all, float iso, DmcChunks chunks)
 {
-    const uint2 tot = *total;
-    const bool fits = tot.x <= vcap && (unsigned long long)tot.y * 6ull <= icap;
-    const unsigned items = lists.counters[1];
+    const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    const DmcGrid<S>& g = m.g;
+    const DmcLists& lists = m.lists;
+    const DmcChunk& chunk = chunks.chunk[blockIdx.y];
+    const MeshVertex* verts = chunk.verts;
+    const uint2 tot = *m.total();
+    const bool fits = tot.x <= chunk.vcap && (unsigned long long)tot.y * 6ull <= chunk.icap;
+    const unsigned items = lists.counters[kDmcLine];
     unsigned air = 0xFFFFFFFFu, solid = 0u;
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < items; j += gridDim.x * blockDim.x) {
         const unsigned it = lists.quad_items[j];
         const DmcCell w = dmc_unpack(it, g.size);
         const unsigned t = w.t;
-        const int a = (int)(it >> 24), x = w.x, y = w.y, z = w.z;
-        const unsigned own = dmc_case_at(g, x, y, z);
-        const bool inside = !(own & 1u);                      // density <= iso; cut, so also density < neighbour
-        const unsigned quad = offsets[t].y + __popc(dmc_axes(own) & ((1u << a) - 1u));
+        const unsigned edges = lists.quad_refs[j];
+        const int a = (int)((it >> 24) & 3u);
+        const bool inside = (it >> 26) & 1u;                  // density <= iso; cut, so also density < neighbour
+        const unsigned quad = m.tile_at[t / kDmcTile].z + j;
         unsigned q[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const DmcRef r = dmc_ref(g, x, y, z, a, s);
-            const unsigned first = dmc_first_use(g, r.wx, r.wy, r.wz, r.c, r.p);
-            const unsigned c = first / 12u, bit = first - c * 12u;
-            q[s] = offsets[c].x + __popc(masks[c] & ((1u << bit) - 1u));
+            const unsigned e = (edges >> (4 * s)) & 0xFu, off = dmc_use_offset(e);
+            const int cx = w.x + dmc_slot_offset(a, s, 0) + (int)(off & 1u), cy = w.y + dmc_slot_offset(a, s, 1) + (int)((off >> 1) & 1u),
+                      cz = w.z + dmc_slot_offset(a, s, 2) + (int)(off >> 2);         // the cell whose quad creates the vertex
+            q[s] = dmc_vertex_index(m, (unsigned)((cz * g.size + cy) * g.size + cx), dmc_use_slot_of(e));
             if (a == 1) {                       // the stored vertex's y: offset of the quad that created it
                 // the vertex pass wrote exactly this value when the buffers fit
-                const int cy = (int)((c / (unsigned)g.size) % (unsigned)g.size);
-                const float vy = fits ? verts[q[s]].y
-                                      : dmc_point(g, dmc_index(g, r.wx, r.wy, r.wz), __ldg(&kDmc.code[r.c][r.p]), iso).y +
-                                            dmc_offset(pos.y, cy, r.wy);
+                float vy;
+                if (fits) vy = verts[q[s]].y;
+                else {
+                    const DmcRef r = dmc_ref(g, w.x, w.y, w.z, a, s);
+                    vy = dmc_point(g, dmc_index(g, r.wx, r.wy, r.wz), __ldg(&kDmc.code[r.c][r.p]), iso).y + dmc_offset(chunk.y, cy, r.wy);
+                }
                 if (inside) solid = max(solid, enc(vy));
                 else air = min(air, enc(vy));
             }
@@ -1002,7 +1023,7 @@ __global__ void dmc_quads(DmcGrid<S> g, int3 pos, float iso, const unsigned* mas
         if (fits) {
             const unsigned rot = fabsf(verts[q[0]].light - verts[q[3]].light) > fabsf(verts[q[1]].light - verts[q[2]].light) ? 2u : 0u;
             const unsigned flip = inside ? 2u : 0u;
-            unsigned* o = idx + (size_t)quad * 6u;
+            unsigned* o = chunk.idx + (size_t)quad * 6u;
             o[0] = q[flip];
             o[1] = q[3u - rot];
             o[2] = q[2u - flip];
@@ -1020,8 +1041,8 @@ __global__ void dmc_quads(DmcGrid<S> g, int3 pos, float iso, const unsigned* mas
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { air = min(air, s_air[w]); solid = max(solid, s_solid[w]); }
-        if (air != 0xFFFFFFFFu) atomicMin(&airsolid[0], air);
-        if (solid != 0u) atomicMax(&airsolid[1], solid);
+        if (air != 0xFFFFFFFFu) atomicMin(&m.airsolid()[0], air);
+        if (solid != 0u) atomicMax(&m.airsolid()[1], solid);
     }
 }
 
@@ -1043,8 +1064,10 @@ __device__ __forceinline__ void mark_run(unsigned* need, int start, int len, uns
 // The density index of every created vertex's cell (its base corner) -- marked in `cells`;
 // need_dilate then adds the densities the vertex and quad passes read around them.
 template <class S>
-__global__ void dmc_mark_cells(DmcGrid<S> g, DmcLists lists, unsigned* cells)
+__global__ void dmc_mark_cells(DmcPass<S> pass, unsigned* cells)
 {
+    const DmcGrid<S>& g = pass.g;
+    const DmcLists& lists = pass.lists;
     const unsigned items = lists.counters[0];
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < items; j += gridDim.x * blockDim.x) {
         const unsigned it = lists.vert_items[j], bit = it >> 24;
@@ -1207,62 +1230,90 @@ cudaError_t launch_heightmap(const float* dens, int size, float px, float pz, fl
     return cudaGetLastError();
 }
 
-cudaError_t launch_dmc(const float* dens, int size, bool up_axis_z, int px, int py, int pz, float iso, const float* dminmax,
-                       DmcScratch& s, MeshVertex* verts, unsigned vcap, unsigned* idx, unsigned icap, cudaStream_t stream)
+size_t dmc_scratch(int size, unsigned chunks, char* block, DmcScratch& s)
+{
+    const size_t n = (size_t)size * size * size, v = (size_t)(size + 1) * (size + 1) * (size + 1), tiles = (n + kDmcTile - 1) / kDmcTile;
+    size_t at = 0;
+    auto take = [&](auto*& p, size_t per_chunk) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(block + at);
+        at += (per_chunk * chunks * sizeof(*p) + 15) / 16 * 16;
+    };
+    take(s.tile_at, tiles);
+    take(s.tile_sums, tiles);
+    take(s.tile_lists, tiles);
+    take(s.marks, n);
+    take(s.counters, 2 * kDmcLine);
+    take(s.vert_items, 4 * v);
+    take(s.quad_items, 3 * n);
+    take(s.quad_refs, 3 * n);
+    take(s.cases, v);
+    take(s.cell_axes, tiles * kDmcTile);
+    return at;
+}
+
+namespace {
+
+template <class S>
+DmcPass<S> dmc_pass(const S& src, int size, bool up_axis_z, const DmcScratch& s)
 {
     const int sg = size + 4;
-    const DmcGrid<DenseSrc> g{DenseSrc{dens}, 1, up_axis_z ? sg * sg : sg, up_axis_z ? sg : sg * sg, size, s.cases};
-    const DmcLists lists{s.vert_items, s.quad_items, s.counters, s.tile_sums};
-    const unsigned n = (unsigned)size * size * size;
-    const unsigned tiles = (n + kDmcTile - 1) / kDmcTile;
-    const int3 pos = make_int3(px, py, pz);
-    dmc_clear<<<(tiles + 255u) / 256u, 256, 0, stream>>>(lists, tiles, s.airsolid);
-    dmc_cases<<<case_grid(size), 256, 0, stream>>>(g, iso, dminmax, s.masks, s.cell_axes, lists);
-    // one thread per quad / vertex: the lists hold a few items per surface cell
-    dmc_count<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, s.masks, lists);
-    dmc_scan_tiles<<<1, kScanBlock, 0, stream>>>(s.tile_sums, tiles, s.total);
-    dmc_scan_cells<<<tiles, 256, 0, stream>>>(s.cell_axes, s.masks, s.offsets, n, s.tile_sums, s.total);
-    dmc_vertices<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, pos, iso, s.masks, s.offsets, s.total, lists, verts, vcap);
-    dmc_quads<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, pos, iso, s.masks, s.offsets, s.total, lists, verts, vcap, idx, icap,
-                                                        s.airsolid);
+    return DmcPass<S>{{src, 1, up_axis_z ? sg * sg : sg, up_axis_z ? sg : sg * sg, size, s.cases},
+                      0xFFFFFFFFu / (unsigned)size + 1u, s.marks, s.cell_axes, s.tile_at, s.tile_sums, s.tile_lists,
+                      {s.vert_items, s.quad_items, s.quad_refs, s.counters}, s.result};
+}
+
+// cases, quads and created vertices of every chunk, and where each cell's begin
+template <class S>
+void dmc_number(const DmcPass<S>& m, float iso, unsigned count, cudaStream_t stream)
+{
+    dmc_cases<S><<<dim3(case_grid(m.g.size), count), 256, 0, stream>>>(m, iso);
+    dmc_count<S><<<dim3(m.tiles(), count), kDmcThreads, 0, stream>>>(m, iso);
+    dmc_scan_tiles<S><<<dim3(1, count), kScanBlock, 0, stream>>>(m);
+}
+
+template <class S>
+void dmc_write(const DmcPass<S>& m, float iso, const DmcChunk* chunks, unsigned count, cudaStream_t stream)
+{
+    DmcChunks c;
+    for (unsigned k = 0; k < count; ++k) c.chunk[k] = chunks[k];
+    // One thread per vertex / quad: the lists hold a few items per surface cell.  About two waves of
+    // blocks for all chunks together (18 blocks per SM; eight 128^3 chunks: 8192 blocks 582 us, 4096
+    // 573, 2728 570, 2048 569, 1024 580), since most of more would find no items.
+    const int each = (grid_for(1u << 30, 256) * 9 / 4 + (int)count - 1) / (int)count;
+    const dim3 grid(std::min(grid_for(m.cells() / 8, 256), each), count);
+    dmc_vertices<S><<<grid, 256, 0, stream>>>(m, iso, dmc_light_dir(), c);
+    dmc_quads<S><<<grid, 256, 0, stream>>>(m, iso, c);
+}
+
+}  // namespace
+
+cudaError_t launch_dmc(const float* dens, size_t dens_stride, int size, bool up_axis_z, float iso, const DmcChunk* chunks,
+                       unsigned count, DmcScratch& s, cudaStream_t stream)
+{
+    const DmcPass<DenseSrc> m = dmc_pass(DenseSrc{dens, dens_stride}, size, up_axis_z, s);
+    dmc_number(m, iso, count, stream);
+    dmc_write(m, iso, chunks, count, stream);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dmc_sparse_prepare(SparseScratch& sp, int size, bool up_axis_z, float iso, const float* dminmax, DmcScratch& s,
-                                      cudaStream_t stream)
+cudaError_t launch_dmc_sparse_prepare(SparseScratch& sp, int size, bool up_axis_z, float iso, DmcScratch& s, cudaStream_t stream)
 {
     const int sg = size + 4;
-    const unsigned n_dens = (unsigned)sg * sg * sg;
-    const DmcGrid<SparseSrc> g{sparse_src(sp), 1, up_axis_z ? sg * sg : sg, up_axis_z ? sg : sg * sg, size, s.cases};
-    const DmcLists lists{s.vert_items, s.quad_items, s.counters, s.tile_sums};
-    const unsigned n = (unsigned)size * size * size;
-    const unsigned tiles = (n + kDmcTile - 1) / kDmcTile;
-    const unsigned nwords = (n_dens + 31u) / 32u;
+    const unsigned n_dens = (unsigned)sg * sg * sg, nwords = (n_dens + 31u) / 32u;
+    const DmcPass<SparseSrc> m = dmc_pass(sparse_src(sp), size, up_axis_z, s);
     const cudaError_t e = cudaMemsetAsync(sp.cells, 0, nwords * sizeof(unsigned), stream);
     if (e != cudaSuccess) return e;
-    dmc_clear<<<(tiles + 255u) / 256u, 256, 0, stream>>>(lists, tiles, s.airsolid);
-    dmc_cases<<<case_grid(size), 256, 0, stream>>>(g, iso, dminmax, s.masks, s.cell_axes, lists);
-    dmc_count<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, s.masks, lists);
-    dmc_scan_tiles<<<1, kScanBlock, 0, stream>>>(s.tile_sums, tiles, s.total);
-    dmc_scan_cells<<<tiles, 256, 0, stream>>>(s.cell_axes, s.masks, s.offsets, n, s.tile_sums, s.total);
-    dmc_mark_cells<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, lists, sp.cells);
-    need_dilate<<<grid_for(nwords, 256), 256, 0, stream>>>(sp.cells, sp.need, sp.counts, n_dens, g.sy, g.sz);
+    dmc_number(m, iso, 1, stream);
+    dmc_mark_cells<<<grid_for(m.cells() / 8, 256), 256, 0, stream>>>(m, sp.cells);
+    need_dilate<<<grid_for(nwords, 256), 256, 0, stream>>>(sp.cells, sp.need, sp.counts, n_dens, m.g.sy, m.g.sz);
     need_list(sp, n_dens, true, stream);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dmc_sparse_finish(const SparseScratch& sp, int size, bool up_axis_z, int px, int py, int pz, float iso,
-                                     DmcScratch& s, MeshVertex* verts, unsigned vcap, unsigned* idx, unsigned icap,
-                                     cudaStream_t stream)
+cudaError_t launch_dmc_sparse_finish(const SparseScratch& sp, int size, bool up_axis_z, float iso, const DmcChunk& chunk,
+                                     DmcScratch& s, cudaStream_t stream)
 {
-    const int sg = size + 4;
-    const DmcGrid<SparseSrc> g{sparse_src(sp), 1, up_axis_z ? sg * sg : sg, up_axis_z ? sg : sg * sg, size, s.cases};
-    const DmcLists lists{s.vert_items, s.quad_items, s.counters, s.tile_sums};
-    const unsigned n = (unsigned)size * size * size;
-    const int3 pos = make_int3(px, py, pz);
-    dmc_vertices<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, pos, iso, s.masks, s.offsets, s.total, lists, verts, vcap);
-    dmc_quads<<<grid_for(n / 8, 256), 256, 0, stream>>>(g, pos, iso, s.masks, s.offsets, s.total, lists, verts, vcap, idx, icap,
-                                                        s.airsolid);
+    dmc_write(dmc_pass(sparse_src(sp), size, up_axis_z, s), iso, &chunk, 1, stream);
     return cudaGetLastError();
 }
 

@@ -20,20 +20,35 @@ struct MeshScratch {
     size_t cap_voxels = 0;
 };
 
-// Per-thread device scratch of the dual marching cubes mesher.
+// Per-thread device scratch of the dual marching cubes mesher: one slice per chunk meshed
+// together in each array (dmc_scratch lays them out).
 struct DmcScratch {
-    uint2* offsets = nullptr;          // per cell: first vertex it creates, first quad it emits (tiles that hold quads)
-    uint2* tile_sums = nullptr;        // per 2048 cells: vertices, quads; then scanned into tile offsets
-    uint2* total = nullptr;            // vertices, quads in the chunk
-    unsigned* masks = nullptr;         // per cell: which of its 12 quad slots create a vertex
-    unsigned* airsolid = nullptr;      // order-preserving min air y / max solid y
-    unsigned* counters = nullptr;      // work items listed: vertices, quads
+    uint4* tile_at = nullptr;          // per tile of 2048 cells: its first vertex; its first vertex and quad less where they are listed
+    uint2* tile_sums = nullptr;        // per tile: vertices it creates, quads
+    uint2* tile_lists = nullptr;       // per tile: where its vertices and quads are listed
+    unsigned* marks = nullptr;         // per cell with quads: bits 0-11 which of its quad slots create a vertex, 12- vertices
+                                       // its tile's earlier cells create
+    unsigned* counters = nullptr;      // work items listed: vertices, quads (a cache line each)
     unsigned* vert_items = nullptr;    // 4 (size+1)^3: every (vertex cell, piece) at most once
     unsigned* quad_items = nullptr;    // 3 size^3: every cut edge at most once
-    unsigned char* cases = nullptr;    // (size+1)^3 marching-cubes cases
-    unsigned char* cell_axes = nullptr;   // per cell: its cut axes
-    size_t cap_cells = 0;
+    unsigned short* quad_refs = nullptr;   // per quad item: the edges through which its 4 vertices are first used
+    unsigned char* cases = nullptr;    // (size+1)^3 marching-cubes cases, of the cells that the surface cuts
+    unsigned char* cell_axes = nullptr;   // per cell: its cut axes (slices of whole tiles)
+    unsigned* result = nullptr;        // 8 words per chunk: vertices, quads, lowest air and highest solid height
+                                       // (order-preserving), OutputMinMax (two floats, read here), unused
 };
+
+// Lay the arrays of `chunks` chunks out in `block`; returns the bytes they take (block may be null).
+size_t dmc_scratch(int size, unsigned chunks, char* block, DmcScratch& s);
+
+// One of the chunks that are meshed together, and where its mesh goes.
+struct DmcChunk {
+    int x, y, z;
+    unsigned vcap, icap;
+    MeshVertex* verts;
+    unsigned* idx;
+};
+constexpr unsigned kDmcChunks = 32;    // most chunks of one launch_dmc
 
 // The sparse density form of a chunk (no density array): two classification bitmasks of
 // every density (bit i of word i / 32), written by the tree's fnjit_solid kernel; the needed
@@ -75,18 +90,17 @@ cudaError_t launch_bloxel_sparse_emit(const SparseScratch& sp, int size, bool up
 cudaError_t launch_heightmap(const float* dens, int size, float px, float pz, float mul, MeshVertex* verts, unsigned vcap,
                              unsigned* idx, unsigned icap, cudaStream_t stream);
 
-// Dual marching cubes chunk: size^3 cells over (size+4)^3 densities (a two-voxel
-// apron).  Vertices and indices are written only when both fit (vcap / icap);
-// the vertex and quad totals land in s.total either way.
-cudaError_t launch_dmc(const float* dens, int size, bool up_axis_z, int px, int py, int pz, float iso, const float* dminmax,
-                       DmcScratch& s, MeshVertex* verts, unsigned vcap, unsigned* idx, unsigned icap, cudaStream_t stream);
+// Dual marching cubes chunks: size^3 cells over (size+4)^3 densities (a two-voxel apron) each;
+// chunk k's densities start at dens + k * dens_stride, and their OutputMinMax is in s.result.
+// Vertices and indices are written only when both fit (vcap / icap); the totals land in
+// s.result either way.
+cudaError_t launch_dmc(const float* dens, size_t dens_stride, int size, bool up_axis_z, float iso, const DmcChunk* chunks,
+                       unsigned count, DmcScratch& s, cudaStream_t stream);
 
-// Dual marching cubes on the sparse form: prepare (cases, quads, vertices, scans, the needed
-// list: the densities around every created vertex's cell), then the vertex and quad passes.
-cudaError_t launch_dmc_sparse_prepare(SparseScratch& sp, int size, bool up_axis_z, float iso, const float* dminmax, DmcScratch& s,
-                                      cudaStream_t stream);
-cudaError_t launch_dmc_sparse_finish(const SparseScratch& sp, int size, bool up_axis_z, int px, int py, int pz, float iso,
-                                     DmcScratch& s, MeshVertex* verts, unsigned vcap, unsigned* idx, unsigned icap,
-                                     cudaStream_t stream);
+// Dual marching cubes on the sparse form, one chunk: prepare (cases, quads, vertices, scans, the
+// needed list: the densities around every created vertex's cell), then the vertex and quad passes.
+cudaError_t launch_dmc_sparse_prepare(SparseScratch& sp, int size, bool up_axis_z, float iso, DmcScratch& s, cudaStream_t stream);
+cudaError_t launch_dmc_sparse_finish(const SparseScratch& sp, int size, bool up_axis_z, float iso, const DmcChunk& chunk,
+                                     DmcScratch& s, cudaStream_t stream);
 
 }  // namespace fn
