@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "fn_eval.cuh"
 #include "fn_mesh.h"
 
 namespace fn {
@@ -782,6 +783,8 @@ template <class S>
 __global__ void __launch_bounds__(256) dmc_cases(DmcPass<S> all, float iso)
 {
     const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    fne::let_stream_continue();
+    fne::wait_for_stream();
     if (blockIdx.x == 0 && threadIdx.x < 2) {        // what the later passes add to
         m.lists.counters[threadIdx.x * kDmcLine] = 0u;
         m.airsolid()[threadIdx.x] = threadIdx.x == 0 ? 0xFFFFFFFFu : 0u;
@@ -850,6 +853,8 @@ __global__ void __launch_bounds__(kDmcThreads) dmc_count(DmcPass<S> all, float i
     const DmcPass<S> m = all.of_chunk(blockIdx.y);
     const DmcGrid<S>& g = m.g;
     const unsigned n = m.cells(), size = (unsigned)g.size, first = blockIdx.x * kDmcTile, own = threadIdx.x * kDmcOwn;
+    fne::let_stream_continue();
+    fne::wait_for_stream();
     unsigned axes[4] = {0u, 0u, 0u, 0u};
     if (first + own < n && !early_out(m.minmax(), iso)) {
         const uint4 v = *reinterpret_cast<const uint4*>(m.cell_axes + first + own);
@@ -928,6 +933,8 @@ template <class S>
 __global__ void __launch_bounds__(kScanBlock) dmc_scan_tiles(DmcPass<S> all)
 {
     const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    fne::let_stream_continue();
+    fne::wait_for_stream();
     const unsigned tiles = m.tiles();
     __shared__ uint2 ws[32];
     uint2 carry = make_uint2(0u, 0u);
@@ -959,6 +966,8 @@ template <class S>
 __global__ void dmc_vertices(DmcPass<S> all, float iso, float3 nl, DmcChunks chunks)
 {
     const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    fne::let_stream_continue();
+    fne::wait_for_stream();
     const DmcGrid<S>& g = m.g;
     const DmcChunk& chunk = chunks.chunk[blockIdx.y];
     if (m.total()->x > chunk.vcap) return;
@@ -985,6 +994,8 @@ template <class S>
 __global__ void dmc_quads(DmcPass<S> all, float iso, DmcChunks chunks)
 {
     const DmcPass<S> m = all.of_chunk(blockIdx.y);
+    fne::let_stream_continue();
+    fne::wait_for_stream();
     const DmcGrid<S>& g = m.g;
     const DmcLists& lists = m.lists;
     const DmcChunk& chunk = chunks.chunk[blockIdx.y];
@@ -1253,6 +1264,23 @@ size_t dmc_scratch(int size, unsigned chunks, char* block, DmcScratch& s)
 
 namespace {
 
+// A pass's launch may take the slots that the launch before it leaves free; every pass waits for
+// that launch before it touches memory.  One chunk of 32^3 72 -> 65 us a call, of 128^3 123 -> 120 us.
+template <class... P, class... A>
+void launch_pass(void (*kernel)(P...), dim3 grid, unsigned block, cudaStream_t stream, const A&... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <class S>
 DmcPass<S> dmc_pass(const S& src, int size, bool up_axis_z, const DmcScratch& s)
 {
@@ -1266,9 +1294,9 @@ DmcPass<S> dmc_pass(const S& src, int size, bool up_axis_z, const DmcScratch& s)
 template <class S>
 void dmc_number(const DmcPass<S>& m, float iso, unsigned count, cudaStream_t stream)
 {
-    dmc_cases<S><<<dim3(case_grid(m.g.size), count), 256, 0, stream>>>(m, iso);
-    dmc_count<S><<<dim3(m.tiles(), count), kDmcThreads, 0, stream>>>(m, iso);
-    dmc_scan_tiles<S><<<dim3(1, count), kScanBlock, 0, stream>>>(m);
+    launch_pass(dmc_cases<S>, dim3(case_grid(m.g.size), count), 256, stream, m, iso);
+    launch_pass(dmc_count<S>, dim3(m.tiles(), count), kDmcThreads, stream, m, iso);
+    launch_pass(dmc_scan_tiles<S>, dim3(1, count), kScanBlock, stream, m);
 }
 
 template <class S>
@@ -1281,8 +1309,8 @@ void dmc_write(const DmcPass<S>& m, float iso, const DmcChunk* chunks, unsigned 
     // 573, 2728 570, 2048 569, 1024 580), since most of more would find no items.
     const int each = (grid_for(1u << 30, 256) * 9 / 4 + (int)count - 1) / (int)count;
     const dim3 grid(std::min(grid_for(m.cells() / 8, 256), each), count);
-    dmc_vertices<S><<<grid, 256, 0, stream>>>(m, iso, dmc_light_dir(), c);
-    dmc_quads<S><<<grid, 256, 0, stream>>>(m, iso, c);
+    launch_pass(dmc_vertices<S>, grid, 256, stream, m, iso, dmc_light_dir(), c);
+    launch_pass(dmc_quads<S>, grid, 256, stream, m, iso, c);
 }
 
 }  // namespace
