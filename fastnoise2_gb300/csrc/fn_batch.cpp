@@ -249,8 +249,10 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     double column_work = 0;                         // their 32-point steps
     for (size_t i = 0; jit && i < n; ++i) {
         const JitKernels& jk = trees[tree_of_[i]].jk;
-        if (jk.batch_column && jit_column_grid(items[i].args, jk, columns_[i]))
-            column_work += (double)columns_[i].steps * column_chunks(columns_[i]);
+        ColumnShape shape;
+        if (!jk.batch_column || !jit_column_grid(items[i].args, jk, shape) || !column_pays(shape, jk)) continue;
+        columns_[i] = shape;
+        column_work += (double)shape.steps * column_chunks(shape);
     }
     // Column units: about four rounds of 16 warps per SM over the whole batch, so that short
     // batches still spread, and at most 64 steps (longer ones gain under 5 % of set-up).

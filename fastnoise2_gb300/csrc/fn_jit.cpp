@@ -118,7 +118,7 @@ ColPlan column_plan(const CompiledProgram& prog)
     auto generic_cost = [&](const FnInstr& I) -> double {
         const int d = I.dim - 2;
         static const double simplex[3] = {90, 130, 230}, super[3] = {130, 380, 900}, lattice[3] = {90, 200, 440}, warp[3] = {70, 190, 500},
-                            cells[3] = {420, 1300, 2400};
+                            cells[3] = {440, 1300, 2400};
         switch (I.op) {
         case FN_OP_NOISE: return I.aux == FN_NOISE_SIMPLEX ? simplex[d] : I.aux == FN_NOISE_SUPERSIMPLEX ? super[d] : lattice[d];
         case FN_OP_WARP_GRAD: return warp[d];
@@ -1535,20 +1535,20 @@ bool column_cut_alone(ColumnShape& s, const JitKernels& jk, OutputMemory memory)
 {
     const unsigned n = s.steps, chunks = column_chunks(s), slots = 8u * (unsigned)num_sms(),
                    fill = (unsigned)std::max(1, jk.column_resident);
-    unsigned best = 1;
+    unsigned best = 1, best_load = 1;
     float best_cost = 1e30f;
     for (unsigned w = 1; w <= 16; ++w) {
         const unsigned fit = std::min(n, std::max(1u, w * slots / chunks)), len = (n + fit - 1) / fit;
         const unsigned long long units = (unsigned long long)chunks * ((n + len - 1) / len);
         const unsigned load = (unsigned)((units + slots - 1) / slots);
         const float cost = (float)std::max(fill, load) * (jk.column_setup + (float)len);
-        if (cost < best_cost) { best_cost = cost; best = len; }
+        if (cost < best_cost) { best_cost = cost; best = len; best_load = std::max(fill, load); }
         if (len == 1) break;
     }
     // microseconds, at ~9000 warp instructions per SM and microsecond, or ~500 of one warp
     const float points = (float)s.plane * (float)s.steps;
     float point_us = points / 32.0f * jk.point_cost / (9000.0f * (float)num_sms());
-    float column_us = best_cost * 8.0f * jk.column_step / 9000.0f;
+    float column_us = (float)best_load * (kColSetupWork * jk.column_setup + (float)best) * 8.0f * jk.column_step / 9000.0f;
     if (memory == kDeviceMemory) {
         point_us = std::max(point_us, 3.0f);
         column_us += 4.0f;

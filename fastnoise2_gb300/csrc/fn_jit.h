@@ -107,6 +107,19 @@ struct ColumnShape {
 bool jit_column_grid(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
 inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
 unsigned column_tiles(ColumnShape& shape, unsigned len);
+// Setting a unit up takes this much of the work that `column_setup` steps are (FBm(Perlin) 600000 x 3
+// takes 35 us in columns, 25 with the point kernel, and would seem to take 25 and 25).
+constexpr float kColSetupWork = 1.4f;
+
+// Whether columns pay in a batch: a plane that is no multiple of 32 leaves lanes idle at every
+// step, so the steps' instructions (units of 16 steps) are set against the points', with 15 % for
+// the estimates.  128 requests, columns / points, us: FBm(Perlin) 2 x 50000 1409 / 228, 12 x 8000 287 / 219,
+// 24 x 4000 167 / 219; terrain 3 x 3 x 10000 2299 / 955, 33 x 3000 664 / 481.
+inline bool column_pays(const ColumnShape& s, const JitKernels& jk)
+{
+    const float len = s.steps < 16 ? (float)s.steps : 16.0f;
+    return 32.0f * (float)column_chunks(s) * jk.column_step * (1.0f + kColSetupWork * jk.column_setup / len) < 0.85f * (float)s.plane * jk.point_cost;
+}
 void column_args(PointArgs& args, const ColumnShape& shape);
 
 // Queue a background build of the batch variants of `prog` (a tuning table loaded in this
