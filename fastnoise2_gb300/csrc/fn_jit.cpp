@@ -114,13 +114,13 @@ ColPlan column_plan(const CompiledProgram& prog)
     // Instructions of setting a state up and of a step of it, and of a step of the other
     // instructions, roughly (from instruction counts of the kernels): their ratio decides how
     // short a unit may be.
-    double setup = 30, step = 15, other = 0, point = 100;
+    double setup = 30, step = 15, other = 0, point = prog.dim == 2 ? 160 : 100;
     auto generic_cost = [&](const FnInstr& I) -> double {
         const int d = I.dim - 2;
         static const double simplex[3] = {90, 130, 230}, super[3] = {130, 380, 900}, lattice[3] = {90, 200, 440}, warp[3] = {70, 190, 500},
-                            cells[3] = {440, 1300, 2400};
+                            cells[3] = {380, 1300, 2400};
         switch (I.op) {
-        case FN_OP_NOISE: return I.aux == FN_NOISE_SIMPLEX ? simplex[d] : I.aux == FN_NOISE_SUPERSIMPLEX ? super[d] : lattice[d];
+        case FN_OP_NOISE: return I.aux == FN_NOISE_SIMPLEX ? simplex[d] : I.aux == FN_NOISE_SUPERSIMPLEX ? super[d] : d == 2 && I.aux == FN_NOISE_VALUE ? 250 : lattice[d];
         case FN_OP_WARP_GRAD: return warp[d];
         case FN_OP_WARP_SIMPLEX: return 2 * warp[d];
         case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: return cells[d];
@@ -1500,6 +1500,7 @@ bool jit_column_grid(const PointArgs& a, const JitKernels& jk, ColumnShape& shap
     shape.plane = (unsigned)plane;
     shape.steps = a.base || a.total != plane * a.count[a.dim - 1] ? (unsigned)(a.total / plane) : (unsigned)a.count[a.dim - 1];
     shape.first = a.base ? a.base / (unsigned)plane : 0u;
+    shape.rate = jk.n_column_rates ? rate / (float)jk.n_column_rates : 0.0f;
     return true;
 }
 
@@ -1548,7 +1549,7 @@ bool column_cut_alone(ColumnShape& s, const JitKernels& jk, OutputMemory memory)
     // microseconds, at ~9000 warp instructions per SM and microsecond, or ~500 of one warp
     const float points = (float)s.plane * (float)s.steps;
     float point_us = points / 32.0f * jk.point_cost / (9000.0f * (float)num_sms());
-    float column_us = (float)best_load * (kColSetupWork * jk.column_setup + (float)best) * 8.0f * jk.column_step / 9000.0f;
+    float column_us = (float)best_load * column_unit_work(s, jk, best) * 8.0f * jk.column_step / 9000.0f;
     if (memory == kDeviceMemory) {
         point_us = std::max(point_us, 3.0f);
         column_us += 4.0f;

@@ -99,6 +99,7 @@ bool jit_batch_kernel(uint64_t hash, int variant, BatchKernel& out);
 // (0: not walked in columns), steps along it and the index of the first, steps per unit, units.
 struct ColumnShape {
     unsigned plane = 0, steps = 0, first = 0, len = 0, units = 0;
+    float rate = 0;                   // mean crossings of a state per step
 };
 
 // Whether a grid is to be walked in columns by the kernels `jk` (fn_column.cuh); if so `shape`
@@ -107,18 +108,27 @@ struct ColumnShape {
 bool jit_column_grid(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
 inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
 unsigned column_tiles(ColumnShape& shape, unsigned len);
-// Setting a unit up takes this much of the work that `column_setup` steps are (FBm(Perlin) 600000 x 3
-// takes 35 us in columns, 25 with the point kernel, and would seem to take 25 and 25).
-constexpr float kColSetupWork = 1.4f;
+// Work of a unit of `len` steps, in steps: setting it up, and rebuilding what a crossing leaves (a crossing
+// costs about 1.3 of a state's set-up: FBm(Perlin) 32^4 takes 20, 24, 38, 54 us at 0.06, 0.12, 0.31, 0.51
+// crossings a step; with the set-up not weighted, FBm(Perlin) 600000 x 3 seemed to take 25 us for 35).
+inline float column_unit_work(const ColumnShape& s, const JitKernels& jk, unsigned len)
+{
+    return 1.4f * jk.column_setup + (float)len * (1.0f + 1.3f * jk.column_setup * s.rate);
+}
 
-// Whether columns pay in a batch: a plane that is no multiple of 32 leaves lanes idle at every
-// step, so the steps' instructions (units of 16 steps) are set against the points', with 15 % for
-// the estimates.  128 requests, columns / points, us: FBm(Perlin) 2 x 50000 1409 / 228, 12 x 8000 287 / 219,
-// 24 x 4000 167 / 219; terrain 3 x 3 x 10000 2299 / 955, 33 x 3000 664 / 481.
+// Whether columns pay in a batch: the instructions of the steps (in units as column_tiles cuts
+// them, about 520 for claiming and closing one; a third less goes through where only one block fits on an
+// SM) against the points', with 15 % for the estimates.  A plane that is no multiple of 32 leaves
+// lanes idle at every step.  Columns / points, us: 128 requests of FBm(Perlin) 2 x 50000 1409 / 228,
+// 12 x 8000 287 / 219, 24 x 4000 167 / 219; of terrain 3 x 3 x 10000 2299 / 955, 33 x 3000 664 / 481; 64 of
+// FBm(Perlin) 32 x 32 x 32 x 2 380 / 250, 1000 x 62 at 0.5 crossings 111 / 92.
 inline bool column_pays(const ColumnShape& s, const JitKernels& jk)
 {
-    const float len = s.steps < 16 ? (float)s.steps : 16.0f;
-    return 32.0f * (float)column_chunks(s) * jk.column_step * (1.0f + kColSetupWork * jk.column_setup / len) < 0.85f * (float)s.plane * jk.point_cost;
+    const unsigned chunks = column_chunks(s);
+    unsigned len = s.steps < 16u ? s.steps : 16u;
+    if ((unsigned long long)chunks * s.steps < 8ull * len) len = (chunks * s.steps + 7u) / 8u;
+    const float unit = column_unit_work(s, jk, len) * jk.column_step + 520.0f, slow = jk.column_resident > 1 ? 1.0f : 1.5f;
+    return slow * 32.0f * (float)chunks * unit / (float)len < 0.85f * (float)s.plane * jk.point_cost;
 }
 void column_args(PointArgs& args, const ColumnShape& shape);
 
