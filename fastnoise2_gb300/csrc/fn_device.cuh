@@ -565,14 +565,11 @@ FND float supersimplex3(int seed, float x, float y, float z)
     return value;
 }
 
-// One copy per kernel where specialised: ~750 instructions inlined once per octave overflowed the
-// instruction cache (warps waited for instructions a third of the time): tileable terrain
-// 1024^2 208 -> 190 us.
-#ifdef FN_GRADIENT_TABLE
-__device__ __noinline__
-#else
-FND
-#endif
+// One copy per kernel: ~750 instructions inlined once per octave overflowed the instruction cache
+// of specialised kernels (warps waited for instructions a third of the time): tileable terrain
+// 1024^2 208 -> 185 us.  In the interpreter it keeps the other nodes closer together: terrain 100^3
+// 315 -> 276 us, SuperSimplex 4D 157 -> 158 us.
+static __device__ __noinline__
 float supersimplex4(int seed, float x, float y, float z, float w)
 {
     constexpr double kSkew4 = 1.0 / (kRoot5 + 1.0);
