@@ -62,6 +62,26 @@ def test_positions_written_just_before(setup):
         assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32)), k
 
 
+@pytest.mark.parametrize("n", [4096, 30_720, 300_032])
+def test_positions_rewritten_by_the_kernel_between(setup, n):
+    """A grid call writes the array that the position calls before and after it read."""
+    torch, nodes = setup
+    stream = torch.cuda.Stream()
+    steps = 30
+    x, rest = torch.zeros(n, device="cuda"), [torch.rand(n, device="cuda") * 50 for _ in range(2)]
+    outs = [torch.empty(n, device="cuda") for _ in range(steps)]
+    torch.cuda.synchronize()
+    for k in range(steps):
+        nodes["fbm"].gen_uniform_grid_device(x.data_ptr(), (0.0,) * 3, (n // 32, 32, 1), (9.0,) * 3, k, 0, stream.cuda_stream)
+        nodes["cells"].gen_position_array_device(outs[k].data_ptr(), n, [x.data_ptr(), rest[0].data_ptr(), rest[1].data_ptr()],
+                                                 (0.0,) * 3, 9, 0, stream.cuda_stream)
+    stream.synchronize()
+    for k in range(steps):
+        px, _ = nodes["fbm"].gen_uniform_grid((0.0,) * 3, (n // 32, 32, 1), (9.0,) * 3, k)
+        ref, _ = nodes["cells"].gen_position_array([px] + [r.cpu().numpy() for r in rest], (0.0,) * 3, 9)
+        assert np.array_equal(outs[k].cpu().numpy().view(np.uint32), ref.view(np.uint32)), k
+
+
 def test_captured_calls_replay(setup):
     torch, nodes = setup
     count = (40, 33, 20)
