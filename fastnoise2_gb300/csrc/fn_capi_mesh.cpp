@@ -454,7 +454,7 @@ int fnBuildChunkMeshHeightmap(const void* node, int size, int posX, int posZ, in
     if (!ensure_runnable(prog)) return FN_ERR_COMPILE;
     const int sg = size + 1;
     MeshCtx& m = t_mesh;
-    if (!m.reserve((size_t)sg * sg, 0)) return FN_ERR_CUDA;
+    if (!m.reserve((size_t)sg * sg, 0) || !m.reserve_host(1)) return FN_ERR_CUDA;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     MinMaxWork* work = work_for_stream(s);
     if (!work) return FN_ERR_CUDA;
