@@ -205,11 +205,13 @@ ColPlan column_plan(const CompiledProgram& prog)
             break;
         case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: {
             // constant jitter, no size jitter, distances that are sums of squares (the 2D value
-            // walk takes the root of Euclidean ones), the closest cell or two
+            // walk takes the root of Euclidean ones), the closest cell or two.  A jitter whose
+            // square could overflow is left to the point function, which keeps its initial result
+            // (hash or cell point 0) where every distance is infinite.
             const int df = I.aux & 15, slots = I.op == FN_OP_CELL_DIST ? std::max((I.aux >> 4) & 3, (I.aux >> 8) & 3) + 1 : ((I.aux >> 4) & 3) + 1;
             const Reg jit = R[I.b];
             const bool sums = df == 1 || (df == 0 && !(I.op == FN_OP_CELL_VALUE && D == 2));
-            if (D < 4 && sums && jit.kind == Reg::kConst && std::isfinite(jit.scale) && I.c == FN_REG_NONE && I.d == FN_REG_NONE &&
+            if (D < 4 && sums && jit.kind == Reg::kConst && std::fabs(jit.scale) <= 1e9f && I.c == FN_REG_NONE && I.d == FN_REG_NONE &&
                 (I.op == FN_OP_CELL_LOOKUP || slots <= (I.op == FN_OP_CELL_DIST ? 2 : 1))) {
                 const std::string kind = I.op == FN_OP_CELL_VALUE ? "kColValue" : I.op == FN_OP_CELL_DIST ? "kColDistance" : "kColLookup";
                 // CellCol's part of the table (kTable there)
