@@ -114,6 +114,7 @@ def _declare(L):
         "fnJitSetCacheDir": (c_int, [ctypes.c_char_p]),
         "fnJitGetCacheInfo": (c_int, [ctypes.c_char_p, c_int, ctypes.POINTER(ctypes.c_ulonglong), ctypes.POINTER(ctypes.c_ulonglong)]),
         "fnSetJitEnabled": (c_int, [c_int]),
+        "fnSetGridRoute": (c_int, [c_int, c_int]),
         "fnSetAutoSpecialise": (c_int, [c_int]),
         "fnAutoSpecialiseWait": (c_int, [c_int]),
         "fnJitIsSpecialised": (c_int, [vp, c_int]),
@@ -294,6 +295,18 @@ def jit_compile(pairs) -> None:
     nodes, dims = _jit_arrays(pairs)
     if lib().fnJitCompile(nodes, dims, len(pairs)) != 0:
         _check()
+
+
+GRID_ROUTE_AUTO, GRID_ROUTE_POINTS, GRID_ROUTE_COLUMNS = 0, 1, 2
+
+
+def set_grid_route(route: int, column_steps: int = 0) -> int:
+    """fnSetGridRoute: which kernel this thread's grids take; returns how many it walked in columns
+    since the last call."""
+    n = lib().fnSetGridRoute(int(route), int(column_steps))
+    if n < 0:
+        _check()
+    return n
 
 
 MESH_DENSITY_ARRAY, MESH_DENSITY_SPARSE = 0, 1

@@ -250,7 +250,8 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     for (size_t i = 0; jit && i < n; ++i) {
         const JitKernels& jk = trees[tree_of_[i]].jk;
         ColumnShape shape;
-        if (!jk.batch_column || !jit_column_grid(items[i].args, jk, shape) || !column_pays(shape, jk)) continue;
+        if (!jit_batch_columns(items[i].args, jk, shape)) continue;
+        ++grid_route().columns;
         columns_[i] = shape;
         column_work += (double)shape.steps * column_chunks(shape);
     }

@@ -1703,6 +1703,21 @@ int fnJitCheckBatchVariants(const void* const* nodes, const int* dims, int count
     return FN_OK;
 }
 
+int fnSetGridRoute(int route, int columnSteps)
+{
+    clear_error();
+    if (route < FN_GRID_ROUTE_AUTO || route > FN_GRID_ROUTE_COLUMNS || columnSteps < 0) {
+        set_error(FN_ERR_ARG, "invalid grid route");
+        return FN_ERR_ARG;
+    }
+    GridRoute& r = grid_route();
+    const int columns = (int)r.columns;
+    r.route = route;
+    r.steps = (unsigned)columnSteps;
+    r.columns = 0;
+    return columns;
+}
+
 int fnSetJitEnabled(int enabled)
 {
     const int was = jit_enabled() ? 1 : 0;

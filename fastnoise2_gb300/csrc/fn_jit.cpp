@@ -23,6 +23,7 @@
 #include <sys/stat.h>
 #include <unistd.h>
 
+#include "FastNoise/FastNoise_C.h"
 #include "fn_kernels.cuh"
 #include "fn_runtime.h"
 
@@ -1478,14 +1479,33 @@ bool jit_auto_wait(int timeout_ms)
 
 constexpr double kColMaxGroups = 3.0;
 
-// A tree without a column kernel, other point sources and partial planes are not walked.
-bool jit_column_grid(const PointArgs& a, const JitKernels& jk, ColumnShape& shape)
+GridRoute& grid_route()
+{
+    thread_local GridRoute r;
+    return r;
+}
+
+namespace {
+
+// The plane and steps of a grid.  A tree without a column kernel, other point sources and partial
+// planes are not walked.
+bool column_shape(const PointArgs& a, const JitKernels& jk, ColumnShape& shape)
 {
     if (a.src != kSrcGrid || a.total <= 0 || a.total > (1ll << 31) || !jk.column) return false;
     long long plane = 1;
     for (int k = 0; k < a.dim - 1; ++k) plane *= a.count[k];
     if (plane <= 0) return false;
-    if ((a.base || a.total != plane * a.count[a.dim - 1]) && (a.total % plane || a.base % plane)) return false;
+    const bool whole = !a.base && a.total == plane * a.count[a.dim - 1];
+    if (!whole && (a.total % plane || a.base % plane)) return false;
+    shape.plane = (unsigned)plane;
+    shape.steps = whole ? (unsigned)a.count[a.dim - 1] : (unsigned)(a.total / plane);
+    shape.first = a.base ? a.base / (unsigned)plane : 0u;
+    return true;
+}
+
+// How often its steps enter other cells, and whether that is seldom enough.
+bool column_rate(const PointArgs& a, const JitKernels& jk, ColumnShape& shape)
+{
     // A step that crosses into another lattice cell rebuilds a Perlin state at about the cost
     // of the point function: FBm(Perlin) 128^3 (69.7 us with the point kernel) takes 27, 39, 53,
     // 70 and 86 us at 0.06, 0.25, 0.40, 0.62 and 0.79 crossings a step.  Value states never lose.
@@ -1506,14 +1526,9 @@ bool jit_column_grid(const PointArgs& a, const JitKernels& jk, ColumnShape& shap
         rate += r < 1.0f ? r : 1.0f;
     }
     if (jk.n_column_rates && !(rate < 0.6f * (float)jk.n_column_rates)) return false;
-    shape.plane = (unsigned)plane;
-    shape.steps = a.base || a.total != plane * a.count[a.dim - 1] ? (unsigned)(a.total / plane) : (unsigned)a.count[a.dim - 1];
-    shape.first = a.base ? a.base / (unsigned)plane : 0u;
     shape.rate = jk.n_column_rates ? rate / (float)jk.n_column_rates : 0.0f;
     return true;
 }
-
-namespace {
 
 // Cut the columns into units of at most `len` steps, evenly.
 void column_cut(ColumnShape& s, unsigned len)
@@ -1523,8 +1538,8 @@ void column_cut(ColumnShape& s, unsigned len)
     s.units = column_chunks(s) * ((s.steps + s.len - 1) / s.len);
 }
 
-// Cut a launch that has the GPU to itself, and say whether it should be walked in columns at
-// all (false: the point kernel).
+// Cut a launch that has the GPU to itself, and say whether walking it in columns is faster than
+// the point kernel.
 //
 // Steps per unit: setting a unit up costs `column_setup` steps (about 7 for FBm(Perlin): 256^3
 // takes 221, 170, 147 us at 8, 16, 32 steps a unit; a fraction of one for a terrain tree), and an
@@ -1567,15 +1582,37 @@ bool column_cut_alone(ColumnShape& s, const JitKernels& jk, OutputMemory memory)
         column_us = std::max(column_us, (jk.column_setup + (float)best) * jk.column_step / 500.0f) + 0.7f;
         if (memory == kPageable) column_us = std::max(column_us, points * 4.0f / 130e3f);
     }
-    if (!(column_us < point_us)) return false;
     column_cut(s, best);
-    return true;
+    return column_us < point_us;
+}
+
+// Whether a launch of its own walks a grid in columns, and its shape if so.
+bool column_alone(const PointArgs& a, const JitKernels& jk, OutputMemory memory, ColumnShape& s)
+{
+    const GridRoute& r = grid_route();
+    if (r.route == FN_GRID_ROUTE_POINTS || !column_shape(a, jk, s)) return false;
+    const bool asked = r.route == FN_GRID_ROUTE_COLUMNS;
+    if (!column_rate(a, jk, s) && !asked) return false;
+    const bool faster = column_cut_alone(s, jk, memory);
+    if (r.steps) column_cut(s, r.steps);
+    return faster || asked;
 }
 
 }  // namespace
 
+bool jit_batch_columns(const PointArgs& a, const JitKernels& jk, ColumnShape& s)
+{
+    const GridRoute& r = grid_route();
+    if (!jk.batch_column || r.route == FN_GRID_ROUTE_POINTS || !column_shape(a, jk, s)) return false;
+    return r.route == FN_GRID_ROUTE_COLUMNS || (column_rate(a, jk, s) && column_pays(s, jk));
+}
+
 unsigned column_tiles(ColumnShape& s, unsigned len)
 {
+    if (grid_route().steps) {
+        column_cut(s, grid_route().steps);
+        return (s.units + 7) / 8;
+    }
     // a request with fewer units than a block has warps is cut finer
     const unsigned long long work = (unsigned long long)column_chunks(s) * s.steps;
     column_cut(s, (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(len, (work + 7) / 8)));
@@ -1616,7 +1653,8 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     if (args.total <= 0 || args.total > (1ll << 31) || !jit_lookup(hash, jk)) return false;
     const int which = args.src == kSrcGrid ? 0 : args.src == kSrcPositions ? 1 : 2;
     ColumnShape shape;
-    if (which == 0 && jit_column_grid(args, jk, shape) && column_cut_alone(shape, jk, memory)) {
+    if (which == 0 && column_alone(args, jk, memory, shape)) {
+        ++grid_route().columns;
         PointArgs c = args;
         column_args(c, shape);
         const unsigned grid = std::min<unsigned>((shape.units + 7) / 8, (unsigned)kMaxReduceBlocks);

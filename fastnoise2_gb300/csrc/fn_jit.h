@@ -102,10 +102,19 @@ struct ColumnShape {
     float rate = 0;                   // mean crossings of a state per step
 };
 
-// Whether a grid is to be walked in columns by the kernels `jk` (fn_column.cuh); if so `shape`
-// gets its plane and steps.  column_tiles cuts it into units of at most `len` steps and returns
-// a batch's work items for it (eight units each).
-bool jit_column_grid(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
+// The calling thread's route for grids of trees that have a column kernel (fnSetGridRoute): by
+// estimate, or always through the point or the column kernel; steps per unit (0: by estimate).
+struct GridRoute {
+    int route = 0;                    // FN_GRID_ROUTE_*
+    unsigned steps = 0;
+    unsigned columns = 0;             // grids walked in columns since the route was last set
+};
+GridRoute& grid_route();
+
+// Whether a request of a batch is to be walked in columns by the kernels `jk` (fn_column.cuh); if
+// so `shape` gets its plane and steps.  column_tiles cuts it into units of at most `len` steps and
+// returns the batch's work items for it (eight units each).
+bool jit_batch_columns(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
 inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
 unsigned column_tiles(ColumnShape& shape, unsigned len);
 // Work of a unit of `len` steps, in steps: setting it up, and rebuilding what a crossing leaves (a crossing

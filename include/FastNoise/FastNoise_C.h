@@ -449,6 +449,19 @@ FASTNOISE_API int fnJitCheckBatchVariants(const void* const* nodes, const int* d
  * Returns the previous setting. */
 FASTNOISE_API int fnSetJitEnabled(int enabled);
 
+/* How the calling thread's uniform grids run (no counterpart in the reference; for tests and
+ * measurements).  A specialised tree with separable lattice noise has two kernels for grids, one
+ * that evaluates points and one that walks columns along the last axis; the results are the same
+ * bit for bit, and by default the library takes the one it estimates to be faster.  POINTS and
+ * COLUMNS ask for one of them, for calls and for requests of fnGenBatchDevice (a tree that has no
+ * column kernel keeps to points); columnSteps is the number of steps a unit of columns takes (0:
+ * as estimated).  Returns the number of grids that this thread has walked in columns since it last
+ * called this, or FN_ERR_ARG. */
+#define FN_GRID_ROUTE_AUTO 0
+#define FN_GRID_ROUTE_POINTS 1
+#define FN_GRID_ROUTE_COLUMNS 2
+FASTNOISE_API int fnSetGridRoute(int route, int columnSteps);
+
 /* No counterpart in the reference.  fnGenUniformGrid3DDevice for callers that
  * cannot let the library allocate device memory: applications whose own pool
  * allocator takes all device memory at start-up (a library cudaMalloc would then
