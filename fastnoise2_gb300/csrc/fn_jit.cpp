@@ -629,11 +629,12 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax)\n{\n"
           << "    __shared__ float4 tab[8][" << plan.table << "];\n"
           << "    __shared__ float smn[8], smx[8];\n"
-          << "    fne::let_stream_continue();\n"
+          << "    if (A.early) fne::let_stream_continue();\n"
           << gradient_setup(prog, &plan)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
           << "        fnjit_colunit_" << id << "(A, out, u, tab[threadIdx.x >> 5], mn, mx);\n"
+          << "    fne::let_stream_continue();\n"
           << "    fne::grid_minmax(mn, mx, work, dminmax, smn, smx);\n"
           << "}\n\n";
     }
@@ -643,17 +644,14 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
     call += ")";
 
     auto kernel = [&](const char* name, const std::string& prologue, const std::string& position) {
-        // prologue: before the first point.  A kernel that reads the caller's arrays waits there, and
-        // where its blocks leave SMs free it lets the next launch begin only behind its own
-        // points: blocks that begin earlier only wait too, and crowd onto some SMs (terrain 4D at
-        // 30000 positions 42 us back to back, 25 so; with the SMs full the early start is
-        // slightly better: blend at 1 M positions 15.7 against 15.9 us).
+        // prologue: before the first point (a kernel that reads the caller's arrays waits there).  See
+        // begin_early for A.early.
         const bool waits = !prologue.empty();
         o << "extern \"C\" __global__ void __launch_bounds__(256, 4) " << name << "_" << k
           << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned ppl)\n{\n"
           << "    __shared__ float4 stage[8][32];\n"
           << "    __shared__ float smn[8], smx[8];\n"
-          << (waits ? "    if (gridDim.x > 512u) fne::let_stream_continue();\n" : "    fne::let_stream_continue();\n")
+          << (waits ? "    if (A.early) fne::let_stream_continue();\n" : "    fne::let_stream_continue();\n")
           << gradient_setup(prog)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    const unsigned total = (unsigned)A.total;\n"
@@ -1645,6 +1643,14 @@ cudaError_t launch_overlapped(cudaKernel_t k, unsigned grid, void** params, cuda
     return cudaLaunchKernelExC(&cfg, (const void*)k, params);
 }
 
+// Whether the launch behind a column or position kernel of `blocks` may begin at once: where its
+// blocks fill the SMs.  Where they leave SMs free, the next launch's blocks would take what is left of the
+// occupied SMs too, run with them and crowd there, launch after launch; so it begins behind the
+// points.  Back to back, us, at once / behind: terrain 2D 669 x 1365 in units of 32 steps (0.7
+// blocks per SM) 104 / 52, of 16 (1.5) 62 / 35; CellularLookup 2D 1054 x 519 15.0 / 8.8; terrain 4D
+// at 30000 positions 42 / 25; blend at 1 M positions (SMs full) 15.7 / 15.9.
+unsigned begin_early(unsigned blocks, int resident) { return blocks >= (unsigned)(num_sms() * std::max(1, resident)) ? 1u : 0u; }
+
 bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* work, float* dminmax, cudaStream_t stream,
                 cudaError_t& err, OutputMemory memory)
 {
@@ -1658,6 +1664,7 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
         PointArgs c = args;
         column_args(c, shape);
         const unsigned grid = std::min<unsigned>((shape.units + 7) / 8, (unsigned)kMaxReduceBlocks);
+        c.early = begin_early(grid, jk.column_resident);
         void* params[] = {&c, &out, &work, &dminmax};
         err = launch_overlapped(jk.column, grid, params, stream);
         return true;
@@ -1683,6 +1690,7 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     if (blocks > kMaxReduceBlocks) blocks = kMaxReduceBlocks;
     if (blocks < 1) blocks = 1;
     PointArgs a = args;
+    a.early = begin_early((unsigned)blocks, jk.resident[which]);
     void* params[] = {&a, &out, &work, &dminmax, &ppl};
     err = launch_overlapped(k, (unsigned)blocks, params, stream);
     return true;
