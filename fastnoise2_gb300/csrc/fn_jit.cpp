@@ -626,10 +626,10 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
         const std::string id = std::to_string(k);
         emit_column_unit(prog, "fnjit_ceval_" + id, "fnjit_colunit_" + id, o);
         o << "extern \"C\" __global__ void __launch_bounds__(256, " << column_blocks(plan) << ") fnjit_col_" << id
-          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax)\n{\n"
+          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned early)\n{\n"
           << "    __shared__ float4 tab[8][" << plan.table << "];\n"
           << "    __shared__ float smn[8], smx[8];\n"
-          << "    if (A.early) fne::let_stream_continue();\n"
+          << "    if (early) fne::let_stream_continue();\n"
           << gradient_setup(prog, &plan)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
@@ -645,13 +645,13 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
 
     auto kernel = [&](const char* name, const std::string& prologue, const std::string& position) {
         // prologue: before the first point (a kernel that reads the caller's arrays waits there).  See
-        // begin_early for A.early.
+        // begin_early for early.
         const bool waits = !prologue.empty();
         o << "extern \"C\" __global__ void __launch_bounds__(256, 4) " << name << "_" << k
-          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned ppl)\n{\n"
+          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned ppl, unsigned early)\n{\n"
           << "    __shared__ float4 stage[8][32];\n"
           << "    __shared__ float smn[8], smx[8];\n"
-          << (waits ? "    if (A.early) fne::let_stream_continue();\n" : "    fne::let_stream_continue();\n")
+          << (waits ? "    if (early) fne::let_stream_continue();\n" : "    fne::let_stream_continue();\n")
           << gradient_setup(prog)
           << "    float mn = fne::inf(), mx = -fne::inf();\n"
           << "    const unsigned total = (unsigned)A.total;\n"
@@ -1664,8 +1664,8 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
         PointArgs c = args;
         column_args(c, shape);
         const unsigned grid = std::min<unsigned>((shape.units + 7) / 8, (unsigned)kMaxReduceBlocks);
-        c.early = begin_early(grid, jk.column_resident);
-        void* params[] = {&c, &out, &work, &dminmax};
+        unsigned early = begin_early(grid, jk.column_resident);
+        void* params[] = {&c, &out, &work, &dminmax, &early};
         err = launch_overlapped(jk.column, grid, params, stream);
         return true;
     }
@@ -1690,8 +1690,8 @@ bool jit_launch(uint64_t hash, const PointArgs& args, float* out, MinMaxWork* wo
     if (blocks > kMaxReduceBlocks) blocks = kMaxReduceBlocks;
     if (blocks < 1) blocks = 1;
     PointArgs a = args;
-    a.early = begin_early((unsigned)blocks, jk.resident[which]);
-    void* params[] = {&a, &out, &work, &dminmax, &ppl};
+    unsigned early = begin_early((unsigned)blocks, jk.resident[which]);
+    void* params[] = {&a, &out, &work, &dminmax, &ppl, &early};
     err = launch_overlapped(k, (unsigned)blocks, params, stream);
     return true;
 }

@@ -32,9 +32,6 @@ struct PointArgs {
     // Column launches (grids walked along their last axis): points of the plane across it, steps
     // of this launch along it and the index of the first, steps per work unit and units.
     unsigned int col_plane, col_steps, col_first, col_len, col_units;
-    // Per-call launches of column and position kernels: whether the stream's next launch may begin at
-    // once (1) or behind this one's points.
-    unsigned int early;
 };
 
 // Per-launch reduction workspace.  Every block folds its min/max into the two
