@@ -97,6 +97,7 @@ private:
     // per request of a launch, kept to save their allocation: tree, column shape, work items, group
     std::vector<uint32_t> tree_of_, tiles_, group_of_;
     std::vector<ColumnShape> columns_;
+    std::vector<float> saved_;
     std::map<cudaKernel_t, int> occupancy_;
     uint64_t signature_ = 0;
     uint64_t points_ = 0;

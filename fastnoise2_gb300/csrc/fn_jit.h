@@ -25,8 +25,10 @@ namespace fn {
 
 constexpr int kMaxColumnStates = 10;
 
-struct ColumnRate {                   // lattice cells per unit along the grid's axes, of one column state
-    float scale[4] = {};
+struct ColumnRate {                   // of one column state
+    float scale[4] = {};              // lattice cells per unit along the grid's axes
+    float enter = 0, step = 0;        // issue slots of entering a cell (per neighbourhood if cellular), of a step,
+    float point = 0;                  // and of the point function
     bool cellular = false;
 };
 
@@ -38,10 +40,9 @@ struct JitKernels {
     cudaKernel_t list = nullptr;      // chunk meshing (3D programs): grid values at listed point indices
     cudaKernel_t column = nullptr;    // grids walked along their last axis (trees with separable lattice noise)
     cudaKernel_t batch_column = nullptr;   // the same for a batch's grid requests
-    ColumnRate column_rates[kMaxColumnStates];   // of its Perlin and cellular states
+    ColumnRate column_rates[kMaxColumnStates];   // of its states
     int n_column_rates = 0;
-    float column_setup = 1.0f;        // set-up of a unit of columns, in steps
-    float column_step = 1.0f, point_cost = 1.0f;   // instructions of a step of a column, of a point otherwise
+    float column_step = 1.0f, point_cost = 1.0f;   // issue slots of a step of a column, of a point otherwise
     int column_resident = 1;          // its 256-thread blocks per SM at once
     int slot = -1;                    // index in the module's batch kernel
     int resident[3] = {1, 1, 1};      // 256-thread blocks per SM of grid / positions / tileable at once
@@ -99,7 +100,9 @@ bool jit_batch_kernel(uint64_t hash, int variant, BatchKernel& out);
 // (0: not walked in columns), steps along it and the index of the first, steps per unit, units.
 struct ColumnShape {
     unsigned plane = 0, steps = 0, first = 0, len = 0, units = 0;
-    float rate = 0;                   // mean crossings of a state per step
+    // issue slots of a step, and of entering cells at a unit's first step and per step after it;
+    // how long a step of one warp takes
+    float step = 0, enter = 0, cross = 0, step_us = 0;
 };
 
 // The calling thread's route for grids of trees that have a column kernel (fnSetGridRoute): by
@@ -111,34 +114,13 @@ struct GridRoute {
 };
 GridRoute& grid_route();
 
-// Whether a request of a batch is to be walked in columns by the kernels `jk` (fn_column.cuh); if
-// so `shape` gets its plane and steps.  column_tiles cuts it into units of at most `len` steps and
-// returns the batch's work items for it (eight units each).
-bool jit_batch_columns(const PointArgs& args, const JitKernels& jk, ColumnShape& shape);
+// Whether a request of a batch can be walked in columns by the kernels `jk` (fn_column.cuh); if so
+// `shape` gets its plane and steps, and `saved_us` the time that saves (negative: loses).  column_tiles
+// cuts it into units of at most `len` steps and returns the batch's work items for it (eight units
+// each).
+bool jit_batch_columns(const PointArgs& args, const JitKernels& jk, ColumnShape& shape, float& saved_us);
 inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
 unsigned column_tiles(ColumnShape& shape, unsigned len);
-// Work of a unit of `len` steps, in steps: setting it up, and rebuilding what a crossing leaves (a crossing
-// costs about 1.3 of a state's set-up: FBm(Perlin) 32^4 takes 20, 24, 38, 54 us at 0.06, 0.12, 0.31, 0.51
-// crossings a step; with the set-up not weighted, FBm(Perlin) 600000 x 3 seemed to take 25 us for 35).
-inline float column_unit_work(const ColumnShape& s, const JitKernels& jk, unsigned len)
-{
-    return 1.4f * jk.column_setup + (float)len * (1.0f + 1.3f * jk.column_setup * s.rate);
-}
-
-// Whether columns pay in a batch: the instructions of the steps (in units as column_tiles cuts
-// them, about 520 for claiming and closing one; a third less goes through where only one block fits on an
-// SM) against the points', with 15 % for the estimates.  A plane that is no multiple of 32 leaves
-// lanes idle at every step.  Columns / points, us: 128 requests of FBm(Perlin) 2 x 50000 1409 / 228,
-// 12 x 8000 287 / 219, 24 x 4000 167 / 219; of terrain 3 x 3 x 10000 2299 / 955, 33 x 3000 664 / 481; 64 of
-// FBm(Perlin) 32 x 32 x 32 x 2 380 / 250, 1000 x 62 at 0.5 crossings 111 / 92.
-inline bool column_pays(const ColumnShape& s, const JitKernels& jk)
-{
-    const unsigned chunks = column_chunks(s);
-    unsigned len = s.steps < 16u ? s.steps : 16u;
-    if ((unsigned long long)chunks * s.steps < 8ull * len) len = (chunks * s.steps + 7u) / 8u;
-    const float unit = column_unit_work(s, jk, len) * jk.column_step + 520.0f, slow = jk.column_resident > 1 ? 1.0f : 1.5f;
-    return slow * 32.0f * (float)chunks * unit / (float)len < 0.85f * (float)s.plane * jk.point_cost;
-}
 void column_args(PointArgs& args, const ColumnShape& shape);
 
 // Queue a background build of the batch variants of `prog` (a tuning table loaded in this

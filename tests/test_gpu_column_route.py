@@ -128,25 +128,39 @@ def test_captured_column_calls(columns):
         assert_parity(outs[k].cpu().numpy(), tuple(mm[k].tolist()), ref, rmm, label=name)
 
 
-# (tree, grid, step along every axis, walked in columns alone / in a batch): the estimate's side of each
-RULE = [("FBmPerlin", (256, 256, 256), 1.0, 1, 1), ("FBmPerlin", (16, 16, 16), 1.0, 0, 1), ("FBmPerlin", (128, 128, 128), 40.0, 0, 0),
-        ("Terrain", (128, 128, 128), 1.0, 1, 1), ("Terrain", (3, 3, 2000), 1.0, 0, 0), ("CellValue", (160, 160, 160), 1.0, 1, 1),
-        ("CellValue", (160, 160, 160), 60.0, 0, 0), ("CellLookup", (2, 2, 2), 1.0, 0, 0), ("Value", (1024, 1024), 1.0, None, 1),
-        ("FBmPerlin", (2, 50000), 1.0, 0, 0)]
+# (tree, grid, step along every axis, requests, walked in columns alone / in a batch of as many): the
+# estimate's side of each.  The last are grids that columns take longer over than points: Value states
+# that often enter cells, warps with more neighbourhoods than the table holds, 4D super-simplex
+# beside a column state, batches too small to gain a column kernel's longer first and last units.
+RULE = [("FBmPerlin", (256, 256, 256), 1.0, 1, 1, 1), ("FBmPerlin", (16, 16, 16), 1.0, 1, 0, 0), ("FBmPerlin", (32, 32, 32), 1.0, 200, 0, 1),
+        ("Terrain", (128, 128, 128), 1.0, 4, 1, 1), ("CellValue", (160, 160, 160), 1.0, 2, 1, 1), ("Value", (1024, 1024), 1.0, 12, None, 1),
+        ("CellLookup", (97, 90, 101), 1.0, 8, 1, 1),
+        ("FBmPerlin", (128, 128, 128), 40.0, 4, 0, 0), ("Terrain", (3, 3, 2000), 1.0, 64, 0, 0), ("FBmPerlin", (2, 50000), 1.0, 16, 0, 0),
+        ("FBmValueShort", (1076, 2092), 3.3, 4, 0, 0), ("FBmValueShort", (691, 284), 2.92, 42, 0, 0), ("CellValue", (160, 160, 160), 60.0, 2, 0, 0),
+        ("CellValue", (26, 64, 144), 1.4, 1, 0, 0), ("FadeSuper4D", (75, 37, 21, 58), 1.0, 1, 0, None), ("FBmPerlin2", (95, 227), 2.9, 64, 0, 0),
+        ("CellLookup", (2, 2, 2), 1.0, 8, 0, 0)]
+RULE_TREES = {"FBmValueShort": lambda: N("FractalFBm", Source=N("Value", Feature_Scale=9.0), Octaves=5),
+              "FBmPerlin2": lambda: N("FractalFBm", Source=N("Perlin", Feature_Scale=20.0), Octaves=2),
+              "FadeSuper4D": lambda: N("Fade", A=N("FractalFBm", Source=N("SuperSimplex", Feature_Scale=30.0), Octaves=2),
+                                       B=N("CellularDistance", Feature_Scale=30.0), Fade=N("Perlin", Feature_Scale=50.0))}
 
 
-@pytest.mark.parametrize("name,count,step,alone,batch", RULE)
-def test_the_estimates_route(columns, name, count, step, alone, batch):
-    node, dim = columns[name], len(count)
+@pytest.mark.parametrize("name,count,step,requests,alone,batch", RULE)
+def test_the_estimates_route(columns, name, count, step, requests, alone, batch):
+    dim = len(count)
+    node = columns[name] if name in columns else trees.to_product(RULE_TREES[name]())
+    if name not in columns:
+        fn.jit_compile([(node, dim)])
     out = torch.empty(int(np.prod(count)), device="cuda")
     fn.set_grid_route(fn.GRID_ROUTE_AUTO)
     node.gen_uniform_grid_device(out.data_ptr(), (0.0,) * dim, count, (step,) * dim, 3)
     walked = fn.set_grid_route(fn.GRID_ROUTE_AUTO)
     assert alone is None or walked == alone
-    kind = {2: fn.KIND_GRID2D, 3: fn.KIND_GRID3D}[dim]
-    fn.gen_batch([fn.make_request(node, kind, out.data_ptr(), 3, count, (0.0,) * dim, (step,) * dim)])
-    assert fn.set_grid_route(fn.GRID_ROUTE_AUTO) == batch
-    fn.set_grid_route(fn.GRID_ROUTE_POINTS)
+    kind = {2: fn.KIND_GRID2D, 3: fn.KIND_GRID3D, 4: fn.KIND_GRID4D}[dim]
+    outs = torch.empty((requests, out.numel()), device="cuda")
+    fn.gen_batch([fn.make_request(node, kind, o.data_ptr(), 3, count, (0.0,) * dim, (step,) * dim) for o in outs])
+    walked = fn.set_grid_route(fn.GRID_ROUTE_POINTS)
+    assert batch is None or walked == batch * requests
     node.gen_uniform_grid_device(out.data_ptr(), (0.0,) * dim, count, (step,) * dim, 3)
     torch.cuda.synchronize()
     assert fn.set_grid_route(fn.GRID_ROUTE_AUTO) == 0
