@@ -699,7 +699,7 @@ constexpr unsigned kDmcLine = 32;          // words between counters
 // blockIdx.y): one after another, a chunk's passes are too short to fill the GPU and each waits
 // for the one before, and beside the density kernels of other chunks they wait for those blocks
 // to end (eight 128^3 chunks of a terrain surface: on
-// four streams 714 us; together, with the passes as they now are, 570 us).
+// four streams 714 us; together 570 us).
 template <class S>
 struct DmcPass {
     DmcGrid<S> g;
@@ -961,6 +961,12 @@ __device__ __forceinline__ unsigned dmc_vertex_index(const DmcPass<S>& m, unsign
     return m.tile_at[cell / kDmcTile].x + (marks >> 12) + __popc(marks & ((1u << bit) - 1u));
 }
 
+// Whether a chunk's vertices and indices both fit its buffers: it writes all of them or none.
+__device__ __forceinline__ bool dmc_fits(uint2 total, const DmcChunk& chunk)
+{
+    return total.x <= chunk.vcap && (unsigned long long)total.y * 6ull <= chunk.icap;
+}
+
 // Vertex pass: one thread per created vertex; a tile's go to consecutive places.
 template <class S>
 __global__ void dmc_vertices(DmcPass<S> all, float iso, float3 nl, DmcChunks chunks)
@@ -970,7 +976,7 @@ __global__ void dmc_vertices(DmcPass<S> all, float iso, float3 nl, DmcChunks chu
     fne::wait_for_stream();
     const DmcGrid<S>& g = m.g;
     const DmcChunk& chunk = chunks.chunk[blockIdx.y];
-    if (m.total()->x > chunk.vcap) return;
+    if (!dmc_fits(*m.total(), chunk)) return;
     const unsigned items = m.lists.counters[0];
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < items; j += gridDim.x * blockDim.x) {
         const unsigned it = m.lists.vert_items[j];
@@ -1000,8 +1006,7 @@ __global__ void dmc_quads(DmcPass<S> all, float iso, DmcChunks chunks)
     const DmcLists& lists = m.lists;
     const DmcChunk& chunk = chunks.chunk[blockIdx.y];
     const MeshVertex* verts = chunk.verts;
-    const uint2 tot = *m.total();
-    const bool fits = tot.x <= chunk.vcap && (unsigned long long)tot.y * 6ull <= chunk.icap;
+    const bool fits = dmc_fits(*m.total(), chunk);
     const unsigned items = lists.counters[kDmcLine];
     unsigned air = 0xFFFFFFFFu, solid = 0u;
     for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < items; j += gridDim.x * blockDim.x) {
