@@ -121,6 +121,16 @@ struct MeshCtx {
         return true;
     }
 
+    // Gives the density and mesher arrays back, so that smaller ones can take their place.
+    void release_arrays()
+    {
+        if (dens) cudaFree(dens);
+        if (dmc_block) cudaFree(dmc_block);
+        dens = nullptr;
+        dmc_block = nullptr;
+        dens_cap = dmc_cap = 0;
+    }
+
     bool reserve_host(size_t chunks)
     {
         if (chunks <= host_cap) return true;
@@ -285,6 +295,7 @@ bool enqueue_dmc_chunks(const DeviceProgram& prog, MeshCtx& m, cudaStream_t s, i
     while (!m.reserve(stride * group, 0) || !m.reserve_dmc(size, (unsigned)group)) {
         if (group == 1) return false;
         group = (group + 1) / 2;                // no memory for so many: fewer together
+        m.release_arrays();
         cudaGetLastError();
         clear_error();
     }
