@@ -173,7 +173,7 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     struct Tree {
         DeviceProgram prog;
         BatchKernel kernel;            // its specialised batch kernel
-        JitKernels jk;                 // its column kernel, unless a variant is forced
+        JitKernels jk;                 // its column kernel
         int group[2] = {-1, -1};       // launch group of its point / column requests
         double won = 0, lost = 0;      // microseconds that columns save over its requests, and lose
         bool column = false, split = false;
@@ -215,21 +215,20 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     }
     // Specialised batch kernels when every program of the batch has one: each tree's tuned
     // variant when it is built (a variant not built yet is queued for a background build and
-    // variant 0 runs meanwhile), or the variant a tuning run forces.
-    const int forced = tuning_in ? tuning_in->variant : -1;
+    // variant 0 runs meanwhile).
     for (size_t t = 0; jit && t < trees.size(); ++t) {
         Tree& tr = trees[t];
         const uint64_t hash = tr.prog.hash;
-        const int v = forced >= 0 ? forced : Autotuner::instance().tree_variant(hash);
+        const int v = Autotuner::instance().tree_variant(hash);
         bool ok = jit_batch_kernel(hash, v, tr.kernel);
         if (!ok && !jit_is_specialised(hash) && jit_try_cached(tr.prog.host))   // an earlier process built it
             ok = jit_batch_kernel(hash, v, tr.kernel);
         if (!ok && v != 0) {
-            if (forced < 0) jit_request_batch_variants(tr.prog.host);
+            jit_request_batch_variants(tr.prog.host);
             ok = jit_batch_kernel(hash, 0, tr.kernel);
         }
         if (!ok) { jit = false; break; }
-        if (forced >= 0 || !jit_lookup(hash, tr.jk)) tr.jk = JitKernels();   // a forced variant is run as asked
+        if (!jit_lookup(hash, tr.jk)) tr.jk = JitKernels();
     }
     if (!jit)                                       // interpreter batch: count a use of each program
         for (size_t t = 0; t < trees.size(); ++t) {
@@ -325,6 +324,9 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         n_items += tiles_[i];
     }
     if (n_items > 0xFFFFFFFFull) { set_error(-4, "batch too large"); return -4; }
+    point_trees_.clear();
+    for (const Tree& tr : trees)
+        if (tr.group[0] >= 0) point_trees_.push_back(tr.prog.hash);
     if (!reserve(n, n_items)) return -3;
 
     // The staging buffer is reused: the previous launch's upload must have been consumed.
@@ -465,7 +467,7 @@ std::vector<BatchTuning> Autotuner::candidates() const
 {
     std::vector<BatchTuning> c;
     for (uint32_t tp : {1024u, 2048u, 4096u, 8192u})
-        for (int ctas : {0, 1}) c.push_back(BatchTuning{tp, ctas, -1});
+        for (int ctas : {0, 1}) c.push_back(BatchTuning{tp, ctas});
     return c;
 }
 
@@ -474,6 +476,12 @@ int Autotuner::tree_variant(uint64_t program_hash)
     std::lock_guard<std::mutex> lk(mu_);
     auto it = trees_.find(program_hash);
     return it == trees_.end() ? 0 : it->second.first;
+}
+
+bool Autotuner::tree_tuned(uint64_t program_hash)
+{
+    std::lock_guard<std::mutex> lk(mu_);
+    return trees_.count(program_hash) != 0;
 }
 
 void Autotuner::store_tree(uint64_t program_hash, int variant, double ms)
@@ -507,7 +515,7 @@ bool Autotuner::load(const std::string& path)
             unsigned tp;
             int ctas;
             double ms;
-            if (in >> tp >> ctas >> ms) table_[sig] = {BatchTuning{tp, ctas, -1}, ms};
+            if (in >> tp >> ctas >> ms) table_[sig] = {BatchTuning{tp, ctas}, ms};
         }
     }
     return true;

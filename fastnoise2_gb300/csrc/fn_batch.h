@@ -27,7 +27,6 @@ struct BatchItem {
 struct BatchTuning {
     uint32_t tile_points = 2048;
     int ctas_per_sm = 0;               // 0 = occupancy limit
-    int variant = -1;                  // specialised kernel variant for every tree; -1 = each tree's tuned choice
 };
 
 // Owns the device/pinned descriptor buffers and a captured graph; not thread safe
@@ -56,6 +55,8 @@ public:
     int last_grid() const { return grid_; }
     bool last_specialised() const { return specialised_; }
     int last_kernels() const { return (int)groups_.size(); }
+    // Program hashes of the trees whose requests ran, all or some, on the point kernel.
+    const std::vector<uint64_t>& last_point_trees() const { return point_trees_; }
 
 private:
     // One kernel launch of a batch: the interpreter's batch kernel over all items
@@ -98,6 +99,7 @@ private:
     std::vector<uint32_t> tree_of_, tiles_, group_of_;
     std::vector<ColumnShape> columns_;
     std::vector<float> saved_;
+    std::vector<uint64_t> point_trees_;
     std::map<cudaKernel_t, int> occupancy_;
     uint64_t signature_ = 0;
     uint64_t points_ = 0;
@@ -118,6 +120,7 @@ public:
     void store(uint64_t signature, const BatchTuning& t, double ms);
     std::vector<BatchTuning> candidates() const;
     int tree_variant(uint64_t program_hash);                 // 0 when the tree has not been tuned
+    bool tree_tuned(uint64_t program_hash);
     void store_tree(uint64_t program_hash, int variant, double ms);
     bool load(const std::string& path);
     bool save(const std::string& path) const;

@@ -1227,12 +1227,14 @@ int fnAutotuneBatch(const fnGenRequest* requests, int count, void* stream)
         if (ms < best_ms) { best_ms = ms; best = t; }
     }
     Autotuner::instance().store(sig, best, best_ms / 2);
+    const std::vector<uint64_t> point_trees = t_batch->runner.last_point_trees();
 
     // Per tree: the variant of its specialised batch kernel (register bound, block size, points
     // in flight per thread).  The trees' kernels run concurrently, so a variant is judged by the
     // whole batch: coordinate descent over the trees (most points first), each variant of one
     // tree tried with the others' current choices, kept when the batch gets faster by more than
-    // the timing noise (0.5 %).
+    // the timing noise (0.5 %).  A tree whose requests are all walked in columns runs none of
+    // them: it keeps what it has.
     int rc = FN_OK;
     if (jit_enabled()) {
         std::map<uint64_t, std::pair<const CompiledProgram*, long long>> trees;   // hash -> program, points
@@ -1249,6 +1251,10 @@ int fnAutotuneBatch(const fnGenRequest* requests, int count, void* stream)
         std::vector<const CompiledProgram*> progs;
         for (auto& kv : trees)
             if (jit_is_specialised(kv.first)) {
+                if (std::find(point_trees.begin(), point_trees.end(), kv.first) == point_trees.end()) {
+                    if (!Autotuner::instance().tree_tuned(kv.first)) Autotuner::instance().store_tree(kv.first, 0, best_ms / 2);
+                    continue;
+                }
                 progs.push_back(kv.second.first);
                 order.push_back({kv.second.second, kv.first});
             }
