@@ -302,6 +302,7 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     const unsigned col_len = (unsigned)std::min(64.0, std::max(4.0, column_work / (64.0 * num_sms())));
     // One group per distinct kernel, in first-appearance order (the interpreter: one for all).
     std::vector<BatchKernel> gkernel;
+    std::vector<char> gcolumn;                      // whether it walks columns
     std::vector<size_t> gitems;                     // work items per group
     tiles_.resize(n);
     group_of_.resize(n);
@@ -316,6 +317,7 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
             for (g = 0; g < (int)gkernel.size() && gkernel[(size_t)g].kernel != bk.kernel; ++g) {}
             if (g == (int)gkernel.size()) {
                 gkernel.push_back(bk);
+                gcolumn.push_back(column);
                 gitems.push_back(0);
             }
         }
@@ -383,7 +385,9 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         grps[g].item_end = gr.item_end;
         grps[g].head = 0;
         grps[g].pad = 0;
-        int occ = tuning.ctas_per_sm;
+        // A tuned number of CTAs goes with the tuned tile size: column groups, whose items are cut
+        // otherwise, take what fits on an SM.
+        int occ = gcolumn[g] ? 0 : tuning.ctas_per_sm;
         if (occ <= 0 && gr.jit) {
             int& known = occupancy_[gr.jit];
             if (!known && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&known, (const void*)gr.jit, gr.threads, 0) != cudaSuccess || known < 1))

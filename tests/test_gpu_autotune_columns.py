@@ -29,6 +29,7 @@ def column_trees_keep_their_variant(path):
     fn.jit_compile([(n, 3) for n in nodes])
     outs = [torch.empty(COUNT, device="cuda") for _ in range(64)]
     reqs = [fn.make_request(nodes[k % 2], fn.KIND_GRID3D, o.data_ptr(), k, COUNT, (32.0 * k, 0.0, -7.0)) for k, o in enumerate(outs)]
+    torch.cuda.synchronize()
     fn.set_grid_route(fn.GRID_ROUTE_COLUMNS)
     built = fn.jit_cache_info()["misses"]
     fn.autotune_batch(reqs)
@@ -40,6 +41,17 @@ def column_trees_keep_their_variant(path):
     fn.autotune_load(path)
     fn.autotune_batch(reqs)
     assert _tree_lines(fn, path) == {h: 3 for h in tuned}
+    # a tuned number of CTAs per SM, which goes with tiles of points, does not bind columns
+    fn.gen_batch(reqs)
+    free = fn.batch_info()["ctas"]
+    fn.autotune_save(path)
+    signatures = [ln.split() for ln in path.read_text().splitlines() if not ln.startswith("tree ")]
+    assert signatures
+    for ctas in (1, 0):
+        path.write_text("".join(f"{ln[0]} 2048 {ctas} 1.0\n" for ln in signatures))
+        fn.autotune_load(path)
+        fn.gen_batch(reqs)
+        assert fn.batch_info()["ctas"] == free > 0
     # as points they are tuned
     fn.set_grid_route(fn.GRID_ROUTE_POINTS)
     fn.autotune_batch(reqs)
