@@ -1693,18 +1693,13 @@ int fnJitCheckBatchVariants(const void* const* nodes, const int* dims, int count
     int rc = jit_programs(nodes, dims, count, store, progs);
     if (rc) return rc;
     const int nv = (int)batch_variants().size();
-    std::vector<std::vector<char>> cubins((size_t)nv);
-    std::vector<std::string> logs((size_t)nv);
-    std::vector<char> ok((size_t)nv, 1);
-    std::vector<std::thread> pool;                 // one NVRTC compilation per variant, concurrently
-    for (int v = 1; v < nv; ++v)
-        pool.emplace_back([&, v] { ok[(size_t)v] = jit_compile_cubin(jit_batch_source(progs, v), cubins[(size_t)v], logs[(size_t)v]) ? 1 : 0; });
-    for (auto& t : pool) t.join();
+    std::vector<ModuleSource> modules;
+    for (int v = 1; v < nv; ++v) modules.push_back(jit_batch_module(progs, v));
+    std::vector<std::vector<char>> cubins;
+    std::string err;
+    if (!jit_compile_modules(modules, cubins, err)) { set_error(FN_ERR_COMPILE, err); return FN_ERR_COMPILE; }
     size_t bytes = 0;
-    for (int v = 1; v < nv; ++v) {
-        if (!ok[(size_t)v]) { set_error(FN_ERR_COMPILE, "NVRTC: " + logs[(size_t)v].substr(0, 4000)); return FN_ERR_COMPILE; }
-        bytes += cubins[(size_t)v].size();
-    }
+    for (auto& c : cubins) bytes += c.size();
     if (cubinBytes) *cubinBytes = bytes > 0x7FFFFFFF ? 0x7FFFFFFF : (int)bytes;
     return FN_OK;
 }

@@ -613,6 +613,24 @@ void emit_column_unit(const CompiledProgram& prog, const std::string& eval, cons
 // registers) 105 us with four, 109 with two.
 int column_blocks(const ColPlan& plan) { return plan.regs <= 20 ? 4 : plan.regs <= 104 ? 2 : 1; }
 
+// The per-call kernel that walks a grid in columns.
+void emit_percall_column(const CompiledProgram& prog, const ColPlan& plan, std::ostringstream& o)
+{
+    emit_column_unit(prog, "fnjit_ceval_0", "fnjit_colunit_0", o);
+    o << "extern \"C\" __global__ void __launch_bounds__(256, " << column_blocks(plan) << ") fnjit_col_0"
+      << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned early)\n{\n"
+      << "    __shared__ float4 tab[8][" << plan.table << "];\n"
+      << "    __shared__ float smn[8], smx[8];\n"
+      << "    if (early) fne::let_stream_continue();\n"
+      << gradient_setup(prog, &plan)
+      << "    float mn = fne::inf(), mx = -fne::inf();\n"
+      << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
+      << "        fnjit_colunit_0(A, out, u, tab[threadIdx.x >> 5], mn, mx);\n"
+      << "    fne::let_stream_continue();\n"
+      << "    fne::grid_minmax(mn, mx, work, dminmax, smn, smx);\n"
+      << "}\n\n";
+}
+
 // Per-call kernels for program k: grid / position array / tileable.
 //
 // Each warp owns chunks of 32*ppl consecutive points (ppl = points per lane,
@@ -621,25 +639,10 @@ int column_blocks(const ColPlan& plan) { return plan.regs <= 20 ? 4 : plan.regs 
 // parks the values in shared memory; with ppl == 4 the warp then writes the
 // chunk as 32 float4 stores (512 contiguous bytes per warp).  Small calls use
 // ppl == 1 so that their few points spread over as many SMs as possible.
-void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::ostringstream& o)
+enum PercallKernels : unsigned { kGridKernel = 1, kPositionKernel = 2, kOtherKernels = 4 };
+void emit_percall(const CompiledProgram& prog, int k, unsigned which, std::ostringstream& o)
 {
     const int D = prog.dim;
-    if (!plan.states.empty()) {
-        const std::string id = std::to_string(k);
-        emit_column_unit(prog, "fnjit_ceval_" + id, "fnjit_colunit_" + id, o);
-        o << "extern \"C\" __global__ void __launch_bounds__(256, " << column_blocks(plan) << ") fnjit_col_" << id
-          << "(fn::PointArgs A, float* __restrict__ out, fn::MinMaxWork* work, float* dminmax, unsigned early)\n{\n"
-          << "    __shared__ float4 tab[8][" << plan.table << "];\n"
-          << "    __shared__ float smn[8], smx[8];\n"
-          << "    if (early) fne::let_stream_continue();\n"
-          << gradient_setup(prog, &plan)
-          << "    float mn = fne::inf(), mx = -fne::inf();\n"
-          << "    for (unsigned u = blockIdx.x * 8u + (threadIdx.x >> 5); u < A.col_units; u += gridDim.x * 8u)\n"
-          << "        fnjit_colunit_" << id << "(A, out, u, tab[threadIdx.x >> 5], mn, mx);\n"
-          << "    fne::let_stream_continue();\n"
-          << "    fne::grid_minmax(mn, mx, work, dminmax, smn, smx);\n"
-          << "}\n\n";
-    }
     const char* pv[4] = {"px", "py", "pz", "pw"};
     std::string call = "fnjit_eval_" + std::to_string(k) + "(A.seed";
     for (int j = 0; j < 4; ++j) call += std::string(", ") + (j < D ? pv[j] : "0.0f");
@@ -706,18 +709,18 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
             pos << "                const float " << pv[j] << " = fmaf(fnd::cvtf((int)i" << ax[j] << "), A.step[" << j << "], A.offset[" << j << "]);\n";
         }
         gridpos = pos.str();
-        kernel("fnjit_grid", "", gridpos);
+        if (which & kGridKernel) kernel("fnjit_grid", "", gridpos);
     }
     // position arrays: Generator.inl:256-350, pos_k = offset_k + array_k[i].  Plain loads: the arrays
     // may be written while this kernel already waits, so they are not read-only to it.
-    {
+    if (which & kPositionKernel) {
         std::ostringstream pos;
         for (int j = 0; j < D; ++j)
             pos << "                const float " << pv[j] << " = A.offset[" << j << "] + A.pos[" << j << "][i + A.base];\n";
         kernel("fnjit_pos", "    fne::wait_for_stream();\n", pos.str());
     }
     // tileable (4D programs): Generator.inl:370-433
-    if (D == 4) {
+    if (D == 4 && (which & kOtherKernels)) {
         std::ostringstream pos;
         pos << "                const unsigned g = i + A.base;\n"
             << "                const unsigned iy = fne::fast_div(g, A.divm[0], A.divs[0]), ix = g - iy * (unsigned)A.count[0];\n"
@@ -734,7 +737,7 @@ void emit_percall(const CompiledProgram& prog, int k, const ColPlan& plan, std::
     //  fnjit_solid: the grid's two classification bitmasks (bit i of word i / 32; the warp's
     //    32 consecutive points form one word) and OutputMinMax -- no density leaves registers;
     //  fnjit_list: the grid's values at listed point indices (count read from the device).
-    if (D == 3) {
+    if (D == 3 && (which & kOtherKernels)) {
         o << "extern \"C\" __global__ void __launch_bounds__(256, 4) fnjit_solid_" << k
           << "(fn::PointArgs A, unsigned* __restrict__ above, unsigned* __restrict__ solid, fn::MinMaxWork* work, float* dminmax,\n"
           << "    float iso, unsigned ppl)\n{\n"
@@ -899,56 +902,83 @@ void emit_batch_column(const CompiledProgram& prog, size_t k, const ColPlan& pla
          "    }\n}\n\n";
 }
 
+// A module's loaded programs.
 struct Module {
-    cudaLibrary_t lib = nullptr;
-    std::vector<uint64_t> hashes;
+    std::vector<cudaLibrary_t> parts;
+    Module() = default;
+    Module(const Module&) = delete;
+    Module& operator=(const Module&) = delete;
+    ~Module()
+    {
+        for (cudaLibrary_t lib : parts) cudaLibraryUnload(lib);
+    }
 };
 
 std::mutex g_jit_mu;
 std::unordered_map<uint64_t, JitKernels> g_kernels;
-std::vector<std::unique_ptr<Module>> g_modules;
+std::vector<std::unique_ptr<Module>>& g_modules = *new std::vector<std::unique_ptr<Module>>;   // never unloaded
 std::unordered_map<uint64_t, cudaKernel_t> g_batch_kernels;   // per-tree batch kernel (variant 0)
 std::unordered_map<uint64_t, std::vector<BatchKernel>> g_batch_variant_kernels;   // per tree: every variant built
 std::atomic<bool> g_enabled{true};
 
 }  // namespace
 
-std::string jit_batch_source(const std::vector<const CompiledProgram*>& progs, int variant)
+namespace {
+
+std::string module_head(const std::string& what)
 {
-    std::ostringstream o;
-    o << "// generated by fn_jit.cpp: batch module, variant " << variant << "\n#define FN_GRADIENT_TABLE\n" << embedded_device_source() << "\n";
-    for (size_t k = 0; k < progs.size(); ++k) emit_eval(*progs[k], "fnjit_eval_" + std::to_string(k), o);
-    emit_batch(progs, o, variant);
-    if (variant == 0)
-        for (size_t k = 0; k < progs.size(); ++k) {
-            const ColPlan plan = column_plan(*progs[k]);
-            if (plan.states.empty()) continue;
-            emit_eval(*progs[k], "fnjit_ceval_" + std::to_string(k), o, &plan);
-            emit_batch_column(*progs[k], k, plan, o);
-        }
-    return o.str();
+    return "// generated by fn_jit.cpp: " + what + "\n#define FN_GRADIENT_TABLE\n" + embedded_device_source() + "\n";
 }
 
-std::string jit_percall_source(const CompiledProgram& prog)
+}  // namespace
+
+ModuleSource jit_batch_module(const std::vector<const CompiledProgram*>& progs, int variant)
 {
     std::ostringstream o;
-    o << "// generated by fn_jit.cpp: per-call module\n#define FN_GRADIENT_TABLE\n" << embedded_device_source() << "\n";
-    emit_eval(prog, "fnjit_eval_0", o);
+    for (size_t k = 0; k < progs.size(); ++k) emit_eval(*progs[k], "fnjit_eval_" + std::to_string(k), o);
+    emit_batch(progs, o, variant);
+    ModuleSource m{module_head("batch module, variant " + std::to_string(variant)), {o.str()}};
+    for (size_t k = 0; variant == 0 && k < progs.size(); ++k) {
+        const ColPlan plan = column_plan(*progs[k]);
+        if (plan.states.empty()) continue;
+        std::ostringstream c;
+        emit_eval(*progs[k], "fnjit_ceval_" + std::to_string(k), c, &plan);
+        emit_batch_column(*progs[k], k, plan, c);
+        m.parts.push_back(c.str());
+    }
+    return m;
+}
+
+ModuleSource jit_percall_module(const CompiledProgram& prog)
+{
     const ColPlan plan = column_plan(prog);
-    if (!plan.states.empty()) emit_eval(prog, "fnjit_ceval_0", o, &plan);
-    emit_percall(prog, 0, plan, o);
-    return o.str();
+    std::ostringstream eval;
+    emit_eval(prog, "fnjit_eval_0", eval);
+    ModuleSource m{module_head("per-call module") + eval.str(), {}};
+    for (unsigned which : {(unsigned)kGridKernel, (unsigned)kPositionKernel, (unsigned)kOtherKernels}) {
+        std::ostringstream o;
+        emit_percall(prog, 0, which, o);
+        if (!o.str().empty()) m.parts.push_back(o.str());
+    }
+    if (!plan.states.empty()) {
+        std::ostringstream c;
+        emit_eval(prog, "fnjit_ceval_0", c, &plan);
+        emit_percall_column(prog, plan, c);
+        m.parts.push_back(c.str());
+    }
+    return m;
 }
 
 // ---------------------------------------------------------------- on-disk module cache
 // Compiled modules are kept on disk, keyed by their CUDA source (which embeds the node
 // library's device code), the NVRTC options and the NVRTC version, so a module that any
 // earlier process built loads in milliseconds instead of being compiled again.  File:
-// "FNJC", format version, the 128-bit key, payload size, the cubin, a checksum of the cubin;
-// a file that does not check out is ignored (and replaced by the next compile).
+// "FNJC", format version, the 128-bit key, payload size, the module (its cubins, see
+// pack_parts), a checksum of it; a file that does not check out is ignored (and replaced by the
+// next compile).
 namespace {
 
-constexpr uint32_t kCacheFormat = 1;
+constexpr uint32_t kCacheFormat = 2;
 const char* const kNvrtcOptions[] = {"--gpu-architecture=sm_103a", "-fmad=false", "--std=c++17", "-default-device",
                                      "-lineinfo", "-diag-suppress=177"};
 
@@ -963,15 +993,21 @@ uint64_t fnv1a(const void* data, size_t n, uint64_t h)
     return h;
 }
 
-CacheKey cache_key(const std::string& src)
+CacheKey cache_key(const ModuleSource& src)
 {
     int major = 0, minor = 0;
     nvrtcVersion(&major, &minor);
     std::string salt = "nvrtc " + std::to_string(major) + "." + std::to_string(minor) + " format " + std::to_string(kCacheFormat);
     for (const char* o : kNvrtcOptions) salt += std::string(" ") + o;
     CacheKey k;
-    k.a = fnv1a(src.data(), src.size(), fnv1a(salt.data(), salt.size(), 0xCBF29CE484222325ull));
-    k.b = fnv1a(src.data(), src.size(), fnv1a(salt.data(), salt.size(), 0x84222325CBF29CE4ull ^ 0x9E3779B97F4A7C15ull));
+    k.a = fnv1a(salt.data(), salt.size(), 0xCBF29CE484222325ull);
+    k.b = fnv1a(salt.data(), salt.size(), 0x84222325CBF29CE4ull ^ 0x9E3779B97F4A7C15ull);
+    auto add = [&](const std::string& text) {
+        k.a = fnv1a(text.data(), text.size(), k.a);
+        k.b = fnv1a(text.data(), text.size(), k.b);
+    };
+    add(src.head);
+    for (const std::string& part : src.parts) add(part);
     return k;
 }
 
@@ -1047,7 +1083,7 @@ void cache_write(const std::string& path, const CacheKey& k, const std::vector<c
 }
 
 // A module from the cache only (no compile); false on a miss.
-bool cached_cubin(const std::string& src, std::vector<char>& cubin)
+bool cached_cubin(const ModuleSource& src, std::vector<char>& cubin)
 {
     const std::string dir = cache_dir();
     if (dir.empty()) return false;
@@ -1075,39 +1111,48 @@ void jit_cache_stats(unsigned long long* hits, unsigned long long* misses)
     if (misses) *misses = g_cache_misses.load();
 }
 
-bool jit_compile_all(const std::vector<const CompiledProgram*>& progs, std::vector<std::vector<char>>& cubins, std::string& error)
+namespace {
+
+// A compiled module: the number of programs, their sizes, their cubins, each from a multiple of 16 bytes.
+size_t part_start(size_t pos) { return (pos + 15) / 16 * 16; }
+std::vector<char> pack_parts(const std::vector<std::vector<char>>& parts)
 {
-    // source 0 = the batch module, 1 + k = program k's per-call module; NVRTC
-    // compiles independent programs concurrently, so the sources go to a pool of threads
-    std::vector<std::string> srcs;
-    srcs.push_back(jit_batch_source(progs, 0));
-    for (auto* p : progs) srcs.push_back(jit_percall_source(*p));
-    cubins.assign(srcs.size(), {});
-    std::vector<std::string> logs(srcs.size());
-    std::vector<char> ok(srcs.size(), 0);
-    std::atomic<size_t> next{0};
-    auto worker = [&]() {
-        for (size_t i; (i = next.fetch_add(1)) < srcs.size();) ok[i] = jit_compile_cubin(srcs[i], cubins[i], logs[i]) ? 1 : 0;
-    };
-    unsigned nt = std::thread::hardware_concurrency();
-    nt = std::max(1u, std::min<unsigned>(nt ? nt : 4, (unsigned)srcs.size()));
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < nt; ++t) pool.emplace_back(worker);
-    worker();
-    for (auto& t : pool) t.join();
-    for (size_t i = 0; i < srcs.size(); ++i)
-        if (!ok[i]) { error = "NVRTC: " + logs[i].substr(0, 4000); return false; }
-    return true;
+    std::vector<uint64_t> head{(uint64_t)parts.size()};
+    for (auto& p : parts) head.push_back(p.size());
+    const char* h = reinterpret_cast<const char*>(head.data());
+    std::vector<char> out(h, h + head.size() * sizeof(uint64_t));
+    for (auto& p : parts) {
+        out.resize(part_start(out.size()));
+        out.insert(out.end(), p.begin(), p.end());
+    }
+    return out;
 }
 
-bool jit_compile_cubin(const std::string& src, std::vector<char>& cubin, std::string& log)
+// Whether a compiled module is whole; `at` gets where each cubin begins.
+bool unpack_parts(const std::vector<char>& module, std::vector<size_t>& at)
+{
+    at.clear();
+    uint64_t n = 0, size = 0;
+    if (module.size() < sizeof n) return false;
+    std::memcpy(&n, module.data(), sizeof n);
+    if (n == 0 || n > module.size() / sizeof n - 1) return false;
+    size_t pos = (size_t)(n + 1) * sizeof n;
+    for (uint64_t k = 0; k < n; ++k) {
+        std::memcpy(&size, module.data() + (k + 1) * sizeof n, sizeof size);
+        pos = part_start(pos);
+        if (pos > module.size() || size > module.size() - pos) return false;
+        at.push_back(pos);
+        pos += (size_t)size;
+    }
+    return pos == module.size();
+}
+
+bool compile_program(const std::string& src, std::vector<char>& cubin, std::string& log)
 {
     // FASTNOISE_JIT_VERBOSE=1 prints ptxas' register / spill report of every
     // specialised kernel to stderr (useful when tuning trees); it always compiles.
     const char* verbose = std::getenv("FASTNOISE_JIT_VERBOSE");
     const bool v = verbose && verbose[0] == '1';
-    if (!v && cached_cubin(src, cubin)) return true;
-    const std::string dir = cache_dir();
     nvrtcProgram prog;
     if (nvrtcCreateProgram(&prog, src.c_str(), "fastnoise_jit.cu", 0, nullptr, nullptr) != NVRTC_SUCCESS) {
         log = "nvrtcCreateProgram failed";
@@ -1130,30 +1175,134 @@ bool jit_compile_cubin(const std::string& src, std::vector<char>& cubin, std::st
     cubin.resize(n);
     nvrtcGetCUBIN(prog, cubin.data());
     nvrtcDestroyProgram(&prog);
-    g_cache_misses.fetch_add(1);
-    if (!dir.empty() && n > 0) {
-        const CacheKey k = cache_key(src);
-        cache_write(cache_path(dir, k), k, cubin);
+    return true;
+}
+
+}  // namespace
+
+bool jit_compile_modules(const std::vector<ModuleSource>& modules, std::vector<std::vector<char>>& compiled, std::string& error)
+{
+    const char* verbose = std::getenv("FASTNOISE_JIT_VERBOSE");
+    const bool v = verbose && verbose[0] == '1';
+    compiled.assign(modules.size(), {});
+    // NVRTC compiles independent programs concurrently, so they go to a pool of threads, the longest
+    // first.  A program is a module's head with some of its parts: all of them, and the longest
+    // programs in two until there is one for each thread (or an eighth more than modules: each costs the
+    // head again).  A tree alone takes as long as its longest part; 16 trees of the chunk mix take 1.0
+    // to 1.2 times what their point kernels do, 1.9 times with one program per module.
+    unsigned nt = std::thread::hardware_concurrency();
+    if (!nt) nt = 4;
+    struct Unit {
+        size_t module, first, end, weight;       // its parts
+        std::vector<char> cubin;
+    };
+    std::vector<Unit> todo;
+    auto weigh = [&](size_t m, size_t first, size_t end) {
+        size_t w = 0;
+        for (size_t k = first; k < end; ++k) w += modules[m].parts[k].size();
+        return w;
+    };
+    for (size_t m = 0; m < modules.size(); ++m)
+        todo.push_back(Unit{m, 0, modules[m].parts.size(), weigh(m, 0, modules[m].parts.size()), {}});
+    const size_t most = std::max<size_t>(nt, todo.size() + todo.size() / 8 + 1);
+    while (todo.size() < most) {
+        Unit* longest = nullptr;
+        for (Unit& u : todo)
+            if (u.end - u.first > 1 && (!longest || u.weight > longest->weight)) longest = &u;
+        if (!longest) break;
+        size_t at = longest->first + 1;          // as even as its parts allow, in their order
+        while (at + 1 < longest->end && 2 * weigh(longest->module, longest->first, at) < longest->weight) ++at;
+        Unit rest{longest->module, at, longest->end, weigh(longest->module, at, longest->end), {}};
+        longest->end = at;
+        longest->weight -= rest.weight;
+        todo.push_back(std::move(rest));
+    }
+    std::vector<char> cached(modules.size(), 0);
+    for (size_t m = 0; !v && m < modules.size(); ++m) cached[m] = cached_cubin(modules[m], compiled[m]) ? 1 : 0;
+    todo.erase(std::remove_if(todo.begin(), todo.end(), [&](const Unit& u) { return cached[u.module] != 0; }), todo.end());
+    std::stable_sort(todo.begin(), todo.end(), [](const Unit& a, const Unit& b) { return a.weight > b.weight; });
+    std::vector<std::string> logs(todo.size());
+    std::vector<char> ok(todo.size(), 0);
+    std::atomic<size_t> next{0};
+    auto worker = [&]() {
+        for (size_t i; (i = next.fetch_add(1)) < todo.size();) {
+            const ModuleSource& m = modules[todo[i].module];
+            std::string src = m.head;
+            for (size_t k = todo[i].first; k < todo[i].end; ++k) src += m.parts[k];
+            ok[i] = compile_program(src, todo[i].cubin, logs[i]) ? 1 : 0;
+        }
+    };
+    nt = std::max(1u, std::min<unsigned>(nt, (unsigned)todo.size()));
+    std::vector<std::thread> pool;
+    for (unsigned t = 1; t < nt; ++t) pool.emplace_back(worker);
+    worker();
+    for (auto& t : pool) t.join();
+    for (size_t i = 0; i < todo.size(); ++i)
+        if (!ok[i]) { error = "NVRTC: " + logs[i].substr(0, 4000); return false; }
+    const std::string dir = cache_dir();
+    for (size_t m = 0; m < modules.size(); ++m) {
+        std::vector<std::vector<char>> cubins;
+        for (Unit& u : todo)
+            if (u.module == m) cubins.push_back(std::move(u.cubin));
+        if (cubins.empty()) continue;
+        compiled[m] = pack_parts(cubins);
+        g_cache_misses.fetch_add(1);
+        if (!dir.empty()) {
+            const CacheKey k = cache_key(modules[m]);
+            cache_write(cache_path(dir, k), k, compiled[m]);
+        }
     }
     return true;
 }
 
+bool jit_compile_all(const std::vector<const CompiledProgram*>& progs, std::vector<std::vector<char>>& compiled, std::string& error)
+{
+    std::vector<ModuleSource> modules{jit_batch_module(progs, 0)};
+    for (auto* p : progs) modules.push_back(jit_percall_module(*p));
+    return jit_compile_modules(modules, compiled, error);
+}
+
 namespace {
 
-// Load the batch module (cubins[0]) and the per-call modules (cubins[1 + k]) of `progs` and
-// register their kernels.
-bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vector<std::vector<char>>& cubins, std::string& error)
+// A kernel of a module, whichever of its programs has it; false if none has.
+bool find_kernel(const Module& m, const std::string& name, cudaKernel_t& out)
 {
-    std::vector<std::unique_ptr<Module>> mods;
-    for (auto& c : cubins) {
-        auto mod = std::make_unique<Module>();
-        cudaError_t e = cudaLibraryLoadData(&mod->lib, c.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
+    for (cudaLibrary_t part : m.parts) {
+        if (cudaLibraryGetKernel(&out, part, name.c_str()) == cudaSuccess) return true;
+        cudaGetLastError();
+    }
+    return false;
+}
+
+// Load a compiled module.
+std::unique_ptr<Module> load_module(const std::vector<char>& compiled, std::string& error)
+{
+    std::vector<size_t> at;
+    if (!unpack_parts(compiled, at)) {
+        error = "damaged module";
+        return nullptr;
+    }
+    auto mod = std::make_unique<Module>();
+    for (size_t pos : at) {
+        cudaLibrary_t lib = nullptr;
+        const cudaError_t e = cudaLibraryLoadData(&lib, compiled.data() + pos, nullptr, nullptr, 0, nullptr, nullptr, 0);
         if (e != cudaSuccess) {
             error = std::string("cudaLibraryLoadData: ") + cudaGetErrorString(e);
-            for (auto& m : mods) cudaLibraryUnload(m->lib);
-            return false;
+            return nullptr;
         }
-        mods.push_back(std::move(mod));
+        mod->parts.push_back(lib);
+    }
+    return mod;
+}
+
+// Load the batch module (compiled[0]) and the per-call modules (compiled[1 + k]) of `progs` and
+// register their kernels.
+bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vector<std::vector<char>>& compiled, std::string& error)
+{
+    std::vector<std::unique_ptr<Module>> mods;
+    for (auto& c : compiled) {
+        mods.push_back(load_module(c, error));
+        if (!mods.back()) return false;
     }
     std::unordered_map<uint64_t, JitKernels> found;
     std::unordered_map<uint64_t, cudaKernel_t> batch;
@@ -1161,7 +1310,7 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
     for (auto* p : progs) plans.push_back(column_plan(*p));
     bool ok = true;
     for (size_t k = 0; ok && k < progs.size(); ++k) {
-        cudaLibrary_t lib = mods[1 + k]->lib;
+        const Module& own = *mods[1 + k];
         JitKernels jk;
         jk.slot = (int)k;
         jk.column_step = plans[k].step;
@@ -1169,15 +1318,12 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
         for (auto& st : plans[k].states)
             jk.column_rates[jk.n_column_rates++] = st.rate;
         cudaKernel_t bk = nullptr;
-        ok = cudaLibraryGetKernel(&jk.grid, lib, "fnjit_grid_0") == cudaSuccess &&
-             cudaLibraryGetKernel(&jk.positions, lib, "fnjit_pos_0") == cudaSuccess &&
-             (progs[k]->dim != 4 || cudaLibraryGetKernel(&jk.tileable, lib, "fnjit_tile_0") == cudaSuccess) &&
-             (progs[k]->dim != 3 || (cudaLibraryGetKernel(&jk.solid, lib, "fnjit_solid_0") == cudaSuccess &&
-                                     cudaLibraryGetKernel(&jk.list, lib, "fnjit_list_0") == cudaSuccess)) &&
-             (plans[k].states.empty() ||
-              (cudaLibraryGetKernel(&jk.column, lib, "fnjit_col_0") == cudaSuccess &&
-               cudaLibraryGetKernel(&jk.batch_column, mods[0]->lib, ("fnjit_bcol_" + std::to_string(k)).c_str()) == cudaSuccess)) &&
-             cudaLibraryGetKernel(&bk, mods[0]->lib, ("fnjit_batch_" + std::to_string(k)).c_str()) == cudaSuccess;
+        ok = find_kernel(own, "fnjit_grid_0", jk.grid) && find_kernel(own, "fnjit_pos_0", jk.positions) &&
+             (progs[k]->dim != 4 || find_kernel(own, "fnjit_tile_0", jk.tileable)) &&
+             (progs[k]->dim != 3 || (find_kernel(own, "fnjit_solid_0", jk.solid) && find_kernel(own, "fnjit_list_0", jk.list))) &&
+             (plans[k].states.empty() || (find_kernel(own, "fnjit_col_0", jk.column) &&
+                                          find_kernel(*mods[0], "fnjit_bcol_" + std::to_string(k), jk.batch_column))) &&
+             find_kernel(*mods[0], "fnjit_batch_" + std::to_string(k), bk);
         const cudaKernel_t kern[4] = {jk.grid, jk.positions, jk.tileable, jk.column};
         for (int j = 0; ok && j < 4; ++j) {
             int n = 0;
@@ -1191,7 +1337,6 @@ bool jit_load(const std::vector<const CompiledProgram*>& progs, const std::vecto
     }
     if (!ok) {
         error = "kernel lookup failed in a specialised module";
-        for (auto& m : mods) cudaLibraryUnload(m->lib);
         return false;
     }
     std::lock_guard<std::mutex> lk(g_jit_mu);
@@ -1233,7 +1378,7 @@ bool jit_try_cached(const CompiledProgram* prog)
         if (g_kernels.count(prog->hash) && g_batch_kernels.count(prog->hash)) return true;
     }
     std::vector<std::vector<char>> cubins(2);
-    if (!cached_cubin(jit_batch_source({prog}, 0), cubins[0]) || !cached_cubin(jit_percall_source(*prog), cubins[1])) return false;
+    if (!cached_cubin(jit_batch_module({prog}, 0), cubins[0]) || !cached_cubin(jit_percall_module(*prog), cubins[1])) return false;
     std::string err;
     return jit_load({prog}, cubins, err);
 }
@@ -1253,39 +1398,24 @@ bool jit_build_batch_variants(const std::vector<const CompiledProgram*>& progs, 
     }
     if (todo.empty()) return true;
     // one module per variant, compiled concurrently
-    std::vector<std::string> srcs;
-    for (size_t v = 1; v < nv; ++v) srcs.push_back(jit_batch_source(todo, (int)v));
-    std::vector<std::vector<char>> cubins(srcs.size());
-    std::vector<std::string> logs(srcs.size());
-    std::vector<char> ok(srcs.size(), 0);
-    std::vector<std::thread> pool;
-    for (size_t i = 0; i < srcs.size(); ++i)
-        pool.emplace_back([&, i] { ok[i] = jit_compile_cubin(srcs[i], cubins[i], logs[i]) ? 1 : 0; });
-    for (auto& t : pool) t.join();
-    for (size_t i = 0; i < srcs.size(); ++i)
-        if (!ok[i]) { error = "NVRTC: " + logs[i].substr(0, 4000); return false; }
+    std::vector<ModuleSource> modules;
+    for (size_t v = 1; v < nv; ++v) modules.push_back(jit_batch_module(todo, (int)v));
+    std::vector<std::vector<char>> compiled;
+    if (!jit_compile_modules(modules, compiled, error)) return false;
     std::vector<std::unique_ptr<Module>> mods;
     std::vector<std::vector<BatchKernel>> got(todo.size(), std::vector<BatchKernel>(nv));
-    for (size_t i = 0; i < cubins.size(); ++i) {
-        auto mod = std::make_unique<Module>();
-        cudaError_t e = cudaLibraryLoadData(&mod->lib, cubins[i].data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
-        if (e != cudaSuccess) {
-            error = std::string("cudaLibraryLoadData: ") + cudaGetErrorString(e);
-            for (auto& m : mods) cudaLibraryUnload(m->lib);
-            return false;
-        }
+    for (size_t i = 0; i < compiled.size(); ++i) {
+        mods.push_back(load_module(compiled[i], error));
+        if (!mods.back()) return false;
         const int v = (int)i + 1;
         for (size_t k = 0; k < todo.size(); ++k) {
             cudaKernel_t kern = nullptr;
-            if (cudaLibraryGetKernel(&kern, mod->lib, batch_kernel_name(k, v).c_str()) != cudaSuccess) {
+            if (cudaLibraryGetKernel(&kern, mods.back()->parts[0], batch_kernel_name(k, v).c_str()) != cudaSuccess) {
                 error = "kernel lookup failed in a batch variant module";
-                cudaLibraryUnload(mod->lib);
-                for (auto& m : mods) cudaLibraryUnload(m->lib);
                 return false;
             }
             got[k][(size_t)v] = BatchKernel{kern, batch_variants()[(size_t)v].threads};
         }
-        mods.push_back(std::move(mod));
     }
     std::lock_guard<std::mutex> lk(g_jit_mu);
     for (size_t k = 0; k < todo.size(); ++k) {

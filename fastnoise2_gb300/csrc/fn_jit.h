@@ -65,14 +65,23 @@ struct BatchKernel {
     int threads = 256;
 };
 
-// CUDA source of the batch module for `progs` (slot k = progs[k]) in one variant, and of
-// one program's per-call module.
-std::string jit_batch_source(const std::vector<const CompiledProgram*>& progs, int variant);
-std::string jit_percall_source(const CompiledProgram& prog);
+// CUDA source of a module: a head, and parts that need the head but not each other.
+struct ModuleSource {
+    std::string head;
+    std::vector<std::string> parts;
+};
 
-// NVRTC-compile the batch module and every per-call module (concurrently);
-// cubins[0] = batch, cubins[1 + k] = program k.  Host only, no GPU needed.
-bool jit_compile_all(const std::vector<const CompiledProgram*>& progs, std::vector<std::vector<char>>& cubins,
+// The batch kernels of `progs` (slot k = progs[k]) in one variant (variant 0: and the column kernels
+// of the programs that have them), and one program's per-call module.
+ModuleSource jit_batch_module(const std::vector<const CompiledProgram*>& progs, int variant);
+ModuleSource jit_percall_module(const CompiledProgram& prog);
+
+// NVRTC-compile modules, concurrently; those in the on-disk cache are taken from it.
+// Host only, no GPU needed.
+bool jit_compile_modules(const std::vector<ModuleSource>& modules, std::vector<std::vector<char>>& compiled,
+                         std::string& error);
+// The batch module and every per-call module: compiled[0] = batch, compiled[1 + k] = program k.
+bool jit_compile_all(const std::vector<const CompiledProgram*>& progs, std::vector<std::vector<char>>& compiled,
                      std::string& error);
 
 // Compile and load a module covering `progs`; on success every program gets
@@ -164,8 +173,5 @@ void jit_note_interpreted(const CompiledProgram* prog);
 int jit_set_auto_threshold(int uses);              // returns the previous threshold
 bool jit_auto_wait(int timeout_ms);                // true when no build is queued or running
 bool jit_is_specialised(uint64_t hash);
-
-// Compile NVRTC source for sm_103a to a cubin (host only; used by tests).
-bool jit_compile_cubin(const std::string& src, std::vector<char>& cubin, std::string& log);
 
 }  // namespace fn
