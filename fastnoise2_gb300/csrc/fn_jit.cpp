@@ -925,6 +925,30 @@ std::atomic<bool> g_enabled{true};
 
 namespace {
 
+// What NVRTC takes for a kernel that evaluates `prog` once, beyond the module's head (seconds on a
+// Grace core, roughly: FBm(Perlin) 3D 0.13, 4D 0.9, terrain 3D 0.27).
+float compile_seconds(const CompiledProgram& prog)
+{
+    const FnProgramHeader* h = reinterpret_cast<const FnProgramHeader*>(prog.blob.data());
+    const FnInstr* ins = fn_program_instrs(h);
+    static const float simplex[3] = {7, 14, 21}, super[3] = {14, 35, 40}, perlin[3] = {8, 26, 180}, value[3] = {7, 14, 28}, warp[3] = {7, 14, 35},
+                       cells[3] = {28, 56, 56};
+    float ms = 0;
+    for (int pc = 0; pc < h->n_instr; ++pc) {
+        const FnInstr& I = ins[pc];
+        const int d = I.dim - 2;
+        switch (I.op) {
+        case FN_OP_NOISE: ms += (I.aux == FN_NOISE_SIMPLEX ? simplex : I.aux == FN_NOISE_SUPERSIMPLEX ? super : I.aux == FN_NOISE_PERLIN ? perlin : value)[d]; break;
+        case FN_OP_WARP_GRAD: ms += warp[d]; break;
+        case FN_OP_WARP_SIMPLEX: ms += 3 * warp[d]; break;
+        case FN_OP_CELL_VALUE: case FN_OP_CELL_DIST: case FN_OP_CELL_LOOKUP: ms += cells[d]; break;
+        default: ms += 0.5f; break;
+        }
+    }
+    for (auto& sub : prog.subs) ms += 1e3f * compile_seconds(sub);
+    return 1e-3f * ms;
+}
+
 std::string module_head(const std::string& what)
 {
     return "// generated by fn_jit.cpp: " + what + "\n#define FN_GRADIENT_TABLE\n" + embedded_device_source() + "\n";
@@ -937,14 +961,16 @@ ModuleSource jit_batch_module(const std::vector<const CompiledProgram*>& progs, 
     std::ostringstream o;
     for (size_t k = 0; k < progs.size(); ++k) emit_eval(*progs[k], "fnjit_eval_" + std::to_string(k), o);
     emit_batch(progs, o, variant);
-    ModuleSource m{module_head("batch module, variant " + std::to_string(variant)), {o.str()}};
+    float seconds = 0;
+    for (auto* p : progs) seconds += compile_seconds(*p);
+    ModuleSource m{module_head("batch module, variant " + std::to_string(variant)), {{o.str(), seconds}}};
     for (size_t k = 0; variant == 0 && k < progs.size(); ++k) {
         const ColPlan plan = column_plan(*progs[k]);
         if (plan.states.empty()) continue;
         std::ostringstream c;
         emit_eval(*progs[k], "fnjit_ceval_" + std::to_string(k), c, &plan);
         emit_batch_column(*progs[k], k, plan, c);
-        m.parts.push_back(c.str());
+        m.parts.push_back({c.str(), compile_seconds(*progs[k])});
     }
     return m;
 }
@@ -958,13 +984,13 @@ ModuleSource jit_percall_module(const CompiledProgram& prog)
     for (unsigned which : {(unsigned)kGridKernel, (unsigned)kPositionKernel, (unsigned)kOtherKernels}) {
         std::ostringstream o;
         emit_percall(prog, 0, which, o);
-        if (!o.str().empty()) m.parts.push_back(o.str());
+        if (!o.str().empty()) m.parts.push_back({o.str(), (which == kOtherKernels && prog.dim == 3 ? 2.0f : 1.0f) * compile_seconds(prog)});
     }
     if (!plan.states.empty()) {
         std::ostringstream c;
         emit_eval(prog, "fnjit_ceval_0", c, &plan);
         emit_percall_column(prog, plan, c);
-        m.parts.push_back(c.str());
+        m.parts.push_back({c.str(), compile_seconds(prog)});
     }
     return m;
 }
@@ -1007,7 +1033,7 @@ CacheKey cache_key(const ModuleSource& src)
         k.b = fnv1a(text.data(), text.size(), k.b);
     };
     add(src.head);
-    for (const std::string& part : src.parts) add(part);
+    for (const ModuleSource::Part& part : src.parts) add(part.text);
     return k;
 }
 
@@ -1187,40 +1213,43 @@ bool jit_compile_modules(const std::vector<ModuleSource>& modules, std::vector<s
     compiled.assign(modules.size(), {});
     // NVRTC compiles independent programs concurrently, so they go to a pool of threads, the longest
     // first.  A program is a module's head with some of its parts: all of them, and the longest
-    // programs in two until there is one for each thread (or an eighth more than modules: each costs the
-    // head again).  A tree alone takes as long as its longest part; 16 trees of the chunk mix take 1.0
-    // to 1.2 times what their point kernels do, 1.9 times with one program per module.
+    // programs in two until there is one for each thread (or a third more than modules), while they
+    // take about as long as the head again (0.2 s, and 25 ms where the compiler has the program
+    // cached).  FBm(Perlin) 3D takes 0.38 s (1.02 with one program per module, 0.62 without its column
+    // kernels), the chunk mix's 16 programs 1.9 (4.3, 1.8; cached 0.79, 0.62, 0.47).
     unsigned nt = std::thread::hardware_concurrency();
     if (!nt) nt = 4;
+    constexpr float kWorthSplitting = 0.15f;
     struct Unit {
-        size_t module, first, end, weight;       // its parts
+        size_t module, first, end;               // its parts
+        float seconds;
         std::vector<char> cubin;
     };
     std::vector<Unit> todo;
-    auto weigh = [&](size_t m, size_t first, size_t end) {
-        size_t w = 0;
-        for (size_t k = first; k < end; ++k) w += modules[m].parts[k].size();
-        return w;
+    auto estimate = [&](size_t m, size_t first, size_t end) {
+        float t = 0;
+        for (size_t k = first; k < end; ++k) t += modules[m].parts[k].seconds;
+        return t;
     };
     for (size_t m = 0; m < modules.size(); ++m)
-        todo.push_back(Unit{m, 0, modules[m].parts.size(), weigh(m, 0, modules[m].parts.size()), {}});
-    const size_t most = std::max<size_t>(nt, todo.size() + todo.size() / 8 + 1);
+        todo.push_back(Unit{m, 0, modules[m].parts.size(), estimate(m, 0, modules[m].parts.size()), {}});
+    const size_t most = std::max<size_t>(nt, todo.size() + todo.size() / 3 + 1);
     while (todo.size() < most) {
         Unit* longest = nullptr;
         for (Unit& u : todo)
-            if (u.end - u.first > 1 && (!longest || u.weight > longest->weight)) longest = &u;
+            if (u.end - u.first > 1 && u.seconds > kWorthSplitting && (!longest || u.seconds > longest->seconds)) longest = &u;
         if (!longest) break;
         size_t at = longest->first + 1;          // as even as its parts allow, in their order
-        while (at + 1 < longest->end && 2 * weigh(longest->module, longest->first, at) < longest->weight) ++at;
-        Unit rest{longest->module, at, longest->end, weigh(longest->module, at, longest->end), {}};
+        while (at + 1 < longest->end && 2.0f * estimate(longest->module, longest->first, at) < longest->seconds) ++at;
+        Unit rest{longest->module, at, longest->end, estimate(longest->module, at, longest->end), {}};
         longest->end = at;
-        longest->weight -= rest.weight;
+        longest->seconds -= rest.seconds;
         todo.push_back(std::move(rest));
     }
     std::vector<char> cached(modules.size(), 0);
     for (size_t m = 0; !v && m < modules.size(); ++m) cached[m] = cached_cubin(modules[m], compiled[m]) ? 1 : 0;
     todo.erase(std::remove_if(todo.begin(), todo.end(), [&](const Unit& u) { return cached[u.module] != 0; }), todo.end());
-    std::stable_sort(todo.begin(), todo.end(), [](const Unit& a, const Unit& b) { return a.weight > b.weight; });
+    std::stable_sort(todo.begin(), todo.end(), [](const Unit& a, const Unit& b) { return a.seconds > b.seconds; });
     std::vector<std::string> logs(todo.size());
     std::vector<char> ok(todo.size(), 0);
     std::atomic<size_t> next{0};
@@ -1228,7 +1257,7 @@ bool jit_compile_modules(const std::vector<ModuleSource>& modules, std::vector<s
         for (size_t i; (i = next.fetch_add(1)) < todo.size();) {
             const ModuleSource& m = modules[todo[i].module];
             std::string src = m.head;
-            for (size_t k = todo[i].first; k < todo[i].end; ++k) src += m.parts[k];
+            for (size_t k = todo[i].first; k < todo[i].end; ++k) src += m.parts[k].text;
             ok[i] = compile_program(src, todo[i].cubin, logs[i]) ? 1 : 0;
         }
     };

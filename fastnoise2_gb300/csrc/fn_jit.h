@@ -65,10 +65,15 @@ struct BatchKernel {
     int threads = 256;
 };
 
-// CUDA source of a module: a head, and parts that need the head but not each other.
+// CUDA source of a module: a head, and parts that need the head but not each other, with the
+// time each takes to compile (seconds, roughly).
 struct ModuleSource {
+    struct Part {
+        std::string text;
+        float seconds;
+    };
     std::string head;
-    std::vector<std::string> parts;
+    std::vector<Part> parts;
 };
 
 // The batch kernels of `progs` (slot k = progs[k]) in one variant (variant 0: and the column kernels
