@@ -130,18 +130,37 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
-def read_traffic(name):
-    """DRAM bytes per launch of the dominant kernel from the committed ncu summary."""
+def read_profile(name, column):
+    """A figure of the specialised kernels from the committed ncu summary: column 1 = DRAM bytes
+    per step, 2 = thread instructions executed per point."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.txt")
     if not os.path.exists(path):
         return None
     for line in open(path):
         if line.startswith(name + " "):
             try:
-                return float(line.split()[1])
+                return float(line.split()[column])
             except (IndexError, ValueError):
                 return None
     return None
+
+
+def roofline(workload, kernels, pts, counted, ms, n_sm, sm_max, peak_src, hbm_peak):
+    """Instructions issued against the issue rate: what the specialised kernels execute per point
+    (column kernels share a cell's work between points, and pruned walks skip cells, so the
+    algorithm's counted operations do not say what runs), else the counted operations."""
+    peak = n_sm * 128 * sm_max * 1e6 / 1e12
+    executed = read_profile(workload, 2) if kernels == "jit" else None
+    work = executed if executed else counted
+    achieved = pts * work / (ms * 1e-3) / 1e12
+    hbm_gbs = pts * 4 / (ms * 1e-3) / 1e9
+    return {"bound": "instruction-issue" if executed else "fp32-issue", "achieved": achieved, "peak": peak, "unit": "Tlane-op/s",
+            "frac": achieved / peak, "traffic": read_profile(workload, 1), "work_per_point": work,
+            "work_source": "thread instructions executed per point (ncu sm__inst_executed, profiles/ncu_traffic.txt)" if executed else
+                           "FS-level ops per point counted by oracle/opcount.h",
+            "counted_ops_per_point": counted, "counted_tops": pts * counted / (ms * 1e-3) / 1e12,
+            "peak_source": f"{n_sm} SMs x 128 lanes x {sm_max:.0f} MHz ({peak_src} sm_max_mhz)",
+            "hbm": {"achieved_gbs": hbm_gbs, "peak_gbs": hbm_peak, "frac": hbm_gbs / hbm_peak, "algorithmic_bytes_per_point": 4}}
 
 
 def parse_cpulist(text):
@@ -507,12 +526,9 @@ def run_chunkmix(a, rank, world, local):
     peaks, peak_src = load_peaks()
     sm_max = float(peaks.get("sm_max_mhz", 2070.0))
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
-    peak_lane = n_sm * 128 * sm_max * 1e6 / 1e12
     tree_ops = [ops_per_point(m(), 3, 1) for m in trees.MIX_TREES]
     tree_ops2 = [ops_per_point(m(), 2, 1) for m in trees.MIX_TREES]
     work = sum(c.points * (tree_ops[c.tree] if len(c.count) == 3 else tree_ops2[c.tree]) for c in chunks)
-    achieved = work / (batch_ms * 1e-3) / 1e12
-    hbm_gbs = pts * 4 / (batch_ms * 1e-3) / 1e9
     cpu = cpu_baseline("chunk-mix", a.cpu_passes, 3.0, rank) if a.cpu_passes > 0 else None
     if cpu is not None and served is not None and a.cpu_rates:
         served["cpu_open_loop"] = cpu_open_loop(chunks, a, rank)
@@ -537,12 +553,7 @@ def run_chunkmix(a, rank, world, local):
             "variants": "0: 256 threads, 64 regs; 1: 256, 80 regs; 2: 256, 128 regs; 3: 128, 64 regs; "
                         "4: 256, 128 regs, 2 points in flight"},
         "served": served,
-        "roofline": {"bound": "fp32-issue", "achieved": achieved, "peak": peak_lane, "unit": "Tlane-op/s",
-                     "frac": achieved / peak_lane, "traffic": read_traffic("chunk-mix"),
-                     "work_per_point": work / pts, "work_source": "FS-level ops per point counted by oracle/opcount.h, per tree and dimensionality",
-                     "peak_source": f"{n_sm} SMs x 128 FP32 lanes x {sm_max:.0f} MHz ({peak_src} sm_max_mhz)",
-                     "hbm": {"achieved_gbs": hbm_gbs, "peak_gbs": float(peaks.get("hbm_gbs", 6800.0)),
-                             "frac": hbm_gbs / float(peaks.get("hbm_gbs", 6800.0)), "algorithmic_bytes_per_point": 4}},
+        "roofline": roofline("chunk-mix", a.kernels, pts, work / pts, batch_ms, n_sm, sm_max, peak_src, float(peaks.get("hbm_gbs", 6800.0))),
         "e2e": {"value": pts * world / (e2e_ms * 1e-3) / 1e6 if e2e_ms else None, "unit": "Mpoints/s",
                 "h2d_bytes_per_step": hinfo["uploadBytes"], "d2h_bytes_per_step": pts * 4 + 8 * len(chunks),
                 "ms_per_step": e2e_ms, "d2h_copy_gbs": d2h_gbs,
@@ -887,10 +898,7 @@ def run_grid(a, rank, world, local):
     peaks, peak_src = load_peaks()
     sm_max = float(peaks.get("sm_max_mhz", 2070.0))
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
-    peak_lane = n_sm * 128 * sm_max * 1e6 / 1e12
     ops = ops_per_point(root, 4 if kind == "tile" else len(args[1]), seed)
-    achieved = pts * ops / (ms * 1e-3) / 1e12
-    hbm_gbs = pts * 4 / (ms * 1e-3) / 1e9
     line = {
         "metric": "Mpoints/s", "value": value, "unit": "Mpoints/s", "n_gpus": world, "steps": a.steps,
         "warmup": a.warmup, "ms_per_step": ms_max, "higher_is_better": True, "scaling": "weak",
@@ -899,12 +907,7 @@ def run_grid(a, rank, world, local):
                    "l2": "flushed between steps (256 MiB write outside the timed events)",
                    "path": "per-call " + ("specialised kernel (fnJitCompile)" if a.kernels == "jit" else "interpreter kernel")
                            + ", device-resident output"},
-        "roofline": {"bound": "fp32-issue", "achieved": achieved, "peak": peak_lane, "unit": "Tlane-op/s",
-                     "frac": achieved / peak_lane, "traffic": read_traffic(a.workload), "work_per_point": ops,
-                     "work_source": "FS-level ops per point counted by oracle/opcount.h",
-                     "peak_source": f"{n_sm} SMs x 128 FP32 lanes x {sm_max:.0f} MHz ({peak_src} sm_max_mhz)",
-                     "hbm": {"achieved_gbs": hbm_gbs, "peak_gbs": float(peaks.get("hbm_gbs", 6800.0)),
-                             "frac": hbm_gbs / float(peaks.get("hbm_gbs", 6800.0)), "algorithmic_bytes_per_point": 4}},
+        "roofline": roofline(a.workload, a.kernels, pts, ops, ms, n_sm, sm_max, peak_src, float(peaks.get("hbm_gbs", 6800.0))),
         "e2e": {"value": pts * world / (e2e_ms * 1e-3) / 1e6 if e2e_ms else None, "unit": "Mpoints/s",
                 "h2d_bytes_per_step": 0, "d2h_bytes_per_step": pts * 4 + 8, "ms_per_step": e2e_ms,
                 "api": "fnGenUniformGrid3D / fnGenTileable2D into pinned host memory",

@@ -369,9 +369,10 @@ FASTNOISE_API int fnBuildChunkMeshDmc(const void* node, int size, int posX, int 
                                       float isoSurface, int upAxisZ, fnChunkMesh* mesh, void* stream);
 /* Many chunks of one tree in one call (what the editor's mesh worker threads do chunk by
  * chunk): positions holds (x, y, z) per chunk, meshes one fnChunkMesh per chunk, each with its
- * own buffers.  The chunks run on several internal streams, ordered after earlier work on
- * `stream`; the call returns when every chunk is done.  FN_ERR_CAPACITY when any chunk's
- * buffers were too small (that chunk's counts are filled; the others are complete). */
+ * own buffers.  Dual marching cubes chunks are meshed together on `stream` (in the sparse form, and
+ * bloxel chunks, on several internal streams ordered after earlier work on it); the call returns
+ * when every chunk is done.  FN_ERR_CAPACITY when any chunk's buffers were too small (that chunk's
+ * counts are filled; the others are complete). */
 FASTNOISE_API int fnBuildChunkMeshesBloxel(const void* node, int size, int count, const int* positions, int seed,
                                            float isoSurface, int upAxisZ, fnChunkMesh* meshes, void* stream);
 FASTNOISE_API int fnBuildChunkMeshesDmc(const void* node, int size, int count, const int* positions, int seed,
