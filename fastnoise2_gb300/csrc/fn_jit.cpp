@@ -1796,7 +1796,7 @@ bool jit_batch_columns(const PointArgs& a, const JitKernels& jk, ColumnShape& s,
     const float column = (float)chunks * (float)((s.steps + len - 1) / len) * column_unit_work(s, len) / column_slots_per_us(jk);
     const float point = (float)s.plane * (float)s.steps / 32.0f * jk.point_cost / slots_per_us();
     saved_us = r.route == FN_GRID_ROUTE_COLUMNS ? 1e30f : 0.9f * point - column;
-    return true;
+    return std::isfinite(saved_us);              // infinite and NaN steps: points
 }
 
 unsigned column_tiles(ColumnShape& s, unsigned len)

@@ -166,6 +166,23 @@ def test_the_estimates_route(columns, name, count, step, requests, alone, batch)
     assert fn.set_grid_route(fn.GRID_ROUTE_AUTO) == 0
 
 
+def test_steps_without_an_estimate_do_not_change_the_other_requests(columns):
+    """Infinite and NaN steps have no estimate: such requests run as points, the others of their tree
+    in columns as without them."""
+    inf, nan = float("inf"), float("nan")
+    odd = [((1, 5, 9), (inf, 1.0, 1.0)), ((7, 5, 9), (nan, 1.0, 1.0)), ((40, 3, 20), (inf, 1.0, inf)), ((5, 1, 9), (1.0, nan, nan))]
+    for name in ("CellValue", "Terrain", "FBmPerlin"):
+        grids = [((32, 32, 32), (1.0, 1.0, 1.0))] * 100 + odd
+        outs = [torch.empty(int(np.prod(c)), device="cuda") for c, _ in grids]
+        fn.set_grid_route(fn.GRID_ROUTE_AUTO)
+        fn.gen_batch([fn.make_request(columns[name], fn.KIND_GRID3D, o.data_ptr(), 5, c, (0.0, 2.0, -3.0), s) for o, (c, s) in zip(outs, grids)])
+        assert 100 <= fn.set_grid_route(fn.GRID_ROUTE_AUTO) <= 104, name
+        oracle = OracleTree(TREES[name]())
+        for o, (c, s) in list(zip(outs, grids))[99:]:
+            ref, rmm = oracle.grid((0.0, 2.0, -3.0), c, s, 5)
+            assert_parity(o.cpu().numpy(), rmm, ref, rmm, label=f"{name} {c} {s}")
+
+
 def test_every_batch_variant_of_the_point_kernels(columns, tmp_path):
     """Tuned variants serve the requests that are not walked in columns; asked to take points, every
     request of every tree runs each variant."""
