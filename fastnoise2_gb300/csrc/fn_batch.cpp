@@ -5,12 +5,15 @@
 #include "fn_jit.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <sstream>
 #include <unordered_map>
+
+#include "FastNoise/FastNoise_C.h"
 
 namespace fn {
 
@@ -178,15 +181,21 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
         BatchKernel kernel;            // its specialised batch kernel
         JitKernels jk;                 // its column kernel
         int group[2] = {-1, -1};       // launch group of its point / column requests
-        double won = 0, lost = 0;      // microseconds that columns save over its requests, and lose
-        bool column = false, split = false;
+        // its requests that can be walked in columns: microseconds of each route, what columns save
+        // over those that gain and lose over the others, and the 32-point steps
+        double point_us = 0, column_us = 0, won = 0, lost = 0;
+        double work = 0, gain_work = 0;
+        long long largest = 0;         // points of the largest
+        unsigned longest = 0;          // steps of the longest unit
+        float step_us = 0, enter_us = 0;
+        enum Walk : char { kPoints, kGains, kColumns } plan = kPoints, walk = kPoints;   // kGains: those that gain
         // the estimates of its last grid shapes: a batch's requests have few (100 ns each otherwise)
         struct Estimate {
             int count[4];
             float step[4];
             bool column;
             ColumnShape shape;
-            float saved;
+            float point_us, column_us;
         };
         std::vector<Estimate> estimates;
         size_t next_estimate = 0;
@@ -258,11 +267,6 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
     if (tuning_in) tuning = *tuning_in;
     else Autotuner::instance().lookup(signature_, tuning);
     const uint32_t tp = std::max<uint32_t>(256, tuning.tile_points);
-    // Grid requests that are better walked in columns.  A tree's requests stay together unless those
-    // that would lose lose more than a second group costs (in the 4096-request chunk mix the 155
-    // smallest 2D grids, 4840 against 4550 us), and a batch has to gain more than a column kernel's
-    // longer first step and last units take (64 requests of FBm(Perlin) 2D 95 x 227 at step 2.9:
-    // 37 us in columns, 30 as points).
     columns_.assign(n, ColumnShape());
     saved_.assign(n, 0.0f);
     for (size_t i = 0; jit && i < n; ++i) {
@@ -277,32 +281,74 @@ int BatchRunner::launch(const std::vector<BatchItem>& items, cudaStream_t stream
             Tree::Estimate& k = tr.estimates[tr.next_estimate++ % 8];
             std::memcpy(k.count, a.count, sizeof k.count);
             std::memcpy(k.step, a.step, sizeof k.step);
-            k.column = jit_batch_columns(a, tr.jk, k.shape, k.saved);
+            k.column = jit_batch_columns(a, tr.jk, k.shape, k.point_us, k.column_us);
             e = &k;
         }
         if (!e->column) continue;
         columns_[i] = e->shape;
-        saved_[i] = e->saved;
-        (e->saved > 0.0f ? tr.won : tr.lost) += e->saved;
+        saved_[i] = e->point_us - e->column_us;
+        const double work = (double)e->shape.steps * column_chunks(e->shape);
+        tr.point_us += e->point_us;
+        tr.column_us += e->column_us;
+        (saved_[i] > 0.0f ? tr.won : tr.lost) += saved_[i];
+        tr.work += work;
+        if (saved_[i] > 0.0f) tr.gain_work += work;
+        tr.largest = std::max(tr.largest, (long long)a.total);
+        tr.longest = std::max(tr.longest, (unsigned)std::min(64.0, std::ceil(work / 8.0)));
+        tr.step_us = std::max(tr.step_us, e->shape.step_us);
+        tr.enter_us = std::max(tr.enter_us, e->shape.enter / 3000.0f);
     }
-    constexpr double kGroupUs = 10.0, kBatchUs = 6.0;
-    double saved_us = 0;
-    for (Tree& tr : trees) {
-        tr.split = tr.lost < -kGroupUs;
-        tr.column = tr.won + (tr.split ? 0.0 : tr.lost) > 0.0;
-        if (tr.column) saved_us += tr.won + (tr.split ? 0.0 : tr.lost);
+    // Column units: about four rounds of 16 warps per SM over the whole batch, so that short
+    // batches still spread, and at most 64 steps (longer ones gain under 5 % of set-up).
+    auto unit_steps = [](double work) { return (unsigned)std::min(64.0, std::max(4.0, work / (64.0 * num_sms()))); };
+    // Which grid requests are walked in columns: none, those of the trees that issue less so, or all
+    // that can be.  A batch of one tree takes what its requests issue, and not less than its longest
+    // tile, whose threads take their points one after another, or its longest unit, whose warp takes
+    // its steps so; columns add 3 us, a longer first step and last units.  Large batches are decided by
+    // what they issue, small ones by the longest tile or unit: 4 requests of terrain 32^3 59 us as
+    // points, 28 in columns, of CellularValue 45 / 21; 106 of FBm(Perlin) 34 x 47 25 / 36.
+    //
+    // Several trees are decided by what they issue, and have to gain 6 us.  The longest tile would often
+    // speak for columns there too (8 requests of 8 trees, 40 000 points, 58 / 32 us), but a server's
+    // batches of that size then end before the next is submitted, and no longer run beside each other.
+    //
+    // A tree's requests stay together unless those that would lose lose more than a second group costs
+    // (the 155 smallest 2D grids of the 4096-request chunk mix: split off 4840 us, together 4550).
+    constexpr double kGroupUs = 10.0, kPointUs = 1.0 / 500.0;   // a warp's points: us per issue slot
+    const bool one = trees.size() == 1;
+    const double columns_us = one ? 3.0 : 6.0;
+    double best_us = 1e30;
+    for (int plan = 0; plan < 3; ++plan) {
+        if (grid_route().route == FN_GRID_ROUTE_COLUMNS && plan < 2) continue;
+        double issue = 0, chain = 0, work = 0;
+        for (Tree& tr : trees) {
+            tr.plan = plan == 2 ? Tree::kColumns : Tree::kPoints;
+            if (plan == 1 && tr.lost < -kGroupUs && tr.won > 0.0) tr.plan = Tree::kGains;
+            else if (plan == 1 && tr.won + tr.lost > 0.0) tr.plan = Tree::kColumns;
+            issue += tr.plan == Tree::kPoints ? tr.point_us : tr.plan == Tree::kGains ? tr.point_us - tr.won : tr.column_us;
+            work += tr.plan == Tree::kPoints ? 0.0 : tr.plan == Tree::kGains ? tr.gain_work : tr.work;
+        }
+        const unsigned len = unit_steps(work);
+        for (const Tree& tr : trees) {
+            if (!one) break;
+            if (tr.plan != Tree::kColumns)
+                chain = std::max(chain, (double)((std::min<long long>(tr.largest, tp) + 255) / 256) * tr.jk.point_cost * kPointUs);
+            if (tr.plan != Tree::kPoints) chain = std::max(chain, (double)(std::min(len, tr.longest) * tr.step_us + tr.enter_us));
+        }
+        const double us = std::max(issue, chain) + (plan ? columns_us : 0.0);
+        if (us >= best_us) continue;
+        best_us = us;
+        for (Tree& tr : trees) tr.walk = tr.plan;
     }
-    double column_work = 0;                         // 32-point steps of columns
+    double column_work = 0;
     for (size_t i = 0; i < n; ++i) {
         const Tree& tr = trees[tree_of_[i]];
-        if (!tr.column || (tr.split && !(saved_[i] > 0.0f)) || saved_us < kBatchUs) columns_[i] = ColumnShape();
+        if (tr.walk == Tree::kPoints || (tr.walk == Tree::kGains && !(saved_[i] > 0.0f))) columns_[i] = ColumnShape();
         if (!columns_[i].plane) continue;
         column_work += (double)columns_[i].steps * column_chunks(columns_[i]);
         ++grid_route().columns;
     }
-    // Column units: about four rounds of 16 warps per SM over the whole batch, so that short
-    // batches still spread, and at most 64 steps (longer ones gain under 5 % of set-up).
-    const unsigned col_len = (unsigned)std::min(64.0, std::max(4.0, column_work / (64.0 * num_sms())));
+    const unsigned col_len = unit_steps(column_work);
     // One group per distinct kernel, in first-appearance order (the interpreter: one for all).
     std::vector<BatchKernel> gkernel;
     std::vector<char> gcolumn;                      // whether it walks columns

@@ -1785,7 +1785,7 @@ bool column_alone(const PointArgs& a, const JitKernels& jk, OutputMemory memory,
 // points, us: 128 requests of FBm(Perlin) 2 x 50000 1409 / 228, 12 x 8000 287 / 219, 24 x 4000
 // 167 / 219; of terrain 3 x 3 x 10000 2299 / 955, 33 x 3000 664 / 481; 64 of FBm(Perlin)
 // 32 x 32 x 32 x 2 380 / 250, 1000 x 62 at 0.5 crossings 111 / 92.
-bool jit_batch_columns(const PointArgs& a, const JitKernels& jk, ColumnShape& s, float& saved_us)
+bool jit_batch_columns(const PointArgs& a, const JitKernels& jk, ColumnShape& s, float& point_us, float& column_us)
 {
     const GridRoute& r = grid_route();
     if (!jk.batch_column || r.route == FN_GRID_ROUTE_POINTS || !column_shape(a, jk, s)) return false;
@@ -1793,10 +1793,9 @@ bool jit_batch_columns(const PointArgs& a, const JitKernels& jk, ColumnShape& s,
     const unsigned chunks = column_chunks(s);
     unsigned len = s.steps < 16u ? s.steps : 16u;
     if ((unsigned long long)chunks * s.steps < 8ull * len) len = (chunks * s.steps + 7u) / 8u;
-    const float column = (float)chunks * (float)((s.steps + len - 1) / len) * column_unit_work(s, len) / column_slots_per_us(jk);
-    const float point = (float)s.plane * (float)s.steps / 32.0f * jk.point_cost / slots_per_us();
-    saved_us = r.route == FN_GRID_ROUTE_COLUMNS ? 1e30f : 0.9f * point - column;
-    return std::isfinite(saved_us);              // infinite and NaN steps: points
+    column_us = (float)chunks * (float)((s.steps + len - 1) / len) * column_unit_work(s, len) / column_slots_per_us(jk);
+    point_us = 0.9f * (float)s.plane * (float)s.steps / 32.0f * jk.point_cost / slots_per_us();
+    return std::isfinite(point_us - column_us);   // infinite and NaN steps: points
 }
 
 unsigned column_tiles(ColumnShape& s, unsigned len)

@@ -129,10 +129,10 @@ struct GridRoute {
 GridRoute& grid_route();
 
 // Whether a request of a batch can be walked in columns by the kernels `jk` (fn_column.cuh); if so
-// `shape` gets its plane and steps, and `saved_us` the time that saves (negative: loses).  column_tiles
-// cuts it into units of at most `len` steps and returns the batch's work items for it (eight units
-// each).
-bool jit_batch_columns(const PointArgs& args, const JitKernels& jk, ColumnShape& shape, float& saved_us);
+// `shape` gets its plane and steps, and `point_us` and `column_us` the time that the GPU takes to issue
+// it either way.  column_tiles cuts it into units of at most `len` steps and returns the batch's work
+// items for it (eight units each).
+bool jit_batch_columns(const PointArgs& args, const JitKernels& jk, ColumnShape& shape, float& point_us, float& column_us);
 inline unsigned column_chunks(const ColumnShape& s) { return (s.plane + 31) / 32; }
 unsigned column_tiles(ColumnShape& shape, unsigned len);
 void column_args(PointArgs& args, const ColumnShape& shape);

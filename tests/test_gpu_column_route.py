@@ -132,13 +132,15 @@ def test_captured_column_calls(columns):
 # estimate's side of each.  The last are grids that columns take longer over than points: Value states
 # that often enter cells, warps with more neighbourhoods than the table holds, 4D super-simplex
 # beside a column state, batches too small to gain a column kernel's longer first and last units.
-RULE = [("FBmPerlin", (256, 256, 256), 1.0, 1, 1, 1), ("FBmPerlin", (16, 16, 16), 1.0, 1, 0, 0), ("FBmPerlin", (32, 32, 32), 1.0, 200, 0, 1),
+# Small batches of heavy points take columns: their longest tile takes longer than the longest unit.
+RULE = [("FBmPerlin", (256, 256, 256), 1.0, 1, 1, 1), ("FBmPerlin", (16, 16, 16), 1.0, 1, 0, 1), ("FBmPerlin", (32, 32, 32), 1.0, 200, 0, 1),
         ("Terrain", (128, 128, 128), 1.0, 4, 1, 1), ("CellValue", (160, 160, 160), 1.0, 2, 1, 1), ("Value", (1024, 1024), 1.0, 12, None, 1),
         ("CellLookup", (97, 90, 101), 1.0, 8, 1, 1),
         ("FBmPerlin", (128, 128, 128), 40.0, 4, 0, 0), ("Terrain", (3, 3, 2000), 1.0, 64, 0, 0), ("FBmPerlin", (2, 50000), 1.0, 16, 0, 0),
         ("FBmValueShort", (1076, 2092), 3.3, 4, 0, 0), ("FBmValueShort", (691, 284), 2.92, 42, 0, 0), ("CellValue", (160, 160, 160), 60.0, 2, 0, 0),
-        ("CellValue", (26, 64, 144), 1.4, 1, 0, 0), ("FadeSuper4D", (75, 37, 21, 58), 1.0, 1, 0, None), ("FBmPerlin2", (95, 227), 2.9, 64, 0, 0),
-        ("CellLookup", (2, 2, 2), 1.0, 8, 0, 0)]
+        ("CellValue", (26, 64, 144), 1.4, 1, 0, 1), ("FadeSuper4D", (75, 37, 21, 58), 1.0, 1, 0, None), ("FBmPerlin2", (95, 227), 2.9, 64, 0, 0),
+        ("CellLookup", (2, 2, 2), 1.0, 8, 0, 0), ("Terrain", (32, 32, 32), 1.0, 4, None, 1), ("CellValue", (32, 32, 32), 1.0, 4, None, 1),
+        ("CellLookup", (9, 10, 15), 0.75, 18, None, 1), ("FBmPerlin", (2, 2000), 1.0, 16, None, 0)]
 RULE_TREES = {"FBmValueShort": lambda: N("FractalFBm", Source=N("Value", Feature_Scale=9.0), Octaves=5),
               "FBmPerlin2": lambda: N("FractalFBm", Source=N("Perlin", Feature_Scale=20.0), Octaves=2),
               "FadeSuper4D": lambda: N("Fade", A=N("FractalFBm", Source=N("SuperSimplex", Feature_Scale=30.0), Octaves=2),
